@@ -95,6 +95,23 @@ def lib():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The tensor-level calls into the library (csrc/fst_host.cpp); raises when not built."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _fst_host
+        except ImportError as e:
+            raise RuntimeError(f"{_PKG}/_fst_host.so cannot be loaded ({e}): run "
+                               "`python -m fstattention_b200.build`. There is no fallback.") from e
+        _host = _fst_host
+    return _host
+
+
 def status_string(code: int) -> str:
     return lib().fst_status_string(int(code)).decode()
 

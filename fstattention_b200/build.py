@@ -1,10 +1,11 @@
-"""Build libfstattn_b200.so in-tree with nvcc for sm_100a.
+"""Build libfstattn_b200.so (nvcc, sm_100a) and the Python host module on top of it, in-tree.
 
   python -m fstattention_b200.build [--force]
 
 One object per .cu file, compiled in parallel, then linked into
-``fstattention_b200/libfstattn_b200.so``.  Nothing is rebuilt when the library is newer than
-every source file.
+``fstattention_b200/libfstattn_b200.so``; ``csrc/fst_host.cpp`` becomes ``_fst_host.so`` (a CPython
+extension against torch's headers, linked to the library).  Nothing is rebuilt when the outputs
+are newer than every source file.
 """
 from __future__ import annotations
 
@@ -18,6 +19,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 LIB = os.path.join(PKG, "libfstattn_b200.so")
+HOST = os.path.join(PKG, "_fst_host.so")
+HOST_SRC = os.path.join(CSRC, "fst_host.cpp")
 OBJ = os.path.join(PKG, "build")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -42,10 +45,30 @@ def _deps():
 
 
 def up_to_date() -> bool:
-    if not os.path.exists(LIB):
+    if not (os.path.exists(LIB) and os.path.exists(HOST)):
         return False
-    t = os.path.getmtime(LIB)
-    return all(os.path.getmtime(p) <= t for p in sources() + _deps() + [os.path.abspath(__file__)])
+    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST))
+    return all(os.path.getmtime(p) <= t for p in sources() + _deps() + [HOST_SRC, os.path.abspath(__file__)])
+
+
+def _build_host() -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cxx = os.environ.get("CXX") or shutil.which("g++")
+    if not cxx:
+        raise RuntimeError("g++ not found; set CXX or put it on PATH")
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = cpp_extension.include_paths() + [os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", INCLUDE, *(x for d in inc for x in ("-isystem", d)), HOST_SRC, "-o", HOST,
+           LIB, "-Wl,-rpath,$ORIGIN", "-L", lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
+           "-lc10_cuda", "-L", os.path.join(cuda, "lib64"), "-lcudart"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{res.stdout}\n{res.stderr}")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -72,9 +95,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
         objs = list(pool.map(compile_one, sources()))
-    res = subprocess.run([nvcc, "-shared", "-cudart", "static", "-o", LIB, *objs], capture_output=True, text=True)
+    res = subprocess.run([nvcc, "-shared", "-cudart", "static", "-Xlinker", "-soname=libfstattn_b200.so", "-o", LIB, *objs], capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _build_host()
     return LIB
 
 

@@ -1,0 +1,556 @@
+// Host path of the Python package: tensors in, library calls out.
+//
+// A decoder calls fst_attention once per layer and the attention of a small tree takes about 5 us
+// on the GPU, so what a call costs on the host decides the step time of eager programs: reading
+// shapes, strides and pointers through Python attributes, building two dozen ctypes arguments and
+// allocating through the dispatcher took 12-15 us per call.  Here the same checks and the same
+// library calls (include/fstattn_b200.h) are made from C++ on the tensors' own fields.
+//
+// Everything follows torch's rules: outputs and workspaces come from torch's caching allocator on
+// the current stream, launches go to the current stream of q's device, errors are Python
+// exceptions.  Nothing here computes anything.
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <atomic>
+#include <cmath>
+#include <mutex>
+#include <optional>
+
+#include "fstattn_b200.h"
+
+namespace {
+
+struct PyError {};                                        // a Python exception is set
+
+[[noreturn]] void raise(PyObject *type, const char *what) {
+    PyErr_SetString(type, what);
+    throw PyError{};
+}
+void check_status(int rc, const char *what) {
+    if (rc == FST_OK) return;
+    PyErr_Format(PyExc_RuntimeError, "%s: %s (status %d)", what, fst_status_string(rc), rc);
+    throw PyError{};
+}
+
+// ---- argument access -------------------------------------------------------------------------
+const at::Tensor &tensor(PyObject *o) {
+    if (!THPVariable_Check(o)) raise(PyExc_TypeError, "a torch.Tensor is expected");
+    return THPVariable_Unpack(o);
+}
+long long integer(PyObject *o) {
+    const long long v = PyLong_AsLongLong(o);
+    if (v == -1 && PyErr_Occurred()) throw PyError{};
+    return v;
+}
+double real(PyObject *o) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw PyError{};
+    return v;
+}
+
+at::Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Device &dev) {
+    return at::detail::empty_cuda(size, type, dev, std::nullopt);
+}
+
+// Attention launches on a device share one status record (the first problem seen stays until it
+// is cleared).  Records live as long as the process.
+at::Tensor *const *status_slots() {
+    static at::Tensor *slots[64] = {};
+    return slots;
+}
+at::Tensor *status_of(const at::Device &dev, bool create) {
+    static std::mutex mutex;
+    at::Tensor **slots = const_cast<at::Tensor **>(status_slots());
+    const int i = dev.index();
+    if (i < 0 || i >= 64) raise(PyExc_RuntimeError, "device index out of range");
+    std::lock_guard<std::mutex> lock(mutex);
+    if (slots[i] == nullptr && create)
+        slots[i] = new at::Tensor(at::zeros({4}, at::TensorOptions().dtype(at::kInt).device(dev)));
+    return slots[i];
+}
+
+int sm_count(int device) {
+    static std::atomic<int> cached[64];
+    int n = cached[device & 63].load(std::memory_order_acquire);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 148;
+        cached[device & 63].store(n, std::memory_order_release);
+    }
+    return n;
+}
+
+// ---- the runs a shared prefix is cut into -------------------------------------------------------
+// Only the tensor-core kernels split.  With head_dim 64 or 128 and at least 256 prefix rows the
+// prefix goes to the tcgen05 kernel: one CTA per 128 query rows, head, batch element and run.  Its
+// shared memory allows one CTA per SM, so the automatic choice is as many runs as keep the grid
+// within one wave, each at least 256 rows.  Otherwise the tree kernel walks the prefix itself,
+// split to about four CTAs per SM.
+struct Splits {
+    int runs;
+    bool workspace;
+};
+Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, int64_t Z, int64_t H, int64_t n_q,
+                   int64_t D, int64_t prefix, int64_t block_m, int kernel, int device) {
+    if ((type != at::kHalf && type != at::kBFloat16) || (D != 64 && D != 128) ||
+        (block_m != 32 && block_m != 64 && block_m != 128) || kernel == FST_KERNEL_SIMT || kernel == FST_KERNEL_MMA ||
+        prefix <= 0)
+        return {1, false};
+    const int64_t cap = 65535 / std::max<int64_t>(Z, 1);
+    const auto clamp = [&](int64_t v) { return int(std::max<int64_t>(1, std::min(v, cap))); };
+    if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && prefix >= 256)) {
+        if (asked) return {clamp(*asked), true};
+        const int64_t ctas = Z * H * ((n_q + 127) / 128);
+        return {clamp(std::min(sm_count(device) / std::max<int64_t>(ctas, 1), prefix / 256)), true};
+    }
+    int runs;
+    if (asked) {
+        runs = clamp(*asked);
+    } else {
+        const int64_t ctas = Z * H * ((n_q + block_m - 1) / block_m);
+        runs = clamp(std::min(4 * sm_count(device) / std::max<int64_t>(ctas, 1), prefix / 512));
+    }
+    return {runs, runs > 1};
+}
+std::optional<long long> optional_int(PyObject *o) {
+    if (o == Py_None) return std::nullopt;
+    return integer(o);
+}
+
+// ---- attention ----------------------------------------------------------------------------------
+int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kHalf: return FST_F16;
+        case at::kBFloat16: return FST_BF16;
+        case at::kFloat: return FST_F32;
+        default: return -1;
+    }
+}
+void head_contiguous(const at::Tensor &t) {
+    if (t.stride(3) != 1) raise(PyExc_ValueError, "the head dimension must be contiguous");
+}
+
+struct Call {
+    at::Tensor q, k, v, o, lse;
+    int64_t Z, H, H_kv, n_q, n_kv, D;
+    float scale;
+    int dtype;
+};
+
+// The checks every attention call makes, in the order callers rely on (the reference asserts the
+// head dimensions, fstattention.py:155-157), and the output tensors.
+Call open_call(PyObject *q, PyObject *k, PyObject *v, PyObject *out, PyObject *scale, bool want_lse) {
+    Call c;
+    c.q = tensor(q); c.k = tensor(k); c.v = tensor(v);
+    if (c.q.dim() != 4 || c.k.dim() != 4 || c.v.dim() != 4) raise(PyExc_ValueError, "q, k, v must have four dimensions");
+    c.D = c.q.size(3);
+    if (c.D != c.k.size(3) || c.k.size(3) != c.v.size(3)) raise(PyExc_AssertionError, "q, k, v must have equal head dimensions");
+    if (c.D != 16 && c.D != 32 && c.D != 64 && c.D != 128) raise(PyExc_AssertionError, "head dimension must be 16, 32, 64 or 128");
+    if (!c.q.is_cuda() || !c.k.is_cuda() || !c.v.is_cuda())
+        raise(PyExc_RuntimeError, "fst_attention runs on CUDA tensors only; there is no CPU path");
+    const at::ScalarType type = c.q.scalar_type();
+    c.dtype = dtype_code(type);
+    if (c.dtype < 0 || c.k.scalar_type() != type || c.v.scalar_type() != type)
+        raise(PyExc_TypeError, "q, k, v must share one dtype out of float16, bfloat16, float32");
+    c.Z = c.q.size(0); c.H = c.q.size(1); c.n_q = c.q.size(2);
+    c.H_kv = c.k.size(1); c.n_kv = c.k.size(2);
+    if (c.k.size(0) != c.Z || c.v.sizes() != c.k.sizes() || c.n_kv < c.n_q || c.H_kv < 1 || c.H % c.H_kv)
+        raise(PyExc_ValueError, "k and v must be [Z, H_kv, P + N, D] with P >= 0 and H a multiple of H_kv");
+    if (out == Py_None) {
+        c.o = c.q.is_contiguous() ? empty(c.q.sizes(), type, c.q.device()) : at::empty_like(c.q);
+    } else {
+        c.o = tensor(out);
+        if (c.o.sizes() != c.q.sizes() || c.o.scalar_type() != type || !c.o.is_cuda()) raise(PyExc_ValueError, "out must match q");
+    }
+    const double s = real(scale);
+    if (!std::isfinite(s)) raise(PyExc_ValueError, "sm_scale must be finite");
+    c.scale = float(s);
+    head_contiguous(c.q); head_contiguous(c.k); head_contiguous(c.v); head_contiguous(c.o);
+    if (want_lse) c.lse = empty({c.Z * c.H, c.n_q}, at::kFloat, c.q.device());
+    return c;
+}
+PyObject *results(const Call &c) {
+    if (!c.lse.defined()) return THPVariable_Wrap(c.o);
+    PyObject *o = THPVariable_Wrap(c.o), *l = THPVariable_Wrap(c.lse);
+    PyObject *pair = PyTuple_Pack(2, o, l);
+    Py_DECREF(o);
+    Py_DECREF(l);
+    return pair;
+}
+float *lse_ptr(const Call &c) { return c.lse.defined() ? static_cast<float *>(c.lse.data_ptr()) : nullptr; }
+
+#define FST_STRIDES(t) (t).stride(0), (t).stride(1), (t).stride(2)
+
+PyObject *launch(Call &c, const void *packed, size_t tree_stride, int64_t block_m, int64_t ma, int kernel,
+                 const std::optional<long long> &kv_splits, void *status, void *stream) {
+    const at::Device dev = c.q.device();
+    const Splits sp = pick_splits(kv_splits, c.q.scalar_type(), c.Z, c.H, c.n_q, c.D, c.n_kv - c.n_q, block_m,
+                                  kernel & FST_KERNEL_MASK, dev.index());
+    at::Tensor ws;
+    size_t ws_bytes = 0;
+    if (sp.workspace) {
+        ws_bytes = fst_attention_split_workspace_bytes(int(c.Z), int(c.H), int(c.n_q), int(c.D), sp.runs);
+        ws = empty({int64_t(ws_bytes)}, at::kByte, dev);
+    }
+    int rc;
+    {
+        pybind11::gil_scoped_release no_gil;
+        rc = fst_attention_fwd_gqa(c.q.data_ptr(), c.k.data_ptr(), c.v.data_ptr(), c.o.data_ptr(), lse_ptr(c), packed,
+                                   tree_stride, int(c.Z), int(c.H), int(c.H_kv), int(c.n_q), int(c.n_kv), int(c.D),
+                                   FST_STRIDES(c.q), FST_STRIDES(c.k), FST_STRIDES(c.v), FST_STRIDES(c.o), int(block_m),
+                                   int(ma), c.scale, c.dtype, kernel, sp.runs, ws.defined() ? ws.data_ptr() : nullptr,
+                                   ws_bytes, static_cast<int32_t *>(status), stream);
+    }
+    check_status(rc, "fst_attention_fwd");
+    return results(c);
+}
+
+template <PyObject *(*F)(PyObject *const *, Py_ssize_t)>
+PyObject *guarded(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    try {
+        return F(args, n);
+    } catch (const PyError &) {
+        return nullptr;
+    }
+    END_HANDLE_TH_ERRORS
+}
+void want_args(Py_ssize_t n, Py_ssize_t want) {
+    if (n != want) raise(PyExc_TypeError, "wrong number of arguments");
+}
+
+// attention(q, k, v, out, packed, tree_stride, n_trees, n_blocks, block_m, max_ancestors, sm_scale,
+//           kernel, kv_splits, return_lse)
+PyObject *attention(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 14);
+    Call c = open_call(a[0], a[1], a[2], a[3], a[10], a[13] == Py_True);
+    const int64_t n_trees = integer(a[6]), n_blocks = integer(a[7]), bm = integer(a[8]), ma = integer(a[9]);
+    if (n_trees != 1 && n_trees != c.Z) raise(PyExc_ValueError, "metadata must describe one tree or one tree per batch element");
+    if (n_blocks != (c.n_q + bm - 1) / bm) raise(PyExc_ValueError, "metadata block count does not match q");
+    const at::Device dev = c.q.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    void *status = status_of(dev, true)->data_ptr();
+    void *stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    return launch(c, tensor(a[4]).data_ptr(), n_trees > 1 ? size_t(integer(a[5])) : 0, bm, ma, int(integer(a[11])),
+                  optional_int(a[12]), status, stream);
+}
+
+// The reference's three tensors (fstattention.py:153) in packed form, one launch; index_base (the prefix
+// length) is what the caller has added to the indices, as the reference's test does, sentinels included.
+struct Packed {
+    at::Tensor blob;
+    size_t stride;
+    int64_t n_trees;
+};
+Packed pack_reference(PyObject *idx, PyObject *mask, PyObject *leaf, int64_t Z, int64_t n_q, int64_t index_base, int64_t bm,
+                      int64_t ma, const at::Device &dev, int32_t *status, void *stream) {
+    if (mask == Py_None || leaf == Py_None) raise(PyExc_TypeError, "ancestor_mask and leaf_idx are required with plain tensors");
+    at::Tensor ai = tensor(idx), am = tensor(mask), li = tensor(leaf);
+    if (!ai.is_cuda() || !am.is_cuda() || !li.is_cuda())
+        raise(PyExc_RuntimeError, "metadata tensors must be on the GPU (call .to('cuda') as the reference does)");
+    if (bm <= 0 || ma <= 0) raise(PyExc_ValueError, "metadata shapes do not match BLOCK_M / MAX_ANCESTORS / q");
+    const int64_t nb = (n_q + bm - 1) / bm, n_meta = ai.dim() == 3 ? ai.size(0) : 1;
+    const auto shaped = [](const at::Tensor &t, at::IntArrayRef want) {
+        return t.dim() >= int64_t(want.size()) && t.sizes().slice(t.dim() - want.size()) == want;
+    };
+    if (!shaped(ai, {nb, ma}) || !shaped(am, {nb, bm, ma}) || !shaped(li, {nb, bm}))
+        raise(PyExc_ValueError, "metadata shapes do not match BLOCK_M / MAX_ANCESTORS / q");
+    if (ai.scalar_type() != at::kLong || li.scalar_type() != at::kLong ||
+        (am.scalar_type() != at::kBool && am.scalar_type() != at::kByte))
+        raise(PyExc_TypeError, "metadata dtypes must be int64 / bool / int64");
+    if (n_meta != 1 && n_meta != Z) raise(PyExc_ValueError, "metadata must describe one tree or one tree per batch element");
+    ai = ai.contiguous(); am = am.contiguous(); li = li.contiguous();
+    Packed p;
+    p.n_trees = n_meta;
+    p.stride = fst_packed_meta_bytes(int(nb), int(bm), int(ma));
+    p.blob = empty({n_meta, int64_t(p.stride)}, at::kByte, dev);
+    check_status(fst_pack_metadata(static_cast<const int64_t *>(ai.data_ptr()), static_cast<const uint8_t *>(am.data_ptr()),
+                                   static_cast<const int64_t *>(li.data_ptr()), int(n_meta), int(nb), int(bm), int(ma),
+                                   index_base, p.blob.data_ptr(), p.stride, status, stream),
+                 "fst_pack_metadata");
+    return p;
+}
+
+// attention_ref(q, k, v, out, ancestor_idx, ancestor_mask, leaf_idx, block_m, max_ancestors, sm_scale,
+//               kernel, kv_splits, return_lse)
+PyObject *attention_ref(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 13);
+    Call c = open_call(a[0], a[1], a[2], a[3], a[9], a[12] == Py_True);
+    const at::Device dev = c.q.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    int32_t *status = static_cast<int32_t *>(status_of(dev, true)->data_ptr());
+    void *stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    const int64_t bm = integer(a[7]), ma = integer(a[8]);
+    const Packed p = pack_reference(a[4], a[5], a[6], c.Z, c.n_q, c.n_kv - c.n_q, bm, ma, dev, status, stream);
+    return launch(c, p.blob.data_ptr(), p.n_trees > 1 ? p.stride : 0, bm, ma, int(integer(a[10])), optional_int(a[11]),
+                  status, stream);
+}
+
+// pack(ancestor_idx, ancestor_mask, leaf_idx, Z, n_q, index_base, block_m, max_ancestors) -> (packed, tree_stride, n_trees)
+PyObject *pack(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 8);
+    const at::Device dev = tensor(a[0]).device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const Packed p = pack_reference(a[0], a[1], a[2], integer(a[3]), integer(a[4]), integer(a[5]), integer(a[6]), integer(a[7]),
+                                    dev, static_cast<int32_t *>(status_of(dev, true)->data_ptr()),
+                                    c10::cuda::getCurrentCUDAStream(dev.index()).stream());
+    return Py_BuildValue("(NnL)", THPVariable_Wrap(p.blob), Py_ssize_t(p.stride), (long long)p.n_trees);
+}
+
+// attention_paged(q, k_tree, v_tree, out, packed, tree_stride, n_trees, n_blocks, block_m, max_ancestors,
+//                 k_pool, v_pool, nhd, block_table, prefix_lens, max_prefix, sm_scale, kv_splits, return_lse)
+PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 19);
+    const at::Tensor &q = tensor(a[0]), &kt = tensor(a[1]), &vt = tensor(a[2]), &kp = tensor(a[10]), &vp = tensor(a[11]),
+                     &table = tensor(a[13]), &lens = tensor(a[14]);
+    for (const at::Tensor *t : {&q, &kt, &vt, &kp, &vp, &table, &lens})
+        if (!t->is_cuda()) raise(PyExc_RuntimeError, "fst_attention_paged runs on CUDA tensors only; there is no CPU path");
+    const at::ScalarType type = q.scalar_type();
+    bool same = type == at::kHalf || type == at::kBFloat16;
+    for (const at::Tensor *t : {&kt, &vt, &kp, &vp}) same = same && t->scalar_type() == type;
+    if (!same) raise(PyExc_TypeError, "q, k_tree, v_tree and the pools must share one dtype out of float16, bfloat16");
+    if (q.dim() != 4 || kt.dim() != 4 || vt.dim() != 4) raise(PyExc_ValueError, "q, k_tree, v_tree must have four dimensions");
+    const int64_t Z = q.size(0), H = q.size(1), n_q = q.size(2), D = q.size(3), H_kv = kt.size(1);
+    if (kt.size(0) != Z || kt.size(2) != n_q || kt.size(3) != D || vt.sizes() != kt.sizes() || H_kv < 1 || H % H_kv)
+        raise(PyExc_ValueError, "k_tree and v_tree must be [Z, H_kv, N, D] with H a multiple of H_kv");
+    const bool nhd = a[12] == Py_True;
+    const int row_dim = nhd ? 1 : 2, head_dim = nhd ? 2 : 1;
+    if (kp.dim() != 4 || vp.sizes() != kp.sizes() || kp.size(head_dim) != H_kv || kp.size(3) != D ||
+        kp.strides() != vp.strides() || kp.stride(3) != 1)
+        raise(PyExc_ValueError, "pools must be two equally laid out [n_pages, page_size, H_kv, D] (or HND) tensors");
+    if (table.scalar_type() != at::kInt || lens.scalar_type() != at::kInt || table.dim() != 2 || table.size(0) != Z ||
+        lens.dim() != 1 || lens.size(0) != Z || !table.is_contiguous())
+        raise(PyExc_ValueError, "block_table must be contiguous int32 [Z, pages], prefix_lens int32 [Z]");
+    const int64_t n_trees = integer(a[6]), n_blocks = integer(a[7]), bm = integer(a[8]), ma = integer(a[9]);
+    if ((n_trees != 1 && n_trees != Z) || n_blocks != (n_q + bm - 1) / bm) raise(PyExc_ValueError, "metadata does not match q");
+    Call c = open_call(a[0], a[1], a[2], a[3], a[16], a[18] == Py_True);
+    const int64_t max_prefix = integer(a[15]);
+    const at::Device dev = q.device();
+    std::optional<long long> asked = optional_int(a[17]);
+    if (!asked) {
+        const int64_t ctas = Z * H * ((n_q + 127) / 128);
+        asked = std::max<int64_t>(1, std::min({sm_count(dev.index()) / std::max<int64_t>(ctas, 1), max_prefix / 256, 65535 / Z}));
+    }
+    const c10::cuda::CUDAGuard guard(dev);
+    int32_t *status = static_cast<int32_t *>(status_of(dev, true)->data_ptr());
+    const size_t ws_bytes = fst_attention_split_workspace_bytes(int(Z), int(H), int(n_q), int(D), int(*asked));
+    const at::Tensor ws = empty({int64_t(ws_bytes)}, at::kByte, dev);
+    void *stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    const size_t tree_stride = n_trees > 1 ? size_t(integer(a[5])) : 0;
+    const void *packed = tensor(a[4]).data_ptr();
+    int rc;
+    {
+        pybind11::gil_scoped_release no_gil;
+        rc = fst_attention_fwd_paged(q.data_ptr(), kt.data_ptr(), vt.data_ptr(), c.o.data_ptr(), lse_ptr(c), packed,
+                                     tree_stride, kp.data_ptr(), vp.data_ptr(), static_cast<const int32_t *>(table.data_ptr()),
+                                     int(table.size(1)), static_cast<const int32_t *>(lens.data_ptr()), int(max_prefix),
+                                     int(kp.size(row_dim)), int(kp.size(0)), kp.stride(0), kp.stride(row_dim),
+                                     kp.stride(head_dim), int(Z), int(H), int(H_kv), int(n_q), int(D), FST_STRIDES(q),
+                                     FST_STRIDES(kt), FST_STRIDES(vt), FST_STRIDES(c.o), int(bm), int(ma), c.scale, c.dtype,
+                                     int(*asked), ws.data_ptr(), ws_bytes, status, stream);
+    }
+    check_status(rc, "fst_attention_fwd_paged");
+    return results(c);
+}
+
+// ---- trees ---------------------------------------------------------------------------------------
+// precompute(parent, block_m, max_ancestors, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx)
+//   -> None; parent is a contiguous int32 CUDA tensor [N] or [T, N], the buffers belong to the caller and
+//   the last three may be None.
+// new_metadata(parent, block_m, max_ancestors, reference_format)
+//   -> (n_trees, n_nodes, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx), buffers made here.
+void run_precompute(const at::Tensor &par, int64_t n_trees, int64_t n_nodes, int64_t bm, int64_t ma, const at::Tensor &packed,
+                    size_t stride, const at::Tensor &status, const at::Tensor &ai, const at::Tensor &am,
+                    const at::Tensor &li) {
+    const at::Device dev = par.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    if (cudaMemsetAsync(status.data_ptr(), 0, 16, stream) != cudaSuccess) check_status(FST_ERR_CUDA, "fst_precompute");
+    check_status(fst_precompute(static_cast<const int32_t *>(par.data_ptr()), int(n_trees), int(n_nodes), int(bm), int(ma),
+                                ai.defined() ? static_cast<int64_t *>(ai.data_ptr()) : nullptr,
+                                am.defined() ? static_cast<uint8_t *>(am.data_ptr()) : nullptr,
+                                li.defined() ? static_cast<int64_t *>(li.data_ptr()) : nullptr, packed.data_ptr(), stride,
+                                static_cast<int32_t *>(status.data_ptr()), stream),
+                 "fst_precompute");
+}
+const at::Tensor &parent_arg(PyObject *o) {
+    const at::Tensor &par = tensor(o);
+    if ((par.dim() != 1 && par.dim() != 2) || par.numel() == 0)
+        raise(PyExc_ValueError, "parent must be a non-empty [N] or [T, N] array");
+    if (!par.is_cuda() || par.scalar_type() != at::kInt || !par.is_contiguous())
+        raise(PyExc_ValueError, "parent must be a contiguous int32 CUDA tensor");
+    return par;
+}
+at::Tensor optional_tensor(PyObject *o) { return o == Py_None ? at::Tensor() : tensor(o); }
+
+PyObject *precompute(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 9);
+    const at::Tensor &par = parent_arg(a[0]);
+    run_precompute(par, par.dim() == 2 ? par.size(0) : 1, par.size(-1), integer(a[1]), integer(a[2]), tensor(a[3]),
+                   size_t(integer(a[4])), tensor(a[5]), optional_tensor(a[6]), optional_tensor(a[7]), optional_tensor(a[8]));
+    Py_RETURN_NONE;
+}
+
+PyObject *wrap_or_none(const at::Tensor &t) {
+    if (t.defined()) return THPVariable_Wrap(t);
+    Py_RETURN_NONE;
+}
+
+PyObject *new_metadata(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 4);
+    const at::Tensor &par = parent_arg(a[0]);
+    const int64_t bm = integer(a[1]), ma = integer(a[2]);
+    const int64_t n_trees = par.dim() == 2 ? par.size(0) : 1, n_nodes = par.size(-1);
+    if (bm <= 0 || ma <= 0) raise(PyExc_ValueError, "block_m and max_ancestors must be positive");
+    const int64_t nb = (n_nodes + bm - 1) / bm;
+    const size_t stride = fst_packed_meta_bytes(int(nb), int(bm), int(ma));
+    const at::Device dev = par.device();
+    const at::Tensor packed = empty({n_trees, int64_t(stride)}, at::kByte, dev), status = empty({4}, at::kInt, dev);
+    at::Tensor ai, am, li;
+    if (a[3] == Py_True) {
+        if (par.dim() == 2) {
+            ai = empty({n_trees, nb, ma}, at::kLong, dev);
+            am = empty({n_trees, nb, bm, ma}, at::kBool, dev);
+            li = empty({n_trees, nb, bm}, at::kLong, dev);
+        } else {
+            ai = empty({nb, ma}, at::kLong, dev);
+            am = empty({nb, bm, ma}, at::kBool, dev);
+            li = empty({nb, bm}, at::kLong, dev);
+        }
+    }
+    run_precompute(par, n_trees, n_nodes, bm, ma, packed, stride, status, ai, am, li);
+    return Py_BuildValue("(LLNnNNNN)", (long long)n_trees, (long long)n_nodes, THPVariable_Wrap(packed), Py_ssize_t(stride),
+                         THPVariable_Wrap(status), wrap_or_none(ai), wrap_or_none(am), wrap_or_none(li));
+}
+
+// dfs_order(parent) -> (order, new_parent, status)
+PyObject *dfs_order(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 1);
+    const at::Tensor &par = parent_arg(a[0]);
+    const at::Device dev = par.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const at::Tensor order = empty(par.sizes(), at::kInt, dev), npar = empty(par.sizes(), at::kInt, dev),
+                     status = empty({4}, at::kInt, dev);
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    if (cudaMemsetAsync(status.data_ptr(), 0, 16, stream) != cudaSuccess) check_status(FST_ERR_CUDA, "fst_dfs_order");
+    check_status(fst_dfs_order(static_cast<const int32_t *>(par.data_ptr()), int(par.dim() == 2 ? par.size(0) : 1),
+                               int(par.size(-1)), static_cast<int32_t *>(order.data_ptr()),
+                               static_cast<int32_t *>(npar.data_ptr()), static_cast<int32_t *>(status.data_ptr()), stream),
+                 "fst_dfs_order");
+    return Py_BuildValue("(NNN)", THPVariable_Wrap(order), THPVariable_Wrap(npar), THPVariable_Wrap(status));
+}
+
+// build_tree_topk(scores, depth, topk, left_weight_factor, n, return_choice, return_scores)
+//   -> (parent, choice or None, node scores or None)
+PyObject *build_tree_topk(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 7);
+    const at::Tensor sc = tensor(a[0]).contiguous();
+    const bool batched = sc.dim() == 3;
+    const int64_t n_trees = batched ? sc.size(0) : 1, nodes = integer(a[4]);
+    const at::Device dev = sc.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const auto made = [&](at::ScalarType t) { return batched ? empty({n_trees, nodes}, t, dev) : empty({nodes}, t, dev); };
+    const at::Tensor parent = made(at::kInt);
+    const at::Tensor choice = a[5] == Py_True ? made(at::kInt) : at::Tensor(), score = a[6] == Py_True ? made(at::kFloat) : at::Tensor();
+    check_status(fst_build_tree_topk(static_cast<const float *>(sc.data_ptr()), int(n_trees), int(integer(a[1])),
+                                     int(integer(a[2])), real(a[3]), int(nodes), static_cast<int32_t *>(parent.data_ptr()),
+                                     choice.defined() ? static_cast<int32_t *>(choice.data_ptr()) : nullptr,
+                                     score.defined() ? static_cast<float *>(score.data_ptr()) : nullptr,
+                                     c10::cuda::getCurrentCUDAStream(dev.index()).stream()),
+                 "fst_build_tree_topk");
+    return Py_BuildValue("(NNN)", THPVariable_Wrap(parent), wrap_or_none(choice), wrap_or_none(score));
+}
+
+// parents_of_lineage(lineage, level_lookup, mutate) -> int32 parent array on the host (pinned), for int64 CPU
+// tensors: parent[k] = lineage[k, level[k] - 1], -1 on level 0 (utils.py:42-44 of the reference).  The
+// reference's side effect (utils.py:124-125) - every node written into its own lineage row - is a second call.
+PyObject *parents_of_lineage(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 2);
+    const at::Tensor &lin = tensor(a[0]), &lvl = tensor(a[1]);
+    const int64_t N = lin.size(0), W = lin.size(1), s0 = lin.stride(0), s1 = lin.stride(1), t0 = lvl.stride(0);
+    const int64_t *L = static_cast<const int64_t *>(lin.data_ptr()), *V = static_cast<const int64_t *>(lvl.data_ptr());
+    const at::Tensor parent = at::empty({N}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));   // torch's pinned pool
+    int32_t *P = static_cast<int32_t *>(parent.data_ptr());
+    for (int64_t k = 0; k < N; ++k) {
+        const int64_t lv = V[k * t0];
+        if (lv > W) raise(PyExc_IndexError, "level_lookup points past the lineage columns");
+        P[k] = lv > 0 ? int32_t(L[k * s0 + (lv - 1) * s1]) : -1;
+    }
+    return THPVariable_Wrap(parent);
+}
+
+// write_self(lineage, level_lookup): lineage[k, level[k]] = k (utils.py:124-125), int64 CPU tensors
+PyObject *write_self(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 2);
+    const at::Tensor &lin = tensor(a[0]), &lvl = tensor(a[1]);
+    const int64_t N = lin.size(0), W = lin.size(1), s0 = lin.stride(0), s1 = lin.stride(1), t0 = lvl.stride(0);
+    int64_t *L = static_cast<int64_t *>(lin.data_ptr());
+    const int64_t *V = static_cast<const int64_t *>(lvl.data_ptr());
+    for (int64_t k = 0; k < N; ++k) {
+        const int64_t lv = V[k * t0];
+        if (lv < 0 || lv >= W) raise(PyExc_IndexError, "level_lookup points past the lineage columns");
+        L[k * s0 + lv * s1] = k;
+    }
+    lin.unsafeGetTensorImpl()->bump_version();
+    Py_RETURN_NONE;
+}
+
+// read_status(record) -> its four words, once everything ahead on the current stream has run
+PyObject *read_status(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 1);
+    const at::Tensor &t = tensor(a[0]);
+    const at::Device dev = t.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    int32_t w[4] = {};
+    cudaError_t e;
+    {
+        pybind11::gil_scoped_release no_gil;
+        e = cudaMemcpyAsync(w, t.data_ptr(), sizeof(w), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    }
+    if (e != cudaSuccess) {
+        PyErr_Format(PyExc_RuntimeError, "reading a status record: %s", cudaGetErrorString(e));
+        throw PyError{};
+    }
+    return Py_BuildValue("(iiii)", w[0], w[1], w[2], w[3]);
+}
+
+// status_record(device_index) -> the attention status record of that device, or None before its first launch
+PyObject *status_record(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 1);
+    const at::Tensor *t = status_of(at::Device(at::kCUDA, at::DeviceIndex(integer(a[0]))), false);
+    if (t == nullptr) Py_RETURN_NONE;
+    return THPVariable_Wrap(*t);
+}
+// attention_status(device_index) -> the same, made on first use
+PyObject *attention_status(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 1);
+    return THPVariable_Wrap(*status_of(at::Device(at::kCUDA, at::DeviceIndex(integer(a[0]))), true));
+}
+
+// splits(q, prefix, block_m, kernel, kv_splits) -> (runs, whether a workspace is needed)
+PyObject *splits(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 5);
+    const at::Tensor &q = tensor(a[0]);
+    const Splits s = pick_splits(optional_int(a[4]), q.scalar_type(), q.size(0), q.size(1), q.size(2), q.size(3), integer(a[1]),
+                                 integer(a[2]), int(integer(a[3])), q.device().index());
+    return Py_BuildValue("(iO)", s.runs, s.workspace ? Py_True : Py_False);
+}
+
+#define FST_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(&guarded<name>)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    FST_METHOD(attention),      FST_METHOD(attention_ref), FST_METHOD(attention_paged), FST_METHOD(pack),
+    FST_METHOD(precompute),     FST_METHOD(new_metadata),  FST_METHOD(dfs_order),
+    FST_METHOD(build_tree_topk), FST_METHOD(parents_of_lineage), FST_METHOD(write_self), FST_METHOD(read_status), FST_METHOD(status_record), FST_METHOD(attention_status),
+    FST_METHOD(splits),         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fst_host", "tensor-level calls into libfstattn_b200.so", -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__fst_host() { return PyModule_Create(&module); }

@@ -9,7 +9,7 @@ decoder that rebuilds its tree every step has.
 """
 from __future__ import annotations
 
-import math
+import weakref
 from typing import Optional, Sequence, Union
 
 import torch
@@ -37,22 +37,25 @@ class TreeMetadata:
                  ancestor_idx=None, ancestor_mask=None, leaf_idx=None, batched=False):
         self.n_trees, self.n_nodes = n_trees, n_nodes
         self.block_m, self.max_ancestors = block_m, max_ancestors
-        self.n_blocks = math.ceil(n_nodes / block_m)
+        self.n_blocks = -(-n_nodes // block_m)
         self.packed, self.tree_stride, self.status = packed, tree_stride, status
         self.ancestor_idx, self.ancestor_mask, self.leaf_idx = ancestor_idx, ancestor_mask, leaf_idx
         self.batched = batched
-        self._versions = self._current_versions()
         # attention launches that have read the packed form since it was last written: from the
         # second one on, the launch ahead of the call in the stream cannot be the writer
         self.reads_since_build = 0
+        self._twin = None if ancestor_idx is None else _PackedTwin(self)
 
-    def _current_versions(self):
-        return tuple(t._version if t is not None else -1
-                     for t in (self.ancestor_idx, self.ancestor_mask, self.leaf_idx))
+    def _rebuilt(self) -> None:
+        """The buffers have just been written (again)."""
+        self.reads_since_build = 0
+        if self._twin is not None:
+            self._twin.reads_since_build = 0
+            self._twin.versions = _versions((self.ancestor_idx, self.ancestor_mask, self.leaf_idx))
 
     def tensors_untouched(self) -> bool:
         """True while nobody has modified the three reference-format tensors in place."""
-        return self._versions == self._current_versions()
+        return self._twin is None or self._twin.versions == _versions((self.ancestor_idx, self.ancestor_mask, self.leaf_idx))
 
     def __iter__(self):
         if self.ancestor_idx is None:
@@ -61,7 +64,7 @@ class TreeMetadata:
 
     def check(self) -> "TreeMetadata":
         """Read the device status record (synchronises) and raise on a recorded problem."""
-        code, where, detail, _ = self.status.tolist()
+        code, where, detail, _ = _lib.host().read_status(self.status)
         if code == _lib.DEV_ANCESTOR_OVERFLOW:
             raise RuntimeError(
                 f"block {where % 65536} of tree {where // 65536} has {detail} unique ancestors, "
@@ -77,16 +80,39 @@ class TreeMetadata:
         return self.packed.device
 
 
-# The three tensors handed out by the precompute remember the metadata they came from, so that
+def _versions(tensors):
+    return tuple(t._version for t in tensors)
+
+
+# The three tensors handed out by the precompute remember the packed form they came with, so that
 # fst_attention(q, k, v, ancestor_idx, ancestor_mask, leaf_idx, ...) can skip re-packing them.
 _ORIGIN_ATTR = "_fst_tree_metadata"
 
 
-def metadata_of(ancestor_idx, ancestor_mask, leaf_idx) -> Optional[TreeMetadata]:
-    meta = getattr(ancestor_idx, _ORIGIN_ATTR, None)
-    if (meta is not None and meta.ancestor_idx is ancestor_idx and meta.ancestor_mask is ancestor_mask
-            and meta.leaf_idx is leaf_idx and meta.tensors_untouched()):
-        return meta
+class _PackedTwin:
+    """What ``ancestor_idx`` carries: the packed form, and weak references to the three tensors it
+    belongs to.  (A strong reference back would be a cycle, and buffers as large as a tree's mask
+    would then wait for the garbage collector instead of going back to the allocator: building a
+    131068-node tree over and over spent more on fresh allocations than on the kernel.)"""
+    __slots__ = ("n_trees", "n_blocks", "block_m", "max_ancestors", "packed", "tree_stride", "reads_since_build",
+                 "versions", "tensors")
+
+    def __init__(self, meta: TreeMetadata):
+        three = (meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx)
+        self.n_trees, self.n_blocks = meta.n_trees, meta.n_blocks
+        self.block_m, self.max_ancestors = meta.block_m, meta.max_ancestors
+        self.packed, self.tree_stride = meta.packed, meta.tree_stride
+        self.reads_since_build = 0
+        self.versions = _versions(three)
+        self.tensors = tuple(weakref.ref(t) for t in three)
+
+
+def metadata_of(ancestor_idx, ancestor_mask, leaf_idx) -> Optional[_PackedTwin]:
+    """The packed form of three tensors handed out together, while nobody has changed them."""
+    twin = getattr(ancestor_idx, _ORIGIN_ATTR, None)
+    three = (ancestor_idx, ancestor_mask, leaf_idx)
+    if twin is not None and all(r() is t for r, t in zip(twin.tensors, three)) and twin.versions == _versions(three):
+        return twin
     return None
 
 
@@ -95,6 +121,10 @@ def _as_parent_tensor(parent: TreeLike, device) -> torch.Tensor:
         parent = torch.tensor(parent, dtype=torch.int32)
     if parent.dim() not in (1, 2) or parent.numel() == 0:
         raise ValueError("parent must be a non-empty [N] or [T, N] array")
+    if parent.is_cuda and parent.dtype == torch.int32 and parent.is_contiguous() and device is None:
+        return parent
+    if device is None:
+        device = parent.device if parent.is_cuda else "cuda"
     return parent.to(device=device, dtype=torch.int32, non_blocking=True).contiguous()
 
 
@@ -114,46 +144,22 @@ def build_tree_metadata(parent: TreeLike, block_m: int = 64, max_ancestors: int 
     status record, which avoids a device synchronisation; call ``.check()`` later.  ``out``
     reuses the buffers of an earlier result of the same shape (nothing is allocated then).
     """
-    if device is None:
-        device = parent.device if torch.is_tensor(parent) and parent.is_cuda else "cuda"
     par = _as_parent_tensor(parent, device)
-    batched = par.dim() == 2
-    n_trees, n_nodes = (par.shape if batched else (1, par.shape[0]))
-    nb = math.ceil(n_nodes / block_m)
-    lib = _lib.lib()
-    dev = par.device
-    if out is not None:
-        if (out.n_trees, out.n_nodes, out.block_m, out.max_ancestors) != (n_trees, n_nodes, block_m, max_ancestors):
-            raise ValueError("out= metadata has a different shape")
-        meta = out
-        meta.status.zero_()
+    host = _lib._host or _lib.host()
+    if out is None:
+        n_trees, n_nodes, packed, stride, status, ai, am, li = host.new_metadata(par, block_m, max_ancestors,
+                                                                                 bool(reference_format))
+        meta = TreeMetadata(n_trees, n_nodes, block_m, max_ancestors, packed, stride, status, ai, am, li, par.dim() == 2)
+        if ai is not None:
+            setattr(ai, _ORIGIN_ATTR, meta._twin)
     else:
-        stride = packed_meta_bytes(nb, block_m, max_ancestors)
-        if stride == 0:
-            raise ValueError("block_m and max_ancestors must be positive")
-        packed = torch.empty((n_trees, stride), dtype=torch.uint8, device=dev)
-        status = torch.zeros(_lib.STATUS_WORDS, dtype=torch.int32, device=dev)
-        ai = am = li = None
-        if reference_format:
-            lead = (n_trees,) if batched else ()
-            ai = torch.empty(lead + (nb, max_ancestors), dtype=torch.long, device=dev)
-            am = torch.empty(lead + (nb, block_m, max_ancestors), dtype=torch.bool, device=dev)
-            li = torch.empty(lead + (nb, block_m), dtype=torch.long, device=dev)
-        meta = TreeMetadata(n_trees, n_nodes, block_m, max_ancestors, packed, stride, status,
-                            ai, am, li, batched)
-        if reference_format:
-            setattr(ai, _ORIGIN_ATTR, meta)
-    with torch.cuda.device(dev):
-        rc = lib.fst_precompute(
-            par.data_ptr(), n_trees, n_nodes, block_m, max_ancestors,
-            meta.ancestor_idx.data_ptr() if meta.ancestor_idx is not None else None,
-            meta.ancestor_mask.data_ptr() if meta.ancestor_mask is not None else None,
-            meta.leaf_idx.data_ptr() if meta.leaf_idx is not None else None,
-            meta.packed.data_ptr(), meta.tree_stride, meta.status.data_ptr(),
-            torch.cuda.current_stream(dev).cuda_stream)
-    _lib.check(rc, "fst_precompute")
-    meta._versions = meta._current_versions()
-    meta.reads_since_build = 0
+        meta = out
+        n_trees, n_nodes = par.shape if par.dim() == 2 else (1, par.shape[0])
+        if (meta.n_trees, meta.n_nodes, meta.block_m, meta.max_ancestors) != (n_trees, n_nodes, block_m, max_ancestors):
+            raise ValueError("out= metadata has a different shape")
+        host.precompute(par, block_m, max_ancestors, meta.packed, meta.tree_stride, meta.status,
+                        meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx)
+        meta._rebuilt()
     if check:
         meta.check()
     return meta
@@ -186,30 +192,17 @@ def build_tree_topk(scores: torch.Tensor, depth: Optional[int] = None, topk: Opt
     """
     if not scores.is_cuda or scores.dtype != torch.float32 or scores.dim() not in (2, 3):
         raise TypeError("scores must be a CUDA float32 tensor [depth + 1, topk] or [T, depth + 1, topk]")
-    batched = scores.dim() == 3
     levels, k = scores.shape[-2:]
     depth = levels - 1 if depth is None else depth
     topk = k if topk is None else topk
     if (depth + 1, topk) != (levels, k):
         raise ValueError("scores must have depth + 1 rows of topk entries")
-    n_trees = scores.shape[0] if batched else 1
     total = tree_topk_nodes(depth, topk, left_weight_factor)
     n = total if max_nodes is None else int(max_nodes)
     if n <= 0:
         raise ValueError("max_nodes must be positive")
-    sc = scores.contiguous()
-    dev = sc.device
-    lead = (n_trees,) if batched else ()
-    parent = torch.empty(lead + (n,), dtype=torch.int32, device=dev)
-    choice = torch.empty(lead + (n,), dtype=torch.int32, device=dev) if return_choice else None
-    nscore = torch.empty(lead + (n,), dtype=torch.float32, device=dev) if return_scores else None
-    with torch.cuda.device(dev):
-        rc = _lib.lib().fst_build_tree_topk(
-            sc.data_ptr(), n_trees, depth, topk, float(left_weight_factor), n, parent.data_ptr(),
-            choice.data_ptr() if choice is not None else None,
-            nscore.data_ptr() if nscore is not None else None,
-            torch.cuda.current_stream(dev).cuda_stream)
-    _lib.check(rc, "fst_build_tree_topk")
+    parent, choice, nscore = (_lib._host or _lib.host()).build_tree_topk(
+        scores, depth, topk, float(left_weight_factor), n, bool(return_choice), bool(return_scores))
     extra = tuple(t for t in (choice, nscore) if t is not None)
     return (parent,) + extra if extra else parent
 
@@ -220,6 +213,10 @@ def parent_from_lineage(lineage: torch.Tensor, level_lookup: torch.Tensor) -> to
     col = (lvl - 1).clamp_min(0).unsqueeze(1)
     par = lineage.gather(1, col).squeeze(1)
     return torch.where(lvl > 0, par, torch.full_like(par, -1))
+
+
+def _on_host(t, dim: int) -> bool:
+    return t.device.type == "cpu" and t.dtype == torch.long and t.dim() == dim
 
 
 def create_fst_attention_kernel_inputs(lineage: torch.Tensor, level_lookup: torch.Tensor,
@@ -233,9 +230,12 @@ def create_fst_attention_kernel_inputs(lineage: torch.Tensor, level_lookup: torc
     ancestors.  Like the reference (utils.py:124-125) it writes every node into its own lineage
     row as a side effect; pass ``mutate_lineage=False`` to leave ``lineage`` alone.
     """
-    parent = parent_from_lineage(lineage, level_lookup)
+    native = _on_host(lineage, 2) and _on_host(level_lookup, 1) and lineage.shape[0] == level_lookup.shape[0]
+    parent = _lib.host().parents_of_lineage(lineage, level_lookup) if native else parent_from_lineage(lineage, level_lookup)
     meta = build_tree_metadata(parent, block_m, max_ancestors, reference_format=True, check=True)
-    if mutate_lineage:
+    if mutate_lineage and native:
+        _lib.host().write_self(lineage, level_lookup)
+    elif mutate_lineage:
         n = lineage.shape[0]
         rows = torch.arange(n, device=lineage.device)
         lineage[rows, level_lookup.to(lineage.device).long()] = rows
@@ -362,22 +362,12 @@ def dfs_order_device(parent: TreeLike, *, check: bool = True,
     ``dfs_order`` gives them; ``new_parent`` goes straight into ``build_tree_metadata``.
     ``check=False`` skips reading the status record (no device synchronisation); a malformed
     tree then leaves both outputs uninitialised."""
-    if device is None:
-        device = parent.device if torch.is_tensor(parent) and parent.is_cuda else "cuda"
     par = _as_parent_tensor(parent, device)
-    n_trees, n_nodes = (par.shape if par.dim() == 2 else (1, par.shape[0]))
-    order = torch.empty_like(par)
-    new_parent = torch.empty_like(par)
-    status = torch.zeros(_lib.STATUS_WORDS, dtype=torch.int32, device=par.device)
-    with torch.cuda.device(par.device):
-        rc = _lib.lib().fst_dfs_order(par.data_ptr(), n_trees, n_nodes, order.data_ptr(), new_parent.data_ptr(),
-                                      status.data_ptr(), torch.cuda.current_stream(par.device).cuda_stream)
-    _lib.check(rc, "fst_dfs_order")
+    order, new_parent, status = (_lib._host or _lib.host()).dfs_order(par)
     if check:
-        code, where, detail, _ = status.tolist()
+        code, where, detail, _ = _lib.host().read_status(status)
         if code == _lib.DEV_MALFORMED_TREE:
             raise ValueError(f"parent[{where}] = {detail} is neither -1 nor an earlier node")
         if code != 0:
             raise RuntimeError(f"fst_dfs_order: device status {code}")
     return order, new_parent
-
