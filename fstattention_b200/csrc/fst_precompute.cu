@@ -284,15 +284,264 @@ precompute_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int bm, i
         }
 }
 
+// The same for large trees.  precompute_kernel keeps the parents of every node below the block's last row
+// in shared memory, so a block of a 131068-node tree reads half a megabyte to follow fifteen links per
+// row, one CTA to an SM.  Here
+//   * the rows climb through L2 (the parent array fits it many times over) and stop at the first node that
+//     another row has been to; a bitmap of the nodes below the block is the only thing that grows with
+//     the tree, and everything that walks it skips its empty words 32 at a time;
+//   * the mask is inherited instead of climbed for again: a slot's row is its parent slot's row and its own
+//     bit, by pointer doubling over the (at most max_ancestors) slots, and a block row's mask is its
+//     parent's;
+// so that a CTA's time is one climb and its shared memory lets seven share an SM.  131068 nodes, block_m 128, with
+// the reference-format tensors: 161 us with precompute_kernel.
+constexpr int WIDE_THREADS = 256, WIDE_WARPS = WIDE_THREADS / 32;
+
+// 32-bit words of shared memory: bitmap and 16-bit ranks of Wp words, masks of slots or rows, block masks,
+// parent and own slot of every row, and of every slot its node and parent slot
+__host__ __device__ inline size_t wide_smem_words(size_t Wp, int bm, int ma, bool inherit) {
+    const size_t maw = (ma + 31) / 32, bw = (bm + 31) / 32;
+    return Wp + Wp / 2 + size_t(inherit && ma > bm ? ma : bm) * maw + size_t(bm) * bw + size_t(bm) * 2 + (inherit ? size_t(ma) * 2 : 0);
+}
+
+__global__ void __launch_bounds__(WIDE_THREADS, 7)
+precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int bm, int ma, int inherit_ok,
+                       int64_t *__restrict__ anc_idx_all, uint8_t *__restrict__ anc_mask_all,
+                       int64_t *__restrict__ leaf_idx_all, unsigned char *__restrict__ packed_all,
+                       size_t packed_stride, int32_t *status) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_warp[WIDE_WARPS], s_ext[WIDE_WARPS];
+    const int b = blockIdx.x, tree = blockIdx.y, nb = gridDim.x;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int row0 = b * bm, maw = (ma + 31) >> 5, bw = (bm + 31) >> 5;
+    // bitmap words, phantom rows included; every warp scans a run of whole 32-word groups
+    const int per_warp = (((row0 + bm + 31) >> 5) + 32 * WIDE_WARPS - 1) / (32 * WIDE_WARPS) * 32, W = per_warp * WIDE_WARPS;
+
+    uint32_t *bitmap = reinterpret_cast<uint32_t *>(smem_raw);       // [W]
+    uint16_t *rank = reinterpret_cast<uint16_t *>(bitmap + W);       // [W] set bits below word w (only where w has any)
+    uint32_t *bits = bitmap + W + W / 2;                             // inherited: [slot][maw], else [row][maw]
+    uint32_t *blkmask = bits + size_t(inherit_ok && ma > bm ? ma : bm) * maw;   // [bm][bw] over block rows
+    int *up = reinterpret_cast<int *>(blkmask + size_t(bm) * bw);    // [bm] parent of row j, then its slot
+    int *self = up + bm;                                             // [bm] slot of row j itself, -1: nobody's ancestor
+    int *node_of = self + bm, *jump = node_of + ma;                  // [ma] (inherited only)
+
+    const int32_t *parent = parent_all + size_t(tree) * n_nodes;
+    auto par = [&](int x) -> int {                        // a malformed entry is reported and treated as a root
+        const int p = __ldg(parent + x);
+        if (p >= x || p < -1) {
+            report(status, FST_DEV_MALFORMED_TREE, x, p);
+            return -1;
+        }
+        return p;
+    };
+    for (int i = tid; i < W / 4; i += WIDE_THREADS) reinterpret_cast<uint4 *>(bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i < bm * bw; i += WIDE_THREADS) blkmask[i] = 0u;
+    __syncthreads();
+
+    // 1. every row climbs until it meets a marked node
+    for (int j = tid; j < bm; j += WIDE_THREADS) {
+        int x = row0 + j < n_nodes ? par(row0 + j) : -1;
+        up[j] = x;
+        while (x >= 0) {
+            const int next = par(x);                      // under way while x is marked
+            const uint32_t bit = 1u << (x & 31);
+            if (atomicOr(&bitmap[x >> 5], bit) & bit) break;
+            x = next;
+        }
+    }
+    __syncthreads();
+
+    // 2. ranks: set bits before every word that has some
+    int mine = 0;
+    for (int i = 0; i < per_warp; i += 32) mine += __popc(bitmap[wid * per_warp + i + lane]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    if (lane == 0) s_warp[wid] = mine;
+    __syncthreads();
+    int base = 0, n_anc = 0;
+#pragma unroll
+    for (int w = 0; w < WIDE_WARPS; ++w) {
+        if (w < wid) base += s_warp[w];
+        n_anc += s_warp[w];
+    }
+    const int n_keep = min(n_anc, ma);
+    const bool inherit = inherit_ok && n_anc <= ma;
+    if (n_anc > ma && tid == 0) report(status, FST_DEV_ANCESTOR_OVERFLOW, tree * 65536 + b, n_anc);
+
+    const PackedLayout L = packed_layout(nb, bm, ma);
+    unsigned char *blob = packed_all ? packed_all + size_t(tree) * packed_stride : nullptr;
+    int32_t *p_idx = blob ? reinterpret_cast<int32_t *>(blob + L.off_idx) + size_t(b) * ma : nullptr;
+    const size_t blk = size_t(tree) * nb + b;
+    int64_t *o_idx = anc_idx_all ? anc_idx_all + blk * ma : nullptr;
+
+    // 3. ascending ancestor list, a lane per word
+    int ext = 0;                                          // listed nodes below the block
+    for (int i = 0; i < per_warp; i += 32) {
+        const int w = wid * per_warp + i + lane;
+        uint32_t word = bitmap[w];
+        if (__ballot_sync(0xffffffffu, word != 0u) == 0u) continue;
+        const int own = __popc(word);
+        int before = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= o) before += v;
+        }
+        const int group = __shfl_sync(0xffffffffu, before, 31);
+        int pos = base + before - own;
+        rank[w] = uint16_t(min(pos, 0xffff));
+        for (; word != 0u; word &= word - 1u, ++pos) {
+            const int node = w * 32 + __ffs(word) - 1;
+            if (node < row0) ++ext;
+            if (pos < ma) {
+                if (p_idx && node < row0) p_idx[pos] = node;
+                if (o_idx) o_idx[pos] = node;
+                if (inherit) node_of[pos] = node;
+            }
+        }
+        base += group;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ext += __shfl_xor_sync(0xffffffffu, ext, o);
+    if (lane == 0) s_ext[wid] = ext;
+    if (!inherit)
+        for (int i = tid; i < bm * maw; i += WIDE_THREADS) bits[i] = 0u;
+    __syncthreads();
+    int n_ext = 0;
+#pragma unroll
+    for (int w = 0; w < WIDE_WARPS; ++w) n_ext += s_ext[w];
+    n_ext = min(n_ext, ma);
+    if (p_idx)
+        for (int i = n_ext + tid; i < ma; i += WIDE_THREADS) p_idx[i] = -1;
+    if (o_idx)
+        for (int i = n_keep + tid; i < ma; i += WIDE_THREADS) o_idx[i] = -1;
+    if (tid == 0 && blob) reinterpret_cast<int32_t *>(blob + L.off_count)[b] = n_ext;
+
+    // 4. masks.  Slot of a node, -1 when it is nobody's ancestor here
+    auto slot_of = [&](int x) -> int {
+        const uint32_t word = bitmap[x >> 5], bit = 1u << (x & 31);
+        return word & bit ? int(rank[x >> 5]) + __popc(word & (bit - 1u)) : -1;
+    };
+    if (inherit) {
+        for (int s = tid; s < n_keep; s += WIDE_THREADS) {
+            const int p = par(node_of[s]);
+            jump[s] = p < 0 ? -1 : slot_of(p);
+            for (int w = 0; w < maw; ++w) bits[s * maw + w] = w == (s >> 5) ? 1u << (s & 31) : 0u;
+        }
+        for (int j = tid; j < bm; j += WIDE_THREADS) {
+            const int p = up[j];
+            up[j] = p < 0 ? -1 : slot_of(p);
+            self[j] = row0 + j < n_nodes ? slot_of(row0 + j) : -1;
+        }
+        __syncthreads();
+        constexpr int PER = 2;                            // (slot, word) pairs per thread: 128 slots of 4 words
+        const int pairs = n_keep * maw;
+        for (;;) {
+            bool any = false;
+            uint32_t got[PER];
+            int far[PER];
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const int i = tid + k * WIDE_THREADS;
+                got[k] = 0u;
+                far[k] = -1;
+                if (i < pairs) {
+                    const int s = i / maw, w = i - s * maw, to = jump[s];
+                    if (to >= 0) {
+                        got[k] = bits[to * maw + w];
+                        far[k] = jump[to];
+                        any = true;
+                    }
+                } else {
+                    break;
+                }
+            }
+            if (!__syncthreads_or(any)) break;
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const int i = tid + k * WIDE_THREADS;
+                if (i >= pairs) break;
+                bits[i] |= got[k];
+                if (i % maw == 0) jump[i / maw] = far[k];
+            }
+            __syncthreads();
+        }
+    } else {                                              // too many ancestors, or too wide a mask: climb again
+        for (int j = tid; j < bm; j += WIDE_THREADS)
+            for (int x = row0 + j < n_nodes ? row0 + j : -1; x >= 0; x = par(x)) {
+                const int pos = slot_of(x);
+                if (pos < 0) continue;
+                if (pos < ma) bits[j * maw + (pos >> 5)] |= 1u << (pos & 31);
+                if (x >= row0) blkmask[j * bw + ((x - row0) >> 5)] |= 1u << ((x - row0) & 31);
+            }
+        __syncthreads();
+    }
+    auto row_word = [&](int j, int w) -> uint32_t {       // word w of row j's mask over all of A_b
+        if (!inherit) return bits[j * maw + w];
+        const uint32_t above = up[j] >= 0 ? bits[up[j] * maw + w] : 0u;
+        return above | (self[j] >= 0 && (self[j] >> 5) == w ? 1u << (self[j] & 31) : 0u);
+    };
+    for (int j = tid; j < bm; j += WIDE_THREADS) {
+        blkmask[j * bw + (j >> 5)] |= 1u << (j & 31);     // every row attends to itself
+        if (inherit)                                      // and to its ancestors inside the block
+            for (int s = n_ext; s < n_keep; ++s)
+                if ((row_word(j, s >> 5) >> (s & 31)) & 1u) {
+                    const int c = node_of[s] - row0;
+                    blkmask[j * bw + (c >> 5)] |= 1u << (c & 31);
+                }
+    }
+
+    if (blob) {
+        uint32_t *p_emask = reinterpret_cast<uint32_t *>(blob + L.off_emask) + size_t(b) * bm * maw;
+        for (int i = tid; i < bm * maw; i += WIDE_THREADS) {
+            const int j = i / maw, w = i - j * maw, lo = w * 32;      // keep the bits of external slots only
+            const uint32_t keep = n_ext >= lo + 32 ? 0xffffffffu : (n_ext > lo ? (1u << (n_ext - lo)) - 1u : 0u);
+            p_emask[i] = row_word(j, w) & keep;
+        }
+    }
+    if (anc_mask_all) {
+        uint8_t *o_mask = anc_mask_all + blk * size_t(bm) * ma;
+        if ((ma & 15) == 0 && (reinterpret_cast<uintptr_t>(o_mask) & 15) == 0) {   // sixteen bool bytes per store
+            const int pieces = ma / 16;
+            for (int i = tid; i < bm * pieces; i += WIDE_THREADS) {
+                const int j = i / pieces, at = (i - j * pieces) * 16;
+                const uint32_t half = row_word(j, at >> 5) >> (at & 31);
+                auto four = [&](int k) {                  // bits 4 k .. 4 k + 3 as bytes
+                    const uint32_t nib = (half >> (4 * k)) & 0xfu;
+                    return (nib & 1u) | ((nib & 2u) << 7) | ((nib & 4u) << 14) | ((nib & 8u) << 21);
+                };
+                reinterpret_cast<uint4 *>(o_mask)[i] = make_uint4(four(0), four(1), four(2), four(3));
+            }
+        } else {
+            for (int i = tid; i < bm * ma; i += WIDE_THREADS) {
+                const int j = i / ma, at = i - j * ma;
+                o_mask[i] = (row_word(j, at >> 5) >> (at & 31)) & 1u;
+            }
+        }
+    }
+    // 5. leaves: block rows that are not in the ancestor set (rows past the last node too)
+    if (leaf_idx_all)
+        for (int j = tid; j < bm; j += WIDE_THREADS) {
+            const int k = row0 + j;
+            leaf_idx_all[blk * bm + j] = ((bitmap[k >> 5] >> (k & 31)) & 1u) ? int64_t(-1) : int64_t(k);
+        }
+    __syncthreads();
+    if (blob) {
+        uint32_t *p_bmask = reinterpret_cast<uint32_t *>(blob + L.off_bmask) + size_t(b) * bm * bw;
+        for (int i = tid; i < bm * bw; i += WIDE_THREADS) p_bmask[i] = blkmask[i];
+    }
+}
+
 // -------------------------------------------------------------------------------------------
 // reference-format tensors -> packed blob
 // -------------------------------------------------------------------------------------------
-constexpr int PACK_THREADS = 128;
+constexpr int PACK_THREADS = 512;
+constexpr int PACK_WORDS = 64;         // mask words of a row held in shared memory, half for each mask
 
 __global__ void __launch_bounds__(PACK_THREADS)
 pack_kernel(const int64_t *__restrict__ anc_idx_all, const uint8_t *__restrict__ anc_mask_all,
             const int64_t *__restrict__ leaf_idx_all, int bm, int ma, int64_t index_base,
-            unsigned char *__restrict__ packed_all, size_t packed_stride, int32_t *status) {
+            unsigned char *__restrict__ packed_all, size_t packed_stride, int32_t *status, int wide_words) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int b = blockIdx.x, tree = blockIdx.y, nb = gridDim.x;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -300,6 +549,8 @@ pack_kernel(const int64_t *__restrict__ anc_idx_all, const uint8_t *__restrict__
     // slot -> external position (>= 0), or -1 - column for an ancestor inside the block, or
     // INT_MIN for padding
     int *slot_map = reinterpret_cast<int *>(smem_raw);               // [ma]
+    uint32_t *s_wide = reinterpret_cast<uint32_t *>(slot_map + ma);  // [wide_words] the block's two masks
+    __shared__ uint32_t s_bits[PACK_THREADS / 32][PACK_WORDS];
     __shared__ int s_warp[PACK_THREADS / 32];
     __shared__ int s_base;
     if (tid == 0) s_base = 0;
@@ -316,6 +567,23 @@ pack_kernel(const int64_t *__restrict__ anc_idx_all, const uint8_t *__restrict__
     const uint8_t *g_mask = anc_mask_all + blk * size_t(bm) * ma;
     const int64_t *g_leaf = leaf_idx_all + blk * bm;
     const int64_t row0 = int64_t(b) * bm;
+
+    // The mask's bytes are asked for first, sixteen at a time: nothing but their use depends on the slot
+    // map (row after row, a warp each, with loads behind the map, took 8.4 us at 64 x 64).
+    constexpr int AHEAD = 2;
+    const bool wide = wide_words > 0;                     // both masks of the block fit shared memory
+    const int pieces = ma / 16, n_pieces = bm * pieces;
+    uint4 bytes[AHEAD];
+    if (wide) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(g_mask);
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+            const int i = tid + k * PACK_THREADS;
+            bytes[k] = i < n_pieces ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        for (int i = tid; i < wide_words; i += PACK_THREADS) s_wide[i] = 0u;
+    }
+    const int64_t my_leaf = tid < bm ? __ldg(g_leaf + tid) : -1;
 
     // external slots keep their order; an exclusive scan of the "is external" flags places them
     for (int a0 = 0; a0 < ma; a0 += PACK_THREADS) {
@@ -359,22 +627,67 @@ pack_kernel(const int64_t *__restrict__ anc_idx_all, const uint8_t *__restrict__
     for (int a = n_ext + tid; a < ma; a += PACK_THREADS) p_idx[a] = -1;
     if (tid == 0) p_count[b] = n_ext;
 
-    // one thread per row: scatter its mask bytes into the two bit masks
-    for (int j = tid; j < bm; j += PACK_THREADS) {
-        uint32_t *er = p_emask + size_t(j) * maw, *br = p_bmask + size_t(j) * bw;
-        for (int w = 0; w < maw; ++w) er[w] = 0u;
-        for (int w = 0; w < bw; ++w) br[w] = 0u;
+    if (wide) {
+        uint32_t *e = s_wide, *m = s_wide + size_t(bm) * maw;
+        for (int j = tid; j < bm; j += PACK_THREADS) {
+            const int64_t leaf = j == tid ? my_leaf : __ldg(g_leaf + j);
+            if (leaf < 0 || leaf < index_base) continue;
+            if (leaf - index_base != row0 + j) report(status, FST_DEV_INDEX_RANGE, tree * 65536 + b, -1 - j);
+            atomicOr(&m[j * bw + (j >> 5)], 1u << (j & 31));
+        }
+        auto scatter = [&](int i, const uint4 &v) {
+            const int j = i / pieces, a0 = (i - j * pieces) * 16;
+            const uint32_t part[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                for (uint32_t rest = part[q]; rest != 0u;) {
+                    const int k = (__ffs(rest) - 1) >> 3;     // the next byte that is not zero
+                    rest &= ~(0xffu << (8 * k));
+                    const int code = slot_map[a0 + q * 4 + k];
+                    if (code >= 0) atomicOr(&e[j * maw + (code >> 5)], 1u << (code & 31));
+                    else if (code != INT_MIN) atomicOr(&m[j * bw + ((-1 - code) >> 5)], 1u << ((-1 - code) & 31));
+                }
+        };
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k)
+            if (tid + k * PACK_THREADS < n_pieces) scatter(tid + k * PACK_THREADS, bytes[k]);
+        for (int i = tid + AHEAD * PACK_THREADS; i < n_pieces; i += PACK_THREADS)
+            scatter(i, __ldg(reinterpret_cast<const uint4 *>(g_mask) + i));
+        __syncthreads();
+        for (int i = tid; i < bm * maw; i += PACK_THREADS) p_emask[i] = e[i];
+        for (int i = tid; i < bm * bw; i += PACK_THREADS) p_bmask[i] = m[i];
+        return;
+    }
+    // Scatter the mask bytes into the two bit masks: a warp per row, a lane per byte, and the few bits
+    // that are set go through shared memory (one thread per row, byte after byte, took 8 us at
+    // 64 x 64; the loads of a whole row are now one access).
+    uint32_t *er = s_bits[wid];
+    uint32_t *br = er + PACK_WORDS / 2;
+    const bool small = maw <= PACK_WORDS / 2 && bw <= PACK_WORDS / 2;
+    for (int j = wid; j < bm; j += PACK_THREADS / 32) {
+        uint32_t *e_out = p_emask + size_t(j) * maw, *b_out = p_bmask + size_t(j) * bw;
+        uint32_t *e = small ? er : e_out, *m = small ? br : b_out;   // very wide masks: straight to memory
+        for (int w = lane; w < maw; w += 32) e[w] = 0u;
+        for (int w = lane; w < bw; w += 32) m[w] = 0u;
+        __syncwarp();
         const int64_t leaf = g_leaf[j];
         const bool is_leaf = leaf >= 0 && leaf >= index_base;
-        if (is_leaf && leaf - index_base != row0 + j)
-            report(status, FST_DEV_INDEX_RANGE, tree * 65536 + b, -1 - j);
-        if (is_leaf) br[j >> 5] |= 1u << (j & 31);
+        if (lane == 0 && is_leaf) {
+            if (leaf - index_base != row0 + j) report(status, FST_DEV_INDEX_RANGE, tree * 65536 + b, -1 - j);
+            atomicOr(&m[j >> 5], 1u << (j & 31));
+        }
         const uint8_t *src = g_mask + size_t(j) * ma;
-        for (int a = 0; a < ma; ++a) {
+        for (int a = lane; a < ma; a += 32) {
             if (!src[a]) continue;
             const int code = slot_map[a];
-            if (code >= 0) er[code >> 5] |= 1u << (code & 31);
-            else if (code != INT_MIN) br[(-1 - code) >> 5] |= 1u << ((-1 - code) & 31);
+            if (code >= 0) atomicOr(&e[code >> 5], 1u << (code & 31));
+            else if (code != INT_MIN) atomicOr(&m[(-1 - code) >> 5], 1u << ((-1 - code) & 31));
+        }
+        __syncwarp();
+        if (small) {
+            for (int w = lane; w < maw; w += 32) e_out[w] = e[w];
+            for (int w = lane; w < bw; w += 32) b_out[w] = m[w];
+            __syncwarp();
         }
     }
 }
@@ -382,6 +695,8 @@ pack_kernel(const int64_t *__restrict__ anc_idx_all, const uint8_t *__restrict__
 // largest dynamic shared memory enabled so far, per device and kernel variant
 static std::atomic<size_t> g_pre_smem_set[2][kMaxDevices];
 static std::atomic<size_t> g_pack_smem_set[kMaxDevices];
+static std::atomic<size_t> g_wide_smem_set[kMaxDevices];
+constexpr int kWideNodes = 8192;
 
 cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, int bm, int ma,
                               int64_t *anc_idx, uint8_t *anc_mask, int64_t *leaf_idx,
@@ -397,6 +712,26 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
     int depth_cap = int((48 * 1024) / (size_t(bm) * 4));
     if (depth_cap > 1024) depth_cap = 1024;
     if (depth_cap < 1) depth_cap = 1;
+    // Large trees: when a block's share of the parent array outgrows what one pass of the CTA stages in the
+    // time a climb through L2 takes (see precompute_wide_kernel).
+    const int slot = current_device_slot();
+    if (slot < 0) return cudaErrorInvalidDevice;
+    if (n_nodes > kWideNodes) {
+        const size_t Ww = (W + 32 * WIDE_WARPS - 1) / (32 * WIDE_WARPS) * (32 * WIDE_WARPS);
+        const bool inherit = ma <= 128;                   // masks of all slots: 2 KB, two words per thread
+        const size_t smem = wide_smem_words(Ww, bm, ma, inherit) * 4;
+        if (smem <= budget) {
+            if (smem > 48 * 1024 && smem > g_wide_smem_set[slot].load(std::memory_order_acquire)) {
+                cudaError_t e = cudaFuncSetAttribute(precompute_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+                if (e != cudaSuccess) return e;
+                g_wide_smem_set[slot].store(smem, std::memory_order_release);
+            }
+            precompute_wide_kernel<<<dim3(nb, n_trees), WIDE_THREADS, smem, stream>>>(
+                parent, n_nodes, bm, ma, inherit ? 1 : 0, anc_idx, anc_mask, leaf_idx, static_cast<unsigned char *>(packed),
+                packed_stride, status);
+            return cudaGetLastError();
+        }
+    }
     // Byte flags (one byte per node below the last row) while they leave room to stage a good
     // part of the parent array; beyond that the walkers set bitmap bits with atomics.
     bool byte_flags = base + W * 32 + size_t(depth_cap) * bm * 4 + 16 * 1024 <= budget;
@@ -409,8 +744,6 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
     const size_t cap = (budget - fixed) / 4;
     const int par_cap = int(cap < size_t(n_nodes) ? cap : size_t(n_nodes));
     const size_t smem = fixed + size_t(par_cap) * 4;
-    const int slot = current_device_slot();
-    if (slot < 0) return cudaErrorInvalidDevice;
     auto kernel = byte_flags ? precompute_kernel<true> : precompute_kernel<false>;
     std::atomic<size_t> &enabled = g_pre_smem_set[byte_flags ? 1 : 0][slot];
     if (smem > 48 * 1024 && smem > enabled.load(std::memory_order_acquire)) {
@@ -428,7 +761,9 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
 cudaError_t launch_pack(const int64_t *anc_idx, const uint8_t *anc_mask, const int64_t *leaf_idx,
                         int n_trees, int nb, int bm, int ma, int64_t index_base, void *packed,
                         size_t packed_stride, int32_t *status, cudaStream_t stream) {
-    const size_t smem = size_t(ma) * 4;
+    const size_t words = size_t(bm) * ((ma + 31) / 32 + (bm + 31) / 32);
+    const bool wide = words <= 8192 && ma % 16 == 0 && (reinterpret_cast<uintptr_t>(anc_mask) & 15) == 0;
+    const size_t smem = size_t(ma) * 4 + (wide ? words * 4 : 0);
     const int slot = current_device_slot();
     if (slot < 0) return cudaErrorInvalidDevice;
     if (smem > 48 * 1024 && smem > g_pack_smem_set[slot].load(std::memory_order_acquire)) {
@@ -439,7 +774,7 @@ cudaError_t launch_pack(const int64_t *anc_idx, const uint8_t *anc_mask, const i
     dim3 grid(nb, n_trees);
     pack_kernel<<<grid, PACK_THREADS, smem, stream>>>(
         anc_idx, anc_mask, leaf_idx, bm, ma, index_base, static_cast<unsigned char *>(packed),
-        packed_stride, status);
+        packed_stride, status, wide ? int(words) : 0);
     return cudaGetLastError();
 }
 
