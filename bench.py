@@ -143,7 +143,8 @@ def kernel_source_digest():
     sources it was taken from."""
     h = hashlib.sha1()
     csrc = os.path.join(ROOT, "fstattention_b200", "csrc")
-    for name in ("fst_attention_tma.cuh", "fst_attention_persist.cuh", "fst_attention_mma.cuh", "fst_prefix_umma.cu"):
+    for name in ("fst_attention_tma.cuh", "fst_attention_persist.cuh", "fst_attention_mma.cuh", "fst_prefix_umma.cu",
+                 "fst_tree_umma.cuh"):
         try:
             with open(os.path.join(csrc, name), "rb") as f:
                 h.update(f.read())
@@ -379,7 +380,7 @@ def measure_case(fst, w, layers_n, reps, dev, kernel="auto", case=None):
     peak, peak_kind = measured_hbm_peak()
     kv = info["gathered_kv_bytes_per_call"]
     traffic, source = ncu_traffic(case or w.name)
-    plan = fst.launch_plan(layers[0][0], w.prefix, w.block_m, kernel)
+    plan = fst.launch_plan(layers[0][0], w.prefix, w.block_m, kernel, max_ancestors=w.max_ancestors)
     resident = sum(t.numel() * t.element_size() for trip in layers for t in trip) / 1e6
     out = {"config": workload_config(w, layers_n), "us_per_call": us, "precompute_us": pre_us,
            "gathered_kv_bytes_per_call": kv, "q_o_bytes_per_call": info["q_o_bytes_per_call"],
@@ -873,7 +874,7 @@ def run_ours(args, rank, world):
     # the bound is the tensor cores.  Algorithmic flops: every query block forms block_m x rows
     # scores and as many products with V, 2 * head_dim flops each.
     probe = torch.empty((T, H, N, D), device=dev, dtype=dtype)
-    plan = fst.launch_plan(probe, w.prefix, w.block_m, args.kernel)
+    plan = fst.launch_plan(probe, w.prefix, w.block_m, args.kernel, max_ancestors=w.max_ancestors)
     del probe
     traffic, traffic_source = ncu_traffic(w.name)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

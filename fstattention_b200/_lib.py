@@ -15,7 +15,7 @@ STATUS_WORDS = 4
 DTYPE_F16, DTYPE_BF16, DTYPE_F32 = 0, 1, 2
 KERNEL_FLAG_META_STABLE = 0x100
 KERNELS = {"auto": 0, "simt": 1, "mma": 2, "tma": 3, "tma_t32": 4, "tma_t64": 5,
-           "tma_umma": 6, "persist": 7}
+           "tma_umma": 6, "persist": 7, "tree_umma": 8}
 DEV_MALFORMED_TREE, DEV_ANCESTOR_OVERFLOW, DEV_INDEX_RANGE = 16, 17, 18
 
 # every symbol include/fstattn_b200.h declares
@@ -24,7 +24,7 @@ EXPORTS = ("fst_version", "fst_status_string", "fst_packed_meta_bytes", "fst_pre
            "fst_attention_fwd_ref", "fst_attention_fwd_ref_static",
            "fst_attention_split_workspace_bytes", "fst_attention_fwd_splitkv", "fst_attention_fwd_gqa", "fst_dfs_order",
            "fst_attention_fwd_paged", "fst_selftest_wait_timeout", "fst_tree_topk_nodes",
-           "fst_build_tree_topk", "fst_attention_fwd_scatter")
+           "fst_build_tree_topk", "fst_attention_fwd_scatter", "fst_attention_tree_kernel")
 STATIC_SCRATCH_BYTES = 512 * 1024
 
 _lib = None
@@ -50,6 +50,8 @@ def _declare(lib):
     lib.fst_attention_fwd_scatter.restype = _i
     lib.fst_attention_fwd_scatter.argtypes = ([_p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _p, _sz, _i, _i, _i, _i, _i]
                                               + _TENSOR_STRIDES + [_i, _i, _f, _i, _i, _p, _p])
+    lib.fst_attention_tree_kernel.restype = _i
+    lib.fst_attention_tree_kernel.argtypes = [_i, _i, _i, _i, _i, _i]
     lib.fst_attention_split_workspace_bytes.restype = _sz
     lib.fst_attention_split_workspace_bytes.argtypes = [_i, _i, _i, _i, _i]
     lib.fst_attention_fwd_splitkv.restype = _i

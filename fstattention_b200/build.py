@@ -63,7 +63,7 @@ def _build_host() -> None:
     inc = cpp_extension.include_paths() + [os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           "-I", INCLUDE, *(x for d in inc for x in ("-isystem", d)), HOST_SRC, "-o", HOST,
+           "-I", INCLUDE, "-I", CSRC, *(x for d in inc for x in ("-isystem", d)), HOST_SRC, "-o", HOST,
            LIB, "-Wl,-rpath,$ORIGIN", "-L", lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
            "-lc10_cuda", "-L", os.path.join(cuda, "lib64"), "-lcudart"]
     res = subprocess.run(cmd, capture_output=True, text=True)

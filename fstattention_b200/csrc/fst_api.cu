@@ -4,6 +4,7 @@
 #include <cstdio>
 
 #include "fst_common.cuh"
+#include "fst_plan.h"
 
 namespace fst {
 cudaError_t launch_mma_f16_d64(const AttnArgs &, int, cudaStream_t);
@@ -29,6 +30,16 @@ cudaError_t launch_attention_mma(const AttnArgs &a, int dtype, int variant, cuda
     if (dtype == FST_BF16 && a.D == 64) return launch_mma_bf16_d64(a, variant, stream);
     if (dtype == FST_BF16 && a.D == 128) return launch_mma_bf16_d128(a, variant, stream);
     return cudaErrorNotSupported;
+}
+
+cudaError_t launch_tree_umma_f16_d64(const AttnArgs &, cudaStream_t);
+cudaError_t launch_tree_umma_f16_d128(const AttnArgs &, cudaStream_t);
+cudaError_t launch_tree_umma_bf16_d64(const AttnArgs &, cudaStream_t);
+cudaError_t launch_tree_umma_bf16_d128(const AttnArgs &, cudaStream_t);
+
+static cudaError_t launch_tree_umma(const AttnArgs &a, int dtype, cudaStream_t stream) {
+    if (dtype == FST_F16) return a.D == 64 ? launch_tree_umma_f16_d64(a, stream) : launch_tree_umma_f16_d128(a, stream);
+    return a.D == 64 ? launch_tree_umma_bf16_d64(a, stream) : launch_tree_umma_bf16_d128(a, stream);
 }
 
 static int elem_size(int dtype) { return dtype == FST_F32 ? 4 : 2; }
@@ -195,6 +206,13 @@ int fst_pack_metadata(const int64_t *ancestor_idx, const uint8_t *ancestor_mask,
                                    static_cast<cudaStream_t>(stream)));
 }
 
+int fst_attention_tree_kernel(int Z, int H, int n_q, int head_dim, int block_m, int max_ancestors) {
+    if (Z <= 0 || H <= 0 || n_q <= 0 || block_m <= 0 || max_ancestors <= 0) return FST_KERNEL_AUTO;
+    if ((head_dim != 64 && head_dim != 128) || (block_m != 16 && block_m != 32 && block_m != 64 && block_m != 128))
+        return FST_KERNEL_SIMT;
+    return block_m >= 32 && tree_umma_pays(Z, H, n_q, head_dim, block_m, max_ancestors) ? FST_KERNEL_TREE_UMMA : FST_KERNEL_TMA;
+}
+
 size_t fst_attention_split_workspace_bytes(int Z, int H, int n_q, int head_dim, int kv_splits) {
     if (Z <= 0 || H <= 0 || n_q <= 0 || head_dim <= 0 || kv_splits < 1) return 0;
     return size_t(kv_splits + 1) * Z * H * n_q * (size_t(head_dim) + 1) * sizeof(float);
@@ -288,9 +306,19 @@ static int attention_fwd_impl(const void *q, const void *k, const void *v, void 
     if (automatic)
         choice = (mma_ok(dtype, head_dim, block_m) && rows_aligned) ? FST_KERNEL_TMA : FST_KERNEL_SIMT;
     if (choice == FST_KERNEL_SIMT) return cuda_status(launch_attention_simt(a, dtype, st));
-    if (choice < FST_KERNEL_MMA || choice > FST_KERNEL_PERSIST) return FST_ERR_INVALID_ARG;
+    if (choice < FST_KERNEL_MMA || choice > FST_KERNEL_TREE_UMMA) return FST_ERR_INVALID_ARG;
     if (!mma_ok(dtype, head_dim, block_m)) return FST_ERR_UNSUPPORTED;
     if (!rows_aligned) return FST_ERR_ALIGNMENT;
+
+    if (choice == FST_KERNEL_TREE_UMMA) {
+        if (a.prefix != 0 || block_m < 32 || sm_scale <= 0.f) return FST_ERR_UNSUPPORTED;
+        return cuda_status(launch_tree_umma(a, dtype, st));
+    }
+
+    if (automatic && a.prefix == 0 && block_m >= 32 && sm_scale > 0.f && tree_umma_pays(Z, H, n_q, head_dim, block_m, max_ancestors)) {
+        const cudaError_t e = launch_tree_umma(a, dtype, st);
+        if (e != cudaErrorNotSupported) return cuda_status(e);
+    }
 
     // A shared prefix with a workspace: either the tcgen05 prefix kernel takes it in kv_splits runs
     // while the tree kernel does the tree part (head_dim 64 or 128; chosen automatically from 256

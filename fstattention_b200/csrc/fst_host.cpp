@@ -22,6 +22,7 @@
 #include <mutex>
 #include <optional>
 
+#include "fst_plan.h"
 #include "fstattn_b200.h"
 
 namespace {
@@ -87,15 +88,13 @@ int sm_count(int device) {
 
 // ---- the runs a shared prefix is cut into -------------------------------------------------------
 // Only the tensor-core kernels split.  With head_dim 64 or 128 and at least 256 prefix rows the
-// prefix goes to the tcgen05 kernel: one CTA per 128 query rows, head, batch element and run.  Its
-// shared memory allows one CTA per SM, so the automatic choice is as many runs as keep the grid
-// within one wave, each at least 256 rows.  Otherwise the tree kernel walks the prefix itself,
-// split to about four CTAs per SM.
+// prefix goes to the tcgen05 kernel (fst_plan.h says into how many runs).  Otherwise the tree kernel
+// walks the prefix itself, split to about four CTAs per SM.
 struct Splits {
     int runs;
     bool workspace;
 };
-Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, int64_t Z, int64_t H, int64_t n_q,
+Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, int64_t Z, int64_t H, int64_t H_kv, int64_t n_q,
                    int64_t D, int64_t prefix, int64_t block_m, int kernel, int device) {
     if ((type != at::kHalf && type != at::kBFloat16) || (D != 64 && D != 128) ||
         (block_m != 32 && block_m != 64 && block_m != 128) || kernel == FST_KERNEL_SIMT || kernel == FST_KERNEL_MMA ||
@@ -105,8 +104,7 @@ Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, i
     const auto clamp = [&](int64_t v) { return int(std::max<int64_t>(1, std::min(v, cap))); };
     if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && prefix >= 256)) {
         if (asked) return {clamp(*asked), true};
-        const int64_t ctas = Z * H * ((n_q + 127) / 128);
-        return {clamp(std::min(sm_count(device) / std::max<int64_t>(ctas, 1), prefix / 256)), true};
+        return {clamp(fst::prefix_runs(Z, H, H_kv, n_q, prefix, sm_count(device))), true};
     }
     int runs;
     if (asked) {
@@ -189,7 +187,7 @@ float *lse_ptr(const Call &c) { return c.lse.defined() ? static_cast<float *>(c.
 PyObject *launch(Call &c, const void *packed, size_t tree_stride, int64_t block_m, int64_t ma, int kernel,
                  const std::optional<long long> &kv_splits, void *status, void *stream) {
     const at::Device dev = c.q.device();
-    const Splits sp = pick_splits(kv_splits, c.q.scalar_type(), c.Z, c.H, c.n_q, c.D, c.n_kv - c.n_q, block_m,
+    const Splits sp = pick_splits(kv_splits, c.q.scalar_type(), c.Z, c.H, c.H_kv, c.n_q, c.D, c.n_kv - c.n_q, block_m,
                                   kernel & FST_KERNEL_MASK, dev.index());
     at::Tensor ws;
     size_t ws_bytes = 0;
@@ -332,10 +330,7 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
     const int64_t max_prefix = integer(a[15]);
     const at::Device dev = q.device();
     std::optional<long long> asked = optional_int(a[17]);
-    if (!asked) {
-        const int64_t ctas = Z * H * ((n_q + 127) / 128);
-        asked = std::max<int64_t>(1, std::min({sm_count(dev.index()) / std::max<int64_t>(ctas, 1), max_prefix / 256, 65535 / Z}));
-    }
+    if (!asked) asked = fst::prefix_runs(Z, H, H_kv, n_q, max_prefix, sm_count(dev.index()));
     const c10::cuda::CUDAGuard guard(dev);
     int32_t *status = static_cast<int32_t *>(status_of(dev, true)->data_ptr());
     const size_t ws_bytes = fst_attention_split_workspace_bytes(int(Z), int(H), int(n_q), int(D), int(*asked));
@@ -360,17 +355,47 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
 
 // ---- trees ---------------------------------------------------------------------------------------
 // precompute(parent, block_m, max_ancestors, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx)
-//   -> None; parent is a contiguous int32 CUDA tensor [N] or [T, N], the buffers belong to the caller and
+//   -> the status record of this build; parent is a contiguous int32 CUDA tensor [N] or [T, N], the buffers belong to the caller and
 //   the last three may be None.
 // new_metadata(parent, block_m, max_ancestors, reference_format)
 //   -> (n_trees, n_nodes, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx), buffers made here.
+// A cleared status record.  Clearing one per call is a launch (about a microsecond in front of a five
+// microsecond kernel), so a thread takes them from a block that it cleared in one go on the same stream;
+// a new block is made for another stream or device and when one is used up (256 records, 4 KB,
+// returned to the allocator with the last record).  A call that is being captured into a graph
+// clears its record in the graph, for every replay: `old` if it is given.
+at::Tensor clear_record(const at::Device &dev, cudaStream_t stream, const at::Tensor &old, const char *what) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) check_status(FST_ERR_CUDA, what);
+    if (capturing != cudaStreamCaptureStatusNone) {
+        at::Tensor t = old.defined() ? old : empty({4}, at::kInt, dev);
+        if (cudaMemsetAsync(t.data_ptr(), 0, 16, stream) != cudaSuccess) check_status(FST_ERR_CUDA, what);
+        return t;
+    }
+    constexpr int64_t kRecords = 256;
+    struct Block {
+        at::Tensor words;
+        cudaStream_t stream = nullptr;
+        int64_t next = kRecords;
+    };
+    static thread_local Block *block = new Block();       // (never destroyed: torch may be gone by then)
+    if (block->next == kRecords || block->stream != stream || block->words.device() != dev) {
+        block->words = empty({kRecords * 4}, at::kInt, dev);
+        block->stream = stream;
+        block->next = 0;
+        if (cudaMemsetAsync(block->words.data_ptr(), 0, kRecords * 16, stream) != cudaSuccess) {
+            block->next = kRecords;
+            check_status(FST_ERR_CUDA, what);
+        }
+    }
+    return block->words.narrow(0, 4 * block->next++, 4);
+}
+
 void run_precompute(const at::Tensor &par, int64_t n_trees, int64_t n_nodes, int64_t bm, int64_t ma, const at::Tensor &packed,
                     size_t stride, const at::Tensor &status, const at::Tensor &ai, const at::Tensor &am,
                     const at::Tensor &li) {
     const at::Device dev = par.device();
-    const c10::cuda::CUDAGuard guard(dev);
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    if (cudaMemsetAsync(status.data_ptr(), 0, 16, stream) != cudaSuccess) check_status(FST_ERR_CUDA, "fst_precompute");
     check_status(fst_precompute(static_cast<const int32_t *>(par.data_ptr()), int(n_trees), int(n_nodes), int(bm), int(ma),
                                 ai.defined() ? static_cast<int64_t *>(ai.data_ptr()) : nullptr,
                                 am.defined() ? static_cast<uint8_t *>(am.data_ptr()) : nullptr,
@@ -391,9 +416,12 @@ at::Tensor optional_tensor(PyObject *o) { return o == Py_None ? at::Tensor() : t
 PyObject *precompute(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 9);
     const at::Tensor &par = parent_arg(a[0]);
+    const at::Device dev = par.device();
+    const c10::cuda::CUDAGuard guard(dev);
+    const at::Tensor status = clear_record(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), tensor(a[5]), "fst_precompute");
     run_precompute(par, par.dim() == 2 ? par.size(0) : 1, par.size(-1), integer(a[1]), integer(a[2]), tensor(a[3]),
-                   size_t(integer(a[4])), tensor(a[5]), optional_tensor(a[6]), optional_tensor(a[7]), optional_tensor(a[8]));
-    Py_RETURN_NONE;
+                   size_t(integer(a[4])), status, optional_tensor(a[6]), optional_tensor(a[7]), optional_tensor(a[8]));
+    return THPVariable_Wrap(status);
 }
 
 PyObject *wrap_or_none(const at::Tensor &t) {
@@ -410,7 +438,9 @@ PyObject *new_metadata(PyObject *const *a, Py_ssize_t n) {
     const int64_t nb = (n_nodes + bm - 1) / bm;
     const size_t stride = fst_packed_meta_bytes(int(nb), int(bm), int(ma));
     const at::Device dev = par.device();
-    const at::Tensor packed = empty({n_trees, int64_t(stride)}, at::kByte, dev), status = empty({4}, at::kInt, dev);
+    const c10::cuda::CUDAGuard guard(dev);
+    const at::Tensor packed = empty({n_trees, int64_t(stride)}, at::kByte, dev),
+                     status = clear_record(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), at::Tensor(), "fst_precompute");
     at::Tensor ai, am, li;
     if (a[3] == Py_True) {
         if (par.dim() == 2) {
@@ -434,10 +464,9 @@ PyObject *dfs_order(PyObject *const *a, Py_ssize_t n) {
     const at::Tensor &par = parent_arg(a[0]);
     const at::Device dev = par.device();
     const c10::cuda::CUDAGuard guard(dev);
-    const at::Tensor order = empty(par.sizes(), at::kInt, dev), npar = empty(par.sizes(), at::kInt, dev),
-                     status = empty({4}, at::kInt, dev);
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    if (cudaMemsetAsync(status.data_ptr(), 0, 16, stream) != cudaSuccess) check_status(FST_ERR_CUDA, "fst_dfs_order");
+    const at::Tensor order = empty(par.sizes(), at::kInt, dev), npar = empty(par.sizes(), at::kInt, dev),
+                     status = clear_record(dev, stream, at::Tensor(), "fst_dfs_order");
     check_status(fst_dfs_order(static_cast<const int32_t *>(par.data_ptr()), int(par.dim() == 2 ? par.size(0) : 1),
                                int(par.size(-1)), static_cast<int32_t *>(order.data_ptr()),
                                static_cast<int32_t *>(npar.data_ptr()), static_cast<int32_t *>(status.data_ptr()), stream),
@@ -538,7 +567,7 @@ PyObject *attention_status(PyObject *const *a, Py_ssize_t n) {
 PyObject *splits(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 5);
     const at::Tensor &q = tensor(a[0]);
-    const Splits s = pick_splits(optional_int(a[4]), q.scalar_type(), q.size(0), q.size(1), q.size(2), q.size(3), integer(a[1]),
+    const Splits s = pick_splits(optional_int(a[4]), q.scalar_type(), q.size(0), q.size(1), q.size(1), q.size(2), q.size(3), integer(a[1]),
                                  integer(a[2]), int(integer(a[3])), q.device().index());
     return Py_BuildValue("(iO)", s.runs, s.workspace ? Py_True : Py_False);
 }

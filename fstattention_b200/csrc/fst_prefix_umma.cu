@@ -23,13 +23,17 @@
 // shared memory and written as one partial result per run (normalised rows in fp32 plus base-2
 // log-sum-exp) in the layout the tree kernel writes; combine_splits_kernel merges the runs.
 //
+// With grouped-query attention a small tree's rows of several heads share a query tile (see
+// prefix_heads_per_tile): the tile is loaded as one box per head and its rows go to their heads at the end.
+//
 // PAGED = true reads the prefix rows from a page pool through a block table (a KV cache): a
 // tile is 128 / page_size pages and lane j of the loading warp requests page j.
 //
 // Every wait is bounded in time (mbar_wait): on expiry the kernel records FST_DEV_TIMEOUT, stops
 // issuing, frees its tensor memory and returns.
 
-#include "fst_attention_tma.cuh"
+#include "fst_plan.h"
+#include "fst_umma.cuh"
 
 namespace fst {
 
@@ -37,7 +41,6 @@ namespace umma {
 
 constexpr int QM = 128;                // query rows per CTA (MMA M)
 constexpr int KN = 128;                // K/V rows per tile (MMA N of the first product)
-constexpr int HALF = QM * 128;         // bytes of one 64-column half of a 128-row tile
 constexpr int TILE_P = 2 * HALF;       // bytes of a P tile (128 x 128 fp16)
 
 // Shared-memory map for head dimension D (64 or 128): a Q / K / V tile is 128 rows of D columns,
@@ -53,68 +56,6 @@ struct Geo {
     static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;   // + barriers, TMEM address, 1 KB alignment slack
 };
 
-// shared-memory matrix descriptor: 128-byte swizzle, 8-row groups 1 KB apart
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes) {
-    uint64_t d = 0;
-    d |= uint64_t((addr >> 4) & 0x3fff);                 // start address
-    d |= uint64_t((lbo_bytes >> 4) & 0x3fff) << 16;      // leading byte offset
-    d |= uint64_t((1024 >> 4) & 0x3fff) << 32;           // stride byte offset
-    d |= uint64_t(1) << 46;                              // descriptor version (Blackwell)
-    d |= uint64_t(2) << 61;                              // SWIZZLE_128B
-    return d;
-}
-
-// instruction descriptor: f32 accumulate, M=128, N=n, A K-major, B K- or MN-major
-__device__ __forceinline__ uint32_t instr_desc(bool bf16, bool b_mn_major, int n) {
-    const uint32_t fmt = bf16 ? 1u : 0u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | (uint32_t(b_mn_major) << 16) |
-           (uint32_t(n >> 3) << 17) | (uint32_t(QM >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        bool accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(uint32_t(accumulate)) : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
-}
-// asynchronous: the registers are valid after tmem_ld_wait()
-__device__ __forceinline__ void tmem_ld32(uint32_t (&r)[32], uint32_t taddr) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32"
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15,"
-                 " %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr));
-}
-// The loaded registers pass through the wait as read-write operands, so that no use of them can
-// be scheduled ahead of it.
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
-                   "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
-                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
-                 :: "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0],"
-                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16,"
-                 " %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-                   "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-                   "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-                 : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-
 }  // namespace umma
 
 // Arguments of the prefix kernel beyond AttnArgs: where this launch's partial results start.
@@ -127,6 +68,7 @@ struct PrefixArgs {
     const int32_t *block_table;
     const int32_t *prefix_lens;
     int table_stride, page_size, n_pages;
+    int pack, pack_shift;                // heads per query tile; a head's rows are 1 << pack_shift of the tile's
 };
 
 constexpr int PFX_SOFTMAX = 256;       // eight softmax warps: two groups of 128, one thread per query row each
@@ -148,7 +90,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     extern __shared__ unsigned char smem_raw[];
     const uint32_t s_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char *smem = smem_raw + (s_base - smem_u32(smem_raw));
-    const int qt = blockIdx.x, h = blockIdx.y, hk = h / a.kv_group;   // query tile, head, K/V head
+    const int qt = blockIdx.x, h = blockIdx.y * pa.pack, hk = h / a.kv_group;   // query tile, (first) head, K/V head
     const int z = blockIdx.z / pa.n_runs, run = blockIdx.z - z * pa.n_runs;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int n_q = a.n_q;
@@ -218,9 +160,10 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         if (nt > 0 && (PAGED || lane == 0)) {
             if (lane == 0) {
                 mbar_arrive_expect_tx(bar_q, TILE);
+                for (int i = 0; i < pa.pack; ++i)
 #pragma unroll
-                for (int hf = 0; hf < DH; ++hf)
-                    tma_load_4d(s_base + OFF_Q + hf * HALF, &tm_q, hf * 64, qt * QM, h, z, bar_q);
+                    for (int hf = 0; hf < DH; ++hf)
+                        tma_load_4d(s_base + OFF_Q + hf * HALF + (i << pa.pack_shift) * 128, &tm_q, hf * 64, qt * QM, h + i, z, bar_q);
             }
             const int page0 = my_page(0), page1 = nt > 1 ? my_page(1) : 0;
             load_k(0, page0);
@@ -232,9 +175,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         }
     }
     if (warp == 9) {                                      // tensor memory: two S buffers and two accumulators, 128 columns each
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
-                     ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+        umma::tmem_alloc_all(smem_u32(tmem_slot));
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -470,20 +411,20 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
             f0 = w0 * inv;
             f1 = w1 * inv;
-            const int grow = qt * QM + rr;
+            const int grow = qt * QM + (rr & ((1 << pa.pack_shift) - 1)), hr = h + (rr >> pa.pack_shift);
             if (lane < RPW && grow < n_q)
-                a.part_lse[((slot * a.Z + z) * a.H + h) * n_q + grow] = l_all > 0.f ? mu_all + log2f(l_all) : -INFINITY;
+                a.part_lse[((slot * a.Z + z) * a.H + hr) * n_q + grow] = l_all > 0.f ? mu_all + log2f(l_all) : -INFINITY;
         }
 #pragma unroll 4
         for (int i = 0; i < RPW; ++i) {
-            const int rr = warp * RPW + i, grow = qt * QM + rr;
+            const int rr = warp * RPW + i, grow = qt * QM + (rr & ((1 << pa.pack_shift) - 1)), hr = h + (rr >> pa.pack_shift);
             const float g0 = __shfl_sync(0xffffffffu, f0, i), g1 = __shfl_sync(0xffffffffu, f1, i);
             if (lane >= D / 4) continue;                  // a row is D / 4 chunks of four floats
             const int sw = (lane ^ (rr & 7)) << 2;
             const float4 v0 = *reinterpret_cast<const float4 *>(stage + rr * D + sw);
             const float4 v1 = *reinterpret_cast<const float4 *>(stage + (128 + rr) * D + sw);
             if (grow < n_q) {
-                const size_t prow_g = ((slot * a.Z + z) * a.H + h) * n_q + grow;
+                const size_t prow_g = ((slot * a.Z + z) * a.H + hr) * n_q + grow;
                 reinterpret_cast<float4 *>(a.part_o + prow_g * D)[lane] =
                     make_float4(v0.x * g0 + v1.x * g1, v0.y * g0 + v1.y * g1, v0.z * g0 + v1.z * g1, v0.w * g0 + v1.w * g1);
             }
@@ -492,8 +433,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
 
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 9)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512) : "memory");
+    if (warp == 9) umma::tmem_free_all(tmem_base);
 }
 
 // rank-4 map with 64-column x 128-row boxes (kept in the calling thread's table of maps)
@@ -522,7 +462,8 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
                                    cudaStream_t stream) {
     constexpr bool bf16 = !std::is_same<T, __half>::value;
     alignas(64) CUtensorMap tq, tk, tv;
-    if (!make_map_rows128(&tq, a.q, bf16, D, a.n_q, a.H, a.Z, a.qs_n, a.qs_h, a.qs_z)) return cudaErrorNotSupported;
+    const int pack = prefix_heads_per_tile(a.H, a.H / a.kv_group, a.n_q);
+    if (!make_map(&tq, a.q, bf16, D, a.n_q, a.H, a.Z, a.qs_n, a.qs_h, a.qs_z, umma::QM / pack)) return cudaErrorNotSupported;
     if (PAGED) {
         if (!make_map_pool(&tk, bf16, D, *pg, a.H / a.kv_group, pg->k_pool) ||
             !make_map_pool(&tv, bf16, D, *pg, a.H / a.kv_group, pg->v_pool))
@@ -538,7 +479,8 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
     });
     if (ce != cudaSuccess) return ce;
     if ((long long)a.Z * n_runs > 65535) return cudaErrorInvalidValue;
-    PrefixArgs pa{n_runs, first_slot, nullptr, nullptr, 0, 0, 0};
+    PrefixArgs pa{n_runs, first_slot, nullptr, nullptr, 0, 0, 0, pack, 7};
+    for (int p = pack; p > 1; p /= 2) --pa.pack_shift;
     if (PAGED) {
         pa.block_table = pg->block_table;
         pa.prefix_lens = pg->prefix_lens;
@@ -546,7 +488,7 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
         pa.page_size = pg->page_size;
         pa.n_pages = pg->n_pages;
     }
-    dim3 grid((a.n_q + umma::QM - 1) / umma::QM, a.H, a.Z * n_runs);
+    dim3 grid((a.n_q + umma::QM - 1) / umma::QM, a.H / pack, a.Z * n_runs);
     prefix_umma_kernel<T, D, PAGED><<<grid, PFX_THREADS, umma::Geo<D>::SMEM_BYTES, stream>>>(a, pa, tq, tk, tv);
     return cudaGetLastError();
 }

@@ -59,15 +59,20 @@ def _strides(t):
     return [st[0], st[1], st[2]]
 
 
-def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[int] = None) -> dict:
+def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[int] = None,
+                max_ancestors: int = 64) -> dict:
     """Which kernels one ``fst_attention`` call on packed metadata launches for ``q`` (shape and
     dtype only), a shared prefix of ``prefix`` rows and the given block size, mirroring the
-    dispatch inside the library: ``{"kernels": [...], "prefix_runs": r}``."""
+    dispatch inside the library (for rows on 16-byte boundaries and a positive scale): ``{"kernels":
+    [...], "prefix_runs": r}``.  ``max_ancestors`` is the metadata's ancestor bound."""
     splits, need_ws = _lib.host().splits(q, prefix, block_m, _lib.KERNELS[kernel], kv_splits)
     tensor_core = q.dtype in (torch.float16, torch.bfloat16) and q.shape[-1] in (64, 128) \
         and block_m in (16, 32, 64, 128)
     tree = "attn_simt_kernel" if kernel == "simt" or not tensor_core else \
         "attn_mma_kernel" if kernel == "mma" or block_m == 16 else "attn_tma_kernel"
+    if tree == "attn_tma_kernel" and prefix == 0 and (kernel == "tree_umma" or (kernel == "auto" and _lib.lib().fst_attention_tree_kernel(
+            q.shape[0], q.shape[1], q.shape[2], q.shape[3], block_m, max_ancestors) == _KERNELS["tree_umma"])):
+        tree = "tree_umma_kernel"
     if kernel == "persist" and tree == "attn_tma_kernel" and prefix == 0 and block_m in (64, 128):
         tree = "attn_persist_kernel"                      # by hand only: it measured slower than attn_tma_kernel
     if need_ws and q.shape[-1] in (64, 128) and (kernel == "tma_umma" or (kernel == "auto" and prefix >= 256)):

@@ -157,8 +157,8 @@ def build_tree_metadata(parent: TreeLike, block_m: int = 64, max_ancestors: int 
         n_trees, n_nodes = par.shape if par.dim() == 2 else (1, par.shape[0])
         if (meta.n_trees, meta.n_nodes, meta.block_m, meta.max_ancestors) != (n_trees, n_nodes, block_m, max_ancestors):
             raise ValueError("out= metadata has a different shape")
-        host.precompute(par, block_m, max_ancestors, meta.packed, meta.tree_stride, meta.status,
-                        meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx)
+        meta.status = host.precompute(par, block_m, max_ancestors, meta.packed, meta.tree_stride, meta.status,
+                                      meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx)
         meta._rebuilt()
     if check:
         meta.check()

@@ -61,10 +61,12 @@ enum fst_kernel {
     FST_KERNEL_TMA_T64 = 5,        /* ... forced 64-column tiles (fewest softmax rounds)         */
     FST_KERNEL_TMA_UMMA = 6,       /* tree part as FST_KERNEL_TMA, shared prefix by the tcgen05  */
                                    /* kernel (head_dim 64 / 128, fst_attention_fwd_splitkv only) */
-    FST_KERNEL_PERSIST = 7         /* persistent CTAs, a producer warp streaming tiles through a */
+    FST_KERNEL_PERSIST = 7,        /* persistent CTAs, a producer warp streaming tiles through a */
                                    /* shared-memory ring ahead of the arithmetic: block_m 64 or  */
                                    /* 128, no prefix.  Slower than FST_KERNEL_TMA on every shape */
                                    /* measured, so never the automatic choice                    */
+    FST_KERNEL_TREE_UMMA = 8       /* persistent tcgen05 kernel, 128-row items, TMA gathers: D 64/ */
+                                   /* 128, block_m 32/64/128, no prefix, positive sm_scale         */
 };
 
 /*
@@ -242,6 +244,13 @@ int fst_attention_fwd_scatter(const void *q, const void *k, const void *v, void 
                               int64_t o_stride_z, int64_t o_stride_h, int64_t o_stride_n,
                               int block_m, int max_ancestors, float sm_scale, int dtype, int kernel,
                               int32_t *status, void *stream);
+
+/*
+ * The kernel FST_KERNEL_AUTO takes for the tree part of a 16-bit call without a shared prefix (rows on 16-byte
+ * boundaries, positive sm_scale): FST_KERNEL_TREE_UMMA, FST_KERNEL_TMA, or FST_KERNEL_SIMT where no
+ * tensor-core kernel fits.  FST_KERNEL_AUTO (0) on non-positive sizes.
+ */
+int fst_attention_tree_kernel(int Z, int H, int n_q, int head_dim, int block_m, int max_ancestors);
 
 /*
  * fst_attention_fwd with the shared prefix cut into kv_splits runs of rows, each handled by its

@@ -1,0 +1,102 @@
+"""The tcgen05 tree kernel at the sizes where it can go wrong: rows that do not fill an item or a 16-row step,
+one CTA with several items, ancestor lists that end in either half of a tile or run over many tiles, grouped
+K/V heads, strided tensors, scores that outgrow the first reference point."""
+import pytest
+import torch
+
+from helpers import oracle_attention
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
+
+
+@pytest.fixture(scope="module")
+def fst(built_lib):
+    import fstattention_b200
+    return fstattention_b200
+
+
+def comb(n, teeth):
+    """A chain of ``teeth`` nodes; every later node hangs under one of them in turn: a block's list is as long
+    as the chain, whatever block it is."""
+    return [i - 1 if i < teeth else (i * 7) % teeth for i in range(n)]
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bm", [32, 64, 128])
+@pytest.mark.parametrize("n,teeth", [(1, 1), (17, 3), (127, 20), (128, 33), (129, 64), (200, 65), (385, 130), (640, 300)])
+def test_tree_umma_edges(fst, D, bm, n, teeth):
+    par = comb(n, teeth)
+    meta = fst.build_tree_metadata(par, bm, 512, reference_format=False)
+    dtype = torch.float16 if n % 2 else torch.bfloat16
+    g = torch.Generator().manual_seed(n + bm)
+    q = torch.randn((2, 4, n, D), generator=g).to(dtype)
+    k, v = (torch.randn((2, 2, n, D), generator=g).to(dtype) for _ in range(2))
+    o, lse = fst.fst_attention(q.cuda(), k.cuda(), v.cuda(), meta, sm_scale=D ** -0.5, kernel="tree_umma", return_lse=True)
+    want = oracle_attention(q, k.repeat_interleave(2, 1), v.repeat_interleave(2, 1), par, D ** -0.5,
+                            compute_dtype=torch.float32)
+    assert (o.cpu().float() - want.float()).abs().max().item() <= TOL[dtype]
+    _, ref = fst.fst_attention(q.cuda().float(), k.cuda().float(), v.cuda().float(), meta, sm_scale=D ** -0.5,
+                               kernel="simt", return_lse=True)
+    assert (lse - ref).abs().max().item() <= 1e-3
+    assert fst.last_status() == 0
+
+
+@pytest.mark.parametrize("D,bm", [(64, 32), (64, 128), (128, 64)])
+def test_tree_umma_many_items_strided(fst, D, bm):
+    """Several items per CTA, a tree of its own for every batch element, [Z, N, H, D] storage."""
+    from fstattention_b200 import configs
+    Z, H, n = 6, 40, 300
+    trees = [configs.random_window_tree(s, n, 40) for s in range(Z)]
+    meta = fst.build_tree_metadata(trees, bm, 256, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v = (torch.randn((Z, n, H, D), generator=g, device="cuda").half().permute(0, 2, 1, 3) for _ in range(3))
+    out = torch.empty((Z, n, H, D), dtype=torch.float16, device="cuda").permute(0, 2, 1, 3)
+    for _ in range(3):
+        fst.fst_attention(q, k, v, meta, sm_scale=D ** -0.5, kernel="tree_umma", out=out)
+        want = fst.fst_attention(q.float(), k.float(), v.float(), meta, sm_scale=D ** -0.5, kernel="simt")
+        assert (out.float() - want).abs().max().item() <= 2e-3
+    assert fst.last_status() == 0
+
+
+def test_tree_umma_moving_maximum(fst):
+    """A late ancestor whose score dwarfs the row's own tile: the accumulator is rescaled."""
+    n, D = 400, 128
+    par = comb(n, 200)
+    meta = fst.build_tree_metadata(par, 64, 256, reference_format=False)
+    g = torch.Generator().manual_seed(4)
+    q, k, v = (torch.randn((1, 2, n, D), generator=g) for _ in range(3))
+    k[:, :, 150:160] *= 12.0
+    q, k, v = q.half(), k.half(), v.half()
+    o = fst.fst_attention(q.cuda(), k.cuda(), v.cuda(), meta, sm_scale=0.5, kernel="tree_umma").cpu()
+    want = oracle_attention(q, k, v, par, 0.5, compute_dtype=torch.float32)
+    assert (o.float() - want).abs().max().item() <= 4e-3
+
+
+@pytest.mark.parametrize("n,H,H_kv", [(16, 16, 2), (17, 16, 2), (32, 8, 2), (33, 8, 2), (64, 8, 4), (65, 8, 4), (9, 12, 2)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_prefix_heads_share_a_query_tile(fst, n, H, H_kv, D):
+    """Grouped-query heads packed into one query tile of the prefix kernel, contiguous and paged."""
+    from fstattention_b200 import configs
+    par = configs.random_window_tree(n, n, 8)
+    meta = fst.build_tree_metadata(par, 32, 128, reference_format=False)
+    P, ps = 700, 16
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q = torch.randn((2, H, n, D), generator=g, device="cuda").half()
+    k, v = (torch.randn((2, H_kv, P + n, D), generator=g, device="cuda").half() for _ in range(2))
+    want, lse_w = fst.fst_attention(q, k, v, meta, sm_scale=D ** -0.5, kernel="tma_t32", kv_splits=1, return_lse=True)
+    got, lse = fst.fst_attention(q, k, v, meta, sm_scale=D ** -0.5, kernel="tma_umma", return_lse=True)
+    assert (got.float() - want.float()).abs().max().item() <= 2e-3 and (lse - lse_w).abs().max().item() <= 2e-2
+    pages = -(-P // ps)
+    pool = torch.zeros((2, 2 * pages, ps, H_kv, D), dtype=torch.float16, device="cuda")
+    for kv, src in enumerate((k, v)):
+        for z in range(2):
+            rows = torch.zeros((pages * ps, H_kv, D), dtype=torch.float16, device="cuda")
+            rows[:P] = src[z, :, :P].transpose(0, 1)
+            pool[kv, z * pages:(z + 1) * pages] = rows.view(pages, ps, H_kv, D)
+    table = torch.arange(2 * pages, dtype=torch.int32, device="cuda").view(2, pages)
+    lens = torch.tensor([P, P], dtype=torch.int32, device="cuda")
+    o = fst.fst_attention_paged(q, k[:, :, P:].contiguous(), v[:, :, P:].contiguous(), meta, pool[0], pool[1], table, lens,
+                                D ** -0.5, max_prefix=P)
+    assert (o.float() - want.float()).abs().max().item() <= 2e-3
+    assert fst.last_status() == 0
