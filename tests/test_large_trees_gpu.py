@@ -1,0 +1,95 @@
+"""Metadata of trees beyond the size where the parent array is staged in shared memory, trees with crowded and deep
+levels in the device renumbering, and levels large enough to be sorted in the device-built forest."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import tree_oracle as orc
+from test_precompute_gpu import _topk_forest_cpu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def fst(built_lib):
+    import fstattention_b200
+    return fstattention_b200
+
+
+def sets_of(par, lo, hi):
+    rows = []
+    for k in range(lo, hi):
+        x, anc = int(par[k]), []
+        while x >= 0:
+            anc.append(x)
+            x = int(par[x])
+        rows.append(anc)
+    return rows
+
+
+@pytest.mark.parametrize("n,bm,ma,kind", [(8193, 64, 64, "near"), (8200, 128, 128, "near"), (9000, 32, 100, "near"),
+                                          (20000, 128, 256, "near"), (12001, 64, 128, "inside"), (9000, 24, 40, "near")])
+def test_wide_precompute(fst, n, bm, ma, kind):
+    """Sampled blocks, bit for bit: ancestors outside and inside the block, partial last blocks, bounds of a slot
+    mask's inheritance (128 slots) and past it, odd sizes."""
+    i = np.arange(n)
+    if kind == "near":                                    # a shallow heap of fan-out 7
+        par = np.where(i > 0, (i - 1) // 7, -1)
+    else:                                                 # chains of eight inside every block, under one root
+        par = np.where(i % 8 > 0, i - 1, np.where(i > 0, 0, -1))
+    meta = fst.build_tree_metadata(torch.tensor(par, dtype=torch.int32), bm, ma)
+    ai, am, li = (t.cpu().numpy() for t in meta)
+    packed_only = fst.build_tree_metadata(torch.tensor(par, dtype=torch.int32), bm, ma, reference_format=False)
+    from helpers import decode_packed
+    nb = meta.n_blocks
+    count, p_ai, p_am, p_li = decode_packed(packed_only.packed[0].cpu().numpy(), nb, bm, ma)
+    for b in (0, 1, nb // 3, nb - 2, nb - 1):
+        lo, hi = b * bm, min(n, b * bm + bm)
+        rows = sets_of(par, lo, hi)
+        anc = sorted(set(x for r in rows for x in r))
+        assert len(anc) <= ma
+        want = np.full(ma, -1)
+        want[:len(anc)] = anc
+        mask = np.zeros((bm, ma), bool)
+        for j, r in enumerate(rows):
+            for x in r + ([lo + j] if lo + j in anc else []):
+                mask[j, anc.index(x)] = True
+        leaf = np.array([-1 if k in anc else k for k in range(lo, lo + bm)])
+        for got_i, got_m, got_l in ((ai[b], am[b], li[b]), (p_ai[b], p_am[b], p_li[b])):
+            assert np.array_equal(got_i, want) and np.array_equal(got_m[:hi - lo], mask[:hi - lo]), b
+            assert np.array_equal(got_l, leaf), b
+        assert count[b] == sum(1 for x in anc if x < lo)
+
+
+def test_wide_precompute_reports(fst):
+    n = 10000
+    star = torch.tensor([-1] * 200 + [i % 200 for i in range(200, n)], dtype=torch.int32)
+    with pytest.raises(RuntimeError, match="unique ancestors"):
+        fst.build_tree_metadata(star, 128, 64)
+    bad = star.clone()
+    bad[9000] = 9500
+    with pytest.raises(ValueError, match="malformed"):
+        fst.build_tree_metadata(bad, 64, 128)
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("n", [1024, 1025, 2049, 4097, 8192])
+def test_dfs_order_sizes(fst, n):
+    rng = np.random.default_rng(n)
+    for par in ([-1] + [int(rng.integers(max(0, i - 50), i)) for i in range(1, n)],
+                [-1] + [0 if i < 60 else int(rng.integers(0, 60)) for i in range(1, n)],      # crowded parents
+                [-1] + [i - 1 if i < 300 else int(rng.integers(0, 300)) for i in range(1, n)]):
+        order, new_parent = fst.dfs_order(par)
+        d_order, d_parent = fst.dfs_order_device(par)
+        assert d_order.cpu().tolist() == order and d_parent.cpu().tolist() == new_parent
+
+
+@pytest.mark.parametrize("depth,topk,lwf", [(9, 4, 0.5), (8, 10, 0.2), (3, 600, 0.002), (2, 1024, 0.001)])
+def test_sorted_levels_with_random_scores_and_ties(fst, depth, topk, lwf):
+    rng = np.random.default_rng(depth)
+    scores = np.round(rng.standard_normal((depth + 1, topk)), 1).astype(np.float32)       # many ties, both zeros
+    parent, choice, score = _topk_forest_cpu(scores, topk, lwf)
+    p, c, s = fst.build_tree_topk(torch.tensor(scores, device="cuda"), left_weight_factor=lwf, return_choice=True,
+                                  return_scores=True)
+    assert p.cpu().tolist() == parent and c.cpu().tolist() == choice
+    assert np.array_equal(s.cpu().numpy(), np.array(score, dtype=np.float32))
