@@ -49,39 +49,6 @@ static bool mma_ok(int dtype, int D, int bm) {
            (bm == 16 || bm == 32 || bm == 64 || bm == 128);
 }
 
-// A second stream with a fork and a join event, per host thread and device, so that two
-// independent kernels of one call can run side by side.  Created on first use and kept for the
-// life of the thread; never created while the caller's stream is being captured into a graph
-// (the call then simply runs its kernels in order).
-struct SideStream {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-};
-static SideStream *side_stream(cudaStream_t caller) {
-    thread_local SideStream per_device[kMaxDevices];
-    const int slot = current_device_slot();
-    if (slot < 0) return nullptr;
-    SideStream &s = per_device[slot];
-    if (s.stream != nullptr) return &s;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(caller, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-        (void)cudaGetLastError();
-        return nullptr;
-    }
-    SideStream made;
-    if (cudaStreamCreateWithFlags(&made.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&made.fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&made.join, cudaEventDisableTiming) != cudaSuccess) {
-        if (made.join != nullptr) cudaEventDestroy(made.join);
-        if (made.fork != nullptr) cudaEventDestroy(made.fork);
-        if (made.stream != nullptr) cudaStreamDestroy(made.stream);
-        (void)cudaGetLastError();
-        return nullptr;
-    }
-    s = made;
-    return &s;
-}
-
 static int cuda_status(cudaError_t e) {
     if (e == cudaSuccess) return FST_OK;
     if (e == cudaErrorNotSupported) return FST_ERR_UNSUPPORTED;
@@ -265,7 +232,6 @@ static int attention_fwd_impl(const void *q, const void *k, const void *v, void 
     a.n_splits = 1;
     a.part_o = nullptr;
     a.part_lse = nullptr;
-    a.skip_prefix = 0;
     a.part_slots = 1;
     a.meta_stable = (flags & FST_KERNEL_FLAG_META_STABLE) ? 1 : 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -320,52 +286,34 @@ static int attention_fwd_impl(const void *q, const void *k, const void *v, void 
         if (e != cudaErrorNotSupported) return cuda_status(e);
     }
 
-    // A shared prefix with a workspace: either the tcgen05 prefix kernel takes it in kv_splits runs
-    // while the tree kernel does the tree part (head_dim 64 or 128; chosen automatically from 256
-    // prefix rows on), or the tree kernel itself is launched kv_splits times over the prefix.
-    const bool can_part = a.prefix > 0 && workspace != nullptr && choice != FST_KERNEL_MMA && choice != FST_KERNEL_PERSIST;
+    // A shared prefix: the tcgen05 kernel takes the whole call in kv_splits runs of column tiles (head_dim 64 or 128,
+    // block_m 32 and up; chosen automatically from 256 prefix rows on), or the tree kernel itself walks the prefix,
+    // split over kv_splits CTAs.  More than one run needs the workspace.
     // (the tcgen05 kernel takes Q from shared memory as it arrived, so it cannot flip Q's sign
     // for a negative factor; the tree kernel walks the prefix itself then)
-    const bool want_umma = can_part && (head_dim == 128 || head_dim == 64) && sm_scale > 0.f &&
+    const bool can_part = a.prefix > 0 && choice != FST_KERNEL_MMA && choice != FST_KERNEL_PERSIST;
+    const bool want_umma = can_part && (workspace != nullptr || kv_splits == 1) && block_m >= 32 && sm_scale > 0.f &&
                            (choice == FST_KERNEL_TMA_UMMA || (automatic && a.prefix >= 256));
     if (choice == FST_KERNEL_TMA_UMMA && !want_umma) return FST_ERR_UNSUPPORTED;
-    if (can_part && (want_umma || kv_splits > 1)) {
-        const size_t need = fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits);
-        if (workspace_bytes < need) return FST_ERR_WORKSPACE;
-        if (!aligned16(workspace)) return FST_ERR_ALIGNMENT;
-        a.part_slots = want_umma ? kv_splits + 1 : kv_splits;
-        a.part_o = static_cast<float *>(workspace);
-        a.part_lse = a.part_o + size_t(a.part_slots) * Z * H * n_q * head_dim;
+    if (want_umma || (can_part && workspace != nullptr && kv_splits > 1)) {
+        if (kv_splits > 1) {
+            const size_t need = fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits);
+            if (workspace_bytes < need) return FST_ERR_WORKSPACE;
+            if (!aligned16(workspace)) return FST_ERR_ALIGNMENT;
+            a.part_slots = kv_splits;
+            a.part_o = static_cast<float *>(workspace);
+            a.part_lse = a.part_o + size_t(a.part_slots) * Z * H * n_q * head_dim;
+        }
         cudaError_t e;
         if (want_umma) {
-            // The tree kernel (slot 0) and the prefix kernel (slots 1..) are independent: the tree
-            // kernel runs on a second stream, forked from and joined back into the caller's.  The
-            // prefix kernel is launched first: its CTAs need a whole SM's shared memory each and
-            // would otherwise queue behind the tree kernel's, which fit beside one another.
-            a.skip_prefix = 1;
-            SideStream *side = side_stream(st);
-            cudaStream_t tree_st = st;
-            if (side != nullptr && cudaEventRecord(side->fork, st) == cudaSuccess &&
-                cudaStreamWaitEvent(side->stream, side->fork, 0) == cudaSuccess)
-                tree_st = side->stream;
-            else
-                (void)cudaGetLastError();                 // no fork: same stream, and no stale error for the launches below
-            e = launch_prefix_umma(a, dtype, kv_splits, 1, st);
-            const cudaError_t et = launch_attention_mma(a, dtype, FST_KERNEL_TMA, tree_st);
-            if (tree_st != st) {                          // always join what was forked
-                cudaError_t ej = cudaEventRecord(side->join, tree_st);
-                if (ej == cudaSuccess) ej = cudaStreamWaitEvent(st, side->join, 0);
-                if (e == cudaSuccess) e = ej;
-            }
-            if (e == cudaSuccess) e = et;
+            e = launch_prefix_umma(a, dtype, kv_splits, st);
         } else {
             a.n_splits = kv_splits;
             e = launch_attention_mma(a, dtype, choice, st);
         }
-        if (e == cudaSuccess) e = launch_combine(a, dtype, st);
+        if (e == cudaSuccess && kv_splits > 1) e = launch_combine(a, dtype, st);
         if (e != cudaErrorNotSupported || !automatic) return cuda_status(e);
         a.n_splits = 1;                                   // a tensor map could not be built: fall through
-        a.skip_prefix = 0;
         a.part_slots = 1;
     }
     cudaError_t e = launch_attention_mma(a, dtype, choice == FST_KERNEL_TMA_UMMA ? FST_KERNEL_TMA : choice, st);
@@ -488,33 +436,16 @@ int fst_attention_fwd_paged(const void *q, const void *k_tree, const void *v_tre
     a.scale_log2 = sm_scale * 1.4426950408889634f;
     a.status = status;
     a.n_splits = 1;
-    a.skip_prefix = 1;
-    a.part_slots = kv_splits + 1;
+    a.part_slots = kv_splits;
     a.meta_stable = 0;
     a.part_o = static_cast<float *>(workspace);
     a.part_lse = a.part_o + size_t(a.part_slots) * Z * H * n_q * head_dim;
-    AttnArgs ap = a;                                      // the prefix part: rows come from the page pool
-    ap.prefix = max_prefix;
-    PagedArgs pg{k_pool, v_pool, block_table, prefix_lens, table_stride, page_size, n_pages,
-                 pool_stride_page, pool_stride_row, pool_stride_head};
-
+    a.prefix = max_prefix;                                // the prefix rows come from the page pool
+    const PagedArgs pg{k_pool, v_pool, block_table, prefix_lens, table_stride, page_size, n_pages,
+                       pool_stride_page, pool_stride_row, pool_stride_head};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    SideStream *side = side_stream(st);                   // as in the contiguous prefix path
-    cudaStream_t tree_st = st;
-    if (side != nullptr && cudaEventRecord(side->fork, st) == cudaSuccess &&
-        cudaStreamWaitEvent(side->stream, side->fork, 0) == cudaSuccess)
-        tree_st = side->stream;
-    else
-        (void)cudaGetLastError();
-    cudaError_t e = launch_prefix_umma_paged(ap, pg, dtype, kv_splits, 1, st);
-    const cudaError_t et = launch_attention_mma(a, dtype, FST_KERNEL_TMA, tree_st);
-    if (tree_st != st) {
-        cudaError_t ej = cudaEventRecord(side->join, tree_st);
-        if (ej == cudaSuccess) ej = cudaStreamWaitEvent(st, side->join, 0);
-        if (e == cudaSuccess) e = ej;
-    }
-    if (e == cudaSuccess) e = et;
-    if (e == cudaSuccess) e = launch_combine(a, dtype, st);
+    cudaError_t e = launch_prefix_umma_paged(a, pg, dtype, kv_splits, st);
+    if (e == cudaSuccess && kv_splits > 1) e = launch_combine(a, dtype, st);
     return cuda_status(e);
 }
 

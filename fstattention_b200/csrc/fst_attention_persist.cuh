@@ -407,7 +407,7 @@ cudaError_t launch_persist_inst(const AttnArgs &a, cudaStream_t stream) {
     using CF = PersistCfg<D, BM>;
     constexpr size_t smem = CF::BYTES;
     constexpr bool bf16 = sizeof(T) == 2 && !std::is_same<T, __half>::value;
-    if (a.prefix != 0 || a.n_splits != 1 || a.skip_prefix) return cudaErrorNotSupported;
+    if (a.prefix != 0 || a.n_splits != 1) return cudaErrorNotSupported;
     alignas(64) CUtensorMap tq, tk, tv, to;
     if (!make_map(&tq, a.q, bf16, D, a.n_q, a.H, a.Z, a.qs_n, a.qs_h, a.qs_z) ||
         !make_map(&tk, a.k, bf16, D, a.n_kv, a.H / a.kv_group, a.Z, a.ks_n, a.ks_h, a.ks_z) ||

@@ -165,7 +165,7 @@ attn_tma_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap tm_q,
     // With the prefix split over several CTAs, split 0 also owns the tree part (block rows and
     // external ancestors); every split takes a contiguous run of prefix tiles.
     const bool tree = split == 0;
-    const int pt_total = (PFX && a.skip_prefix) ? 0 : (prefix + TN - 1) / TN, pt_per = (pt_total + n_splits - 1) / n_splits;
+    const int pt_total = (prefix + TN - 1) / TN, pt_per = (pt_total + n_splits - 1) / n_splits;
     const int pt_lo = min(split * pt_per, pt_total), pt_hi = min(pt_lo + pt_per, pt_total);
     const int p_lo = pt_lo * TN, p_end = min(prefix, pt_hi * TN);      // my prefix rows [p_lo, p_end)
     const int nblk = tree ? SM::NBT : 0;
@@ -558,7 +558,7 @@ attn_tma_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap tm_q,
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
     const float inv0 = (l0 > 0.f && alive) ? 1.f / l0 : 0.f, inv1 = (l1 > 0.f && alive) ? 1.f / l1 : 0.f;
-    if (PFX && (n_splits > 1 || a.skip_prefix)) {
+    if (PFX && n_splits > 1) {
         // partial result of this split: normalised rows in fp32 plus their log-sum-exp; the
         // combine kernel weighs the splits against each other
         const size_t prow = ((size_t(split) * a.Z + z) * a.H + h) * n_q + row0;
@@ -638,19 +638,12 @@ combine_splits_kernel(const AttnArgs a) {
     const size_t row = idx / CPR;
     const int c = int(idx - row * CPR) * 4;
     if (row >= rows) return;
-    // Loads go out four slots at a time so that their latencies overlap.
-    constexpr int U = 4;
     float big = -INFINITY;
-    for (int s0 = 0; s0 < a.part_slots; s0 += U) {
-        float ls[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            ls[u] = s0 + u < a.part_slots ? a.part_lse[size_t(s0 + u) * rows + row] : -INFINITY;
-#pragma unroll
-        for (int u = 0; u < U; ++u) big = fmaxf(big, ls[u]);
-    }
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
     float wsum = 0.f;
+    // Four slots at a time, everything of theirs asked for at once; up to four (the usual case) are merged with one
+    // memory latency.
+    constexpr int U = 4;
     for (int s0 = 0; s0 < a.part_slots; s0 += U) {
         float ls[U];
         float4 v[U];
@@ -661,6 +654,14 @@ combine_splits_kernel(const AttnArgs a) {
             v[u] = in ? *reinterpret_cast<const float4 *>(a.part_o + (size_t(s0 + u) * rows + row) * D + c)
                       : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        float top = big;
+#pragma unroll
+        for (int u = 0; u < U; ++u) top = fmaxf(top, ls[u]);
+        if (top == -INFINITY) continue;
+        const float keep = exp2f(big - top);
+        sum.x *= keep; sum.y *= keep; sum.z *= keep; sum.w *= keep;
+        wsum *= keep;
+        big = top;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (ls[u] == -INFINITY) continue;            // an empty run: its O row is not meaningful
@@ -842,7 +843,7 @@ cudaError_t launch_tma_pfx(const AttnArgs &a, cudaStream_t stream) {
     a2.heads_first = (TN == 64 && ctas > sm_count() && ctas <= 8LL * sm_count() && a.nb > 1) ? 1 : 0;
     dim3 grid(a.nb, a.H, a.Z * a.n_splits), block(BM * 2);
     if (a2.heads_first) grid = dim3(a.H, a.nb, a.Z * a.n_splits);
-    const size_t launch_smem = (ctas <= sm_count() && !a.skip_prefix && smem < kExclusive) ? kExclusive : smem;
+    const size_t launch_smem = (ctas <= sm_count() && smem < kExclusive) ? kExclusive : smem;
     // Programmatic stream serialisation: the grid may become resident while the kernel ahead of
     // it in the stream drains (it waits for that kernel before touching global memory).  Worth
     // about 2 % on back-to-back layers.
@@ -855,19 +856,18 @@ cudaError_t launch_tma_pfx(const AttnArgs &a, cudaStream_t stream) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = a.skip_prefix ? 0 : 1;                 // beside the prefix kernel an early, waiting grid would hold the SMs it needs
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, attn_tma_kernel<T, D, BM, TN, PFX, NOUT>, a2, tq, tk, tv, to);
 }
 
 template <typename T, int D, int BM, int TN>
 cudaError_t launch_tma_inst(const AttnArgs &a, cudaStream_t stream) {
     if (a.n_out > 0) {                                    // attention + delivery to every rank; no shared prefix there
-        if (a.prefix > 0 || a.skip_prefix || a.n_splits != 1) return cudaErrorNotSupported;
+        if (a.prefix > 0 || a.n_splits != 1) return cudaErrorNotSupported;
         return launch_tma_pfx<T, D, BM, TN, false, kMaxRanks>(a, stream);
     }
-    // the prefix instantiation also writes partial results (skip_prefix), with or without prefix rows
-    return (a.prefix > 0 || a.skip_prefix) ? launch_tma_pfx<T, D, BM, TN, true, 1>(a, stream)
-                                           : launch_tma_pfx<T, D, BM, TN, false, 1>(a, stream);
+    return a.prefix > 0 ? launch_tma_pfx<T, D, BM, TN, true, 1>(a, stream)
+                        : launch_tma_pfx<T, D, BM, TN, false, 1>(a, stream);
 }
 
 // tile_cols: 32, 64, or 0 = by grid size: 64-column tiles up to about eight CTAs per SM (measured:

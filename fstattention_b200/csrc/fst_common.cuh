@@ -111,10 +111,7 @@ struct AttnArgs {
     int n_splits;
     float *part_o;
     float *part_lse;
-    // skip_prefix: the tree kernel leaves the prefix to the tcgen05 prefix kernel and writes its
-    // own result as partial slot 0; part_slots: how many partial slots the merge kernel reads
-    int skip_prefix;
-    int part_slots;
+    int part_slots;        // how many partial results the merge kernel reads
     // the packed metadata was complete before the launch ahead of this one in the stream began:
     // a kernel launched with programmatic stream serialisation may read it before its dependency wait
     int meta_stable;
@@ -140,10 +137,10 @@ struct PagedArgs {
 cudaError_t launch_attention_simt(const AttnArgs &a, int dtype, cudaStream_t stream);
 // returns cudaErrorNotSupported when no tensor-core instantiation fits
 cudaError_t launch_attention_mma(const AttnArgs &a, int dtype, int variant, cudaStream_t stream);
-// dense prefix on tcgen05: partial results of n_runs runs into slots first_slot..; D = 64 or 128
-cudaError_t launch_prefix_umma(const AttnArgs &a, int dtype, int n_runs, int first_slot, cudaStream_t stream);
-cudaError_t launch_prefix_umma_paged(const AttnArgs &a, const PagedArgs &pg, int dtype, int n_runs, int first_slot,
-                                     cudaStream_t stream);
+// prefix and tree on tcgen05 in n_runs runs of column tiles, D = 64 or 128, block_m 32 and up: the output itself
+// with one run, else n_runs partial results
+cudaError_t launch_prefix_umma(const AttnArgs &a, int dtype, int n_runs, cudaStream_t stream);
+cudaError_t launch_prefix_umma_paged(const AttnArgs &a, const PagedArgs &pg, int dtype, int n_runs, cudaStream_t stream);
 // merge a.part_slots partial results into o (and lse)
 cudaError_t launch_combine(const AttnArgs &a, int dtype, cudaStream_t stream);
 

@@ -21,6 +21,7 @@
 #include <cmath>
 #include <mutex>
 #include <optional>
+#include <vector>
 
 #include "fst_plan.h"
 #include "fstattn_b200.h"
@@ -103,8 +104,9 @@ Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, i
     const int64_t cap = 65535 / std::max<int64_t>(Z, 1);
     const auto clamp = [&](int64_t v) { return int(std::max<int64_t>(1, std::min(v, cap))); };
     if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && prefix >= 256)) {
-        if (asked) return {clamp(*asked), true};
-        return {clamp(fst::prefix_runs(Z, H, H_kv, n_q, prefix, sm_count(device))), true};
+        if (asked) return {clamp(*asked), clamp(*asked) > 1};
+        const int runs = clamp(fst::prefix_runs(Z, H, H_kv, n_q, prefix, sm_count(device)));
+        return {runs, runs > 1};
     }
     int runs;
     if (asked) {
@@ -513,6 +515,33 @@ PyObject *parents_of_lineage(PyObject *const *a, Py_ssize_t n) {
     return THPVariable_Wrap(parent);
 }
 
+// check_tree(parent, block_m, max_ancestors): what the device status record of a metadata build would say, from a
+// parent array on the host (int32, contiguous), so that the caller need not wait for the device to learn it.
+// Every node is marked once per block: the marks of a block are its ancestors.
+PyObject *check_tree(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 3);
+    const at::Tensor &par = tensor(a[0]);
+    const int64_t N = par.size(0), bm = integer(a[1]), ma = integer(a[2]);
+    const int32_t *P = static_cast<const int32_t *>(par.data_ptr());
+    for (int64_t k = 0; k < N; ++k)
+        if (P[k] >= k || P[k] < -1) {
+            PyErr_Format(PyExc_ValueError, "malformed tree: parent[%lld]=%d must be -1 or an earlier node", (long long)k, int(P[k]));
+            throw PyError{};
+        }
+    std::vector<int32_t> seen(N, -1);                     // last block that met the node
+    for (int64_t b = 0; b * bm < N; ++b) {
+        int64_t count = 0;
+        for (int64_t k = b * bm; k < std::min(N, (b + 1) * bm); ++k)
+            for (int32_t x = P[k]; x >= 0 && seen[x] != int32_t(b); x = P[x], ++count) seen[x] = int32_t(b);
+        if (count > ma) {
+            PyErr_Format(PyExc_RuntimeError, "block %lld of tree 0 has %lld unique ancestors, more than max_ancestors=%lld",
+                         (long long)b, (long long)count, (long long)ma);
+            throw PyError{};
+        }
+    }
+    Py_RETURN_NONE;
+}
+
 // write_self(lineage, level_lookup): lineage[k, level[k]] = k (utils.py:124-125), int64 CPU tensors
 PyObject *write_self(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 2);
@@ -576,7 +605,7 @@ PyObject *splits(PyObject *const *a, Py_ssize_t n) {
 PyMethodDef methods[] = {
     FST_METHOD(attention),      FST_METHOD(attention_ref), FST_METHOD(attention_paged), FST_METHOD(pack),
     FST_METHOD(precompute),     FST_METHOD(new_metadata),  FST_METHOD(dfs_order),
-    FST_METHOD(build_tree_topk), FST_METHOD(parents_of_lineage), FST_METHOD(write_self), FST_METHOD(read_status), FST_METHOD(status_record), FST_METHOD(attention_status),
+    FST_METHOD(build_tree_topk), FST_METHOD(parents_of_lineage), FST_METHOD(write_self), FST_METHOD(check_tree), FST_METHOD(read_status), FST_METHOD(status_record), FST_METHOD(attention_status),
     FST_METHOD(splits),         {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fst_host", "tensor-level calls into libfstattn_b200.so", -1, methods};
 

@@ -17,18 +17,19 @@ inline int prefix_heads_per_tile(int64_t H, int64_t H_kv, int64_t n_q) {
     return pack;
 }
 
-// Runs a shared prefix is cut into for the tcgen05 prefix kernel: one CTA per 128 query rows, head (or pack of
+// Runs of column tiles that a call behind a shared prefix is cut into: one CTA per 128 query rows, head (or pack of
 // heads), batch element and run, one CTA per SM.  The choice minimises waves x (tiles of a run + kFixed), with a
-// charge for every further partial result that has to be written and merged: loading the first tiles,
-// merging the two softmax groups and writing a partial result take as long as some eight tiles of the
-// steady state (0.95 us each at D 128), and a grid of 1.2 waves takes two.
+// charge for merging more than one run: loading the first tiles, merging the two softmax groups and writing the
+// result take as long as some eight tiles of the steady state (0.95 us each at D 128), the merge kernel as four
+// and more, and a grid of 1.2 waves takes two.
 inline int prefix_runs(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, int64_t prefix, int sms) {
     const int64_t ctas = std::max<int64_t>(1, Z * (H / prefix_heads_per_tile(H, H_kv, n_q)) * ((n_q + 127) / 128));
-    const int64_t tiles = (prefix + 127) / 128, cap = std::min<int64_t>({prefix / 256, 16, 65535 / std::max<int64_t>(Z, 1)});
-    constexpr int64_t kFixed = 8;
+    const int64_t tiles = (prefix + 127) / 128 + 2, cap = std::min<int64_t>({prefix / 256, 16, 65535 / std::max<int64_t>(Z, 1)});
+    constexpr int64_t kFixed = 8, kMerge = 4;
     int64_t best = 1, best_cost = INT64_MAX;
     for (int64_t runs = 1; runs <= std::max<int64_t>(cap, 1); ++runs) {
-        const int64_t waves = (ctas * runs + sms - 1) / sms, cost = waves * ((tiles + runs - 1) / runs + kFixed) + runs;
+        const int64_t waves = (ctas * runs + sms - 1) / sms,
+                      cost = waves * ((tiles + runs - 1) / runs + kFixed) + (runs > 1 ? kMerge + runs : 0);
         if (cost < best_cost) {
             best_cost = cost;
             best = runs;

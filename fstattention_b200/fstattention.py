@@ -75,8 +75,8 @@ def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[in
         tree = "tree_umma_kernel"
     if kernel == "persist" and tree == "attn_tma_kernel" and prefix == 0 and block_m in (64, 128):
         tree = "attn_persist_kernel"                      # by hand only: it measured slower than attn_tma_kernel
-    if need_ws and q.shape[-1] in (64, 128) and (kernel == "tma_umma" or (kernel == "auto" and prefix >= 256)):
-        return {"kernels": ["prefix_umma_kernel", tree, "combine_splits_kernel"], "prefix_runs": splits}
+    if tensor_core and block_m >= 32 and prefix > 0 and (kernel == "tma_umma" or (kernel == "auto" and prefix >= 256)):
+        tree = "prefix_umma_kernel"                       # prefix and tree in one
     if need_ws:
         return {"kernels": [tree, "combine_splits_kernel"], "prefix_runs": splits}
     return {"kernels": [tree], "prefix_runs": 1}
@@ -97,8 +97,8 @@ def fst_attention(q, k, v, ancestor_idx, ancestor_mask=None, leaf_idx=None, sm_s
     ``Z`` gives every batch element its own tree.  ``k`` and ``v`` may have fewer heads than ``q``
     (grouped-query attention, ``H`` a multiple of ``H_kv``).
 
-    ``kv_splits`` cuts a shared prefix into that many runs handled by separate CTAs and merged
-    afterwards; ``None`` picks a split that fills the GPU when the tree alone does not.
+    ``kv_splits`` cuts a call behind a shared prefix into that many runs handled by separate CTAs and
+    merged afterwards; ``None`` picks a split that fills the GPU when the tree alone does not.
 
     ``scatter`` (see ``sharding.GatheredOutput.target``) makes the kernel deliver this call's
     rows into every rank's copy of a full output tensor instead of a local ``out``; the return

@@ -231,8 +231,12 @@ def create_fst_attention_kernel_inputs(lineage: torch.Tensor, level_lookup: torc
     row as a side effect; pass ``mutate_lineage=False`` to leave ``lineage`` alone.
     """
     native = _on_host(lineage, 2) and _on_host(level_lookup, 1) and lineage.shape[0] == level_lookup.shape[0]
-    parent = _lib.host().parents_of_lineage(lineage, level_lookup) if native else parent_from_lineage(lineage, level_lookup)
-    meta = build_tree_metadata(parent, block_m, max_ancestors, reference_format=True, check=True)
+    host = _lib._host or _lib.host()
+    parent = host.parents_of_lineage(lineage, level_lookup) if native else parent_from_lineage(lineage, level_lookup)
+    meta = build_tree_metadata(parent, block_m, max_ancestors, reference_format=True, check=not native)
+    if native:
+        # the parents are on the host: so is the check, and nobody waits for the device
+        host.check_tree(parent, block_m, max_ancestors)
     if mutate_lineage and native:
         _lib.host().write_self(lineage, level_lookup)
     elif mutate_lineage:

@@ -5,10 +5,7 @@
  * void*.  No function allocates or frees device memory or synchronises; each one enqueues its
  * kernels on the given stream and returns a status code (0 = FST_OK) describing host-side
  * argument checks.  Host-side state the library keeps: per host thread a table of the tensor
- * maps it has built (about 200 KB of host memory, filled as calls come), and - only for calls
- * that hand a shared prefix to the tcgen05 kernel (fst_attention_fwd_splitkv / _gqa / _paged with
- * a workspace) - one extra CUDA stream and two events per host thread and device, created at the
- * first such call outside stream capture and kept until the process ends.  The first call of a
+ * maps it has built (about 200 KB of host memory, filled as calls come).  The first call of a
  * kernel variant on a device also sets that kernel's shared-memory attribute; make one call per
  * shape and dtype before capturing a stream into a graph.
  * Problems that only the GPU can see (a malformed tree, too many ancestors in a block, an
@@ -59,8 +56,8 @@ enum fst_kernel {
                                    /* 32- or 64-column tiles chosen by grid size                 */
     FST_KERNEL_TMA_T32 = 4,        /* ... forced 32-column tiles (three CTAs per SM)             */
     FST_KERNEL_TMA_T64 = 5,        /* ... forced 64-column tiles (fewest softmax rounds)         */
-    FST_KERNEL_TMA_UMMA = 6,       /* tree part as FST_KERNEL_TMA, shared prefix by the tcgen05  */
-                                   /* kernel (head_dim 64 / 128, fst_attention_fwd_splitkv only) */
+    FST_KERNEL_TMA_UMMA = 6,       /* shared prefix and tree by one tcgen05 kernel (head_dim 64  */
+                                   /* / 128, block_m 32 and up, positive sm_scale)               */
     FST_KERNEL_PERSIST = 7,        /* persistent CTAs, a producer warp streaming tiles through a */
                                    /* shared-memory ring ahead of the arithmetic: block_m 64 or  */
                                    /* 128, no prefix.  Slower than FST_KERNEL_TMA on every shape */
@@ -257,10 +254,10 @@ int fst_attention_tree_kernel(int Z, int H, int n_q, int head_dim, int block_m, 
  * own CTA per (block, head, batch) - the decode case, where a long prompt meets a tree too small
  * to fill the GPU (the reference walks the prefix in one program, fstattention.py:113-136).
  * Partial results (fp32) and their log-sum-exps pass through `workspace`
- * (fst_attention_split_workspace_bytes bytes, 16-byte aligned, scratch) and a second kernel merges
- * them.  With head_dim 64 or 128 and at least 256 prefix rows FST_KERNEL_AUTO hands the prefix to a
- * tcgen05/TMEM kernel (128 x 128 tiles, dense) in kv_splits runs and keeps the tree part in the
- * tree kernel; FST_KERNEL_TMA_UMMA forces that, FST_KERNEL_TMA* forces the tree kernel to walk
+ * (fst_attention_split_workspace_bytes bytes, 16-byte aligned, scratch; not needed with one run) and a
+ * second kernel merges them.  With head_dim 64 or 128, block_m 32 and up and at least 256 prefix rows
+ * FST_KERNEL_AUTO hands the call to a tcgen05/TMEM kernel that walks prefix and tree in 128 x 128 tiles,
+ * cut into kv_splits runs; FST_KERNEL_TMA_UMMA forces that, FST_KERNEL_TMA* forces the tree kernel to walk
  * the prefix itself in kv_splits runs.  Without a prefix this is fst_attention_fwd.
  */
 size_t fst_attention_split_workspace_bytes(int Z, int H, int n_q, int head_dim, int kv_splits);
@@ -305,8 +302,8 @@ int fst_attention_fwd_gqa(const void *q, const void *k, const void *v, void *o, 
  * k_pool / v_pool: element (page, row, head, d) at page * pool_stride_page + row * pool_stride_row
  * + head * pool_stride_head + d (element strides, multiples of 8).  page_size 16, 32, 64 or 128;
  * head_dim 64 or 128; fp16 / bf16.  max_prefix >= every prefix_lens[z] (it sizes the grid; lengths
- * above it are cut).  The prefix goes to the tcgen05 kernel in kv_splits runs, the tree part to
- * the tree kernel, partial results through `workspace`
+ * above it are cut).  Prefix and tree go to the tcgen05 kernel in kv_splits runs, partial results
+ * of more than one run through `workspace`
  * (fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits) bytes).  A page number
  * outside [0, n_pages) reads as zeros and sets FST_DEV_INDEX_RANGE.  block_table and prefix_lens
  * are device pointers.  sm_scale must be positive here (the tcgen05 prefix kernel takes Q as it

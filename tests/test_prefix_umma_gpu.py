@@ -1,0 +1,100 @@
+"""The tcgen05 kernel behind a shared prefix, which walks prefix and tree: prefixes that end inside a tile, query
+tiles of one to four blocks, ancestor lists that end inside a tile or run over several, and cuts that leave runs
+without a tile or with the tree's tiles only."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
+
+
+@pytest.fixture(scope="module")
+def fst(built_lib):
+    import fstattention_b200
+    return fstattention_b200
+
+
+def comb(n, teeth):
+    return [i - 1 if i < teeth else (i * 7) % teeth for i in range(n)]
+
+
+@pytest.mark.parametrize("bm", [32, 64, 128])
+@pytest.mark.parametrize("n,teeth,prefix,splits,D", [
+    (1, 1, 1, 1, 128), (17, 3, 127, 1, 64), (33, 8, 128, 2, 128), (64, 20, 129, 3, 128), (65, 40, 300, 2, 64),
+    (128, 33, 256, 8, 128), (129, 64, 700, 2, 128), (200, 65, 513, 3, 64), (257, 30, 384, 1, 128),
+    (385, 130, 1000, 5, 128), (640, 300, 640, 2, 64), (640, 300, 130, 6, 128)])
+def test_prefix_and_tree_in_one(fst, n, teeth, prefix, splits, D, bm):
+    par = comb(n, teeth)
+    meta = fst.build_tree_metadata(par, bm, 512, reference_format=False)
+    dtype = torch.float16 if n % 2 else torch.bfloat16
+    g = torch.Generator().manual_seed(n + bm)
+    q = torch.randn((2, 4, n, D), generator=g).to(dtype)
+    k, v = (torch.randn((2, 2, prefix + n, D), generator=g).to(dtype) for _ in range(2))
+    qc, kc, vc = q.cuda(), k.cuda(), v.cuda()
+    o, lse = fst.fst_attention(qc, kc, vc, meta, sm_scale=D ** -0.5, kernel="tma_umma", kv_splits=splits, return_lse=True)
+    want, ref = fst.fst_attention(qc.float(), kc.float(), vc.float(), meta, sm_scale=D ** -0.5, kernel="simt", return_lse=True)
+    assert (o.float() - want).abs().max().item() <= TOL[dtype]
+    assert (lse - ref).abs().max().item() <= 1e-3
+    assert fst.last_status() == 0
+
+
+@pytest.mark.parametrize("rows", [slice(40, 50), slice(700, 710), slice(1100, 1110)])     # prefix, prefix, tree
+def test_prefix_moving_maximum(fst, rows):
+    """Rows whose scores dwarf the first reference point: the accumulators are rescaled."""
+    n, D, prefix = 300, 128, 1000
+    par = comb(n, 200)
+    meta = fst.build_tree_metadata(par, 64, 256, reference_format=False)
+    g = torch.Generator().manual_seed(4)
+    q = torch.randn((1, 2, n, D), generator=g).half()
+    k, v = (torch.randn((1, 2, prefix + n, D), generator=g) for _ in range(2))
+    k[:, :, rows] *= 12.0
+    q, k, v = q.cuda(), k.half().cuda(), v.half().cuda()
+    for splits in (1, 3):
+        o = fst.fst_attention(q, k, v, meta, sm_scale=0.5, kernel="tma_umma", kv_splits=splits)
+        want = fst.fst_attention(q.float(), k.float(), v.float(), meta, sm_scale=0.5, kernel="simt")
+        assert (o.float() - want).abs().max().item() <= 4e-3
+
+
+def test_paged_lengths_of_their_own(fst):
+    """Sequences without a prefix, with part of a page, and with the longest allowed, next to one another."""
+    Z, H, n, D, ps = 4, 4, 70, 128, 16
+    lens, longest = [0, 5, 130, 640], 640
+    par = comb(n, 20)
+    meta = fst.build_tree_metadata(par, 64, 64, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, kt, vt = (torch.randn((Z, H, n, D), generator=g, device="cuda").half() for _ in range(3))
+    pages = longest // ps
+    pool = torch.randn((2, Z * pages, ps, H, D), generator=g, device="cuda").half()
+    table = torch.randperm(Z * pages, generator=g, device="cuda", dtype=torch.int32).view(Z, pages)
+    for splits in (1, 3):
+        o = fst.fst_attention_paged(q, kt, vt, meta, pool[0], pool[1], table,
+                                    torch.tensor(lens, dtype=torch.int32, device="cuda"), D ** -0.5, max_prefix=longest,
+                                    kv_splits=splits)
+        for z in range(Z):
+            kv = [torch.cat([p[table[z].long()].reshape(-1, H, D)[:lens[z]].transpose(0, 1), t[z]], 1)[None]
+                  for p, t in ((pool[0], kt), (pool[1], vt))]
+            want = fst.fst_attention(q[z:z + 1].float(), kv[0].float(), kv[1].float(), meta, sm_scale=D ** -0.5, kernel="simt")
+            assert (o[z:z + 1].float() - want).abs().max().item() <= 2e-3
+    assert fst.last_status() == 0
+
+
+def test_lineage_on_the_host_is_checked_there(fst):
+    """The bound at which a lineage on the host is refused is the device's, and so is the message."""
+    par = comb(300, 90)
+    lineage, level = fst.lineage_from_parent(par)
+    for bm in (16, 64):
+        bound = 60
+        while True:                                       # the smallest bound that the device accepts
+            try:
+                want = fst.build_tree_metadata(par, bm, bound)
+                break
+            except RuntimeError:
+                bound += 1
+        got = fst.create_fst_attention_kernel_inputs(lineage.clone(), level, bm, bound)
+        assert bound > 60 and all(torch.equal(a, b) for a, b in zip(got, want))
+        with pytest.raises(RuntimeError, match="max_ancestors"):
+            fst.create_fst_attention_kernel_inputs(lineage.clone(), level, bm, bound - 1)
+    bad = lineage.clone()
+    bad[5, level[5] - 1] = 7
+    with pytest.raises(ValueError, match="malformed"):
+        fst.create_fst_attention_kernel_inputs(bad, level, 64, 128)
