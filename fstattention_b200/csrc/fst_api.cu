@@ -288,30 +288,27 @@ static int attention_fwd_impl(const void *q, const void *k, const void *v, void 
 
     // A shared prefix: the tcgen05 kernel takes the whole call in kv_splits runs of column tiles (head_dim 64 or 128,
     // block_m 32 and up; chosen automatically from 256 prefix rows on), or the tree kernel itself walks the prefix,
-    // split over kv_splits CTAs.  More than one run needs the workspace.
+    // split over kv_splits CTAs whose partial results pass through the workspace.
     // (the tcgen05 kernel takes Q from shared memory as it arrived, so it cannot flip Q's sign
     // for a negative factor; the tree kernel walks the prefix itself then)
     const bool can_part = a.prefix > 0 && choice != FST_KERNEL_MMA && choice != FST_KERNEL_PERSIST;
-    const bool want_umma = can_part && (workspace != nullptr || kv_splits == 1) && block_m >= 32 && sm_scale > 0.f &&
+    const bool want_umma = can_part && block_m >= 32 && sm_scale > 0.f &&
                            (choice == FST_KERNEL_TMA_UMMA || (automatic && a.prefix >= 256));
     if (choice == FST_KERNEL_TMA_UMMA && !want_umma) return FST_ERR_UNSUPPORTED;
-    if (want_umma || (can_part && workspace != nullptr && kv_splits > 1)) {
-        if (kv_splits > 1) {
-            const size_t need = fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits);
-            if (workspace_bytes < need) return FST_ERR_WORKSPACE;
-            if (!aligned16(workspace)) return FST_ERR_ALIGNMENT;
-            a.part_slots = kv_splits;
-            a.part_o = static_cast<float *>(workspace);
-            a.part_lse = a.part_o + size_t(a.part_slots) * Z * H * n_q * head_dim;
-        }
-        cudaError_t e;
-        if (want_umma) {
-            e = launch_prefix_umma(a, dtype, kv_splits, st);
-        } else {
-            a.n_splits = kv_splits;
-            e = launch_attention_mma(a, dtype, choice, st);
-        }
-        if (e == cudaSuccess && kv_splits > 1) e = launch_combine(a, dtype, st);
+    if (want_umma) {
+        const cudaError_t e = launch_prefix_umma(a, dtype, kv_splits, st);
+        if (e != cudaErrorNotSupported || !automatic) return cuda_status(e);
+        // a tensor map could not be built: fall through
+    } else if (can_part && workspace != nullptr && kv_splits > 1) {
+        const size_t need = fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits);
+        if (workspace_bytes < need) return FST_ERR_WORKSPACE;
+        if (!aligned16(workspace)) return FST_ERR_ALIGNMENT;
+        a.part_slots = kv_splits;
+        a.part_o = static_cast<float *>(workspace);
+        a.part_lse = a.part_o + size_t(a.part_slots) * Z * H * n_q * head_dim;
+        a.n_splits = kv_splits;
+        cudaError_t e = launch_attention_mma(a, dtype, choice, st);
+        if (e == cudaSuccess) e = launch_combine(a, dtype, st);
         if (e != cudaErrorNotSupported || !automatic) return cuda_status(e);
         a.n_splits = 1;                                   // a tensor map could not be built: fall through
         a.part_slots = 1;
@@ -403,7 +400,7 @@ int fst_attention_fwd_paged(const void *q, const void *k_tree, const void *v_tre
                             int max_ancestors, float sm_scale, int dtype, int kv_splits, void *workspace,
                             size_t workspace_bytes, int32_t *status, void *stream) {
     if (!q || !k_tree || !v_tree || !o || !packed || !k_pool || !v_pool || !block_table || !prefix_lens ||
-        !workspace || Z <= 0 || H <= 0 || H_kv <= 0 || H % H_kv != 0 || n_q <= 0 || block_m <= 0 ||
+        Z <= 0 || H <= 0 || H_kv <= 0 || H % H_kv != 0 || n_q <= 0 || block_m <= 0 ||
         max_ancestors <= 0 || max_prefix <= 0 || n_pages <= 0 || kv_splits < 1 || table_stride <= 0)
         return FST_ERR_INVALID_ARG;
     if ((head_dim != 128 && head_dim != 64) || !mma_ok(dtype, head_dim, block_m)) return FST_ERR_UNSUPPORTED;
@@ -415,12 +412,12 @@ int fst_attention_fwd_paged(const void *q, const void *k_tree, const void *v_tre
                                v_stride_z, v_stride_h, v_stride_n, o_stride_z, o_stride_h, o_stride_n,
                                pool_stride_page, pool_stride_row, pool_stride_head};
     bool ok = aligned16(q) && aligned16(k_tree) && aligned16(v_tree) && aligned16(o) && aligned16(k_pool) &&
-              aligned16(v_pool) && aligned16(packed) && aligned16(workspace) && !(meta_tree_stride & 15);
+              aligned16(v_pool) && aligned16(packed) && !(meta_tree_stride & 15);
     for (int64_t s : strides)
         if ((s * 2) & 15) ok = false;
     if (!ok) return FST_ERR_ALIGNMENT;
-    if (workspace_bytes < fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits))
-        return FST_ERR_WORKSPACE;
+    (void)workspace;                                      // the runs are merged inside the kernel
+    (void)workspace_bytes;
 
     AttnArgs a = {};                                      // the tree part: K/V rows of the tree nodes only
     a.q = q; a.k = k_tree; a.v = v_tree; a.o = o; a.lse = lse;
@@ -436,17 +433,13 @@ int fst_attention_fwd_paged(const void *q, const void *k_tree, const void *v_tre
     a.scale_log2 = sm_scale * 1.4426950408889634f;
     a.status = status;
     a.n_splits = 1;
-    a.part_slots = kv_splits;
+    a.part_slots = 1;
     a.meta_stable = 0;
-    a.part_o = static_cast<float *>(workspace);
-    a.part_lse = a.part_o + size_t(a.part_slots) * Z * H * n_q * head_dim;
     a.prefix = max_prefix;                                // the prefix rows come from the page pool
     const PagedArgs pg{k_pool, v_pool, block_table, prefix_lens, table_stride, page_size, n_pages,
                        pool_stride_page, pool_stride_row, pool_stride_head};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaError_t e = launch_prefix_umma_paged(a, pg, dtype, kv_splits, st);
-    if (e == cudaSuccess && kv_splits > 1) e = launch_combine(a, dtype, st);
-    return cuda_status(e);
+    return cuda_status(launch_prefix_umma_paged(a, pg, dtype, kv_splits, st));
 }
 
 size_t fst_attention_ref_workspace_bytes(int n_meta_trees, int n_q, int block_m, int max_ancestors) {

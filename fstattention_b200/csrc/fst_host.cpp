@@ -104,9 +104,7 @@ Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, i
     const int64_t cap = 65535 / std::max<int64_t>(Z, 1);
     const auto clamp = [&](int64_t v) { return int(std::max<int64_t>(1, std::min(v, cap))); };
     if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && prefix >= 256)) {
-        if (asked) return {clamp(*asked), clamp(*asked) > 1};
-        const int runs = clamp(fst::prefix_runs(Z, H, H_kv, n_q, prefix, sm_count(device)));
-        return {runs, runs > 1};
+        return {fst::prefix_plan(Z, H, H_kv, n_q, prefix, sm_count(device), asked ? clamp(*asked) : 0).runs, false};
     }
     int runs;
     if (asked) {
@@ -332,11 +330,9 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
     const int64_t max_prefix = integer(a[15]);
     const at::Device dev = q.device();
     std::optional<long long> asked = optional_int(a[17]);
-    if (!asked) asked = fst::prefix_runs(Z, H, H_kv, n_q, max_prefix, sm_count(dev.index()));
+    if (!asked && max_prefix > 0) asked = fst::prefix_plan(Z, H, H_kv, n_q, max_prefix, sm_count(dev.index()), 0, kp.size(row_dim)).runs;
     const c10::cuda::CUDAGuard guard(dev);
     int32_t *status = static_cast<int32_t *>(status_of(dev, true)->data_ptr());
-    const size_t ws_bytes = fst_attention_split_workspace_bytes(int(Z), int(H), int(n_q), int(D), int(*asked));
-    const at::Tensor ws = empty({int64_t(ws_bytes)}, at::kByte, dev);
     void *stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     const size_t tree_stride = n_trees > 1 ? size_t(integer(a[5])) : 0;
     const void *packed = tensor(a[4]).data_ptr();
@@ -349,7 +345,7 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
                                      int(kp.size(row_dim)), int(kp.size(0)), kp.stride(0), kp.stride(row_dim),
                                      kp.stride(head_dim), int(Z), int(H), int(H_kv), int(n_q), int(D), FST_STRIDES(q),
                                      FST_STRIDES(kt), FST_STRIDES(vt), FST_STRIDES(c.o), int(bm), int(ma), c.scale, c.dtype,
-                                     int(*asked), ws.data_ptr(), ws_bytes, status, stream);
+                                     int(asked.value_or(1)), nullptr, 0, status, stream);
     }
     check_status(rc, "fst_attention_fwd_paged");
     return results(c);

@@ -17,25 +17,38 @@ inline int prefix_heads_per_tile(int64_t H, int64_t H_kv, int64_t n_q) {
     return pack;
 }
 
-// Runs of column tiles that a call behind a shared prefix is cut into: one CTA per 128 query rows, head (or pack of
-// heads), batch element and run, one CTA per SM.  The choice minimises waves x (tiles of a run + kFixed), with a
-// charge for merging more than one run: loading the first tiles, merging the two softmax groups and writing the
-// result take as long as some eight tiles of the steady state (0.95 us each at D 128), the merge kernel as four
-// and more, and a grid of 1.2 waves takes two.
-inline int prefix_runs(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, int64_t prefix, int sms) {
-    const int64_t ctas = std::max<int64_t>(1, Z * (H / prefix_heads_per_tile(H, H_kv, n_q)) * ((n_q + 127) / 128));
-    const int64_t tiles = (prefix + 127) / 128 + 2, cap = std::min<int64_t>({prefix / 256, 16, 65535 / std::max<int64_t>(Z, 1)});
-    constexpr int64_t kFixed = 8, kMerge = 4;
-    int64_t best = 1, best_cost = INT64_MAX;
-    for (int64_t runs = 1; runs <= std::max<int64_t>(cap, 1); ++runs) {
-        const int64_t waves = (ctas * runs + sms - 1) / sms,
-                      cost = waves * ((tiles + runs - 1) / runs + kFixed) + (runs > 1 ? kMerge + runs : 0);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = runs;
+// How a call behind a shared prefix is laid out: whether a CTA has two query tiles (pair), and into how many runs
+// the column tiles are cut, the runs of a query tile being a cluster of CTAs.  One CTA per SM.
+// The choice minimises waves x (tiles of a run x a tile's time + a CTA's fixed time) + merging.  In tenths of a
+// microsecond at D 128 (4096 prefix rows, 32 heads of 256 query rows; 3001 rows in pages of 16, 8 K/V heads): a tile 10
+// for one query tile and 22 for two, but 18 for one where the tile comes in small pages (a page of 16 rows
+// is a TMA box per 64 columns, and the boxes are what takes the time: two query tiles share them);
+// 140 for loading the first tiles, the last tile's chain and the output; 7 for every run to be merged.
+constexpr int kMaxPrefixRuns = 8;      // portable cluster size
+struct PrefixPlan {
+    int runs;
+    bool pair;
+};
+inline PrefixPlan prefix_plan(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, int64_t prefix, int sms, int64_t asked = 0,
+                              int64_t page = 128) {
+    const int64_t kv_tiles = H / H_kv / prefix_heads_per_tile(H, H_kv, n_q) * ((n_q + 127) / 128);
+    const int64_t tiles = (prefix + 127) / 128 + 2;
+    const int64_t cap = std::max<int64_t>(1, std::min<int64_t>({kMaxPrefixRuns, tiles / 2, 65535 / std::max<int64_t>(Z, 1)}));
+    const int64_t lo = asked > 0 ? std::min<int64_t>(asked, kMaxPrefixRuns) : 1, hi = asked > 0 ? lo : cap;
+    PrefixPlan best{int(lo), false};
+    int64_t best_cost = INT64_MAX;
+    for (int64_t pair = 0; pair < (kv_tiles > 1 ? 2 : 1); ++pair)
+        for (int64_t runs = lo; runs <= hi; ++runs) {
+            const int64_t ctas = Z * H_kv * ((kv_tiles + pair) / (1 + pair)) * runs;
+            const int64_t fit = runs > 4 ? sms * 7 / 8 : runs > 2 ? sms * 9 / 10 : sms;      // clusters stay within a GPC
+            const int64_t waves = (ctas + fit - 1) / fit;
+            const int64_t cost = waves * ((tiles + runs - 1) / runs * (pair ? 22 : page < 32 ? 18 : 10) + 140) + (runs > 1 ? 10 + 7 * runs : 0);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = {int(runs), pair != 0};
+            }
         }
-    }
-    return int(best);
+    return best;
 }
 
 // When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, six kinds of trees, from 64

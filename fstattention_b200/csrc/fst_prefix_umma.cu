@@ -1,31 +1,35 @@
 // Attention behind a shared prefix on the 5th-generation tensor cores (tcgen05 + TMEM).
 //
 // The prefix part of the reference kernel (fstattention.py:113-136) is plain dense attention: every query
-// row attends to every prefix row.  One CTA per (128 query rows, head, batch element, run of column tiles);
+// row attends to every prefix row.  A CTA has one or two query tiles of 128 rows and a run of column tiles;
 // the column tiles of a query tile are the prefix in 128-row tiles, then the tree: one tile with the
 // query tile's own K/V rows and, behind it, tiles of gathered ancestors, in which every block of the query tile has
-// a segment of columns.  Tree tiles are masked by the rows' mask words and cost what a prefix tile costs;
-// run beside this kernel as a launch of its own on a second stream, the tree part took a fork, a join, a
-// further partial result and, at small sizes, most of the call.  Per tile t
-//     S(t) = Q K(t)^T       tcgen05.mma  M=128 N=128 K=16 x D/16, both operands K-major in shared memory
-//     P(t) = softmax part   one thread per query row (TMEM lane = row, so no shuffles): tcgen05.ld
-//                           of S, probabilities against a lazily moved reference point, P written
-//                           to shared memory in the 128-byte-swizzled K-major layout
-//     O_g += P(t) V(t)      tcgen05.mma  A = P, B = V (MN-major: rows of V are the K index)
-// Tensor memory holds two S buffers and two accumulators O_0, O_1 (4 x 128 columns).  K/V tiles
-// arrive by TMA (128-row x 64-column boxes, 128-byte swizzle; gathered rows by cp.async into the same
-// layout) into two stages each.  Head dimension D is 64 or 128: one or two 64-column halves per Q / K / V tile.
+// a segment of columns.  Tree tiles are masked by the rows' mask words and cost what a prefix tile costs.
+// Per query tile and column tile, a step:
+//     S = Q K^T             tcgen05.mma  M=128 N=128 K=16 x D/16, both operands K-major in shared memory
+//     P = softmax part      one thread per query row (TMEM lane = row, so no shuffles): a row of S in 128 registers,
+//                           probabilities against a lazily moved reference point, P back to tensor memory
+//     O += P V              tcgen05.mma  A = P in tensor memory, B = V (MN-major: rows of V are the K index)
+// K/V tiles arrive by TMA (128-row x 64-column boxes, 128-byte swizzle; gathered rows by cp.async into the same
+// layout) in a ring of stages.  Head dimension D is 64 or 128: one or two 64-column halves per Q / K / V tile.
 //
-// Twelve warps.  Warps 0-3 and 4-7 are two softmax groups; group g takes the tiles with t & 1 == g
-// and keeps its own reference point, row sums, P buffer and accumulator O_g, so the groups never
-// wait for one another and one group's barrier waits and tensor-memory latencies hide behind the
-// other's exponentials.  Warp 8 loads K and its lane 0 issues S(t); warp 9 loads V and its lane 0
-// issues O_g += P V; warps 10 and 11 gather the K and the V rows of ancestors when 8 and 9 say that their stage is
-// free.  All hand-offs are mbarriers (TMA completion, tcgen05.commit, or arrivals by
-// the 128 threads of a group); every barrier indexed by t & 1 completes once per two tiles, so a
-// waiter can never fall two phases behind.  At the end the groups' results are merged through
-// shared memory and written: as the output itself when there is one run, else as one partial result per
-// run (normalised rows in fp32 plus base-2 log-sum-exp) that combine_splits_kernel merges.
+// Shared-memory bandwidth is what a tile costs: at D 128 the two products read 96 KB of operands and the tile's
+// K and V come in with 64 KB, against 1024 cycles of tensor work.  Hence P in tensor memory (writing it to and
+// reading it from shared memory took another 64 KB), and hence two query tiles to a CTA where there are two
+// that read the same K and V - neighbouring rows of a tree, or other heads of a grouped-query group: a
+// K/V tile then comes in once for both.  Two softmax groups of four warps take a query tile each; with one
+// query tile they take its column tiles in turn and their results are merged at the end.  Either way a
+// group's barrier waits and tensor-memory latencies hide behind the other's exponentials.
+//
+// Twelve warps.  Warps 0-3 and 4-7 are the softmax groups; warp 8 loads K and V; one lane of warp 9 issues the
+// products, the two groups' in turn: O += P V, then the group's next S (which overwrites P: tcgen05.mma
+// of one thread run in order); warps 10 and 11 gather the K and the V rows of ancestors when warp 8 says that their stage
+// is free.  All hand-offs are mbarriers (TMA completion, tcgen05.commit, or arrivals by the 128 threads of a group).
+// A stage's fills are claimed in order by warp 8 alone, so no waiter is ever two phases behind or one ahead.
+//
+// Runs: the column tiles of a query tile are cut into up to eight runs, one CTA each, which form a
+// cluster.  Every CTA leaves its rows, unnormalised, in its shared memory; each then merges its share of the rows
+// out of all of them and writes the output.  There are no partial results in memory and no second kernel.
 //
 // With grouped-query attention a small tree's rows of several heads share a query tile (see
 // prefix_heads_per_tile): the tile is loaded as one box per head and its rows go to their heads at the end.
@@ -43,39 +47,81 @@ namespace fst {
 
 namespace umma {
 
-constexpr int QM = 128;                // query rows per CTA (MMA M)
+constexpr int QM = 128;                // query rows per tile (MMA M)
 constexpr int KN = 128;                // K/V rows per tile (MMA N of the first product)
-constexpr int TILE_P = 2 * HALF;       // bytes of a P tile (128 x 128 fp16)
 
-// Shared-memory map for head dimension D (64 or 128): a Q / K / V tile is 128 rows of D columns,
-// D / 64 halves.  Q | P x 2 (double buffered) | K x 2 stages | V x 2 stages | barriers.
+// Shared memory for head dimension D (64 or 128): a Q / K / V tile is 128 rows of D columns, D / 64 halves.
+// One or two Q tiles, the rest of the tiles are the ring of K/V stages; then barriers.  At the end the
+// groups' rows (fp32) and their statistics take the tiles' place.
 template <int D>
 struct Geo {
     static constexpr int TILE = (D / 64) * HALF;
-    static constexpr int OFF_Q = 0;
-    static constexpr int OFF_P = OFF_Q + TILE;
-    static constexpr int OFF_K = OFF_P + 2 * TILE_P;
-    static constexpr int OFF_V = OFF_K + 2 * TILE;
-    static constexpr int OFF_BAR = OFF_V + 2 * TILE;
-    static constexpr int SMEM_BYTES = OFF_BAR + 160 + 1024;   // + barriers, TMEM address, 1 KB alignment slack
+    static constexpr int TILES = D == 128 ? 7 : 12;
+    static constexpr int MAX_RING = TILES - 1;
+    static constexpr int OFF_BAR = TILES * TILE;
+    static constexpr int SMEM_BYTES = OFF_BAR + 384 + 1024;   // + barriers, TMEM address, 1 KB alignment slack
+    static constexpr int OFF_STATS = 2 * QM * D * 4;          // [256] (exponent, sum) of the groups' rows, [256] of the CTA's
 };
+static_assert(Geo<128>::OFF_STATS + 4 * QM * 8 <= Geo<128>::OFF_BAR, "merge buffers fit");
+static_assert(Geo<64>::OFF_STATS + 4 * QM * 8 <= Geo<64>::OFF_BAR, "merge buffers fit");
+static_assert(1 + 3 * Geo<64>::MAX_RING + 8 <= 46, "barriers fit");
+
+// the same word of shared memory in CTA `cta` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, int cta) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(cta));
+    return r;
+}
+__device__ __forceinline__ float4 cluster_ld4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 cluster_ld2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+// every thread of every CTA of the cluster; shared memory written before is visible after
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
 
 }  // namespace umma
 
 // Arguments of the prefix kernel beyond AttnArgs.
 struct PrefixArgs {
-    int n_runs;          // runs of column tiles (CTAs per query tile, head, batch element)
+    int n_runs;          // runs of column tiles (CTAs of a cluster)
+    int pair;            // two query tiles to a CTA
+    int q_tiles;         // query tiles of a head (or pack of heads)
+    int kv_tiles;        // query tiles that read one K/V head
+    int pack, pack_shift;                // heads per query tile; a head's rows are 1 << pack_shift of the tile's
     // paged prefix: K/V rows live in pages of page_size rows; block_table[z][i] is the page
     // holding rows [i * page_size, (i + 1) * page_size) of batch element z, prefix_lens[z] its
     // number of prefix rows (AttnArgs::prefix is then the largest of them)
     const int32_t *block_table;
     const int32_t *prefix_lens;
     int table_stride, page_size, n_pages;
-    int pack, pack_shift;                // heads per query tile; a head's rows are 1 << pack_shift of the tile's
 };
 
 constexpr int PFX_SOFTMAX = 256;       // eight softmax warps: two groups of 128, one thread per query row each
-constexpr int PFX_THREADS = PFX_SOFTMAX + 128;  // + two issuing and two gathering warps
+constexpr int PFX_THREADS = PFX_SOFTMAX + 128;  // + loading, issuing and two gathering warps
+
+// A query tile: its nodes [q0, q0 + rows) of heads h .. h + pack - 1 in blocks b0 .. b0 + n_blk - 1, every block
+// with a segment of 1 << seg_shift columns in a gathered tile.
+struct QueryTile {
+    int h, q0, rows, b0, n_blk, seg_shift;
+    __device__ __forceinline__ QueryTile(const AttnArgs &a, const PrefixArgs &pa, int hk, int x) {
+        const int sub = x / pa.q_tiles;
+        h = hk * a.kv_group + sub * pa.pack;
+        q0 = (x - sub * pa.q_tiles) * umma::QM;
+        rows = min(a.n_q - q0, 1 << pa.pack_shift);
+        b0 = q0 / a.bm;
+        n_blk = (rows + a.bm - 1) / a.bm;
+        seg_shift = n_blk > 2 ? 5 : n_blk > 1 ? 6 : 7;
+    }
+};
 
 template <typename T, int D, bool PAGED>
 __global__ void __launch_bounds__(PFX_THREADS, 1)
@@ -87,177 +133,288 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     using G = Geo<D>;
     constexpr bool BF16 = !std::is_same<T, __half>::value;
     constexpr int DH = D / 64;                            // 64-column halves of a Q / K / V tile
-    constexpr int TILE = G::TILE, OFF_Q = G::OFF_Q, OFF_P = G::OFF_P, OFF_K = G::OFF_K, OFF_V = G::OFF_V,
-                  OFF_BAR = G::OFF_BAR;
+    constexpr int TILE = G::TILE;
 
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // the merge kernel may take its place
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     extern __shared__ unsigned char smem_raw[];
     const uint32_t s_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char *smem = smem_raw + (s_base - smem_u32(smem_raw));
-    const int qt = blockIdx.x, h = blockIdx.y * pa.pack, hk = h / a.kv_group;   // query tile, (first) head, K/V head
-    const int z = blockIdx.z / pa.n_runs, run = blockIdx.z - z * pa.n_runs;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int hk = blockIdx.y, z = blockIdx.z / pa.n_runs, run = blockIdx.z - z * pa.n_runs;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, qt = blockIdx.x;
     const int n_q = a.n_q;
-    // prefix rows of my batch element (paged: every batch element has its own count)
-    const int prefix = PAGED ? max(0, min(__ldg(pa.prefix_lens + z), a.prefix)) : a.prefix;
+    const int x0 = pa.pair ? blockIdx.x * 2 : blockIdx.x;
+    const bool two = pa.pair && x0 + 1 < pa.kv_tiles;     // two query tiles ...
+    const bool same = pa.q_tiles == 1;                    // ... of the same nodes, so that tree tiles are shared as well
+    const int ring = G::TILES - (two ? 2 : 1);
+    const uint32_t s_ring = s_base + (two ? 2 : 1) * TILE;
 
-    const int lane = tid & 31;
+    // barriers: Q, full / empty / go (a gathered tile may be written) of every stage, S (landed), P (written), O (all
+    // products done) of either group
+    const uint32_t bar_q = s_base + G::OFF_BAR, bar_full = bar_q + 8, bar_empty = bar_full + G::MAX_RING * 8,
+                   bar_go = bar_empty + G::MAX_RING * 8, bar_s = bar_go + G::MAX_RING * 8, bar_p = bar_s + 16, bar_o = bar_p + 32;    // P: [half][group]
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + G::OFF_BAR + 376);
 
-    // The query tile's nodes [q0, q0 + rows_t) in blocks b0 .. b0 + n_blk - 1, every block with a segment of
-    // seg columns in a gathered tile.  external(s): ancestors of block s outside it.
-    const int q0 = qt * QM, rows_t = min(n_q - q0, 1 << pa.pack_shift), b0 = q0 / a.bm, n_blk = (rows_t + a.bm - 1) / a.bm;
-    const int seg_shift = n_blk > 2 ? 5 : n_blk > 1 ? 6 : 7, seg = 1 << seg_shift;
-    const PackedLayout L = packed_layout(a.nb, a.bm, a.ma);
-    const unsigned char *blob = a.packed + size_t(z) * a.meta_stride;
-    auto external = [&](int s) -> int {
-        return s < n_blk ? min(max(__ldg(reinterpret_cast<const int32_t *>(blob + L.off_count) + b0 + s), 0), a.ma) : 0;
-    };
-    int longest = max(max(external(0), external(1)), max(external(2), external(3)));
-    // My run of column tiles [T0, T0 + nt): tp prefix tiles, the own tile, gathered tiles.  The runs are cut as if
-    // there were one gathered tile, so that no CTA waits for the counts before its first loads; nt_sure
-    // tiles of the run are there whatever they say.
-    const int tp = (prefix + KN - 1) / KN, per = (tp + 2 + pa.n_runs - 1) / pa.n_runs;
-    const int T0 = run * per, T1 = run + 1 == pa.n_runs ? 0x7fffffff : T0 + per;
-    const int nt_sure = max(0, min(T1, tp + 1) - T0);
-
-    // barriers: Q, K[2], V[2] (TMA), S[2] (S product landed in its buffer), O[2] (O += P V done, per P buffer),
-    // P[2] (all softmax threads are through with S(t) and have written P(t)).  Every barrier that is
-    // indexed by t & 1 completes once per two tiles, so a waiter can never fall two phases behind.
-    const uint32_t bar_q = s_base + OFF_BAR, bar_k = bar_q + 8, bar_v = bar_q + 24, bar_s = bar_q + 40,
-                   bar_o = bar_q + 56, bar_p = bar_q + 72, bar_go = bar_q + 88;   // go[K][2], go[V][2]: a gathered tile's stage is free
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + OFF_BAR + 144);
-
-    // Loads are issued by whole warps (8: K, 9: V).  Contiguous prefix: lane 0 requests the two
-    // boxes of a tile.  Paged: a tile is KN / page_size pages, one pair of boxes each, and lane j
-    // takes page j - it reads that page's number from the block table (my_page) a tile before
-    // it requests the boxes, so the table's latency is off the path, and a single thread is
-    // not left to issue sixteen copies one after the other.  Pages past the end of my batch
-    // element's prefix repeat its last page: finite values under columns the softmax masks.
-    const int ps = PAGED ? pa.page_size : KN, npt = KN / ps;
-    const int32_t *table = PAGED ? pa.block_table + size_t(z) * pa.table_stride : nullptr;
-    const int last_page = PAGED ? max(prefix - 1, 0) / ps : 0;
-    auto my_page = [&](int t) -> int {
-        if (!PAGED || lane >= npt) return 0;
-        return __ldg(table + min((T0 + t) * KN / ps + lane, last_page));
-    };
-    auto warp_load = [&](uint32_t dst, const CUtensorMap *map, const CUtensorMap *map_tree, uint32_t bar, uint32_t go, int t, int page) {
-        const int tile = T0 + t;
-        if (tile > tp) {                                     // gathered: the gathering warp's turn
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(go) : "memory");
-            return;
-        }
-        if (lane == 0) mbar_arrive_expect_tx(bar, TILE);
-        if (tile == tp) {                                 // the query tile's own rows
-            if (lane == 0) {
-#pragma unroll
-                for (int hf = 0; hf < DH; ++hf)
-                    tma_load_4d(dst + hf * HALF, map_tree, hf * 64, (PAGED ? 0 : a.prefix) + q0, hk, z, bar);
-            }
-            return;
-        }
-        if (PAGED) __syncwarp();                          // (contiguous: only lane 0 ever comes here)
-        if (PAGED) {
-            if (lane < npt) {
-                if (unsigned(page) >= unsigned(pa.n_pages))       // the boxes then read as zeros
-                    report(a.status, FST_DEV_INDEX_RANGE, z, tile * KN / ps + lane);
-#pragma unroll
-                for (int hf = 0; hf < DH; ++hf)
-                    tma_load_4d(dst + lane * ps * 128 + hf * HALF, map, hf * 64, 0, hk, page, bar);
-            }
-        } else if (lane == 0) {
-#pragma unroll
-            for (int hf = 0; hf < DH; ++hf) tma_load_4d(dst + hf * HALF, map, hf * 64, tile * KN, hk, z, bar);
-        }
-    };
-    auto load_q = [&]() {
-        if (lane != 0) return;
-        mbar_arrive_expect_tx(bar_q, TILE);
-        for (int i = 0; i < pa.pack; ++i)
-#pragma unroll
-            for (int hf = 0; hf < DH; ++hf)
-                tma_load_4d(s_base + OFF_Q + hf * HALF + (i << pa.pack_shift) * 128, &tm_q, hf * 64, q0, h + i, z, bar_q);
-    };
-    auto load_k = [&](int t, int page) {
-        warp_load(s_base + OFF_K + (t & 1) * TILE, &tm_k, &tm_kt, bar_k + (t & 1) * 8, bar_go + (t & 1) * 8, t, page);
-    };
-    auto load_v = [&](int t, int page) {
-        warp_load(s_base + OFF_V + (t & 1) * TILE, &tm_v, &tm_vt, bar_v + (t & 1) * 8, bar_go + 16 + (t & 1) * 8, t, page);
-    };
-    // Warp 8 sets the barriers up and sends the first loads off before the CTA-wide sync, so that
-    // they are under way while warp 9 allocates tensor memory.
     if (warp == 8) {
         if (lane == 0) {
             mbar_init(bar_q, 1);
+            for (int i = 0; i < 3 * G::MAX_RING; ++i) mbar_init(bar_full + i * 8, 1);
             for (int i = 0; i < 2; ++i) {
-                mbar_init(bar_k + i * 8, 1);
-                mbar_init(bar_v + i * 8, 1);
                 mbar_init(bar_s + i * 8, 1);
-                mbar_init(bar_o + i * 8, 1);
                 mbar_init(bar_p + i * 8, PFX_SOFTMAX / 2);
-                mbar_init(bar_go + i * 8, 1);
-                mbar_init(bar_go + 16 + i * 8, 1);
+                mbar_init(bar_p + 16 + i * 8, PFX_SOFTMAX / 2);
+                mbar_init(bar_o + i * 8, 1);
             }
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
         __syncwarp();
+    } else if (warp == 9) {                               // tensor memory: S, O of either group (and P at D 64)
+        tmem_alloc_all(smem_u32(tmem_slot));
+        fence_before_sync();
+    }
+    // Launched with programmatic stream serialisation: wait for the grid ahead before the first access to memory.
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    // the loading warp does not wait for the others: barriers are its own work, its first loads leave at once
+    if (warp == 8) asm volatile("bar.arrive 2, 384;\n" ::: "memory");
+    else asm volatile("bar.sync 2, 384;\n" ::: "memory");
+
+    // prefix rows of my batch element (paged: every batch element has its own count)
+    const int prefix = PAGED ? max(0, min(__ldg(pa.prefix_lens + z), a.prefix)) : a.prefix;
+    const PackedLayout L = packed_layout(a.nb, a.bm, a.ma);
+    const unsigned char *blob = a.packed + size_t(z) * a.meta_stride;
+    // ancestors of the tile's block s that lie outside it
+    auto external = [&](const QueryTile &qt_, int s) -> int {
+        return s < qt_.n_blk ? min(max(__ldg(reinterpret_cast<const int32_t *>(blob + L.off_count) + qt_.b0 + s), 0), a.ma) : 0;
+    };
+    auto gathered_tiles = [&](const QueryTile &qt_) -> int {
+        const int longest = max(max(external(qt_, 0), external(qt_, 1)), max(external(qt_, 2), external(qt_, 3)));
+        return (longest + (1 << qt_.seg_shift) - 1) >> qt_.seg_shift;
+    };
+    // My run of column tiles [T0, T0 + nt): tp prefix tiles, the own tile, gathered tiles.  The runs are cut as if
+    // there were one gathered tile, so that no CTA waits for the counts before its first loads; nt_sure
+    // tiles of the run are there whatever they say.
+    const int tp = (prefix + KN - 1) / KN, per = (tp + 2 + pa.n_runs - 1) / pa.n_runs;
+    const int T0 = run * per, T1 = run + 1 == pa.n_runs ? 0x3fffffff : T0 + per;
+    const int nt_sure = max(0, min(T1, tp + 1) - T0);
+    auto count_tiles = [&]() -> int {
+        int g = gathered_tiles(QueryTile(a, pa, hk, x0));
+        if (two && !same) g = max(g, gathered_tiles(QueryTile(a, pa, hk, x0 + 1)));
+        return max(0, min(T1, tp + 1 + g) - T0);
+    };
+    // Steps j = 0, 1, ...: group j & 1 and column tile T0 + (two ? j >> 1 : j).  K/V tiles (units) are shared by
+    // two steps each in the first 2 * shared steps (all of them when the two query tiles have the same nodes, else those
+    // of the prefix); every other step has a unit of its own.
+    auto n_shared = [&](int nt) -> int { return !two ? 0 : same ? nt : min(max(tp - T0, 0), nt); };
+
+    if (warp == 8) {
+        // ====== loads: unit u is items 2u (K) and 2u + 1 (V) of the ring.  Whole warps for a paged prefix, lane 0
+        // alone otherwise.  Paged: a tile is KN / page_size pages, one pair of boxes each, and lane j takes page j - it
+        // reads that page's number from the block table a tile before it requests the boxes, so the
+        // table's latency is off the path, and a single thread is not left to issue sixteen copies one after
+        // the other.  Pages past the end of my batch element's prefix repeat its last page: finite values
+        // under columns the softmax masks. ======
         if (PAGED || lane == 0) {
-            if (nt_sure > 0) load_q();
-            const int page0 = T0 < tp ? my_page(0) : 0, page1 = T0 + 1 < tp ? my_page(1) : 0;
-            if (nt_sure > 0) {
-                load_k(0, page0);
-                load_v(0, page0);
+            const int ps = PAGED ? pa.page_size : KN, npt = KN / ps;
+            const int32_t *table = PAGED ? pa.block_table + size_t(z) * pa.table_stride : nullptr;
+            const int last_page = PAGED ? max(prefix - 1, 0) / ps : 0;
+            auto my_page = [&](int tile) -> int {
+                return PAGED && lane < npt && tile < tp ? __ldg(table + min(tile * KN / ps + lane, last_page)) : 0;
+            };
+            int page = my_page(T0);
+            bool known = false, alive = true;
+            int nt = nt_sure, st = 0;
+            uint32_t use = 0;                             // fills of the current stage before this one
+            if (lane == 0) {
+                mbar_arrive_expect_tx(bar_q, (two ? 2 : 1) * TILE);
+#pragma unroll 1
+                for (int g = 0; g < (two ? 2 : 1); ++g) {
+                    const QueryTile me(a, pa, hk, x0 + g);
+#pragma unroll 1
+                    for (int i = 0; i < pa.pack; ++i)
+#pragma unroll
+                        for (int hf = 0; hf < DH; ++hf)
+                            tma_load_4d(s_base + g * TILE + hf * HALF + (i << pa.pack_shift) * 128, &tm_q, hf * 64, me.q0, me.h + i, z, bar_q);
+                }
             }
-            if (nt_sure > 1) {
-                load_k(1, page1);
-                load_v(1, page1);
+            const int shared = n_shared(nt_sure);         // the same for the final count: see above
+            int n_units = (two ? 2 : 1) * nt - shared;
+#pragma unroll 1
+            for (int u = 0; alive; ++u) {
+                if (u >= n_units) {                       // only now ask how many gathered tiles there are
+                    if (known) break;
+                    known = true;
+                    nt = count_tiles();
+                    n_units = (two ? 2 : 1) * nt - n_shared(nt);
+                    if (u >= n_units) break;
+                }
+                const int x = u - shared, g = two && !same && x >= 0 ? x & 1 : 0;
+                const int tile = T0 + (two && !same && x >= 0 ? shared + (x >> 1) : u);
+                const int here = page;
+                if (tile + 1 < tp) page = my_page(tile + 1);
+#pragma unroll 1
+                for (int kv = 0; kv < 2; ++kv) {
+                    const uint32_t dst = s_ring + st * TILE, bar = bar_full + st * 8;
+                    if (u == (two ? 1 : 2) && kv == 0 && T0 <= tp) {  // everybody's first steps ahead of the rest
+                        if (lane == 0) alive = mbar_wait(bar_full, 0, a.status, qt);
+                        if (PAGED) alive = __shfl_sync(0xffffffffu, alive, 0);
+                        if (!alive) break;
+                    }
+                    if (use > 0) {
+                        if (lane == 0) alive = mbar_wait(bar_empty + st * 8, (use - 1) & 1, a.status, qt);
+                        if (PAGED) alive = __shfl_sync(0xffffffffu, alive, 0);
+                        if (!alive) break;
+                    }
+                    if (tile > tp) {                      // gathered: the gathering warp's turn
+                        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_go + st * 8) : "memory");
+                    } else {
+                        if (lane == 0) mbar_arrive_expect_tx(bar, TILE);
+                        if (PAGED) __syncwarp();
+                        const bool pool = PAGED && tile < tp;
+                        const CUtensorMap *map = pool ? (kv ? &tm_v : &tm_k) : (kv ? &tm_vt : &tm_kt);
+                        if (pool ? lane < npt : lane == 0) {
+                            if (pool && unsigned(here) >= unsigned(pa.n_pages))   // the boxes then read as zeros
+                                report(a.status, FST_DEV_INDEX_RANGE, z, tile * KN / ps + lane);
+                            const int row = pool ? 0 : tile < tp ? tile * KN : (PAGED ? 0 : a.prefix) + QueryTile(a, pa, hk, x0 + g).q0;
+                            const uint32_t to = dst + (pool ? lane * ps * 128 : 0);
+#pragma unroll
+                            for (int hf = 0; hf < DH; ++hf) tma_load_4d(to + hf * HALF, map, hf * 64, row, hk, pool ? here : z, bar);
+                        }
+                    }
+                    if (++st == ring) {
+                        st = 0;
+                        ++use;
+                    }
+                }
             }
         }
-    }
-    if (warp == 9) {                                      // tensor memory: two S buffers and two accumulators, 128 columns each
-        umma::tmem_alloc_all(smem_u32(tmem_slot));
-    }
-    umma::fence_before_sync();
-    __syncthreads();
-    umma::fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tmem_s0 = tmem_base, tmem_o = tmem_base + 256;   // S(t) at tmem_s0 + (t & 1) * 128, O_g at tmem_o + g * 128
-
-    const int nt = max(0, min(T1, tp + 1 + ((longest + seg - 1) >> seg_shift)) - T0);
-
-    if (warp >= 10) {
+    } else if (warp == 9) {
+        // ====== products: lane 0 issues O += P V of step j, then S of step j + 2 ======
+        if (lane == 0) {
+            fence_after_sync();
+            const uint32_t tmem = *tmem_slot;
+            const int nt = count_tiles(), shared = n_shared(nt), n_steps = (two ? 2 : 1) * nt;
+            const uint32_t idesc_s = instr_desc(BF16, false, KN), idesc_pv = instr_desc(BF16, true, D);
+            // descriptors of the tiles' first 16-wide step; a step further on adds its byte offset / 16
+            const uint64_t dq = smem_desc(s_base, 16), dk = smem_desc(s_ring, 16), dv = smem_desc(s_ring, HALF);
+            int k_st = 0, v_st = 1;                       // stages of the next K and the next V tile
+            uint32_t k_ph = 0, v_ph = 0;
+            auto next = [&](int &st, uint32_t &ph) {
+                st += 2;
+                if (st >= ring) {
+                    st -= ring;
+                    ph ^= 1u;
+                }
+            };
+            bool alive = n_steps > 0 && mbar_wait(bar_q, 0, a.status, qt);
+#pragma unroll 1
+            for (int j = -2; j < n_steps && alive; ++j) {
+                const int g = j & 1;
+                const uint32_t tmem_s = tmem + g * 128, tmem_o = tmem + 256 + g * D, tmem_p = D == 128 ? tmem_s : tmem + 384 + g * 64;
+                if (j >= 0) {
+                    alive = mbar_wait(bar_full + v_st * 8, v_ph, a.status, qt) &&
+                            mbar_wait(bar_p + g * 8, (j >> 1) & 1, a.status, qt);       // the first half of P is in tensor memory
+                    if (!alive) break;
+                    fence_after_sync();
+                    // rows of a gathered tile past the lists' ends were never fetched
+                    const int tile = T0 + (two ? j >> 1 : j);
+                    uint32_t live = 0xffu;
+                    if (tile > tp) {
+                        const QueryTile me(a, pa, hk, x0 + (two && !same ? g : 0));
+                        const int slot0 = (tile - tp - 1) << me.seg_shift;
+                        live = 0u;
+#pragma unroll 1
+                        for (int s = 0; s < me.n_blk; ++s) {
+                            const int left = min(external(me, s) - slot0, 1 << me.seg_shift), steps = left > 0 ? (left + 15) >> 4 : 0;
+                            live |= ((1u << steps) - 1u) << (s << me.seg_shift >> 4);
+                        }
+                    }
+                    const uint64_t dvs = dv + uint64_t(v_st * (TILE >> 4));
+                    bool more = j > 1;
+#pragma unroll
+                    for (int ks = 0; ks < KN / 16; ++ks) {        // 16 rows per step
+                        if (ks == KN / 32) {                      // the rest of P
+                            alive = mbar_wait(bar_p + 16 + g * 8, (j >> 1) & 1, a.status, qt);
+                            fence_after_sync();
+                        }
+                        if (!((live >> ks) & 1u)) continue;
+                        mma_f16_ts(tmem_o, tmem_p + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, more);
+                        more = true;
+                    }
+                    if (j >= 2 * shared || g == 1) {      // the last to read this V
+                        mma_commit(bar_empty + v_st * 8);
+                        next(v_st, v_ph);
+                    }
+                }
+                const int j2 = j + 2;
+                if (j2 >= n_steps) {
+                    if (j >= 0) mma_commit(bar_o + g * 8);        // all of the group's products
+                    continue;
+                }
+                alive = mbar_wait(bar_full + k_st * 8, k_ph, a.status, qt);
+                if (!alive) break;
+                fence_after_sync();
+                const uint64_t dqs = dq + uint64_t((two ? g : 0) * (TILE >> 4)), dks = dk + uint64_t(k_st * (TILE >> 4));
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    const uint64_t koff = ((ks >> 2) * HALF + (ks & 3) * 32) >> 4;
+                    mma_f16(tmem_s, dqs + koff, dks + koff, idesc_s, ks > 0);
+                }
+                mma_commit(bar_s + g * 8);
+                if (j2 >= 2 * shared || g == 1) {         // the last to read this K
+                    mma_commit(bar_empty + k_st * 8);
+                    next(k_st, k_ph);
+                }
+            }
+        }
+    } else if (warp >= 10) {
         // ====== two gathering warps: ancestors' K rows (10) and V rows (11), whole steps of 16 rows at a time ======
+        const int nt = count_tiles(), shared = n_shared(nt), n_units = (two ? 2 : 1) * nt - shared;
+        const int plain = min(max(tp + 1 - T0, 0), nt), u0 = (two ? 2 : 1) * plain - min(shared, plain);
         const T *src = warp == 10 ? static_cast<const T *>(a.k) + z * a.ks_z + hk * a.ks_h
                                   : static_cast<const T *>(a.v) + z * a.vs_z + hk * a.vs_h;
         const int64_t row_stride = warp == 10 ? a.ks_n : a.vs_n;
         constexpr int CH = D / 8, RPP = 32 / CH;          // 16-byte chunks per row, rows per pass of the warp
         const int lr = lane / CH, lc = lane % CH;
         src += (PAGED ? 0 : a.prefix) * row_stride + lc * 8;
-        uint32_t turn = 0;                                // parity of the next hand-over of each stage
+        int st = (2 * u0 + (warp - 10)) % ring, turn = warp - 10;     // stage; items since the first gathered one, mod ring
+        uint32_t go_ph = 0;
+        // The first pass, while the tensor cores are at the prefix, only asks for the rows to be brought into L2: a
+        // unit's count, indices and rows are three memory latencies one after the other.
+        const bool early = u0 > 0;
 #pragma unroll 1
-        for (int t = max(0, tp + 1 - T0); t < nt; ++t) {
-            const int st = t & 1, slot0 = (T0 + t - tp - 1) << seg_shift;
+        for (int v = early ? 2 * u0 - n_units : u0; v < n_units; ++v) {
+            const bool fetch = v >= u0;
+            const int u = fetch ? v : v + n_units - u0, x = u - shared, tile = T0 + (two && !same ? shared + (x >> 1) : u);
+            const QueryTile me(a, pa, hk, x0 + (two && !same ? x & 1 : 0));
+            const int seg = 1 << me.seg_shift, slot0 = (tile - tp - 1) << me.seg_shift;
             // a step's rows: lanes 0-15 those of an even step, lanes 16-31 those of the odd one behind it
             int node[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const int row = k * 32 + lane, s = row >> seg_shift, slot = slot0 + (row & (seg - 1));
+                const int row = k * 32 + lane, s = row >> me.seg_shift, slot = slot0 + (row & (seg - 1));
                 node[k] = -1;
-                if (s < n_blk && slot < external(s)) {
-                    node[k] = __ldg(reinterpret_cast<const int32_t *>(blob + L.off_idx) + size_t(b0 + s) * a.ma + slot);
+                if (s < me.n_blk && slot < external(me, s)) {
+                    node[k] = __ldg(reinterpret_cast<const int32_t *>(blob + L.off_idx) + size_t(me.b0 + s) * a.ma + slot);
                     if (node[k] >= n_q) {
-                        report(a.status, FST_DEV_INDEX_RANGE, b0 + s, slot);
+                        report(a.status, FST_DEV_INDEX_RANGE, me.b0 + s, slot);
                         node[k] = -1;
                     }
                 }
             }
-            const uint32_t go = bar_go + (warp == 10 ? 0 : 16) + st * 8;
-            if (!__all_sync(0xffffffffu, mbar_wait(go, (turn >> st) & 1, a.status, qt))) break;
-            turn ^= 1u << st;
-            const uint32_t dst = s_base + (warp == 10 ? OFF_K : OFF_V) + st * TILE + (lc >> 3) * HALF;
+            if (!fetch) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (node[k] >= 0)
+#pragma unroll
+                        for (int hf = 0; hf < DH; ++hf)
+                            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(src - lc * 8 + node[k] * row_stride + hf * 64));
+                continue;
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_go + st * 8, go_ph, a.status, qt))) break;
+            const uint32_t dst = s_ring + st * TILE + (lc >> 3) * HALF;
 #pragma unroll 1
             for (int step = 0; step < QM / 16; ++step) {
-                const int s = step * 16 >> seg_shift;
-                if (slot0 + (step * 16 & (seg - 1)) >= external(s)) continue;      // nothing there: not used either
+                const int s = step * 16 >> me.seg_shift;
+                if (slot0 + (step * 16 & (seg - 1)) >= external(me, s)) continue;      // nothing there: not used either
                 const int mine = step < 4 ? (step < 2 ? node[0] : node[1]) : (step < 6 ? node[2] : node[3]);
 #pragma unroll
                 for (int i = 0; i < 16 / RPP; ++i) {
@@ -270,307 +427,219 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             cp_async_wait<0>();
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"((warp == 10 ? bar_k : bar_v) + st * 8) : "memory");
-        }
-    } else if (warp >= 8) {
-        // ====== two issuing warps: 8 loads K and issues S = Q K^T, 9 loads V and issues O += P V ======
-        // Lane 0 waits and issues the products; the whole warp takes part in the loads.
-        const uint32_t idesc_s = instr_desc(BF16, false, KN), idesc_pv = instr_desc(BF16, true, D);
-        bool alive = true;
-        if (warp == 8 && nt > 0 && (PAGED || lane == 0)) {     // contiguous: lane 0 alone
-            // descriptors of the tiles' first 16-wide step; a step further on adds its byte offset / 16
-            const uint64_t dq = smem_desc(s_base + OFF_Q, 16), dk = smem_desc(s_base + OFF_K, 16);
-            int page = T0 + 2 < tp ? my_page(2) : 0;      // my page of the tile to be requested next
-            if (nt_sure == 0) load_q();
-            for (int t = nt_sure; t < min(nt, 2); ++t) load_k(t, 0);
-            if (lane == 0) alive = mbar_wait(bar_q, 0, a.status, qt) && alive;
-#pragma unroll 1
-            for (int t = 0; t < nt; ++t) {                // S(t) = Q K(t)^T into S buffer t & 1
-                const int st = t & 1;
-                if (lane == 0 && alive) {
-                    // the buffer is free when the softmax warps are through with tile t-2
-                    if (t > 1) alive = mbar_wait(bar_p + st * 8, ((t >> 1) - 1) & 1, a.status, qt) && alive;
-                    alive = mbar_wait(bar_k + st * 8, (t >> 1) & 1, a.status, qt) && alive;
-                    if (alive) {
-                        umma::fence_after_sync();
-                        const uint64_t dks = dk + uint64_t(st * (TILE >> 4));
-#pragma unroll
-                        for (int ks = 0; ks < D / 16; ++ks) {
-                            const uint64_t koff = ((ks >> 2) * HALF + (ks & 3) * 32) >> 4;
-                            mma_f16(tmem_s0 + st * 128, dq + koff, dks + koff, idesc_s, ks > 0);
-                        }
-                        mma_commit(bar_s + st * 8);
-                        // K stage st is free as soon as S(t) has been formed
-                        if (t + 2 < nt) alive = mbar_wait(bar_s + st * 8, (t >> 1) & 1, a.status, qt) && alive;
-                    }
-                }
-                if (PAGED) alive = __shfl_sync(0xffffffffu, alive, 0);
-                if (!alive) break;
-                if (t + 2 < nt) {
-                    load_k(t + 2, page);
-                    if (T0 + t + 3 < tp) page = my_page(t + 3);
-                }
-            }
-        } else if (warp == 9 && nt > 0 && (PAGED || lane == 0)) {
-            const uint64_t dp = smem_desc(s_base + OFF_P, 16), dv = smem_desc(s_base + OFF_V, HALF);
-            int page = T0 + 2 < tp ? my_page(2) : 0;
-            for (int t = nt_sure; t < min(nt, 2); ++t) load_v(t, 0);
-            const int ext[4] = {external(0), external(1), external(2), external(3)};
-#pragma unroll 1
-            for (int t = 0; t < nt; ++t) {                // O_g += P(t) V(t), g = t & 1
-                const int st = t & 1;
-                if (lane == 0 && alive) {
-                    alive = mbar_wait(bar_p + st * 8, (t >> 1) & 1, a.status, qt) && alive;   // P(t) is in shared memory
-                    alive = mbar_wait(bar_v + st * 8, (t >> 1) & 1, a.status, qt) && alive;
-                    if (alive) {
-                        umma::fence_after_sync();
-                        // rows of a gathered tile past the lists' ends were never fetched
-                        uint32_t live = 0xffu;
-                        if (T0 + t > tp) {
-                            const int slot0 = (T0 + t - tp - 1) << seg_shift;
-                            live = 0u;
-#pragma unroll
-                            for (int s = 0; s < 4; ++s) {
-                                const int left = min(ext[s] - slot0, seg), steps = left > 0 ? (left + 15) >> 4 : 0;
-                                live |= ((1u << steps) - 1u) << (s << seg_shift >> 4);
-                            }
-                        }
-                        bool more = t > 1;
-                        const uint64_t dps = dp + uint64_t(st * (TILE_P >> 4)), dvs = dv + uint64_t(st * (TILE >> 4));
-#pragma unroll
-                        for (int ks = 0; ks < KN / 16; ++ks) {    // 16 prefix rows per step
-                            const uint64_t aoff = ((ks >> 2) * HALF + (ks & 3) * 32) >> 4;
-                            if (!((live >> ks) & 1u)) continue;
-                            mma_f16(tmem_o + st * 128, dps + aoff, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, more);
-                            more = true;
-                        }
-                        mma_commit(bar_o + st * 8);
-                        // V stage st is free once that product has read it
-                        if (t + 2 < nt) alive = mbar_wait(bar_o + st * 8, (t >> 1) & 1, a.status, qt) && alive;
-                    }
-                }
-                if (PAGED) alive = __shfl_sync(0xffffffffu, alive, 0);
-                if (!alive) break;
-                if (t + 2 < nt) {
-                    load_v(t + 2, page);
-                    if (T0 + t + 3 < tp) page = my_page(t + 3);
-                }
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_full + st * 8) : "memory");
+            st += 2;
+            if (st >= ring) st -= ring;
+            turn += 2;
+            if (turn >= ring) {
+                turn -= ring;
+                go_ph ^= 1u;
             }
         }
     } else {
-        // ============ softmax: two groups of 128 threads, one thread per query row, alternating tiles ============
-        // Group g owns the tiles with t & 1 == g: S buffer g, P buffer g and the accumulator O_g,
-        // with its own reference point and row sum, so the groups never wait for one another and
-        // one group's waits and tensor-memory latencies hide behind the other's exponentials.
+        // ====== softmax: two groups of 128 threads, one thread per query row ======
+        fence_after_sync();
+        const uint32_t tmem = *tmem_slot;
         const int r = tid & 127, g = tid >> 7;            // my query row (TMEM lane r) and group
-        const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
-        const uint32_t tmem_s = tmem_s0 + g * 128, tmem_og = tmem_o + g * 128;
-        unsigned char *prow = smem + OFF_P + g * TILE_P + r * 128; // my row of P buffer g
+        const uint32_t lanes = uint32_t((warp & 3) * 32) << 16;
+        const uint32_t tmem_s = tmem + g * 128 + lanes, tmem_o = tmem + 256 + g * D + lanes,
+                       tmem_p = D == 128 ? tmem_s : tmem + 384 + g * 64 + lanes;
         const float c2 = a.scale_log2;
         float m_ref = -INFINITY, l = 0.f;                 // reference point of the exponent, row sum
         bool alive = true;
-        float mx = -INFINITY, l_tile = 0.f, mu = 0.f;     // results / parameter of a sweep
 
         // my node, its block in the query tile and row in the block: where its mask words are
-        const int node = r & ((1 << pa.pack_shift) - 1), sub = node / a.bm, j = node - sub * a.bm;
-        const bool real = node < rows_t;
-        const uint32_t *own_words = reinterpret_cast<const uint32_t *>(blob + L.off_bmask) + (size_t(b0 + sub) * a.bm + j) * L.bw;
-        const uint32_t *ext_words = reinterpret_cast<const uint32_t *>(blob + L.off_emask) + (size_t(b0 + sub) * a.bm + j) * L.maw;
-        uint32_t word[4];                                 // columns of a masked tile that my row attends to
-        auto tile_words = [&](int tile) {
-            if (tile < tp) {                                 // the prefix's last, partial tile
+        const QueryTile me(a, pa, hk, x0 + (two ? g : 0));
+        const int node = r & ((1 << pa.pack_shift) - 1), sub = node / a.bm, jrow = node - sub * a.bm;
+        const bool real = node < me.rows;
+        const int seg = 1 << me.seg_shift;
+        const uint32_t *own_words = reinterpret_cast<const uint32_t *>(blob + L.off_bmask) + (size_t(me.b0 + sub) * a.bm + jrow) * L.bw;
+        const uint32_t *ext_words = reinterpret_cast<const uint32_t *>(blob + L.off_emask) + (size_t(me.b0 + sub) * a.bm + jrow) * L.maw;
+        const int nt = count_tiles(), n_steps = (two ? 2 : 1) * nt;
+
+        if (T1 > tp && real) {                            // on their way while the prefix is walked
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(own_words));
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(ext_words));
+        }
+
+        int n = 0;                                        // tiles my group has taken
+#pragma unroll 1
+        for (int j = g; j < n_steps; j += 2, ++n) {
+            const int tile = T0 + (two ? n : j);
+            const bool full = (tile + 1) * KN <= prefix;
+            uint32_t word[4];                             // columns of a masked tile that my row attends to
+            if (tile < tp) {                              // the prefix's last tile may be partial
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int left = prefix - tile * KN - i * 32;
                     word[i] = left >= 32 ? 0xffffffffu : left > 0 ? (1u << left) - 1u : 0u;
                 }
-                return;
-            }
-            const uint32_t *from = tile == tp ? own_words : ext_words;
-            const int first = tile == tp ? 0 : (tile - tp - 1) << seg_shift >> 5, have = tile == tp ? L.bw : L.maw;
-            const int at = (tile == tp ? sub * a.bm : sub << seg_shift) >> 5, n = (tile == tp ? a.bm : seg) >> 5;
+            } else {
+                const bool own = tile == tp;
+                const uint32_t *from = own ? own_words : ext_words;
+                const int first = own ? 0 : (tile - tp - 1) << me.seg_shift >> 5, have = own ? L.bw : L.maw;
+                const int at = (own ? sub * a.bm : sub << me.seg_shift) >> 5, nw = (own ? a.bm : seg) >> 5;
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                word[i] = real && i >= at && i < at + n && first + i - at < have ? __ldg(from + first + i - at) : 0u;
-        };
-
-        // One sweep over my row of S: row maximum, and (WRITE) probabilities against the reference
-        // point into my row of P plus their sum.  MASK: columns without a bit in word are -inf.  S is read 32
-        // columns at a time, the next load in flight while the current one is processed.
-        auto sweep = [&](auto write_c, auto mask_c) {
-            constexpr bool WRITE = decltype(write_c)::value, MASK = decltype(mask_c)::value;
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, l4[4] = {0.f, 0.f, 0.f, 0.f};
-            uint32_t ra[32], rb[32];
-            tmem_ld32(ra, tmem_s + lane_base);
-            tmem_ld_wait(ra);
+                for (int i = 0; i < 4; ++i)
+                    word[i] = real && i >= at && i < at + nw && first + i - at < have ? __ldg(from + first + i - at) : 0u;
+            }
+            // (S landing says that O += P V of my previous tile is done as well: it was issued before)
+            alive = mbar_wait(bar_s + g * 8, n & 1, a.status, qt) && alive;
+            fence_after_sync();
+            uint32_t s[4][32];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) tmem_ld32(s[c], tmem_s + c * 32);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) tmem_ld_wait(s[c]);
+            if (!full) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if ((word[c] & (1u << i)) == 0u) s[c][i] = 0xff800000u;      // -inf
+            }
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};             // four independent chains
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; i += 2)
+                    mx4[(i >> 1) & 3] = fmaxf(mx4[(i >> 1) & 3], fmaxf(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])));
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            // the reference moves when a row has outgrown it by more than 2^8 (always on the first live tile)
+            const bool up = (mx - m_ref) * c2 > 8.f;      // true from -inf
+            if (__any_sync(0xffffffffu, up)) {
+                if (n > 0) {                              // rescale my row of O in tensor memory
+                    const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < D; c0 += 8) {
+                        uint32_t o[8];
+                        tmem_ld8(o, tmem_o + c0);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st8(tmem_o + c0, o);
+                    }
+                    l *= alpha;
+                }
+                if (up) m_ref = mx;
+            }
+            const float mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
+            const uint64_t scale2 = pair(c2, c2), shift2 = pair(-mu, -mu);
+            uint64_t l2[2] = {0, 0};
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                uint32_t (&cur)[32] = (c & 1) ? rb : ra;
-                uint32_t (&nxt)[32] = (c & 1) ? ra : rb;
-                if (c < 3) tmem_ld32(nxt, tmem_s + lane_base + (c + 1) * 32);
                 uint32_t packed[16];
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) {
-                    float s0 = __uint_as_float(cur[i]), s1 = __uint_as_float(cur[i + 1]);
-                    if (MASK) {
-                        s0 = (word[c] & (1u << i)) != 0u ? s0 : -INFINITY;
-                        s1 = (word[c] & (2u << i)) != 0u ? s1 : -INFINITY;
-                    }
-                    mx4[(i >> 1) & 3] = fmaxf(mx4[(i >> 1) & 3], fmaxf(s0, s1));   // four independent chains
-                    if (WRITE) {
-                        const float p0 = fast_exp2(fmaf(s0, c2, -mu)), p1 = fast_exp2(fmaf(s1, c2, -mu));
-                        l4[(i >> 1) & 3] += p0 + p1;
-                        packed[i >> 1] = MT::pack(p0, p1);
-                    }
+                    const uint64_t x = fma2(pair(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), scale2, shift2);
+                    float p0, p1;
+                    unpair(x, p0, p1);
+                    p0 = fast_exp2(p0);
+                    p1 = fast_exp2(p1);
+                    l2[(i >> 1) & 1] = add2(l2[(i >> 1) & 1], pair(p0, p1));
+                    packed[i >> 1] = MT::pack(p0, p1);
                 }
-                if (WRITE) {
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {      // four 16-byte chunks of my row, swizzled
-                        const int chunk = c * 4 + q4;
-                        *reinterpret_cast<uint4 *>(prow + (chunk >> 3) * HALF + (((chunk & 7) ^ (r & 7)) << 4)) =
-                            make_uint4(packed[q4 * 4], packed[q4 * 4 + 1], packed[q4 * 4 + 2], packed[q4 * 4 + 3]);
-                    }
+                tmem_st16(tmem_p + c * 16, packed);
+                if (c & 1) {                              // half of P: its products may begin
+                    tmem_st_wait();
+                    fence_before_sync();
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_p + (c >> 1) * 16 + g * 8) : "memory");
                 }
-                if (c < 3) tmem_ld_wait(nxt);
             }
-            mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            l_tile = (l4[0] + l4[1]) + (l4[2] + l4[3]);
-        };
-        const std::true_type yes{};
-        const std::false_type no{};
+            float la, lb;
+            unpair(add2(l2[0], l2[1]), la, lb);
+            l += la + lb;
+        }
 
-        int n_mine = 0;                                   // tiles my group has taken
+        // ---- rows of O, unnormalised, and their (exponent, sum) into shared memory, once every product of either
+        // group is done with the operands there; 16-byte chunks swizzled.  Two groups with one query tile
+        // merge here: either reads both accumulators, for every other 32 columns.
+        if (n > 0) alive = mbar_wait(bar_o + g * 8, 0, a.status, qt) && alive;
+        fence_after_sync();
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        float2 *stats = reinterpret_cast<float2 *>(smem + G::OFF_STATS);
+        stats[tid] = make_float2(n > 0 && alive && m_ref != -INFINITY ? m_ref * c2 : -INFINITY, l);
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        const float2 st0 = stats[two ? tid : r], st1 = two ? make_float2(-INFINITY, 0.f) : stats[QM + r];
+        const float mu = fmaxf(st0.x, st1.x);
+        const float w0 = st0.x == -INFINITY ? 0.f : fast_exp2(st0.x - mu), w1 = st1.x == -INFINITY ? 0.f : fast_exp2(st1.x - mu);
+        if (two || g == 0) stats[2 * QM + tid] = make_float2(mu, st0.y * w0 + st1.y * w1);
+        float *srow = reinterpret_cast<float *>(smem) + (two ? tid : r) * D;
+        const uint32_t tmem_first = two ? tmem_o : tmem + 256 + lanes;
 #pragma unroll 1
-        for (int t = g; t < nt; t += 2, ++n_mine) {
-            const bool full = (T0 + t + 1) * KN <= prefix;
-            if (!full) tile_words(T0 + t);
-            alive = mbar_wait(bar_s + g * 8, n_mine & 1, a.status, qt) && alive;
-            // P buffer g and O_g belong to the tensor core until O_g += P V of my previous tile is done
-            if (n_mine > 0) alive = mbar_wait(bar_o + g * 8, (n_mine - 1) & 1, a.status, qt) && alive;
-            umma::fence_after_sync();
-
-            // Probabilities are formed against the current reference point while the row maximum
-            // is tracked (one pass over S).  Only if a row of my warp has outgrown its reference
-            // by more than 2^8 (always on the first tile) is the reference moved, O_g rescaled,
-            // and the tile done again.
-            if (n_mine == 0) {
-                // first tile: the maximum of the first 32 columns is reference enough to start
-                // with (should a later column outgrow it by 2^8 the tile is redone below)
-                uint32_t f[32];
-                tmem_ld32(f, tmem_s + lane_base);
-                tmem_ld_wait(f);
-                mx = -INFINITY;
+        for (int c0 = two ? 0 : g * 32; c0 < D; c0 += two ? 32 : 64) {
+            uint32_t o[32], o1[32];
+            tmem_ld32(o, tmem_first + c0);
+            if (!two) tmem_ld32(o1, tmem_first + D + c0);
+            tmem_ld_wait(o);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = w0 == 0.f ? 0u : __float_as_uint(__uint_as_float(o[i]) * w0);   // without a column: never written
+            if (!two) {
+                tmem_ld_wait(o1);
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
-                    if (full || (word[0] & (1u << i)) != 0u) mx = fmaxf(mx, __uint_as_float(f[i]));
+                    if (w1 != 0.f) o[i] = __float_as_uint(fmaf(__uint_as_float(o1[i]), w1, __uint_as_float(o[i])));
             }
-#pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
-                if (pass == 1 || n_mine == 0) {
-                    const bool up = (mx - m_ref) * c2 > 8.f;          // true from -inf
-                    if (n_mine > 0) {                     // rescale my row of O_g in tensor memory
-                        const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
-#pragma unroll 1
-                        for (int c0 = 0; c0 < D; c0 += 32) {
-                            uint32_t o[32];
-                            tmem_ld32(o, tmem_og + lane_base + c0);
-                            tmem_ld_wait(o);
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                            tmem_st32(tmem_og + lane_base + c0, o);
-                        }
-                        l *= alpha;
-                    }
-                    if (up) m_ref = mx;
-                    mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
-                }
-                if (full) sweep(yes, no);
-                else sweep(yes, yes);
-                if (!__any_sync(0xffffffffu, (mx - m_ref) * c2 > 8.f)) break;
-            }
-            l += l_tile;
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // P visible to the tensor core
-            umma::fence_before_sync();
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_p + g * 8) : "memory");
-        }
-
-        // ---- epilogue: merge the two groups' results; O / l and the log-sum-exp of every row go to
-        // this run's partial-result slot.  Each thread puts its unnormalised row of O_g into shared
-        // memory (the K and V stages, free once every product is done; the (exponent, sum) pairs
-        // go to the P buffers); then each warp merges and writes whole rows, 512 contiguous bytes
-        // per store instruction.
-        if (n_mine > 0) alive = mbar_wait(bar_o + g * 8, (n_mine - 1) & 1, a.status, qt) && alive;
-        umma::fence_after_sync();
-        asm volatile("bar.sync 1, 256;\n" ::: "memory");  // every product of either group is done
-        float2 *stats = reinterpret_cast<float2 *>(smem + OFF_P);            // [2][128]
-        float *stage = reinterpret_cast<float *>(smem + OFF_K);              // [2][128][128], 16-byte chunks swizzled
-        const float my_mu = (n_mine > 0 && alive && m_ref != -INFINITY) ? m_ref * c2 : -INFINITY;
-        stats[g * 128 + r] = make_float2(my_mu, l);
-        {
-            float *srow = stage + (g * 128 + r) * D;
-#pragma unroll 1
-            for (int c0 = 0; c0 < D; c0 += 32) {
-                uint32_t o[32];
-                if (n_mine > 0) {
-                    tmem_ld32(o, tmem_og + lane_base + c0);
-                    tmem_ld_wait(o);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = 0u;
-                }
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    const int chunk = (c0 + i) >> 2;
-                    *reinterpret_cast<uint4 *>(srow + ((chunk ^ (r & 7)) << 2)) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-                }
-            }
-        }
-        asm volatile("bar.sync 1, 256;\n" ::: "memory");
-        const size_t slot = size_t(run);
-        const bool whole = pa.n_runs == 1;                // this is the output already
-        constexpr int RPW = QM / (PFX_SOFTMAX / 32);      // 16 rows per warp: rows warp * 16 ..
-        // lanes 0..15 work out the two groups' weights for one row each; they are handed round by shuffle
-        float f0 = 0.f, f1 = 0.f;
-        {
-            const int rr = warp * RPW + (lane & (RPW - 1));
-            const float2 s0 = stats[rr], s1 = stats[128 + rr];
-            const float mu_all = fmaxf(s0.x, s1.x);
-            const float w0 = s0.x == -INFINITY ? 0.f : fast_exp2(s0.x - mu_all);
-            const float w1 = s1.x == -INFINITY ? 0.f : fast_exp2(s1.x - mu_all);
-            const float l_all = s0.y * w0 + s1.y * w1;
-            const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-            f0 = w0 * inv;
-            f1 = w1 * inv;
-            const int grow = qt * QM + (rr & ((1 << pa.pack_shift) - 1)), hr = h + (rr >> pa.pack_shift);
-            if (lane < RPW && grow < n_q && (!whole || a.lse != nullptr))
-                (whole ? a.lse : a.part_lse)[((slot * a.Z + z) * a.H + hr) * n_q + grow] =
-                    l_all > 0.f ? mu_all + log2f(l_all) : -INFINITY;
-        }
-#pragma unroll 4
-        for (int i = 0; i < RPW; ++i) {
-            const int rr = warp * RPW + i, grow = qt * QM + (rr & ((1 << pa.pack_shift) - 1)), hr = h + (rr >> pa.pack_shift);
-            const float g0 = __shfl_sync(0xffffffffu, f0, i), g1 = __shfl_sync(0xffffffffu, f1, i);
-            if (lane >= D / 4) continue;                  // a row is D / 4 chunks of four floats
-            const int sw = (lane ^ (rr & 7)) << 2;
-            const float4 v0 = *reinterpret_cast<const float4 *>(stage + rr * D + sw);
-            const float4 v1 = *reinterpret_cast<const float4 *>(stage + (128 + rr) * D + sw);
-            if (grow >= n_q) continue;
-            if (whole) {
-                T *to = static_cast<T *>(a.o) + z * a.os_z + hr * a.os_h + grow * a.os_n;
-                reinterpret_cast<uint2 *>(to)[lane] = make_uint2(MT::pack(v0.x * g0 + v1.x * g1, v0.y * g0 + v1.y * g1),
-                                                                 MT::pack(v0.z * g0 + v1.z * g1, v0.w * g0 + v1.w * g1));
-            } else {
-                const size_t prow_g = ((slot * a.Z + z) * a.H + hr) * n_q + grow;
-                reinterpret_cast<float4 *>(a.part_o + prow_g * D)[lane] =
-                    make_float4(v0.x * g0 + v1.x * g1, v0.y * g0 + v1.y * g1, v0.z * g0 + v1.z * g1, v0.w * g0 + v1.w * g1);
+            for (int i = 0; i < 32; i += 4) {
+                const int chunk = (c0 + i) >> 2;
+                *reinterpret_cast<uint4 *>(srow + ((chunk ^ (r & 7)) << 2)) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
             }
         }
     }
 
-    umma::fence_before_sync();
-    __syncthreads();
-    if (warp == 9) umma::tmem_free_all(tmem_base);
+    // ---- merge: a row lies in every CTA of the cluster.  Every CTA takes an equal share of the rows.  Shared memory of
+    // another CTA reads at some 12 bytes per cycle, which is why prefix_plan prefers few runs.
+    const QueryTile tile_a(a, pa, hk, x0), tile_b(a, pa, hk, two ? x0 + 1 : x0);
+    fence_before_sync();
+    __syncwarp();
+    if (pa.n_runs > 1) cluster_sync();
+    else __syncthreads();
+    if (warp == 9) {
+        fence_after_sync();
+        tmem_free_all(*tmem_slot);
+    }
+    const int rows_all = two ? 2 * QM : QM, share = (rows_all + pa.n_runs - 1) / pa.n_runs;
+    const int row_lo = run * share, row_hi = min(rows_all, row_lo + share);
+    // a lane has a 64-byte piece of a row: four chunks of 16 bytes, LPR lanes a row
+    constexpr int LPR = D / 16, RPW = 32 / LPR;
+    const int c = lane % LPR;
+#pragma unroll 1
+    for (int row = row_lo + warp * RPW + lane / LPR; row < row_hi; row += PFX_THREADS / 32 * RPW) {
+        float4 acc[4] = {};
+        float mu = -INFINITY, l = 0.f;
+#pragma unroll 2
+        for (int s = 0; s < pa.n_runs; ++s) {
+            const uint32_t base = cluster_addr(s_base, s);
+            const float2 st = cluster_ld2(base + G::OFF_STATS + (2 * QM + row) * 8);
+            float4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = cluster_ld4(base + row * D * 4 + (((k * LPR + c) ^ (row & 7)) << 4));
+            const float top = fmaxf(mu, st.x), to = top == -INFINITY ? 0.f : top;
+            const float w_old = fast_exp2(mu - to), w = fast_exp2(st.x - to);
+            mu = top;
+            l = l * w_old + st.y * w;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                acc[k].x = acc[k].x * w_old + v[k].x * w;
+                acc[k].y = acc[k].y * w_old + v[k].y * w;
+                acc[k].z = acc[k].z * w_old + v[k].z * w;
+                acc[k].w = acc[k].w * w_old + v[k].w * w;
+            }
+        }
+        const bool first = row < QM;
+        const int node = row & ((1 << pa.pack_shift) - 1), gr = (first ? tile_a.q0 : tile_b.q0) + node;
+        const int h = (first ? tile_a.h : tile_b.h) + ((row & 127) >> pa.pack_shift);
+        if (node >= (first ? tile_a.rows : tile_b.rows)) continue;
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        uint2 *to = reinterpret_cast<uint2 *>(static_cast<T *>(a.o) + z * a.os_z + h * a.os_h + gr * a.os_n);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            to[k * LPR + c] = make_uint2(MT::pack(acc[k].x * inv, acc[k].y * inv), MT::pack(acc[k].z * inv, acc[k].w * inv));
+        if (a.lse != nullptr && c == 0) a.lse[(size_t(z) * a.H + h) * n_q + gr] = l > 0.f ? mu + log2f(l) : -INFINITY;
+    }
+    if (pa.n_runs == 1) return;
+    __syncwarp();
+    cluster_sync();                                       // nobody leaves while its rows are being read
 }
 
 // rank-4 map with 64-column x 128-row boxes (kept in the calling thread's table of maps)
@@ -617,7 +686,17 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
     });
     if (ce != cudaSuccess) return ce;
     if ((long long)a.Z * n_runs > 65535) return cudaErrorInvalidValue;
-    PrefixArgs pa{n_runs, nullptr, nullptr, 0, 0, 0, pack, 7};
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return cudaErrorInvalidDevice;
+    const PrefixPlan plan = prefix_plan(a.Z, a.H, H_kv, a.n_q, a.prefix, sms, n_runs, PAGED ? pg->page_size : 128);
+    PrefixArgs pa = {};
+    pa.n_runs = plan.runs;
+    pa.pair = plan.pair;
+    pa.q_tiles = (a.n_q + umma::QM - 1) / umma::QM;
+    pa.kv_tiles = a.kv_group / pack * pa.q_tiles;
+    pa.pack = pack;
+    pa.pack_shift = 7;
     for (int p = pack; p > 1; p /= 2) --pa.pack_shift;
     if (PAGED) {
         pa.block_table = pg->block_table;
@@ -626,9 +705,20 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
         pa.page_size = pg->page_size;
         pa.n_pages = pg->n_pages;
     }
-    dim3 grid((a.n_q + umma::QM - 1) / umma::QM, a.H / pack, a.Z * n_runs);
-    prefix_umma_kernel<T, D, PAGED><<<grid, PFX_THREADS, umma::Geo<D>::SMEM_BYTES, stream>>>(a, pa, tq, tk, tv, tkt, tvt);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pa.pair ? (pa.kv_tiles + 1) / 2 : pa.kv_tiles, H_kv, a.Z * pa.n_runs);
+    cfg.blockDim = dim3(PFX_THREADS);
+    cfg.dynamicSmemBytes = umma::Geo<D>::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = unsigned(pa.n_runs);
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, prefix_umma_kernel<T, D, PAGED>, a, pa, tq, tk, tv, tkt, tvt);
 }
 
 template <bool PAGED>
@@ -643,8 +733,7 @@ static cudaError_t launch_prefix_any(const AttnArgs &a, const PagedArgs *pg, int
     return cudaErrorNotSupported;
 }
 
-// The whole call - prefix and tree - in n_runs runs of column tiles: the output when there is one, else partial
-// results 0 .. n_runs - 1.
+// The whole call - prefix and tree - in n_runs runs of column tiles (at most kMaxPrefixRuns).
 cudaError_t launch_prefix_umma(const AttnArgs &a, int dtype, int n_runs, cudaStream_t stream) {
     return launch_prefix_any<false>(a, nullptr, dtype, n_runs, stream);
 }
