@@ -206,13 +206,14 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     auto n_shared = [&](int nt) -> int { return !two ? 0 : same ? nt : min(max(tp - T0, 0), nt); };
 
     if (warp == 8) {
-        // ====== loads: unit u is items 2u (K) and 2u + 1 (V) of the ring.  Whole warps for a paged prefix, lane 0
-        // alone otherwise.  Paged: a tile is KN / page_size pages, one pair of boxes each, and lane j takes page j - it
+        // ====== loads: unit u is items 2u (K) and 2u + 1 (V) of the ring.  The whole warp for a paged prefix, one lane
+        // otherwise.  Paged: a tile is KN / page_size pages, one pair of boxes each, and lane j takes page j - it
         // reads that page's number from the block table a tile before it requests the boxes, so the
         // table's latency is off the path, and a single thread is not left to issue sixteen copies one after
         // the other.  Pages past the end of my batch element's prefix repeat its last page: finite values
         // under columns the softmax masks. ======
-        if (PAGED || lane == 0) {
+        const bool lead = elect_one();
+        if (PAGED || lead) {
             const int ps = PAGED ? pa.page_size : KN, npt = KN / ps;
             const int32_t *table = PAGED ? pa.block_table + size_t(z) * pa.table_stride : nullptr;
             const int last_page = PAGED ? max(prefix - 1, 0) / ps : 0;
@@ -223,7 +224,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             bool known = false, alive = true;
             int nt = nt_sure, st = 0;
             uint32_t use = 0;                             // fills of the current stage before this one
-            if (lane == 0) {
+            if (lead) {
                 mbar_arrive_expect_tx(bar_q, (two ? 2 : 1) * TILE);
 #pragma unroll 1
                 for (int g = 0; g < (two ? 2 : 1); ++g) {
@@ -254,23 +255,23 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                 for (int kv = 0; kv < 2; ++kv) {
                     const uint32_t dst = s_ring + st * TILE, bar = bar_full + st * 8;
                     if (u == (two ? 1 : 2) && kv == 0 && T0 <= tp) {  // everybody's first steps ahead of the rest
-                        if (lane == 0) alive = mbar_wait(bar_full, 0, a.status, qt);
-                        if (PAGED) alive = __shfl_sync(0xffffffffu, alive, 0);
+                        if (lead) alive = mbar_wait(bar_full, 0, a.status, qt);
+                        if (PAGED) alive = __all_sync(0xffffffffu, alive);
                         if (!alive) break;
                     }
                     if (use > 0) {
-                        if (lane == 0) alive = mbar_wait(bar_empty + st * 8, (use - 1) & 1, a.status, qt);
-                        if (PAGED) alive = __shfl_sync(0xffffffffu, alive, 0);
+                        if (lead) alive = mbar_wait(bar_empty + st * 8, (use - 1) & 1, a.status, qt);
+                        if (PAGED) alive = __all_sync(0xffffffffu, alive);
                         if (!alive) break;
                     }
                     if (tile > tp) {                      // gathered: the gathering warp's turn
-                        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_go + st * 8) : "memory");
+                        if (lead) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_go + st * 8) : "memory");
                     } else {
-                        if (lane == 0) mbar_arrive_expect_tx(bar, TILE);
+                        if (lead) mbar_arrive_expect_tx(bar, TILE);
                         if (PAGED) __syncwarp();
                         const bool pool = PAGED && tile < tp;
                         const CUtensorMap *map = pool ? (kv ? &tm_v : &tm_k) : (kv ? &tm_vt : &tm_kt);
-                        if (pool ? lane < npt : lane == 0) {
+                        if (pool ? lane < npt : lead) {
                             if (pool && unsigned(here) >= unsigned(pa.n_pages))   // the boxes then read as zeros
                                 report(a.status, FST_DEV_INDEX_RANGE, z, tile * KN / ps + lane);
                             const int row = pool ? 0 : tile < tp ? tile * KN : (PAGED ? 0 : a.prefix) + QueryTile(a, pa, hk, x0 + g).q0;
@@ -287,8 +288,8 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             }
         }
     } else if (warp == 9) {
-        // ====== products: lane 0 issues O += P V of step j, then S of step j + 2 ======
-        if (lane == 0) {
+        // ====== products: one lane issues O += P V of step j, then S of step j + 2 ======
+        if (elect_one()) {
             fence_after_sync();
             const uint32_t tmem = *tmem_slot;
             const int nt = count_tiles(), shared = n_shared(nt), n_steps = (two ? 2 : 1) * nt;

@@ -22,7 +22,7 @@
 // Sixteen warps.  Warps 0-3 and 4-7 are two softmax groups: group g takes the CTA's items g, g + 2, ... and
 // owns an S/P buffer and an accumulator (TMEM: 2 x 128 columns each), so that one group's latencies hide
 // behind the other's work (one group with a tile of lookahead in the products was bound by its own
-// instruction stream: 7000 cycles per 128 rows at D 64).  Lane 0 of warp 8 + g issues the products of
+// instruction stream: 7000 cycles per 128 rows at D 64).  One lane of warp 8 + g issues the products of
 // group g.  Warp 10 loads Q and the own tiles, warps 11-14 gather (cp.async, 16 bytes a lane; TMA's gather4
 // fills the same layout but takes the engine about 100 cycles for its four rows, 6500 per item of 64
 // trees against the 5700 that its HBM bytes take), warp 15 stores O.  All tiles share one pool of 128-row
@@ -303,7 +303,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             for (int kv = 0; kv < 3; ++kv) {              // own K, own V, Q
                 const int b = take();
                 if (!alive) break;
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint32_t bar = kv < 2 ? full_of(g, pos + kv) : q_of(n);
                     if (kv < 2) {
                         buf_of(g, pos + kv) = (unsigned char)b;
@@ -326,7 +326,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             for (int at = pos + 2; alive && at < pos + 2 * tiles - int(narrow); ++at) {
                 const int b = take();
                 if (!alive) break;
-                if (lane == 0) {
+                if (elect_one()) {
                     buf_of(g, at) = (unsigned char)b;
                     arrive(bar_go + (turn % TURNS) * 8);
                 }
@@ -447,7 +447,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 for (int st = 0; st < 2; ++st) {
                     const int row0 = st ? cur.row_b : cur.row_a;
                     if (row0 < 0) break;
-#pragma unroll 4
+#pragma unroll 2
                     for (int i = 0; i < 16 / RPP; ++i) {
                         const int rr = i * RPP + lr, row = row0 + rr;
                         const int nd = __shfl_sync(0xffffffffu, node, st * 16 + rr);
@@ -467,7 +467,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
     } else if (warp == 8 || warp == 9) {
         // ================================ products ================================
         const int g = warp - 8;
-        if (lane == 0) {
+        if (elect_one()) {
             const uint64_t dk = smem_desc(s_base, 16), dv = smem_desc(s_base, HALF), dv_narrow = smem_desc(s_base + TILE / 2, HALF / 2);
             const uint32_t idesc_pv = instr_desc(BF16, true, D), s_col = tmem_base + g * 128, o_col = s_col + 256;
             bool alive = true;
@@ -512,12 +512,12 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                     const uint64_t dvs = (narrow ? dv_narrow : dv) + uint64_t(b * (TILE >> 4));
                     fence_after_sync();
                     bool more = t > 0;
-#pragma unroll
-                    for (int ks = 0; ks < ROWS / 16; ++ks)
-                        if ((steps >> ks) & 1u) {
-                            mma_f16_ts(o_col, s_col + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, more);
-                            more = true;
-                        }
+#pragma unroll 1
+                    for (uint32_t rest = steps; rest != 0u; rest &= rest - 1) {
+                        const int ks = __ffs(rest) - 1;
+                        mma_f16_ts(o_col, s_col + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, more);
+                        more = true;
+                    }
                     mma_commit(bar_empty + b * 8);
                     if (t + 1 == tiles) mma_commit(bar_o + g * 8);
                 }
@@ -525,7 +525,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
         }
     } else if (warp == 15) {
         // ================================ O to global memory ================================
-        if (lane == 0) {
+        if (elect_one()) {
             Where w = first;
             int n = 0;
             if (a.meta_stable) asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -604,95 +604,69 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 if (!alive) break;
                 fence_after_sync();
 
-                // My live words, two at a time: the first pair's scores stay in registers between the two
-                // passes, further pairs (BM 128 only) are read again.
+                // My live words, one at a time.
                 uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
 #pragma unroll
                 for (int i = 0; i < NW; ++i) live |= uint32_t(__any_sync(0xffffffffu, word[i] != 0u)) << i;
-                uint32_t s[2][32];
-                uint32_t wi[2];                           // the pair's word numbers; NW: none
-                auto pair_of = [&](uint32_t &rest) {
+                float sum[2] = {0.f, 0.f}, mu = 0.f, mx = -INFINITY;
+                // First round over the words: the row's maximum, then the reference point.  Second round (or at once,
+                // when there was only one word): probabilities, over S - word i of P covers columns 16 i .. of S,
+                // below the words still to be read; words nobody uses are zeros.  One loop and one word to a
+                // turn: code that runs once per tile and does not stay in the instruction cache costs more than it saves.
+                bool second = false;
+#pragma unroll 1
+                for (uint32_t rest = live; rest != 0u;) {
+                    const int wi = __ffs(rest) - 1;
+                    rest &= rest - 1;
+                    uint32_t s[32];
+                    tmem_ld32(s, tmem_my + wi * 32);
+                    uint32_t w = word[0];
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        wi[k] = rest != 0u ? uint32_t(__ffs(rest) - 1) : uint32_t(NW);
-                        rest &= rest - 1;
+                    for (int i = 1; i < NW; ++i) w = wi == i ? word[i] : w;
+                    tmem_ld_wait(s);
+                    float m2[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+                    for (int c = 0; c < 32; c += 2) {
+                        s[c] = (w & (1u << c)) != 0u ? s[c] : 0xff800000u;
+                        s[c + 1] = (w & (2u << c)) != 0u ? s[c + 1] : 0xff800000u;
+                        m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[c]), __uint_as_float(s[c + 1])));
                     }
-                };
-                auto load_pair = [&]() -> float {         // masked scores of the pair; their maximum
-                    float mx = -INFINITY;
-#pragma unroll
-                    for (int k = 0; k < (NW > 1 ? 2 : 1); ++k)
-                        if (wi[k] < NW) tmem_ld32(s[k], tmem_my + wi[k] * 32);
-#pragma unroll
-                    for (int k = 0; k < (NW > 1 ? 2 : 1); ++k) {
-                        if (wi[k] >= NW) continue;
-                        uint32_t w = word[0];
-#pragma unroll
-                        for (int i = 1; i < NW; ++i) w = wi[k] == i ? word[i] : w;
-                        tmem_ld_wait(s[k]);
-                        float m2[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-                        for (int c = 0; c < 32; c += 2) {
-                            s[k][c] = (w & (1u << c)) != 0u ? s[k][c] : 0xff800000u;
-                            s[k][c + 1] = (w & (2u << c)) != 0u ? s[k][c + 1] : 0xff800000u;
-                            m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[k][c]), __uint_as_float(s[k][c + 1])));
-                        }
+                    if (!second) {
                         mx = fmaxf(mx, fmaxf(m2[0], m2[1]));
-                    }
-                    return mx;
-                };
-                // pass 1: the row's maximum
-                float mx = -INFINITY;
+                        if (rest != 0u) continue;
+                        const bool up = (mx - m_ref) * c2 > 8.f;      // true from -inf
+                        if (__any_sync(0xffffffffu, up)) {
+                            if (t > 0) {                  // rescale my row of O
+                                const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
 #pragma unroll 1
-                for (uint32_t rest = live; rest != 0u;) {
-                    pair_of(rest);
-                    mx = fmaxf(mx, load_pair());
-                }
-                const bool up = (mx - m_ref) * c2 > 8.f;  // true from -inf
-                if (__any_sync(0xffffffffu, up)) {
-                    if (t > 0) {                          // rescale my row of O
-                        const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
-#pragma unroll 1
-                        for (int c0 = 0; c0 < D; c0 += 8) {
-                            uint32_t o[8];
-                            tmem_ld8(o, tmem_o + c0);
+                                for (int c0 = 0; c0 < D; c0 += 8) {
+                                    uint32_t o[8];
+                                    tmem_ld8(o, tmem_o + c0);
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                            tmem_st8(tmem_o + c0, o);
+                                    for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                                    tmem_st8(tmem_o + c0, o);
+                                }
+                                l *= alpha;
+                            }
+                            if (up) m_ref = mx;
                         }
-                        l *= alpha;
-                    }
-                    if (up) m_ref = mx;
-                }
-                // pass 2: probabilities, over S: word i of P covers columns 16 i .. of S, below the words still to
-                // be read; words nobody uses are zeros
-                const float mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
-                float sum[2] = {0.f, 0.f};
-                auto write_pair = [&]() {
-#pragma unroll
-                    for (int k = 0; k < (NW > 1 ? 2 : 1); ++k) {
-                        if (wi[k] >= NW) continue;
-                        uint32_t pk[16];
-#pragma unroll
-                        for (int c = 0; c < 32; c += 2) {
-                            const float p0 = fast_exp2(fmaf(__uint_as_float(s[k][c]), c2, -mu));
-                            const float p1 = fast_exp2(fmaf(__uint_as_float(s[k][c + 1]), c2, -mu));
-                            sum[0] += p0;
-                            sum[1] += p1;
-                            pk[c >> 1] = MT::pack(p0, p1);
+                        mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
+                        second = true;
+                        if ((live & (live - 1)) != 0u) {  // several words: once more from the first
+                            rest = live;
+                            continue;
                         }
-                        tmem_st16(tmem_s + (sub * segw + wi[k]) * 16, pk);
                     }
-                };
-                bool held = __popc(live) <= 2;
-                for (uint32_t rest = live; rest != 0u;) {
-                    if (!held) {
-                        pair_of(rest);
-                        (void)load_pair();
-                    } else {
-                        rest = 0u;
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int c = 0; c < 32; c += 2) {
+                        const float p0 = fast_exp2(fmaf(__uint_as_float(s[c]), c2, -mu));
+                        const float p1 = fast_exp2(fmaf(__uint_as_float(s[c + 1]), c2, -mu));
+                        sum[0] += p0;
+                        sum[1] += p1;
+                        pk[c >> 1] = MT::pack(p0, p1);
                     }
-                    write_pair();
+                    tmem_st16(tmem_s + (sub * segw + wi) * 16, pk);
                 }
                 l += sum[0] + sum[1];
                 {
