@@ -53,14 +53,14 @@ inline PrefixPlan prefix_plan(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, i
 
 // When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, six kinds of trees, from 64
 // items (128 query rows of one head) up, ratios of old to new time:
-//   D 128, block_m 128   1.15 - 1.46 from 256 items, up to 1.95 at 4096; 0.73 - 0.98 below 100
-//   D 128, block_m 64    1.06 - 1.28 from 256 items where the ancestor lists run to several tiles (bound of
-//                        four blocks), 1.05 - 1.25 from 1024 items with a bound of two; 0.93 - 1.04 with one
-//   D 128, block_m 32    1.38 - 1.74 at 256 items, 0.98 - 1.09 above; 0.82 - 0.99 with long lists
-//   D 64, block_m 128    1.16 - 1.32 from 288 to 1248 items, 0.95 - 1.29 above
-//   D 64, block_m 64     1.08 - 1.40 from 1024 items with a bound of two blocks or more, 1.05 - 1.14 from
-//                        4096 with one
-//   D 64, block_m 32     1.12 - 1.33 from 4096 items; 0.53 - 0.88 with long lists
+//   D 128, block_m 128   1.27 - 1.72 from 256 items, up to 2.40 at 5184; 0.82 - 1.12 below 100
+//   D 128, block_m 64    1.04 - 1.32 from 256 items with an ancestor bound of two blocks or more, 1.00 - 1.21
+//                        from 1024 with one (0.99 - 1.13 at 256); 0.63 - 0.75 below 100
+//   D 128, block_m 32    1.19 - 1.83 at 256 items, 1.08 - 1.26 above; 0.89 - 0.97 above with long lists
+//   D 64, block_m 128    1.01 - 1.36 at 256 items, 1.12 - 1.65 above; 0.69 - 0.90 below 100
+//   D 64, block_m 64     1.03 - 1.31 from 4096 items, 1.04 - 1.16 from 1024 with a bound of two or three blocks;
+//                        0.92 - 1.09 otherwise, 0.56 - 0.95 up to 300
+//   D 64, block_m 32     1.01 - 1.43 from 1024 items; 0.64 - 0.85 with long lists, 0.61 - 0.97 up to 300
 // Small grids are bound by one CTA's latency, which is longer here; with one short tile of ancestors per
 // 64 rows at D 128 both kernels wait for the same HBM bytes.
 inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int ma) {
@@ -68,12 +68,12 @@ inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int
     const int bound = ma / bm;                        // tiles of ancestors the caller allows for
     if (D == 128) {
         if (bm == 128) return items >= 200;
-        if (bm == 64) return bound >= 4 ? items >= 256 : bound >= 2 && items >= 1024;
+        if (bm == 64) return items >= (bound >= 2 ? 256 : 1000);
         return items >= 200 && (bound < 8 || items <= 400);
     }
-    if (bm == 128) return items >= 280;
-    if (bm == 64) return bound >= 2 ? items >= 1024 : items >= 3000;
-    return bound < 8 && items >= 2000;
+    if (bm == 128) return items >= 250;
+    if (bm == 64) return items >= (bound == 2 || bound == 3 ? 1000 : 2000);
+    return bound < 8 && items >= 1000;
 }
 
 }  // namespace fst

@@ -604,35 +604,47 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 if (!alive) break;
                 fence_after_sync();
 
-                // My live words, one at a time.
                 uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
 #pragma unroll
                 for (int i = 0; i < NW; ++i) live |= uint32_t(__any_sync(0xffffffffu, word[i] != 0u)) << i;
                 float sum[2] = {0.f, 0.f}, mu = 0.f, mx = -INFINITY;
-                // First round over the words: the row's maximum, then the reference point.  Second round (or at once,
-                // when there was only one word): probabilities, over S - word i of P covers columns 16 i .. of S,
-                // below the words still to be read; words nobody uses are zeros.  One loop and one word to a
-                // turn: code that runs once per tile and does not stay in the instruction cache costs more than it saves.
+                // My live words, WT to a turn.  First round: the row's maximum, then the reference point.  Second round (or
+                // at once, when one turn was all): probabilities, over S - word i of P covers columns 16 i .. of S,
+                // below the words still to be read; words nobody uses are zeros.  One loop and one copy of its
+                // code: what runs once per tile and does not stay in the instruction cache costs more than it saves
+                // (two words to a turn at block_m 128: 1760 -> 1892 us on the forest of 65532 nodes; both words of
+                // a row in one turn at block_m 64: 69.0 -> 67.5 us on the deep tree).
+                constexpr int WT = NW == 2 ? 2 : 1;
                 bool second = false;
 #pragma unroll 1
                 for (uint32_t rest = live; rest != 0u;) {
-                    const int wi = __ffs(rest) - 1;
-                    rest &= rest - 1;
-                    uint32_t s[32];
-                    tmem_ld32(s, tmem_my + wi * 32);
-                    uint32_t w = word[0];
+                    uint32_t s[WT][32];
+                    int wi[WT];                           // the words' numbers; NW: none
 #pragma unroll
-                    for (int i = 1; i < NW; ++i) w = wi == i ? word[i] : w;
-                    tmem_ld_wait(s);
-                    float m2[2] = {-INFINITY, -INFINITY};
+                    for (int k = 0; k < WT; ++k) {
+                        wi[k] = WT == 1 || rest != 0u ? __ffs(rest) - 1 : NW;
+                        rest &= rest - 1;
+                        if (WT == 1 || wi[k] < NW) tmem_ld32(s[k], tmem_my + wi[k] * 32);
+                    }
+                    float m = -INFINITY;
 #pragma unroll
-                    for (int c = 0; c < 32; c += 2) {
-                        s[c] = (w & (1u << c)) != 0u ? s[c] : 0xff800000u;
-                        s[c + 1] = (w & (2u << c)) != 0u ? s[c + 1] : 0xff800000u;
-                        m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[c]), __uint_as_float(s[c + 1])));
+                    for (int k = 0; k < WT; ++k) {
+                        if (WT > 1 && wi[k] >= NW) continue;
+                        uint32_t w = word[0];
+#pragma unroll
+                        for (int i = 1; i < NW; ++i) w = wi[k] == i ? word[i] : w;
+                        tmem_ld_wait(s[k]);
+                        float m2[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+                        for (int c = 0; c < 32; c += 2) {
+                            s[k][c] = (w & (1u << c)) != 0u ? s[k][c] : 0xff800000u;
+                            s[k][c + 1] = (w & (2u << c)) != 0u ? s[k][c + 1] : 0xff800000u;
+                            m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[k][c]), __uint_as_float(s[k][c + 1])));
+                        }
+                        m = fmaxf(m, fmaxf(m2[0], m2[1]));
                     }
                     if (!second) {
-                        mx = fmaxf(mx, fmaxf(m2[0], m2[1]));
+                        mx = fmaxf(mx, m);
                         if (rest != 0u) continue;
                         const bool up = (mx - m_ref) * c2 > 8.f;      // true from -inf
                         if (__any_sync(0xffffffffu, up)) {
@@ -652,21 +664,25 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                         }
                         mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
                         second = true;
-                        if ((live & (live - 1)) != 0u) {  // several words: once more from the first
+                        if (WT < NW && __popc(live) > WT) {       // more than a turn: once again from the first
                             rest = live;
                             continue;
                         }
                     }
-                    uint32_t pk[16];
 #pragma unroll
-                    for (int c = 0; c < 32; c += 2) {
-                        const float p0 = fast_exp2(fmaf(__uint_as_float(s[c]), c2, -mu));
-                        const float p1 = fast_exp2(fmaf(__uint_as_float(s[c + 1]), c2, -mu));
-                        sum[0] += p0;
-                        sum[1] += p1;
-                        pk[c >> 1] = MT::pack(p0, p1);
+                    for (int k = 0; k < WT; ++k) {
+                        if (WT > 1 && wi[k] >= NW) continue;
+                        uint32_t pk[16];
+#pragma unroll
+                        for (int c = 0; c < 32; c += 2) {
+                            const float p0 = fast_exp2(fmaf(__uint_as_float(s[k][c]), c2, -mu));
+                            const float p1 = fast_exp2(fmaf(__uint_as_float(s[k][c + 1]), c2, -mu));
+                            sum[0] += p0;
+                            sum[1] += p1;
+                            pk[c >> 1] = MT::pack(p0, p1);
+                        }
+                        tmem_st16(tmem_s + (sub * segw + wi[k]) * 16, pk);
                     }
-                    tmem_st16(tmem_s + (sub * segw + wi) * 16, pk);
                 }
                 l += sum[0] + sum[1];
                 {
