@@ -96,6 +96,7 @@ struct PrefixArgs {
     int pair;            // two query tiles to a CTA
     int q_tiles;         // query tiles of a head (or pack of heads)
     int kv_tiles;        // query tiles that read one K/V head
+    int bm_shift;                        // block_m is 1 << bm_shift
     int pack, pack_shift;                // heads per query tile; a head's rows are 1 << pack_shift of the tile's
     // paged prefix: K/V rows live in pages of page_size rows; block_table[z][i] is the page
     // holding rows [i * page_size, (i + 1) * page_size) of batch element z, prefix_lens[z] its
@@ -112,13 +113,12 @@ constexpr int PFX_THREADS = PFX_SOFTMAX + 128;  // + loading, issuing and two ga
 // with a segment of 1 << seg_shift columns in a gathered tile.
 struct QueryTile {
     int h, q0, rows, b0, n_blk, seg_shift;
-    __device__ __forceinline__ QueryTile(const AttnArgs &a, const PrefixArgs &pa, int hk, int x) {
-        const int sub = x / pa.q_tiles;
-        h = hk * a.kv_group + sub * pa.pack;
-        q0 = (x - sub * pa.q_tiles) * umma::QM;
+    __device__ __forceinline__ QueryTile(const AttnArgs &a, const PrefixArgs &pa, int head, int first) {
+        h = head;
+        q0 = first;
         rows = min(a.n_q - q0, 1 << pa.pack_shift);
-        b0 = q0 / a.bm;
-        n_blk = (rows + a.bm - 1) / a.bm;
+        b0 = q0 >> pa.bm_shift;
+        n_blk = (rows + a.bm - 1) >> pa.bm_shift;
         seg_shift = n_blk > 2 ? 5 : n_blk > 1 ? 6 : 7;
     }
 };
@@ -145,6 +145,10 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     const int x0 = pa.pair ? blockIdx.x * 2 : blockIdx.x;
     const bool two = pa.pair && x0 + 1 < pa.kv_tiles;     // two query tiles ...
     const bool same = pa.q_tiles == 1;                    // ... of the same nodes, so that tree tiles are shared as well
+    // the two query tiles; query(0) is the one where there is only one
+    const int sub0 = x0 / pa.q_tiles, n0 = x0 - sub0 * pa.q_tiles, h0 = hk * a.kv_group + sub0 * pa.pack;
+    const bool wraps = n0 + 1 == pa.q_tiles;              // the second one is the next heads' first
+    auto query = [&](int g) { return QueryTile(a, pa, g && wraps ? h0 + pa.pack : h0, g ? (wraps ? 0 : n0 + 1) * QM : n0 * QM); };
     const int ring = G::TILES - (two ? 2 : 1);
     const uint32_t s_ring = s_base + (two ? 2 : 1) * TILE;
 
@@ -196,14 +200,15 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     const int T0 = run * per, T1 = run + 1 == pa.n_runs ? 0x3fffffff : T0 + per;
     const int nt_sure = max(0, min(T1, tp + 1) - T0);
     auto count_tiles = [&]() -> int {
-        int g = gathered_tiles(QueryTile(a, pa, hk, x0));
-        if (two && !same) g = max(g, gathered_tiles(QueryTile(a, pa, hk, x0 + 1)));
+        int g = gathered_tiles(query(0));
+        if (two && !same) g = max(g, gathered_tiles(query(1)));
         return max(0, min(T1, tp + 1 + g) - T0);
     };
     // Steps j = 0, 1, ...: group j & 1 and column tile T0 + (two ? j >> 1 : j).  K/V tiles (units) are shared by
     // two steps each in the first 2 * shared steps (all of them when the two query tiles have the same nodes, else those
     // of the prefix); every other step has a unit of its own.
     auto n_shared = [&](int nt) -> int { return !two ? 0 : same ? nt : min(max(tp - T0, 0), nt); };
+    const int nt_all = warp == 8 ? 0 : count_tiles();     // (the loading warp asks when it has nothing else to do)
 
     if (warp == 8) {
         // ====== loads: unit u is items 2u (K) and 2u + 1 (V) of the ring.  The whole warp for a paged prefix, one lane
@@ -228,7 +233,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                 mbar_arrive_expect_tx(bar_q, (two ? 2 : 1) * TILE);
 #pragma unroll 1
                 for (int g = 0; g < (two ? 2 : 1); ++g) {
-                    const QueryTile me(a, pa, hk, x0 + g);
+                    const QueryTile me = query(g);
 #pragma unroll 1
                     for (int i = 0; i < pa.pack; ++i)
 #pragma unroll
@@ -274,7 +279,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                         if (pool ? lane < npt : lead) {
                             if (pool && unsigned(here) >= unsigned(pa.n_pages))   // the boxes then read as zeros
                                 report(a.status, FST_DEV_INDEX_RANGE, z, tile * KN / ps + lane);
-                            const int row = pool ? 0 : tile < tp ? tile * KN : (PAGED ? 0 : a.prefix) + QueryTile(a, pa, hk, x0 + g).q0;
+                            const int row = pool ? 0 : tile < tp ? tile * KN : (PAGED ? 0 : a.prefix) + query(g).q0;
                             const uint32_t to = dst + (pool ? lane * ps * 128 : 0);
 #pragma unroll
                             for (int hf = 0; hf < DH; ++hf) tma_load_4d(to + hf * HALF, map, hf * 64, row, hk, pool ? here : z, bar);
@@ -292,7 +297,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         if (elect_one()) {
             fence_after_sync();
             const uint32_t tmem = *tmem_slot;
-            const int nt = count_tiles(), shared = n_shared(nt), n_steps = (two ? 2 : 1) * nt;
+            const int nt = nt_all, shared = n_shared(nt), n_steps = (two ? 2 : 1) * nt;
             const uint32_t idesc_s = instr_desc(BF16, false, KN), idesc_pv = instr_desc(BF16, true, D);
             // descriptors of the tiles' first 16-wide step; a step further on adds its byte offset / 16
             const uint64_t dq = smem_desc(s_base, 16), dk = smem_desc(s_ring, 16), dv = smem_desc(s_ring, HALF);
@@ -319,7 +324,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                     const int tile = T0 + (two ? j >> 1 : j);
                     uint32_t live = 0xffu;
                     if (tile > tp) {
-                        const QueryTile me(a, pa, hk, x0 + (two && !same ? g : 0));
+                        const QueryTile me = query(two && !same ? g : 0);
                         const int slot0 = (tile - tp - 1) << me.seg_shift;
                         live = 0u;
 #pragma unroll 1
@@ -368,7 +373,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         }
     } else if (warp >= 10) {
         // ====== two gathering warps: ancestors' K rows (10) and V rows (11), whole steps of 16 rows at a time ======
-        const int nt = count_tiles(), shared = n_shared(nt), n_units = (two ? 2 : 1) * nt - shared;
+        const int nt = nt_all, shared = n_shared(nt), n_units = (two ? 2 : 1) * nt - shared;
         const int plain = min(max(tp + 1 - T0, 0), nt), u0 = (two ? 2 : 1) * plain - min(shared, plain);
         const T *src = warp == 10 ? static_cast<const T *>(a.k) + z * a.ks_z + hk * a.ks_h
                                   : static_cast<const T *>(a.v) + z * a.vs_z + hk * a.vs_h;
@@ -385,7 +390,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         for (int v = early ? 2 * u0 - n_units : u0; v < n_units; ++v) {
             const bool fetch = v >= u0;
             const int u = fetch ? v : v + n_units - u0, x = u - shared, tile = T0 + (two && !same ? shared + (x >> 1) : u);
-            const QueryTile me(a, pa, hk, x0 + (two && !same ? x & 1 : 0));
+            const QueryTile me = query(two && !same ? x & 1 : 0);
             const int seg = 1 << me.seg_shift, slot0 = (tile - tp - 1) << me.seg_shift;
             // a step's rows: lanes 0-15 those of an even step, lanes 16-31 those of the odd one behind it
             int node[4];
@@ -417,7 +422,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                 const int s = step * 16 >> me.seg_shift;
                 if (slot0 + (step * 16 & (seg - 1)) >= external(me, s)) continue;      // nothing there: not used either
                 const int mine = step < 4 ? (step < 2 ? node[0] : node[1]) : (step < 6 ? node[2] : node[3]);
-#pragma unroll
+#pragma unroll 4
                 for (int i = 0; i < 16 / RPP; ++i) {
                     const int rr = i * RPP + lr, row = step * 16 + rr;
                     const int nd = __shfl_sync(0xffffffffu, mine, (step & 1) * 16 + rr);
@@ -450,13 +455,13 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         bool alive = true;
 
         // my node, its block in the query tile and row in the block: where its mask words are
-        const QueryTile me(a, pa, hk, x0 + (two ? g : 0));
-        const int node = r & ((1 << pa.pack_shift) - 1), sub = node / a.bm, jrow = node - sub * a.bm;
+        const QueryTile me = query(two ? g : 0);
+        const int node = r & ((1 << pa.pack_shift) - 1), sub = node >> pa.bm_shift, jrow = node - sub * a.bm;
         const bool real = node < me.rows;
         const int seg = 1 << me.seg_shift;
         const uint32_t *own_words = reinterpret_cast<const uint32_t *>(blob + L.off_bmask) + (size_t(me.b0 + sub) * a.bm + jrow) * L.bw;
         const uint32_t *ext_words = reinterpret_cast<const uint32_t *>(blob + L.off_emask) + (size_t(me.b0 + sub) * a.bm + jrow) * L.maw;
-        const int nt = count_tiles(), n_steps = (two ? 2 : 1) * nt;
+        const int nt = nt_all, n_steps = (two ? 2 : 1) * nt;
 
         if (T1 > tp && real) {                            // on their way while the prefix is walked
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(own_words));
@@ -590,7 +595,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
 
     // ---- merge: a row lies in every CTA of the cluster.  Every CTA takes an equal share of the rows.  Shared memory of
     // another CTA reads at some 12 bytes per cycle, which is why prefix_plan prefers few runs.
-    const QueryTile tile_a(a, pa, hk, x0), tile_b(a, pa, hk, two ? x0 + 1 : x0);
+    const QueryTile tile_a = query(0), tile_b = query(two);
     fence_before_sync();
     __syncwarp();
     if (pa.n_runs > 1) cluster_sync();
@@ -608,7 +613,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     for (int row = row_lo + warp * RPW + lane / LPR; row < row_hi; row += PFX_THREADS / 32 * RPW) {
         float4 acc[4] = {};
         float mu = -INFINITY, l = 0.f;
-#pragma unroll 2
+#pragma unroll 1
         for (int s = 0; s < pa.n_runs; ++s) {
             const uint32_t base = cluster_addr(s_base, s);
             const float2 st = cluster_ld2(base + G::OFF_STATS + (2 * QM + row) * 8);
@@ -696,6 +701,7 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
     pa.pair = plan.pair;
     pa.q_tiles = (a.n_q + umma::QM - 1) / umma::QM;
     pa.kv_tiles = a.kv_group / pack * pa.q_tiles;
+    pa.bm_shift = a.bm == 32 ? 5 : a.bm == 64 ? 6 : 7;
     pa.pack = pack;
     pa.pack_shift = 7;
     for (int p = pack; p > 1; p /= 2) --pa.pack_shift;

@@ -113,35 +113,6 @@ __device__ __forceinline__ uint32_t live_steps(int t, int seg, const int (&count
     return steps;
 }
 
-// whether a phase is over, without the suspended wait try_wait may make of it
-__device__ __forceinline__ bool over(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-
-// mbar_wait with its loop out of line (with a copy of it at every wait the kernel outgrew the instruction
-// cache), suspended for up to 20 us at a time
-static __device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, int32_t *status, int where) {
-    unsigned long long since = 0;
-#pragma unroll 1
-    for (int it = 0; it < (1 << 20); ++it) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000) : "memory");
-        if (ok != 0) return true;
-        const unsigned long long now = global_ns();
-        if (since == 0) since = now;
-        else if (now - since > 50000000ull) break;
-    }
-    report(status, FST_DEV_TIMEOUT, where, int(parity));
-    return false;
-}
-__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, int32_t *status, int where) {
-    return over(bar, parity) || wait_slow(bar, parity, status, where);
-}
-
 __device__ __forceinline__ void arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
