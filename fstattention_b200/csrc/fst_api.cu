@@ -296,9 +296,15 @@ static int attention_fwd_impl(const void *q, const void *k, const void *v, void 
                            (choice == FST_KERNEL_TMA_UMMA || (automatic && a.prefix >= 256));
     if (choice == FST_KERNEL_TMA_UMMA && !want_umma) return FST_ERR_UNSUPPORTED;
     if (want_umma) {
+        if (workspace != nullptr && kv_splits > 1) {      // the runs may be spread, their results merged from there
+            if (workspace_bytes < fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits)) return FST_ERR_WORKSPACE;
+            if (!aligned16(workspace)) return FST_ERR_ALIGNMENT;
+            a.part_o = static_cast<float *>(workspace);
+            a.part_lse = a.part_o + size_t(kv_splits) * Z * H * n_q * head_dim;
+        }
         const cudaError_t e = launch_prefix_umma(a, dtype, kv_splits, st);
         if (e != cudaErrorNotSupported || !automatic) return cuda_status(e);
-        // a tensor map could not be built: fall through
+        a.part_o = a.part_lse = nullptr;                  // a tensor map could not be built: fall through
     } else if (can_part && workspace != nullptr && kv_splits > 1) {
         const size_t need = fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits);
         if (workspace_bytes < need) return FST_ERR_WORKSPACE;
@@ -416,8 +422,10 @@ int fst_attention_fwd_paged(const void *q, const void *k_tree, const void *v_tre
     for (int64_t s : strides)
         if ((s * 2) & 15) ok = false;
     if (!ok) return FST_ERR_ALIGNMENT;
-    (void)workspace;                                      // the runs are merged inside the kernel
-    (void)workspace_bytes;
+    if (workspace != nullptr && !aligned16(workspace)) return FST_ERR_ALIGNMENT;
+    if (kv_splits < 2) workspace = nullptr;
+    if (workspace != nullptr && workspace_bytes < fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits))
+        return FST_ERR_WORKSPACE;
 
     AttnArgs a = {};                                      // the tree part: K/V rows of the tree nodes only
     a.q = q; a.k = k_tree; a.v = v_tree; a.o = o; a.lse = lse;
@@ -434,6 +442,10 @@ int fst_attention_fwd_paged(const void *q, const void *k_tree, const void *v_tre
     a.status = status;
     a.n_splits = 1;
     a.part_slots = 1;
+    if (workspace != nullptr) {                           // the runs may be spread, their results merged from there
+        a.part_o = static_cast<float *>(workspace);
+        a.part_lse = a.part_o + size_t(kv_splits) * Z * H * n_q * head_dim;
+    }
     a.meta_stable = 0;
     a.prefix = max_prefix;                                // the prefix rows come from the page pool
     const PagedArgs pg{k_pool, v_pool, block_table, prefix_lens, table_stride, page_size, n_pages,

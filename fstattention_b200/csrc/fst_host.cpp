@@ -104,7 +104,8 @@ Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, i
     const int64_t cap = 65535 / std::max<int64_t>(Z, 1);
     const auto clamp = [&](int64_t v) { return int(std::max<int64_t>(1, std::min(v, cap))); };
     if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && prefix >= 256)) {
-        return {fst::prefix_plan(Z, H, H_kv, n_q, prefix, sm_count(device), asked ? clamp(*asked) : 0).runs, false};
+        const fst::PrefixPlan plan = fst::prefix_plan(Z, H, H_kv, n_q, prefix, sm_count(device), true, asked ? clamp(*asked) : 0);
+        return {plan.runs, plan.spread};
     }
     int runs;
     if (asked) {
@@ -330,8 +331,22 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
     const int64_t max_prefix = integer(a[15]);
     const at::Device dev = q.device();
     std::optional<long long> asked = optional_int(a[17]);
-    if (!asked && max_prefix > 0) asked = fst::prefix_plan(Z, H, H_kv, n_q, max_prefix, sm_count(dev.index()), 0, kp.size(row_dim)).runs;
+    Splits sp{asked ? int(*asked) : 1, false};
+    if (max_prefix > 0 && (!asked || *asked > 0)) {
+        const int64_t cap = 65535 / std::max<int64_t>(Z, 1);
+        if (!asked || *asked <= cap) {                    // (more than the grid holds is the library's error to give)
+            const fst::PrefixPlan plan =
+                fst::prefix_plan(Z, H, H_kv, n_q, max_prefix, sm_count(dev.index()), true, asked.value_or(0), kp.size(row_dim));
+            sp = {plan.runs, plan.spread};
+        }
+    }
     const c10::cuda::CUDAGuard guard(dev);
+    at::Tensor ws;
+    size_t ws_bytes = 0;
+    if (sp.workspace) {
+        ws_bytes = fst_attention_split_workspace_bytes(int(Z), int(H), int(n_q), int(D), sp.runs);
+        ws = empty({int64_t(ws_bytes)}, at::kByte, dev);
+    }
     int32_t *status = static_cast<int32_t *>(status_of(dev, true)->data_ptr());
     void *stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     const size_t tree_stride = n_trees > 1 ? size_t(integer(a[5])) : 0;
@@ -345,7 +360,7 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
                                      int(kp.size(row_dim)), int(kp.size(0)), kp.stride(0), kp.stride(row_dim),
                                      kp.stride(head_dim), int(Z), int(H), int(H_kv), int(n_q), int(D), FST_STRIDES(q),
                                      FST_STRIDES(kt), FST_STRIDES(vt), FST_STRIDES(c.o), int(bm), int(ma), c.scale, c.dtype,
-                                     int(asked.value_or(1)), nullptr, 0, status, stream);
+                                     sp.runs, ws.defined() ? ws.data_ptr() : nullptr, ws_bytes, status, stream);
     }
     check_status(rc, "fst_attention_fwd_paged");
     return results(c);

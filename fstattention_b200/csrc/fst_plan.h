@@ -17,37 +17,46 @@ inline int prefix_heads_per_tile(int64_t H, int64_t H_kv, int64_t n_q) {
     return pack;
 }
 
-// How a call behind a shared prefix is laid out: whether a CTA has two query tiles (pair), and into how many runs
-// the column tiles are cut, the runs of a query tile being a cluster of CTAs.  One CTA per SM.
-// The choice minimises waves x (tiles of a run x a tile's time + a CTA's fixed time) + merging.  In tenths of a
-// microsecond at D 128 (4096 prefix rows, 32 heads of 256 query rows; 3001 rows in pages of 16, 8 K/V heads): a tile 10
-// for one query tile and 22 for two, but 18 for one where the tile comes in small pages (a page of 16 rows
+// How a call behind a shared prefix is laid out: whether a CTA has two query tiles (pair), into how many runs the
+// column tiles are cut, and whether the runs of a query tile are a cluster of CTAs that merges them through
+// distributed shared memory, or spread over the GPU, with partial results in a workspace and a merge kernel.
+// One CTA per SM.  A cluster stays within a GPC, of which there are eight with 16 SMs or more, not all of them
+// with 18: 7 CTAs to a cluster use 112 SMs of 148, and few query tiles behind a long prefix are better
+// spread (18 query tiles, 15100 rows: 47 us as clusters of seven in two waves, 25 spread).
+// The choice minimises waves x (tiles of a run x a tile's time + a CTA's fixed time) + merging, in tenths of a
+// microsecond at D 128 (4096 prefix rows, 32 heads of 256 query rows; 3001 rows in pages of 16, 8 K/V heads): a tile 8
+// for one query tile and 17 for two, but 15 for one where the tile comes in small pages (a page of 16 rows
 // is a TMA box per 64 columns, and the boxes are what takes the time: two query tiles share them);
-// 140 for loading the first tiles, the last tile's chain and the output; 7 for every run to be merged.
-constexpr int kMaxPrefixRuns = 8;      // portable cluster size
+// 120 for loading the first tiles, the last tile's chain and the output; 10 and 7 for every run to merge a
+// cluster's, 45 and 3 for every run to spread them.
+constexpr int kMaxClusterRuns = 8;     // portable cluster size
+constexpr int kMaxSpreadRuns = 16;
 struct PrefixPlan {
     int runs;
-    bool pair;
+    bool pair, spread;
 };
-inline PrefixPlan prefix_plan(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, int64_t prefix, int sms, int64_t asked = 0,
-                              int64_t page = 128) {
+inline PrefixPlan prefix_plan(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, int64_t prefix, int sms, bool may_spread,
+                              int64_t asked = 0, int64_t page = 128) {
     const int64_t kv_tiles = H / H_kv / prefix_heads_per_tile(H, H_kv, n_q) * ((n_q + 127) / 128);
-    const int64_t tiles = (prefix + 127) / 128 + 2;
-    const int64_t cap = std::max<int64_t>(1, std::min<int64_t>({kMaxPrefixRuns, tiles / 2, 65535 / std::max<int64_t>(Z, 1)}));
-    const int64_t lo = asked > 0 ? std::min<int64_t>(asked, kMaxPrefixRuns) : 1, hi = asked > 0 ? lo : cap;
-    PrefixPlan best{int(lo), false};
+    const int64_t tiles = (prefix + 127) / 128 + 2, per_z = 65535 / std::max<int64_t>(Z, 1);
+    const int64_t most = may_spread ? per_z : std::min<int64_t>(kMaxClusterRuns, per_z);
+    const int64_t lo = asked > 0 ? std::min(asked, most) : 1,
+                  hi = asked > 0 ? lo : std::max<int64_t>(1, std::min<int64_t>({may_spread ? kMaxSpreadRuns : kMaxClusterRuns, tiles / 2, per_z}));
+    PrefixPlan best{int(lo), false, lo > kMaxClusterRuns};
     int64_t best_cost = INT64_MAX;
-    for (int64_t pair = 0; pair < (kv_tiles > 1 ? 2 : 1); ++pair)
-        for (int64_t runs = lo; runs <= hi; ++runs) {
-            const int64_t ctas = Z * H_kv * ((kv_tiles + pair) / (1 + pair)) * runs;
-            const int64_t fit = runs > 4 ? sms * 7 / 8 : runs > 2 ? sms * 9 / 10 : sms;      // clusters stay within a GPC
-            const int64_t waves = (ctas + fit - 1) / fit;
-            const int64_t cost = waves * ((tiles + runs - 1) / runs * (pair ? 22 : page < 32 ? 18 : 10) + 140) + (runs > 1 ? 10 + 7 * runs : 0);
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = {int(runs), pair != 0};
+    for (int spread = 0; spread < (may_spread ? 2 : 1); ++spread)
+        for (int pair = 0; pair < (kv_tiles > 1 ? 2 : 1); ++pair)
+            for (int64_t runs = std::max<int64_t>(lo, spread ? 2 : 1); runs <= (spread ? hi : std::min<int64_t>(hi, kMaxClusterRuns)); ++runs) {
+                const int64_t ctas = Z * H_kv * ((kv_tiles + pair) / (1 + pair)) * runs;
+                const int64_t fit = spread || runs == 1 ? sms : runs == 2 ? sms / 18 * 18 : std::max<int64_t>(1, sms / 18 * (16 / runs) * runs);
+                const int64_t waves = (ctas + fit - 1) / fit, tile = pair ? 17 : page < 32 ? 15 : 8;
+                const int64_t merge = runs == 1 ? 0 : spread ? 45 + 3 * runs : 10 + 7 * runs;
+                const int64_t cost = waves * ((tiles + runs - 1) / runs * tile + 120) + merge;
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best = {int(runs), pair != 0, spread != 0};
+                }
             }
-        }
     return best;
 }
 

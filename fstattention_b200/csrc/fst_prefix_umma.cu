@@ -29,7 +29,8 @@
 //
 // Runs: the column tiles of a query tile are cut into up to eight runs, one CTA each, which form a
 // cluster.  Every CTA leaves its rows, unnormalised, in its shared memory; each then merges its share of the rows
-// out of all of them and writes the output.  There are no partial results in memory and no second kernel.
+// out of all of them and writes the output.  There are no partial results in memory and no second kernel -
+// except where clusters would leave SMs idle (prefix_plan): then every run leaves its rows in a workspace.
 //
 // With grouped-query attention a small tree's rows of several heads share a query tile (see
 // prefix_heads_per_tile): the tile is loaded as one box per head and its rows go to their heads at the end.
@@ -92,7 +93,8 @@ __device__ __forceinline__ void cluster_sync() {
 
 // Arguments of the prefix kernel beyond AttnArgs.
 struct PrefixArgs {
-    int n_runs;          // runs of column tiles (CTAs of a cluster)
+    int n_runs;          // runs of column tiles
+    int cluster;         // CTAs of a cluster: n_runs, or 1 where every run leaves a partial result of its own
     int pair;            // two query tiles to a CTA
     int q_tiles;         // query tiles of a head (or pack of heads)
     int kv_tiles;        // query tiles that read one K/V head
@@ -598,14 +600,15 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     const QueryTile tile_a = query(0), tile_b = query(two);
     fence_before_sync();
     __syncwarp();
-    if (pa.n_runs > 1) cluster_sync();
+    if (pa.cluster > 1) cluster_sync();
     else __syncthreads();
     if (warp == 9) {
         fence_after_sync();
         tmem_free_all(*tmem_slot);
     }
-    const int rows_all = two ? 2 * QM : QM, share = (rows_all + pa.n_runs - 1) / pa.n_runs;
-    const int row_lo = run * share, row_hi = min(rows_all, row_lo + share);
+    const int rows_all = two ? 2 * QM : QM, share = (rows_all + pa.cluster - 1) / pa.cluster;
+    const bool partial = pa.cluster < pa.n_runs;          // rows in fp32 for the merge kernel, slot by slot
+    const int row_lo = partial ? 0 : run * share, row_hi = min(rows_all, row_lo + share);
     // a lane has a 64-byte piece of a row: four chunks of 16 bytes, LPR lanes a row
     constexpr int LPR = D / 16, RPW = 32 / LPR;
     const int c = lane % LPR;
@@ -614,7 +617,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         float4 acc[4] = {};
         float mu = -INFINITY, l = 0.f;
 #pragma unroll 1
-        for (int s = 0; s < pa.n_runs; ++s) {
+        for (int s = 0; s < pa.cluster; ++s) {
             const uint32_t base = cluster_addr(s_base, s);
             const float2 st = cluster_ld2(base + G::OFF_STATS + (2 * QM + row) * 8);
             float4 v[4];
@@ -637,13 +640,23 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         const int h = (first ? tile_a.h : tile_b.h) + ((row & 127) >> pa.pack_shift);
         if (node >= (first ? tile_a.rows : tile_b.rows)) continue;
         const float inv = l > 0.f ? 1.f / l : 0.f;
+        const float lse = l > 0.f ? mu + log2f(l) : -INFINITY;
+        if (partial) {
+            const size_t slot_row = ((size_t(run) * a.Z + z) * a.H + h) * n_q + gr;
+            float4 *to = reinterpret_cast<float4 *>(a.part_o + slot_row * D);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                to[k * LPR + c] = make_float4(acc[k].x * inv, acc[k].y * inv, acc[k].z * inv, acc[k].w * inv);
+            if (c == 0) a.part_lse[slot_row] = lse;
+            continue;
+        }
         uint2 *to = reinterpret_cast<uint2 *>(static_cast<T *>(a.o) + z * a.os_z + h * a.os_h + gr * a.os_n);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             to[k * LPR + c] = make_uint2(MT::pack(acc[k].x * inv, acc[k].y * inv), MT::pack(acc[k].z * inv, acc[k].w * inv));
-        if (a.lse != nullptr && c == 0) a.lse[(size_t(z) * a.H + h) * n_q + gr] = l > 0.f ? mu + log2f(l) : -INFINITY;
+        if (a.lse != nullptr && c == 0) a.lse[(size_t(z) * a.H + h) * n_q + gr] = lse;
     }
-    if (pa.n_runs == 1) return;
+    if (pa.cluster == 1) return;
     __syncwarp();
     cluster_sync();                                       // nobody leaves while its rows are being read
 }
@@ -695,9 +708,10 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return cudaErrorInvalidDevice;
-    const PrefixPlan plan = prefix_plan(a.Z, a.H, H_kv, a.n_q, a.prefix, sms, n_runs, PAGED ? pg->page_size : 128);
+    const PrefixPlan plan = prefix_plan(a.Z, a.H, H_kv, a.n_q, a.prefix, sms, a.part_o != nullptr, n_runs, PAGED ? pg->page_size : 128);
     PrefixArgs pa = {};
     pa.n_runs = plan.runs;
+    pa.cluster = plan.spread ? 1 : plan.runs;
     pa.pair = plan.pair;
     pa.q_tiles = (a.n_q + umma::QM - 1) / umma::QM;
     pa.kv_tiles = a.kv_group / pack * pa.q_tiles;
@@ -722,10 +736,14 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = unsigned(pa.n_runs);
+    attr[1].val.clusterDim.z = unsigned(pa.cluster);
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, prefix_umma_kernel<T, D, PAGED>, a, pa, tq, tk, tv, tkt, tvt);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, prefix_umma_kernel<T, D, PAGED>, a, pa, tq, tk, tv, tkt, tvt);
+    if (e != cudaSuccess || !plan.spread) return e;
+    AttnArgs merge = a;
+    merge.part_slots = pa.n_runs;
+    return launch_combine(merge, bf16 ? FST_BF16 : FST_F16, stream);
 }
 
 template <bool PAGED>
@@ -740,7 +758,8 @@ static cudaError_t launch_prefix_any(const AttnArgs &a, const PagedArgs *pg, int
     return cudaErrorNotSupported;
 }
 
-// The whole call - prefix and tree - in n_runs runs of column tiles (at most kMaxPrefixRuns).
+// The whole call - prefix and tree - in n_runs runs of column tiles (without room for partial results, part_o, at most
+// kMaxClusterRuns).
 cudaError_t launch_prefix_umma(const AttnArgs &a, int dtype, int n_runs, cudaStream_t stream) {
     return launch_prefix_any<false>(a, nullptr, dtype, n_runs, stream);
 }

@@ -76,7 +76,8 @@ def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[in
     if kernel == "persist" and tree == "attn_tma_kernel" and prefix == 0 and block_m in (64, 128):
         tree = "attn_persist_kernel"                      # by hand only: it measured slower than attn_tma_kernel
     if tensor_core and block_m >= 32 and prefix > 0 and (kernel == "tma_umma" or (kernel == "auto" and prefix >= 256)):
-        return {"kernels": ["prefix_umma_kernel"], "prefix_runs": splits}      # prefix and tree in one, runs merged inside
+        # prefix and tree in one; its runs merge inside unless they are spread over the GPU
+        return {"kernels": ["prefix_umma_kernel"] + ["combine_splits_kernel"] * need_ws, "prefix_runs": splits}
     if need_ws:
         return {"kernels": [tree, "combine_splits_kernel"], "prefix_runs": splits}
     return {"kernels": [tree], "prefix_runs": 1}

@@ -22,7 +22,7 @@ def comb(n, teeth):
 @pytest.mark.parametrize("n,teeth,prefix,splits,D", [
     (1, 1, 1, 1, 128), (17, 3, 127, 1, 64), (33, 8, 128, 2, 128), (64, 20, 129, 3, 128), (65, 40, 300, 2, 64),
     (128, 33, 256, 8, 128), (129, 64, 700, 2, 128), (200, 65, 513, 3, 64), (257, 30, 384, 1, 128),
-    (385, 130, 1000, 5, 128), (640, 300, 640, 2, 64), (640, 300, 130, 6, 128)])
+    (64, 20, 2500, 16, 128), (129, 64, 3000, 12, 64), (385, 130, 1000, 5, 128), (640, 300, 640, 2, 64), (640, 300, 130, 6, 128)])
 def test_prefix_and_tree_in_one(fst, n, teeth, prefix, splits, D, bm):
     par = comb(n, teeth)
     meta = fst.build_tree_metadata(par, bm, 512, reference_format=False)
