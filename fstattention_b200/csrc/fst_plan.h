@@ -63,8 +63,8 @@ inline PrefixPlan prefix_plan(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, i
 // When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, six kinds of trees, from 64
 // items (128 query rows of one head) up, ratios of old to new time:
 //   D 128, block_m 128   1.27 - 1.72 from 256 items, up to 2.40 at 5184; 0.82 - 1.12 below 100
-//   D 128, block_m 64    1.04 - 1.32 from 256 items with an ancestor bound of two blocks or more, 1.00 - 1.21
-//                        from 1024 with one (0.99 - 1.13 at 256); 0.63 - 0.75 below 100
+//   D 128, block_m 64    1.10 from 256 items with an ancestor bound of two or three blocks, 1.28 - 1.32 from 1024 with
+//                        two or more (0.98 - 1.06 at 256 with long lists), 1.00 - 1.21 with one; 0.63 - 0.75 below 100
 //   D 128, block_m 32    1.19 - 1.83 at 256 items, 1.08 - 1.26 above; 0.89 - 0.97 above with long lists
 //   D 64, block_m 128    1.01 - 1.36 at 256 items, 1.12 - 1.65 above; 0.69 - 0.90 below 100
 //   D 64, block_m 64     1.03 - 1.31 from 4096 items, 1.04 - 1.16 from 1024 with a bound of two or three blocks;
@@ -78,7 +78,7 @@ inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int
     const int bound = ma / bm;                        // tiles of ancestors the caller allows for
     if (D == 128) {
         if (bm == 128) return items >= 200;
-        if (bm == 64) return bound >= 2 && items >= 256;
+        if (bm == 64) return bound >= 4 ? items >= 1000 : bound >= 2 && items >= 256;
         return items >= 200 && (bound < 8 || items <= 400);
     }
     if (bm == 128) return items >= 250;
