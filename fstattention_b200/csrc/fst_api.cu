@@ -287,13 +287,14 @@ static int attention_fwd_impl(const void *q, const void *k, const void *v, void 
     }
 
     // A shared prefix: the tcgen05 kernel takes the whole call in kv_splits runs of column tiles (head_dim 64 or 128,
-    // block_m 32 and up; chosen automatically from 256 prefix rows on), or the tree kernel itself walks the prefix,
+    // block_m 32 and up; chosen automatically by prefix_umma_pays), or the tree kernel itself walks the prefix,
     // split over kv_splits CTAs whose partial results pass through the workspace.
     // (the tcgen05 kernel takes Q from shared memory as it arrived, so it cannot flip Q's sign
     // for a negative factor; the tree kernel walks the prefix itself then)
     const bool can_part = a.prefix > 0 && choice != FST_KERNEL_MMA && choice != FST_KERNEL_PERSIST;
     const bool want_umma = can_part && block_m >= 32 && sm_scale > 0.f &&
-                           (choice == FST_KERNEL_TMA_UMMA || (automatic && a.prefix >= 256));
+                           (choice == FST_KERNEL_TMA_UMMA ||
+                            (automatic && prefix_umma_pays(Z, H, H_kv, n_q, a.prefix, block_m)));
     if (choice == FST_KERNEL_TMA_UMMA && !want_umma) return FST_ERR_UNSUPPORTED;
     if (want_umma) {
         if (workspace != nullptr && kv_splits > 1) {      // the runs may be spread, their results merged from there

@@ -94,6 +94,7 @@ int sm_count(int device) {
 struct Splits {
     int runs;
     bool workspace;
+    bool umma = false;                                    // the tcgen05 prefix kernel takes the call
 };
 Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, int64_t Z, int64_t H, int64_t H_kv, int64_t n_q,
                    int64_t D, int64_t prefix, int64_t block_m, int kernel, int device) {
@@ -103,9 +104,9 @@ Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, i
         return {1, false};
     const int64_t cap = 65535 / std::max<int64_t>(Z, 1);
     const auto clamp = [&](int64_t v) { return int(std::max<int64_t>(1, std::min(v, cap))); };
-    if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && prefix >= 256)) {
+    if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && fst::prefix_umma_pays(Z, H, H_kv, n_q, prefix, block_m))) {
         const fst::PrefixPlan plan = fst::prefix_plan(Z, H, H_kv, n_q, prefix, sm_count(device), true, asked ? clamp(*asked) : 0);
-        return {plan.runs, plan.spread};
+        return {plan.runs, plan.spread, true};
     }
     int runs;
     if (asked) {
@@ -609,7 +610,7 @@ PyObject *splits(PyObject *const *a, Py_ssize_t n) {
     const at::Tensor &q = tensor(a[0]);
     const Splits s = pick_splits(optional_int(a[4]), q.scalar_type(), q.size(0), q.size(1), q.size(1), q.size(2), q.size(3), integer(a[1]),
                                  integer(a[2]), int(integer(a[3])), q.device().index());
-    return Py_BuildValue("(iO)", s.runs, s.workspace ? Py_True : Py_False);
+    return Py_BuildValue("(iOO)", s.runs, s.workspace ? Py_True : Py_False, s.umma ? Py_True : Py_False);
 }
 
 #define FST_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(&guarded<name>)), METH_FASTCALL, nullptr}

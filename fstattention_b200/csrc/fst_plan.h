@@ -60,6 +60,17 @@ inline PrefixPlan prefix_plan(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, i
     return best;
 }
 
+// Whether a call behind a shared prefix goes to the tcgen05 prefix kernel (head_dim 64 or 128, block_m 32 and up) or the
+// tree kernel walks the prefix.  Measured at 33 to 255 prefix rows, ratio of the tree kernel's time to the other's:
+// block_m 128 (250 nodes) 0.85 - 1.09 at 33 rows, 1.02 - 1.32 at 96, 1.30 - 1.61 at 200; block_m 64 (100
+// nodes) 0.74 - 0.91 up to 128, 0.98 - 1.18 at 200; block_m 32 (20 nodes) 0.45 - 0.96 up to 128, 1.00 - 1.22
+// at 200, but 0.60 - 0.64 where more query tiles than SMs are filled to a quarter or less.
+inline bool prefix_umma_pays(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, int64_t prefix, int64_t bm) {
+    const int64_t pack = prefix_heads_per_tile(H, H_kv, n_q);
+    const bool sparse = n_q * pack <= 32 && Z * H / pack > 148;
+    return prefix >= (sparse ? 256 : bm >= 128 ? 96 : 192);
+}
+
 // When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, six kinds of trees, from 64
 // items (128 query rows of one head) up, ratios of old to new time:
 //   D 128, block_m 128   1.27 - 1.72 from 256 items, up to 2.40 at 5184; 0.82 - 1.12 below 100

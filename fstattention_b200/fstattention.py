@@ -65,7 +65,7 @@ def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[in
     dtype only), a shared prefix of ``prefix`` rows and the given block size, mirroring the
     dispatch inside the library (for rows on 16-byte boundaries and a positive scale): ``{"kernels":
     [...], "prefix_runs": r}``.  ``max_ancestors`` is the metadata's ancestor bound."""
-    splits, need_ws = _lib.host().splits(q, prefix, block_m, _lib.KERNELS[kernel], kv_splits)
+    splits, need_ws, umma = _lib.host().splits(q, prefix, block_m, _lib.KERNELS[kernel], kv_splits)
     tensor_core = q.dtype in (torch.float16, torch.bfloat16) and q.shape[-1] in (64, 128) \
         and block_m in (16, 32, 64, 128)
     tree = "attn_simt_kernel" if kernel == "simt" or not tensor_core else \
@@ -75,7 +75,7 @@ def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[in
         tree = "tree_umma_kernel"
     if kernel == "persist" and tree == "attn_tma_kernel" and prefix == 0 and block_m in (64, 128):
         tree = "attn_persist_kernel"                      # by hand only: it measured slower than attn_tma_kernel
-    if tensor_core and block_m >= 32 and prefix > 0 and (kernel == "tma_umma" or (kernel == "auto" and prefix >= 256)):
+    if umma:
         # prefix and tree in one; its runs merge inside unless they are spread over the GPU
         return {"kernels": ["prefix_umma_kernel"] + ["combine_splits_kernel"] * need_ws, "prefix_runs": splits}
     if need_ws:

@@ -255,7 +255,7 @@ int fst_attention_tree_kernel(int Z, int H, int n_q, int head_dim, int block_m, 
  * to fill the GPU (the reference walks the prefix in one program, fstattention.py:113-136).
  * Partial results (fp32) and their log-sum-exps pass through `workspace`
  * (fst_attention_split_workspace_bytes bytes, 16-byte aligned, scratch; not needed with one run) and a
- * second kernel merges them.  With head_dim 64 or 128, block_m 32 and up and at least 256 prefix rows
+ * second kernel merges them.  With head_dim 64 or 128, block_m 32 and up and some 100 to 250 prefix rows or more
  * FST_KERNEL_AUTO hands the call to a tcgen05/TMEM kernel that walks prefix and tree in 128 x 128 tiles,
  * cut into kv_splits runs; FST_KERNEL_TMA_UMMA forces that, FST_KERNEL_TMA* forces the tree kernel to walk
  * the prefix itself in kv_splits runs.  Without a prefix this is fst_attention_fwd.
