@@ -60,15 +60,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int32_t
     report(status, FST_DEV_TIMEOUT, where, int(parity));
     return false;
 }
-// One lane of a converged warp.  The compiler knows that the branch holds a single thread, and the operands of products
-// and TMA copies, which the hardware takes from uniform registers, go there directly; under `lane == 0` it wraps each
-// in a loop over the lanes that might be active (16 products M 128, N 64 with rolled issue: 1568 -> 1037 cycles).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
-    return p != 0;
-}
-
 // one box of a rank-4 tensor (columns, rows, head, batch) into shared memory
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2,
                                             int c3, uint32_t bar) {
@@ -191,7 +182,7 @@ attn_tma_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap tm_q,
     // it has finished asks for its Q and its block's K/V rows to be brought into L2 meanwhile.  No
     // value reaches the SM before the dependency wait below, and L2 is where the other launch's
     // writes land too, so whatever it still writes to those rows is what the loads after the wait see.
-    if (TN == 64 && warp == 0 && elect_one()) {
+    if (TN == 64 && tid == 0) {
         const int hk0 = h / a.kv_group;
 #pragma unroll
         for (int j = 0; j < NB32; ++j)
@@ -263,7 +254,7 @@ attn_tma_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap tm_q,
     if (early_meta) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
     // ---- one thread starts the TMA transfers: Q and block K on one barrier, block V on another
-    if (warp == 0 && elect_one()) {
+    if (tid == 0) {
         mbar_arrive_expect_tx(bar_qk, (tree ? 2 : 1) * NB32 * SM::TILE);
 #pragma unroll
         for (int j = 0; j < NB32; ++j)
@@ -300,7 +291,7 @@ attn_tma_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap tm_q,
                 cp_async16(kd + o, kp + rr * a.ks_n + lc * 8, ok);
                 cp_async16(vd + o, vp + rr * a.vs_n + lc * 8, ok);
             }
-        } else if (warp == 0 && elect_one()) {
+        } else if (tid == 0) {
             const int p0 = p_lo + (e - nt_ext_of<TN>(count, a.ma)) * TN;
             const uint32_t bar = bar_p + st * 8;
             mbar_arrive_expect_tx(bar, 2 * TP * SM::TILE);
@@ -604,7 +595,7 @@ attn_tma_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap tm_q,
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
-    if (warp == 0 && elect_one()) {
+    if (tid == 0) {
         const int n_out = NOUT == 1 ? 1 : a.n_out;
         const int oh = NOUT == 1 ? h : h + a.out_h0, oz = NOUT == 1 ? z : z + a.out_z0;
         // Every rank starts with its own copy and then walks the others in ring order from its
@@ -627,8 +618,7 @@ attn_tma_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap tm_q,
         if (ok0) lse[row0 + r0] = m0 * c2 + log2f(l0);
         if (ok1) lse[row0 + r1] = m1 * c2 + log2f(l1);
     }
-    __syncwarp();
-    if (warp == 0 && elect_one()) {                       // the same lane: elect.sync is deterministic
+    if (tid == 0) {
         if (NOUT == 1) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // smem stays valid until read
         else asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");   // rows bound for other GPUs: until written
     }

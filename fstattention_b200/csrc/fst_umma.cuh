@@ -10,6 +10,15 @@ namespace umma {
 
 constexpr int HALF = 128 * 128;        // bytes of one 64-column half of a 128-row tile, 128-byte swizzle
 
+// One lane of a converged warp.  The compiler knows that the branch holds a single thread, and the operands of products
+// and TMA copies, which the hardware takes from uniform registers, go there directly; under `lane == 0` it wraps each
+// in a loop over the lanes that might be active (16 products M 128, N 64 with rolled issue: 1568 -> 1037 cycles).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+
 // shared-memory matrix descriptor: 128-byte swizzle, 8-row groups 1 KB apart
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes) {
     uint64_t d = 0;
