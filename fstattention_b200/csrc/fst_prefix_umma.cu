@@ -231,18 +231,6 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             bool known = false, alive = true;
             int nt = nt_sure, st = 0;
             uint32_t use = 0;                             // fills of the current stage before this one
-            if (lead) {
-                mbar_arrive_expect_tx(bar_q, (two ? 2 : 1) * TILE);
-#pragma unroll 1
-                for (int g = 0; g < (two ? 2 : 1); ++g) {
-                    const QueryTile me = query(g);
-#pragma unroll 1
-                    for (int i = 0; i < pa.pack; ++i)
-#pragma unroll
-                        for (int hf = 0; hf < DH; ++hf)
-                            tma_load_4d(s_base + g * TILE + hf * HALF + (i << pa.pack_shift) * 128, &tm_q, hf * 64, me.q0, me.h + i, z, bar_q);
-                }
-            }
             const int shared = n_shared(nt_sure);         // the same for the final count: see above
             int n_units = (two ? 2 : 1) * nt - shared;
 #pragma unroll 1
@@ -253,6 +241,18 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                     nt = count_tiles();
                     n_units = (two ? 2 : 1) * nt - n_shared(nt);
                     if (u >= n_units) break;
+                }
+                if (lead && u == 0) {                     // Q, when there is anything to do: nobody would wait for it otherwise
+                    mbar_arrive_expect_tx(bar_q, (two ? 2 : 1) * TILE);
+#pragma unroll 1
+                    for (int g = 0; g < (two ? 2 : 1); ++g) {
+                        const QueryTile me = query(g);
+#pragma unroll 1
+                        for (int i = 0; i < pa.pack; ++i)
+#pragma unroll
+                            for (int hf = 0; hf < DH; ++hf)
+                                tma_load_4d(s_base + g * TILE + hf * HALF + (i << pa.pack_shift) * 128, &tm_q, hf * 64, me.q0, me.h + i, z, bar_q);
+                    }
                 }
                 const int x = u - shared, g = two && !same && x >= 0 ? x & 1 : 0;
                 const int tile = T0 + (two && !same && x >= 0 ? shared + (x >> 1) : u);

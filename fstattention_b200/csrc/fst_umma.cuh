@@ -15,6 +15,7 @@ constexpr int HALF = 128 * 128;        // bytes of one 64-column half of a 128-r
 // in a loop over the lanes that might be active (16 products M 128, N 64 with rolled issue: 1568 -> 1037 cycles).
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
+    __syncwarp();
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
     return p != 0;
 }
