@@ -44,6 +44,7 @@ class TreeMetadata:
         # attention launches that have read the packed form since it was last written: from the
         # second one on, the launch ahead of the call in the stream cannot be the writer
         self.reads_since_build = 0
+        self._captured_status = []
         self._twin = None if ancestor_idx is None else _PackedTwin(self)
 
     def _rebuilt(self) -> None:
@@ -157,8 +158,13 @@ def build_tree_metadata(parent: TreeLike, block_m: int = 64, max_ancestors: int 
         n_trees, n_nodes = par.shape if par.dim() == 2 else (1, par.shape[0])
         if (meta.n_trees, meta.n_nodes, meta.block_m, meta.max_ancestors) != (n_trees, n_nodes, block_m, max_ancestors):
             raise ValueError("out= metadata has a different shape")
-        meta.status = host.precompute(par, block_m, max_ancestors, meta.packed, meta.tree_stride, meta.status,
-                                      meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx)
+        status = host.precompute(par, block_m, max_ancestors, meta.packed, meta.tree_stride, meta.status,
+                                 meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx)
+        if status is meta.status:
+            # captured into a graph, which clears and writes this record at every replay: it lives as long as the
+            # buffers, whatever record a later eager call takes
+            meta._captured_status.append(status)
+        meta.status = status
         meta._rebuilt()
     if check:
         meta.check()
