@@ -98,17 +98,17 @@ def test_sorted_levels_with_random_scores_and_ties(fst, depth, topk, lwf):
 def test_a_captured_build_keeps_its_status_record(fst):
     """A graph writes the record it was captured with; eager calls on other streams take records of their own."""
     par = torch.tensor([-1] + [i // 2 for i in range(255)], dtype=torch.int32, device="cuda")
-    meta = fst.build_tree_metadata(par, 64, 64, reference_format=False)
+    meta = fst.build_tree_metadata(par, 64, 128, reference_format=False)
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
-        fst.build_tree_metadata(par, 64, 64, out=meta, check=False)
+        fst.build_tree_metadata(par, 64, 128, out=meta, check=False)
     torch.cuda.current_stream().wait_stream(side)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        fst.build_tree_metadata(par, 64, 64, out=meta, check=False)
+        fst.build_tree_metadata(par, 64, 128, out=meta, check=False)
     record = meta.status.data_ptr()
-    fst.build_tree_metadata(par, 64, 64, out=meta, check=False)
+    fst.build_tree_metadata(par, 64, 128, out=meta, check=False)
     assert meta.status.data_ptr() != record and any(t.data_ptr() == record for t in meta._captured_status)
     want = meta.packed.clone()
     graph.replay()
