@@ -137,8 +137,8 @@ struct PagedArgs {
 cudaError_t launch_attention_simt(const AttnArgs &a, int dtype, cudaStream_t stream);
 // returns cudaErrorNotSupported when no tensor-core instantiation fits
 cudaError_t launch_attention_mma(const AttnArgs &a, int dtype, int variant, cudaStream_t stream);
-// prefix and tree on tcgen05 in n_runs runs of column tiles, D = 64 or 128, block_m 32 and up: the output itself
-// with one run, else n_runs partial results
+// prefix and tree on tcgen05 in n_runs runs of column tiles, D = 64 or 128, block_m 32 and up; the runs are merged,
+// through a.part_o where that is given and pays
 cudaError_t launch_prefix_umma(const AttnArgs &a, int dtype, int n_runs, cudaStream_t stream);
 cudaError_t launch_prefix_umma_paged(const AttnArgs &a, const PagedArgs &pg, int dtype, int n_runs, cudaStream_t stream);
 // merge a.part_slots partial results into o (and lse)
