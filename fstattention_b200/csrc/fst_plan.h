@@ -82,8 +82,7 @@ inline bool prefix_umma_pays(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, in
 //                        0.92 - 1.09 otherwise, 0.56 - 0.95 up to 300
 //   D 64, block_m 32     1.01 - 1.43 from 1024 items; 0.64 - 0.85 with long lists, 0.61 - 0.97 up to 300
 // Small grids are bound by one CTA's latency, which is longer here.  With one short tile of ancestors per 64 rows at
-// D 128 both kernels wait for the same HBM bytes, and the few per cent are left to the kernel whose
-// exponents always start from the row's own maximum (largest error over 64 trees of 256 nodes 1.8e-3 against 2.3e-3).
+// D 128 both kernels wait for the same HBM bytes and are within a few per cent of one another.
 inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int ma) {
     const int64_t items = (n_q + 127) / 128 * H * Z;
     const int bound = ma / bm;                        // tiles of ancestors the caller allows for
