@@ -372,15 +372,18 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
 //   -> the status record of this build; parent is a contiguous int32 CUDA tensor [N] or [T, N], the buffers belong to the caller and
 //   the last three may be None.
 // new_metadata(parent, block_m, max_ancestors, reference_format)
-//   -> (n_trees, n_nodes, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx), buffers made here.
+//   -> (n_trees, n_nodes, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx, whether the call was
+//   captured into a graph), buffers made here.
 // A cleared status record.  Clearing one per call is a launch (about a microsecond in front of a five
 // microsecond kernel), so a thread takes them from a block that it cleared in one go on the same stream;
 // a new block is made for another stream or device and when one is used up (256 records, 4 KB,
 // returned to the allocator with the last record).  A call that is being captured into a graph
 // clears its record in the graph, for every replay: `old` if it is given.
-at::Tensor clear_record(const at::Device &dev, cudaStream_t stream, const at::Tensor &old, const char *what) {
+at::Tensor clear_record(const at::Device &dev, cudaStream_t stream, const at::Tensor &old, const char *what,
+                        bool *captured = nullptr) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) check_status(FST_ERR_CUDA, what);
+    if (captured != nullptr) *captured = capturing != cudaStreamCaptureStatusNone;
     if (capturing != cudaStreamCaptureStatusNone) {
         at::Tensor t = old.defined() ? old : empty({4}, at::kInt, dev);
         if (cudaMemsetAsync(t.data_ptr(), 0, 16, stream) != cudaSuccess) check_status(FST_ERR_CUDA, what);
@@ -453,8 +456,10 @@ PyObject *new_metadata(PyObject *const *a, Py_ssize_t n) {
     const size_t stride = fst_packed_meta_bytes(int(nb), int(bm), int(ma));
     const at::Device dev = par.device();
     const c10::cuda::CUDAGuard guard(dev);
+    bool captured = false;
     const at::Tensor packed = empty({n_trees, int64_t(stride)}, at::kByte, dev),
-                     status = clear_record(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), at::Tensor(), "fst_precompute");
+                     status = clear_record(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), at::Tensor(), "fst_precompute",
+                                           &captured);
     at::Tensor ai, am, li;
     if (a[3] == Py_True) {
         if (par.dim() == 2) {
@@ -468,8 +473,9 @@ PyObject *new_metadata(PyObject *const *a, Py_ssize_t n) {
         }
     }
     run_precompute(par, n_trees, n_nodes, bm, ma, packed, stride, status, ai, am, li);
-    return Py_BuildValue("(LLNnNNNN)", (long long)n_trees, (long long)n_nodes, THPVariable_Wrap(packed), Py_ssize_t(stride),
-                         THPVariable_Wrap(status), wrap_or_none(ai), wrap_or_none(am), wrap_or_none(li));
+    return Py_BuildValue("(LLNnNNNNO)", (long long)n_trees, (long long)n_nodes, THPVariable_Wrap(packed), Py_ssize_t(stride),
+                         THPVariable_Wrap(status), wrap_or_none(ai), wrap_or_none(am), wrap_or_none(li),
+                         captured ? Py_True : Py_False);
 }
 
 // dfs_order(parent) -> (order, new_parent, status)

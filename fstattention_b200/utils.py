@@ -44,7 +44,7 @@ class TreeMetadata:
         # attention launches that have read the packed form since it was last written: from the
         # second one on, the launch ahead of the call in the stream cannot be the writer
         self.reads_since_build = 0
-        self._captured_status = []
+        self._captured_status = []                        # records that graphs write at their replays
         self._twin = None if ancestor_idx is None else _PackedTwin(self)
 
     def _rebuilt(self) -> None:
@@ -63,9 +63,19 @@ class TreeMetadata:
             raise RuntimeError("metadata was built with reference_format=False")
         return iter((self.ancestor_idx, self.ancestor_mask, self.leaf_idx))
 
+    def _keep_captured(self, status) -> None:
+        """A graph clears and writes this record at every replay: it lives as long as the buffers, whatever record a
+        later eager build takes, and ``check`` reads it too."""
+        if not any(t is status for t in self._captured_status):
+            self._captured_status.append(status)
+
     def check(self) -> "TreeMetadata":
-        """Read the device status record (synchronises) and raise on a recorded problem."""
+        """Read the device status record (synchronises) and raise on a recorded problem - of the last build, eager
+        or replayed from a graph."""
         code, where, detail, _ = _lib.host().read_status(self.status)
+        for record in self._captured_status:
+            if code == 0 and record is not self.status:
+                code, where, detail, _ = _lib.host().read_status(record)
         if code == _lib.DEV_ANCESTOR_OVERFLOW:
             raise RuntimeError(
                 f"block {where % 65536} of tree {where // 65536} has {detail} unique ancestors, "
@@ -148,9 +158,11 @@ def build_tree_metadata(parent: TreeLike, block_m: int = 64, max_ancestors: int 
     par = _as_parent_tensor(parent, device)
     host = _lib._host or _lib.host()
     if out is None:
-        n_trees, n_nodes, packed, stride, status, ai, am, li = host.new_metadata(par, block_m, max_ancestors,
-                                                                                 bool(reference_format))
+        n_trees, n_nodes, packed, stride, status, ai, am, li, captured = host.new_metadata(par, block_m, max_ancestors,
+                                                                                           bool(reference_format))
         meta = TreeMetadata(n_trees, n_nodes, block_m, max_ancestors, packed, stride, status, ai, am, li, par.dim() == 2)
+        if captured:
+            meta._keep_captured(status)
         if ai is not None:
             setattr(ai, _ORIGIN_ATTR, meta._twin)
     else:
@@ -158,12 +170,13 @@ def build_tree_metadata(parent: TreeLike, block_m: int = 64, max_ancestors: int 
         n_trees, n_nodes = par.shape if par.dim() == 2 else (1, par.shape[0])
         if (meta.n_trees, meta.n_nodes, meta.block_m, meta.max_ancestors) != (n_trees, n_nodes, block_m, max_ancestors):
             raise ValueError("out= metadata has a different shape")
+        for record in meta._captured_status:              # what a replay has left there is about an older build
+            if record is not meta.status:
+                record.zero_()
         status = host.precompute(par, block_m, max_ancestors, meta.packed, meta.tree_stride, meta.status,
                                  meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx)
-        if status is meta.status:
-            # captured into a graph, which clears and writes this record at every replay: it lives as long as the
-            # buffers, whatever record a later eager call takes
-            meta._captured_status.append(status)
+        if status is meta.status:                         # captured into a graph
+            meta._keep_captured(status)
         meta.status = status
         meta._rebuilt()
     if check:

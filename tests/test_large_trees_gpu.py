@@ -113,3 +113,35 @@ def test_a_captured_build_keeps_its_status_record(fst):
     want = meta.packed.clone()
     graph.replay()
     assert torch.equal(meta.packed, want) and meta.check() is meta
+
+
+@pytest.mark.parametrize("made_in_graph", [False, True])
+def test_check_sees_what_a_replay_reports(fst, made_in_graph):
+    """A problem that only a replay meets is reported by ``check``, also after an eager build in between; the next
+    build, eager or replayed, starts afresh."""
+    good = torch.tensor([-1] + [i // 2 for i in range(255)], dtype=torch.int32, device="cuda")
+    par = good.clone()
+    build = lambda **kw: fst.build_tree_metadata(par, 64, 128, reference_format=False, check=False, **kw)
+    meta = build()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        meta = build() if made_in_graph else build(out=meta)
+        build(out=meta)
+    build(out=meta)
+    assert len(meta._captured_status) == 1
+    par[100] = 200
+    graph.replay()
+    with pytest.raises(ValueError, match="malformed"):
+        meta.check()
+    par.copy_(good)
+    graph.replay()
+    meta.check()
+    par[0] = 7
+    graph.replay()
+    par.copy_(good)
+    build(out=meta)
+    meta.check()
+    par[:] = torch.arange(-1, 255, device="cuda")         # a chain: 255 ancestors
+    graph.replay()
+    with pytest.raises(RuntimeError, match="unique ancestors"):
+        meta.check()
