@@ -302,7 +302,8 @@ int fst_attention_fwd_gqa(const void *q, const void *k, const void *v, void *o, 
  * k_pool / v_pool: element (page, row, head, d) at page * pool_stride_page + row * pool_stride_row
  * + head * pool_stride_head + d (element strides, multiples of 8).  page_size 16, 32, 64 or 128;
  * head_dim 64 or 128; fp16 / bf16.  max_prefix >= every prefix_lens[z] (it sizes the grid; lengths
- * above it are cut).  Prefix and tree go to the tcgen05 kernel in kv_splits runs, partial results
+ * above it are cut; rows of a page past a
+ * sequence's length may hold anything).  Prefix and tree go to the tcgen05 kernel in kv_splits runs, partial results
  * of more than one run through `workspace`
  * (fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits) bytes).  A page number
  * outside [0, n_pages) reads as zeros and sets FST_DEV_INDEX_RANGE.  block_table and prefix_lens

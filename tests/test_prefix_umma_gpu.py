@@ -78,6 +78,36 @@ def test_paged_lengths_of_their_own(fst):
     assert fst.last_status() == 0
 
 
+@pytest.mark.parametrize("ps", [16, 64, 128])
+@pytest.mark.parametrize("n,H,H_kv,D", [(70, 4, 4, 128), (200, 4, 2, 64), (30, 8, 2, 128), (60, 16, 2, 64)])
+def test_paged_rows_past_the_end(fst, ps, n, H, H_kv, D):
+    """What the pool holds past a sequence's end - NaN, infinities - reaches nobody: the outputs are bit for bit
+    those of a pool of zeros there.  Ends before, in and behind a 16-row step, in the first, a middle and the last tile."""
+    lens = [1, 15, 16, 17, 100, 127, 128, 129, 255, 300, 383, 400]
+    Z, longest = len(lens), 400
+    meta = fst.build_tree_metadata(comb(n, 20), 32, 64, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q = torch.randn((Z, H, n, D), generator=g, device="cuda").bfloat16()
+    kt, vt = (torch.randn((Z, H_kv, n, D), generator=g, device="cuda").bfloat16() for _ in range(2))
+    per_seq = -(-longest // ps)
+    pool = torch.randn((2, Z * per_seq, ps, H_kv, D), generator=g, device="cuda").bfloat16()
+    table = torch.randperm(Z * per_seq, generator=g, device="cuda", dtype=torch.int32).view(Z, per_seq)
+    past = torch.zeros((Z * per_seq, ps), dtype=torch.bool, device="cuda")
+    for z, end in enumerate(lens):
+        for i in range(per_seq):
+            past[table[z, i].long(), max(0, min(ps, end - i * ps)):] = True
+    lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    for splits in (None, 1, 2, 3):
+        outs = []
+        for fill in (0.0, float("nan"), float("inf")):
+            pool[:, past] = fill
+            outs.append(fst.fst_attention_paged(q, kt, vt, meta, pool[0], pool[1], table, lens, D ** -0.5, max_prefix=longest,
+                                                kv_splits=splits, return_lse=True))
+        for o, lse in outs:
+            assert torch.isfinite(o).all() and torch.equal(o, outs[0][0]) and torch.equal(lse, outs[0][1]), splits
+    assert fst.last_status() == 0
+
+
 def test_lineage_on_the_host_is_checked_there(fst):
     """The bound at which a lineage on the host is refused is the device's, and so is the message."""
     par = comb(300, 90)
