@@ -264,6 +264,8 @@ Packed pack_reference(PyObject *idx, PyObject *mask, PyObject *leaf, int64_t Z, 
         (am.scalar_type() != at::kBool && am.scalar_type() != at::kByte))
         raise(PyExc_TypeError, "metadata dtypes must be int64 / bool / int64");
     if (n_meta != 1 && n_meta != Z) raise(PyExc_ValueError, "metadata must describe one tree or one tree per batch element");
+    if (am.numel() < n_meta * nb * bm * ma || li.numel() < n_meta * nb * bm)
+        raise(PyExc_ValueError, "ancestor_mask and leaf_idx must describe as many trees as ancestor_idx");
     ai = ai.contiguous(); am = am.contiguous(); li = li.contiguous();
     Packed p;
     p.n_trees = n_meta;
