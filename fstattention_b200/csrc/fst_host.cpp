@@ -309,8 +309,8 @@ PyObject *pack(PyObject *const *a, Py_ssize_t n) {
 PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 19);
     const at::Tensor &q = tensor(a[0]), &kt = tensor(a[1]), &vt = tensor(a[2]), &kp = tensor(a[10]), &vp = tensor(a[11]),
-                     &table = tensor(a[13]), &lens = tensor(a[14]);
-    for (const at::Tensor *t : {&q, &kt, &vt, &kp, &vp, &table, &lens})
+                     &table = tensor(a[13]), &given_lens = tensor(a[14]);
+    for (const at::Tensor *t : {&q, &kt, &vt, &kp, &vp, &table, &given_lens})
         if (!t->is_cuda()) raise(PyExc_RuntimeError, "fst_attention_paged runs on CUDA tensors only; there is no CPU path");
     const at::ScalarType type = q.scalar_type();
     bool same = type == at::kHalf || type == at::kBFloat16;
@@ -325,8 +325,8 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
     if (kp.dim() != 4 || vp.sizes() != kp.sizes() || kp.size(head_dim) != H_kv || kp.size(3) != D ||
         kp.strides() != vp.strides() || kp.stride(3) != 1)
         raise(PyExc_ValueError, "pools must be two equally laid out [n_pages, page_size, H_kv, D] (or HND) tensors");
-    if (table.scalar_type() != at::kInt || lens.scalar_type() != at::kInt || table.dim() != 2 || table.size(0) != Z ||
-        lens.dim() != 1 || lens.size(0) != Z || !table.is_contiguous())
+    if (table.scalar_type() != at::kInt || given_lens.scalar_type() != at::kInt || table.dim() != 2 || table.size(0) != Z ||
+        given_lens.dim() != 1 || given_lens.size(0) != Z || !table.is_contiguous())
         raise(PyExc_ValueError, "block_table must be contiguous int32 [Z, pages], prefix_lens int32 [Z]");
     const int64_t n_trees = integer(a[6]), n_blocks = integer(a[7]), bm = integer(a[8]), ma = integer(a[9]);
     if ((n_trees != 1 && n_trees != Z) || n_blocks != (n_q + bm - 1) / bm) raise(PyExc_ValueError, "metadata does not match q");
@@ -344,6 +344,7 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
         }
     }
     const c10::cuda::CUDAGuard guard(dev);
+    const at::Tensor lens = given_lens.contiguous();      // the kernel reads length z at word z
     at::Tensor ws;
     size_t ws_bytes = 0;
     if (sp.workspace) {

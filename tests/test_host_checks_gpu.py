@@ -29,3 +29,18 @@ def test_reference_tensors_describe_the_same_trees(fst):
     # one list of ancestors: the first tree of the others, as ever
     assert torch.equal(fst.fst_attention(q, k, v, idx[0], mask, leaf, **args), want)
     assert torch.equal(fst.fst_attention(q, k, v, idx[:1], mask[:1], leaf[0], **args), want)
+
+
+def test_paged_prefix_lengths_of_any_stride(fst):
+    """Lengths out of a column of a table, and one length for all."""
+    Z, H, n, D, ps = 3, 2, 20, 128, 16
+    meta = fst.build_tree_metadata([-1] + [0] * (n - 1), 32, 32, reference_format=False)
+    q, k, v = qkv(Z, H, n, D)
+    pool = torch.randn((2, Z * 8, ps, H, D), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda").half()
+    table = torch.arange(Z * 8, dtype=torch.int32, device="cuda").view(Z, 8)
+    wide = torch.tensor([[100, 0], [7, 128], [128, 3]], dtype=torch.int32, device="cuda")
+    for lens in (wide[:, 0], wide[:1, 0].expand(Z)):
+        assert not lens.is_contiguous()
+        got, want = (fst.fst_attention_paged(q, k, v, meta, pool[0], pool[1], table, x, 0.1, max_prefix=128)
+                     for x in (lens, lens.clone(memory_format=torch.contiguous_format)))
+        assert torch.equal(got, want)
