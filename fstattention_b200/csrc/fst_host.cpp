@@ -131,6 +131,10 @@ int dtype_code(at::ScalarType t) {
         default: return -1;
     }
 }
+// A kernel takes plain addresses: one of another device, or of the host, would be a fault there.
+void on_device(const at::Tensor &t, const at::Device &dev) {
+    if (t.device() != dev) raise(PyExc_RuntimeError, "all tensors of a call must be on one device");
+}
 void head_contiguous(const at::Tensor &t) {
     if (t.stride(3) != 1) raise(PyExc_ValueError, "the head dimension must be contiguous");
 }
@@ -153,6 +157,8 @@ Call open_call(PyObject *q, PyObject *k, PyObject *v, PyObject *out, PyObject *s
     if (c.D != 16 && c.D != 32 && c.D != 64 && c.D != 128) raise(PyExc_AssertionError, "head dimension must be 16, 32, 64 or 128");
     if (!c.q.is_cuda() || !c.k.is_cuda() || !c.v.is_cuda())
         raise(PyExc_RuntimeError, "fst_attention runs on CUDA tensors only; there is no CPU path");
+    on_device(c.k, c.q.device());
+    on_device(c.v, c.q.device());
     const at::ScalarType type = c.q.scalar_type();
     c.dtype = dtype_code(type);
     if (c.dtype < 0 || c.k.scalar_type() != type || c.v.scalar_type() != type)
@@ -166,6 +172,7 @@ Call open_call(PyObject *q, PyObject *k, PyObject *v, PyObject *out, PyObject *s
     } else {
         c.o = tensor(out);
         if (c.o.sizes() != c.q.sizes() || c.o.scalar_type() != type || !c.o.is_cuda()) raise(PyExc_ValueError, "out must match q");
+        on_device(c.o, c.q.device());
     }
     const double s = real(scale);
     if (!std::isfinite(s)) raise(PyExc_ValueError, "sm_scale must be finite");
@@ -234,6 +241,7 @@ PyObject *attention(PyObject *const *a, Py_ssize_t n) {
     if (n_blocks != (c.n_q + bm - 1) / bm) raise(PyExc_ValueError, "metadata block count does not match q");
     const at::Device dev = c.q.device();
     const c10::cuda::CUDAGuard guard(dev);
+    on_device(tensor(a[4]), dev);
     void *status = status_of(dev, true)->data_ptr();
     void *stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     return launch(c, tensor(a[4]).data_ptr(), n_trees > 1 ? size_t(integer(a[5])) : 0, bm, ma, int(integer(a[11])),
@@ -253,6 +261,7 @@ Packed pack_reference(PyObject *idx, PyObject *mask, PyObject *leaf, int64_t Z, 
     at::Tensor ai = tensor(idx), am = tensor(mask), li = tensor(leaf);
     if (!ai.is_cuda() || !am.is_cuda() || !li.is_cuda())
         raise(PyExc_RuntimeError, "metadata tensors must be on the GPU (call .to('cuda') as the reference does)");
+    for (const at::Tensor *t : {&ai, &am, &li}) on_device(*t, dev);
     if (bm <= 0 || ma <= 0) raise(PyExc_ValueError, "metadata shapes do not match BLOCK_M / MAX_ANCESTORS / q");
     const int64_t nb = (n_q + bm - 1) / bm, n_meta = ai.dim() == 3 ? ai.size(0) : 1;
     const auto shaped = [](const at::Tensor &t, at::IntArrayRef want) {
@@ -333,6 +342,7 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
     Call c = open_call(a[0], a[1], a[2], a[3], a[16], a[18] == Py_True);
     const int64_t max_prefix = integer(a[15]);
     const at::Device dev = q.device();
+    for (const at::Tensor *t : {&kp, &vp, &table, &given_lens, &tensor(a[4])}) on_device(*t, dev);
     std::optional<long long> asked = optional_int(a[17]);
     Splits sp{asked ? int(*asked) : 1, false};
     if (max_prefix > 0 && (!asked || *asked > 0)) {
@@ -417,6 +427,8 @@ void run_precompute(const at::Tensor &par, int64_t n_trees, int64_t n_nodes, int
                     size_t stride, const at::Tensor &status, const at::Tensor &ai, const at::Tensor &am,
                     const at::Tensor &li) {
     const at::Device dev = par.device();
+    for (const at::Tensor *t : {&packed, &status, &ai, &am, &li})
+        if (t->defined()) on_device(*t, dev);
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     check_status(fst_precompute(static_cast<const int32_t *>(par.data_ptr()), int(n_trees), int(n_nodes), int(bm), int(ma),
                                 ai.defined() ? static_cast<int64_t *>(ai.data_ptr()) : nullptr,

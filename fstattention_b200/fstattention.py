@@ -163,6 +163,8 @@ def _scattered(q, k, v, meta, tensors, sm_scale, kern, scatter, out, return_lse)
             raise ValueError("metadata must describe one tree or one tree per batch element")
         if meta.n_blocks != -(-n_q // block_m):
             raise ValueError("metadata block count does not match q")
+    if any(t.device != dev for t in (k, v, o, packed)):
+        raise RuntimeError("all tensors of a call must be on one device")
     lse = torch.empty((Z * H, n_q), device=dev, dtype=torch.float32) if return_lse else None
     with torch.cuda.device(dev):
         if meta is not None:

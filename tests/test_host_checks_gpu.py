@@ -44,3 +44,31 @@ def test_paged_prefix_lengths_of_any_stride(fst):
         got, want = (fst.fst_attention_paged(q, k, v, meta, pool[0], pool[1], table, x, 0.1, max_prefix=128)
                      for x in (lens, lens.clone(memory_format=torch.contiguous_format)))
         assert torch.equal(got, want)
+
+
+def test_tensors_of_one_device(fst):
+    """Metadata buffers that were moved to the host (or, with two GPUs, tensors of the other one) are refused."""
+    n = 40
+    par = torch.tensor([-1] + [0] * (n - 1), dtype=torch.int32, device="cuda")
+    meta = fst.build_tree_metadata(par, 32, 32, reference_format=False)
+    q, k, v = qkv(1, 2, n, 128)
+    pool = torch.zeros((4, 16, 2, 128), dtype=torch.float16, device="cuda")
+    table, lens = torch.zeros((1, 4), dtype=torch.int32, device="cuda"), torch.tensor([40], dtype=torch.int32, device="cuda")
+    elsewhere = ["cpu"] + ["cuda:1"] * (torch.cuda.device_count() > 1)
+    for other in elsewhere:
+        meta.packed = meta.packed.to(other)
+        for call in (lambda: fst.fst_attention(q, k, v, meta, sm_scale=0.1),
+                     lambda: fst.fst_attention(q.float(), k.float(), v.float(), meta, sm_scale=0.1),
+                     lambda: fst.fst_attention_paged(q, k, v, meta, pool, pool, table, lens, 0.1, max_prefix=40),
+                     lambda: fst.build_tree_metadata(par, 32, 32, out=meta)):
+            with pytest.raises(RuntimeError, match="one device"):
+                call()
+        meta.packed = meta.packed.to("cuda:0")
+        for i in (1, 2):
+            args = [q, k, v]
+            args[i] = args[i].to(other)
+            with pytest.raises(RuntimeError, match="one device|CUDA tensors"):
+                fst.fst_attention(*args, meta, sm_scale=0.1)
+        with pytest.raises((RuntimeError, ValueError), match="one device|out must match"):
+            fst.fst_attention(q, k, v, meta, sm_scale=0.1, out=q.to(other))
+    fst.fst_attention(q, k, v, meta, sm_scale=0.1)
