@@ -111,6 +111,8 @@ def fst_attention(q, k, v, ancestor_idx, ancestor_mask=None, leaf_idx=None, sm_s
         raise TypeError("sm_scale is required")
     kern = _KERNELS[kernel]
     meta = ancestor_idx if isinstance(ancestor_idx, TreeMetadata) else metadata_of(ancestor_idx, ancestor_mask, leaf_idx)
+    if meta is not None and meta is not ancestor_idx and (meta.block_m != BLOCK_M or meta.max_ancestors != MAX_ANCESTORS):
+        raise ValueError("BLOCK_M / MAX_ANCESTORS differ from the ones the metadata was built with")
     if scatter is not None:
         tensors = (ancestor_idx, ancestor_mask, leaf_idx, BLOCK_M, MAX_ANCESTORS)
         return _scattered(q, k, v, meta, tensors, sm_scale, kern, scatter, out, return_lse)
@@ -119,8 +121,6 @@ def fst_attention(q, k, v, ancestor_idx, ancestor_mask=None, leaf_idx=None, sm_s
         # the reference's three tensors (fstattention.py:153), which the call packs first
         return host.attention_ref(q, k, v, out, ancestor_idx, ancestor_mask, leaf_idx, BLOCK_M, MAX_ANCESTORS,
                                   sm_scale, kern, kv_splits, bool(return_lse))
-    if meta is not ancestor_idx and (meta.block_m != BLOCK_M or meta.max_ancestors != MAX_ANCESTORS):
-        raise ValueError("BLOCK_M / MAX_ANCESTORS differ from the ones the metadata was built with")
     # From the second launch after the precompute on, the launch ahead of this one in the stream
     # cannot be the metadata's writer: the kernel may then fetch its index lists while that launch
     # drains (FST_KERNEL_FLAG_META_STABLE).

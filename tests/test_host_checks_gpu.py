@@ -72,3 +72,23 @@ def test_tensors_of_one_device(fst):
         with pytest.raises((RuntimeError, ValueError), match="one device|out must match"):
             fst.fst_attention(q, k, v, meta, sm_scale=0.1, out=q.to(other))
     fst.fst_attention(q, k, v, meta, sm_scale=0.1)
+
+
+def test_block_size_of_the_metadata_tensors(fst):
+    """Tensors of one block size with another BLOCK_M or MAX_ANCESTORS beside them, with and without ``scatter``."""
+    class Copy:
+        n_ranks, rank, z0, h0 = 1, 0, 0, 0
+
+    import ctypes
+    n = 64
+    three = tuple(fst.build_tree_metadata([-1] + [0] * (n - 1), 32, 64))
+    q, k, v = qkv(1, 2, n, 64)
+    to = Copy()
+    to.local = torch.empty_like(q)
+    to.pointer_array = (ctypes.c_void_p * 1)(to.local.data_ptr())
+    for scatter in (None, to):
+        for bm, ma in ((64, 64), (32, 32), (64, 32)):
+            with pytest.raises(ValueError, match="BLOCK_M / MAX_ANCESTORS"):
+                fst.fst_attention(q, k, v, *three, sm_scale=0.1, BLOCK_M=bm, MAX_ANCESTORS=ma, scatter=scatter)
+    want = fst.fst_attention(q, k, v, *three, sm_scale=0.1, BLOCK_M=32, MAX_ANCESTORS=64)
+    assert torch.equal(fst.fst_attention(q, k, v, *three, sm_scale=0.1, BLOCK_M=32, MAX_ANCESTORS=64, scatter=to), want)
