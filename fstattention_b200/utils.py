@@ -58,6 +58,23 @@ class TreeMetadata:
         """True while nobody has modified the three reference-format tensors in place."""
         return self._twin is None or self._twin.versions == _versions((self.ancestor_idx, self.ancestor_mask, self.leaf_idx))
 
+    # Saved or deep-copied metadata has tensors of its own, and a twin that belongs to them.
+    def __getstate__(self):
+        return dict(self.__dict__, _twin=self.tensors_untouched())
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        self._twin = None if self.ancestor_idx is None else _PackedTwin(self)
+        if not state["_twin"]:
+            self._twin.versions = None
+        elif self._twin is not None:
+            setattr(self.ancestor_idx, _ORIGIN_ATTR, self._twin)
+
+    def __copy__(self):                                   # the same tensors, hence the same twin
+        other = object.__new__(type(self))
+        other.__dict__.update(self.__dict__)
+        return other
+
     def __iter__(self):
         if self.ancestor_idx is None:
             raise RuntimeError("metadata was built with reference_format=False")
@@ -116,6 +133,9 @@ class _PackedTwin:
         self.reads_since_build = 0
         self.versions = _versions(three)
         self.tensors = tuple(weakref.ref(t) for t in three)
+
+    def __reduce__(self):                                 # a tensor saved or copied on its own is a plain one
+        return type(None), ()
 
 
 def metadata_of(ancestor_idx, ancestor_mask, leaf_idx) -> Optional[_PackedTwin]:

@@ -211,3 +211,40 @@ def test_c_program_against_the_library(built_lib, tmp_path):
     assert "max-abs difference" in run.stdout
     assert "host time per fst_attention_fwd call" in run.stdout
     print(run.stdout)
+
+
+def test_metadata_and_its_tensors_can_be_copied_and_saved(built_lib):
+    """Copies keep the packed form only while their own three tensors are as they were handed out."""
+    import copy
+    import io
+    import pickle
+    from fstattention_b200 import utils
+
+    def made():
+        three = torch.zeros(2, 4, dtype=torch.long), torch.zeros(2, 32, 4, dtype=torch.bool), torch.zeros(2, 32, dtype=torch.long)
+        meta = utils.TreeMetadata(1, 64, 32, 4, torch.arange(64, dtype=torch.uint8), 64, torch.zeros(4, dtype=torch.int32), *three)
+        setattr(three[0], utils._ORIGIN_ATTR, meta._twin)
+        return meta
+
+    def saved(x):
+        f = io.BytesIO()
+        torch.save(x, f)
+        f.seek(0)
+        return torch.load(f, weights_only=False)
+
+    for how in (copy.copy, copy.deepcopy, saved, lambda x: pickle.loads(pickle.dumps(x))):
+        meta = made()
+        other = how(meta)
+        assert other.tensors_untouched() and other.n_blocks == meta.n_blocks and torch.equal(other.packed, meta.packed)
+        twin = utils.metadata_of(*other)
+        assert twin is not None and twin is other._twin and twin.packed is other.packed
+        assert utils.metadata_of(*meta) is meta._twin
+        other.ancestor_idx += 1
+        assert not other.tensors_untouched() and utils.metadata_of(*other) is None
+        assert not how(other).tensors_untouched() and utils.metadata_of(*how(other)) is None
+        if how is not copy.copy:
+            assert meta.tensors_untouched()
+            alone = how(meta.ancestor_idx)
+            assert torch.equal(alone, meta.ancestor_idx) and utils.metadata_of(alone, meta.ancestor_mask, meta.leaf_idx) is None
+    plain = utils.TreeMetadata(1, 64, 32, 4, torch.zeros(64, dtype=torch.uint8), 64, torch.zeros(4, dtype=torch.int32))
+    assert saved(plain).tensors_untouched() and saved(plain).ancestor_idx is None
