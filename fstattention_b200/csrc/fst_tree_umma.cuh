@@ -440,6 +440,8 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
     } else if (warp == 8 || warp == 9) {
         // ================================ products ================================
         const int g = warp - 8;
+        // (as every role does before its first bounded wait: the grid ahead may run longer than the bound)
+        if (a.meta_stable) asm volatile("griddepcontrol.wait;\n" ::: "memory");
         if (elect_one()) {
             const uint64_t dk = smem_desc(s_base, 16), dv = smem_desc(s_base, HALF), dv_narrow = smem_desc(s_base + TILE / 2, HALF / 2);
             const uint32_t idesc_pv = instr_desc(BF16, true, D), s_col = tmem_base + g * 128, o_col = s_col + 256;

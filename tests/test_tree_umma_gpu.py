@@ -92,6 +92,30 @@ def test_tree_umma_rounds_like_the_other_kernel(fst, D, bm, dtype):
     assert err["tree_umma"] <= 1.04 * err["tma"], err
 
 
+def test_tree_umma_behind_a_long_launch(fst):
+    """A launch that becomes resident while the one ahead runs for longer than the bound of its waits: no role's
+    bound starts before the launch ahead has ended.  (The launch ahead is one CTA that walks a long prefix.)"""
+    n, D, prefix = 64, 64, 8_000_000
+    meta = fst.build_tree_metadata([-1] + [0] * (n - 1), 64, 64, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(0)
+    long_kv = torch.randn((1, 1, prefix + n, D), generator=g, device="cuda").half()
+    q, k, v = (torch.randn((1, 4, n, D), generator=g, device="cuda").half() for _ in range(3))
+    small = lambda: fst.fst_attention(q, k, v, meta, sm_scale=0.1, kernel="tree_umma")
+    ahead = lambda: fst.fst_attention(q[:, :1], long_kv, long_kv, meta, sm_scale=0.1, kernel="tma", kv_splits=1)
+    small()
+    want = small()
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    start.record()
+    ahead()
+    end.record()
+    torch.cuda.synchronize()
+    assert start.elapsed_time(end) > 75.0                 # half as long again as the bound
+    ahead()
+    got = small()
+    torch.cuda.synchronize()
+    assert fst.last_status() == 0 and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("n,H,H_kv", [(16, 16, 2), (17, 16, 2), (32, 8, 2), (33, 8, 2), (64, 8, 4), (65, 8, 4), (9, 12, 2)])
 @pytest.mark.parametrize("D", [64, 128])
 def test_prefix_heads_share_a_query_tile(fst, n, H, H_kv, D):
