@@ -294,7 +294,7 @@ static int attention_fwd_impl(const void *q, const void *k, const void *v, void 
     const bool can_part = a.prefix > 0 && choice != FST_KERNEL_MMA && choice != FST_KERNEL_PERSIST;
     const bool want_umma = can_part && block_m >= 32 && sm_scale > 0.f &&
                            (choice == FST_KERNEL_TMA_UMMA ||
-                            (automatic && prefix_umma_pays(Z, H, H_kv, n_q, a.prefix, block_m)));
+                            (automatic && prefix_umma_pays(Z, H, H_kv, n_q, a.prefix, block_m, sm_count())));
     if (choice == FST_KERNEL_TMA_UMMA && !want_umma) return FST_ERR_UNSUPPORTED;
     if (want_umma) {
         if (workspace != nullptr && kv_splits > 1) {      // the runs may be spread, their results merged from there

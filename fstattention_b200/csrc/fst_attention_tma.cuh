@@ -787,19 +787,6 @@ inline bool make_map(CUtensorMap *map, const void *base, bool bf16, int D, int r
     });
 }
 
-// number of SMs of the current device (cached)
-inline int sm_count() {
-    static std::atomic<int> cached[kMaxDevices];
-    const int slot = current_device_slot();
-    if (slot < 0) return 148;
-    int n = cached[slot].load(std::memory_order_acquire);
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, slot) != cudaSuccess || n <= 0) n = 148;
-        cached[slot].store(n, std::memory_order_release);
-    }
-    return n;
-}
-
 template <typename T, int D, int BM, int TN, bool PFX, int NOUT>
 cudaError_t launch_tma_pfx(const AttnArgs &a, cudaStream_t stream) {
     using SM = TmaSmem<D, BM, TN>;

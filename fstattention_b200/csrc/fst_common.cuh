@@ -56,6 +56,19 @@ inline int current_device_slot() {
     return dev;
 }
 
+// number of SMs of the current device (cached)
+inline int sm_count() {
+    static std::atomic<int> cached[kMaxDevices];
+    const int slot = current_device_slot();
+    if (slot < 0) return 148;
+    int n = cached[slot].load(std::memory_order_acquire);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, slot) != cudaSuccess || n <= 0) n = 148;
+        cached[slot].store(n, std::memory_order_release);
+    }
+    return n;
+}
+
 // One-time per-device launch set-up of a kernel instantiation (the dynamic shared memory
 // attribute is per device); safe from several host threads.
 struct DeviceOnce {

@@ -104,7 +104,7 @@ Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, i
         return {1, false};
     const int64_t cap = 65535 / std::max<int64_t>(Z, 1);
     const auto clamp = [&](int64_t v) { return int(std::max<int64_t>(1, std::min(v, cap))); };
-    if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && fst::prefix_umma_pays(Z, H, H_kv, n_q, prefix, block_m))) {
+    if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && fst::prefix_umma_pays(Z, H, H_kv, n_q, prefix, block_m, sm_count(device)))) {
         const fst::PrefixPlan plan = fst::prefix_plan(Z, H, H_kv, n_q, prefix, sm_count(device), true, asked ? clamp(*asked) : 0);
         return {plan.runs, plan.spread, true};
     }

@@ -31,6 +31,7 @@ inline int prefix_heads_per_tile(int64_t H, int64_t H_kv, int64_t n_q) {
 // cluster's, 45 and 3 for every run to spread them.
 constexpr int kMaxClusterRuns = 8;     // portable cluster size
 constexpr int kMaxSpreadRuns = 16;
+constexpr int kGpcSms = 18;
 struct PrefixPlan {
     int runs;
     bool pair, spread;
@@ -48,7 +49,8 @@ inline PrefixPlan prefix_plan(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, i
         for (int pair = 0; pair < (kv_tiles > 1 ? 2 : 1); ++pair)
             for (int64_t runs = std::max<int64_t>(lo, spread ? 2 : 1); runs <= (spread ? hi : std::min<int64_t>(hi, kMaxClusterRuns)); ++runs) {
                 const int64_t ctas = Z * H_kv * ((kv_tiles + pair) / (1 + pair)) * runs;
-                const int64_t fit = spread || runs == 1 ? sms : runs == 2 ? sms / 18 * 18 : std::max<int64_t>(1, sms / 18 * (16 / runs) * runs);
+                const int64_t gpcs = sms / kGpcSms;         // (a slice of a GPU may have less than one)
+                const int64_t fit = std::max<int64_t>(1, spread || runs == 1 ? sms : runs == 2 ? gpcs * kGpcSms : gpcs * (16 / runs) * runs);
                 const int64_t waves = (ctas + fit - 1) / fit, tile = pair ? 17 : page < 32 ? 15 : 8;
                 const int64_t merge = runs == 1 ? 0 : spread ? 45 + 3 * runs : 10 + 7 * runs;
                 const int64_t cost = waves * ((tiles + runs - 1) / runs * tile + 120) + merge;
@@ -65,9 +67,9 @@ inline PrefixPlan prefix_plan(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, i
 // block_m 128 (250 nodes) 0.85 - 1.09 at 33 rows, 1.02 - 1.32 at 96, 1.30 - 1.61 at 200; block_m 64 (100
 // nodes) 0.74 - 0.91 up to 128, 0.98 - 1.18 at 200; block_m 32 (20 nodes) 0.45 - 0.96 up to 128, 1.00 - 1.22
 // at 200, but 0.60 - 0.64 where more query tiles than SMs are filled to a quarter or less.
-inline bool prefix_umma_pays(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, int64_t prefix, int64_t bm) {
+inline bool prefix_umma_pays(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, int64_t prefix, int64_t bm, int sms) {
     const int64_t pack = prefix_heads_per_tile(H, H_kv, n_q);
-    const bool sparse = n_q * pack <= 32 && Z * H / pack > 148;
+    const bool sparse = n_q * pack <= 32 && Z * H / pack > sms;
     return prefix >= (sparse ? 256 : bm >= 128 ? 96 : 192);
 }
 

@@ -725,10 +725,7 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
     });
     if (ce != cudaSuccess) return ce;
     if ((long long)a.Z * n_runs > 65535) return cudaErrorInvalidValue;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return cudaErrorInvalidDevice;
-    const PrefixPlan plan = prefix_plan(a.Z, a.H, H_kv, a.n_q, a.prefix, sms, a.part_o != nullptr, n_runs, PAGED ? pg->page_size : 128);
+    const PrefixPlan plan = prefix_plan(a.Z, a.H, H_kv, a.n_q, a.prefix, sm_count(), a.part_o != nullptr, n_runs, PAGED ? pg->page_size : 128);
     PrefixArgs pa = {};
     pa.n_runs = plan.runs;
     pa.cluster = plan.spread ? 1 : plan.runs;

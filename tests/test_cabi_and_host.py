@@ -248,3 +248,43 @@ def test_metadata_and_its_tensors_can_be_copied_and_saved(built_lib):
             assert torch.equal(alone, meta.ancestor_idx) and utils.metadata_of(alone, meta.ancestor_mask, meta.leaf_idx) is None
     plain = utils.TreeMetadata(1, 64, 32, 4, torch.zeros(64, dtype=torch.uint8), 64, torch.zeros(4, dtype=torch.int32))
     assert saved(plain).tensors_untouched() and saved(plain).ancestor_idx is None
+
+
+def test_prefix_plans_on_any_number_of_sms(tmp_path):
+    """A slice of a GPU may have fewer SMs than a GPC: every plan is one that can be launched."""
+    import shutil
+    import subprocess
+    cxx = os.environ.get("CXX") or shutil.which("g++")
+    if not cxx:
+        pytest.skip("no C++ compiler")
+    src = tmp_path / "plans.cpp"
+    src.write_text(r"""
+#include "fst_plan.h"
+#include <cstdio>
+using namespace fst;
+int main() {
+    long long plans = 0;
+    for (int sms : {1, 2, 7, 16, 17, 18, 20, 36, 74, 132, 148, 160})
+        for (int Z : {1, 3, 64, 30000})
+            for (int H_kv : {1, 2, 8})
+                for (int group : {1, 4, 8})
+                    for (int n_q : {1, 16, 64, 129, 1000})
+                        for (int prefix : {1, 128, 5000, 200000})
+                            for (int spread : {0, 1})
+                                for (int asked : {0, 1, 2, 3, 8, 16, 40}) {
+                                    const PrefixPlan p = prefix_plan(Z, H_kv * group, H_kv, n_q, prefix, sms, spread, asked);
+                                    if (p.runs < 1 || (long long)p.runs * Z > 65535 || (p.spread && (!spread || p.runs < 2)) ||
+                                        (!p.spread && p.runs > kMaxClusterRuns) || (asked > 0 && p.runs > asked)) {
+                                        std::printf("sms %d Z %d H %d/%d n_q %d prefix %d: %d runs\n", sms, Z, H_kv * group, H_kv, n_q, prefix, p.runs);
+                                        return 1;
+                                    }
+                                    prefix_umma_pays(Z, H_kv * group, H_kv, n_q, prefix, 64, sms);
+                                    ++plans;
+                                }
+    std::printf("%lld plans\n", plans);
+}
+""")
+    exe = tmp_path / "plans"
+    subprocess.run([cxx, "-O1", "-std=c++17", "-I", os.path.join(ROOT, "fstattention_b200", "csrc"), str(src), "-o", str(exe)], check=True)
+    res = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0 and "plans" in res.stdout, (res.returncode, res.stdout[-500:])
