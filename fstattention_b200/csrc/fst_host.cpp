@@ -88,22 +88,29 @@ int sm_count(int device) {
 }
 
 // ---- the runs a shared prefix is cut into -------------------------------------------------------
-// Only the tensor-core kernels split.  With head_dim 64 or 128 and at least 256 prefix rows the
-// prefix goes to the tcgen05 kernel (fst_plan.h says into how many runs).  Otherwise the tree kernel
-// walks the prefix itself, split to about four CTAs per SM.
+// Only the tensor-core kernels split.  With head_dim 64 or 128, a positive scale and as many prefix rows as
+// prefix_umma_pays asks for, the call goes to the tcgen05 kernel (fst_plan.h says in how many runs).  Otherwise
+// the tree kernel walks the prefix itself: split to about four CTAs per SM, or, where the tcgen05 kernel is
+// ruled out by the scale alone, in runs of 256 rows to about one CTA per SM and 128 query rows (8 heads of
+// 127 rows behind 4096: 21.8 us, 125 unsplit).
 struct Splits {
     int runs;
     bool workspace;
     bool umma = false;                                    // the tcgen05 prefix kernel takes the call
 };
 Splits pick_splits(const std::optional<long long> &asked, at::ScalarType type, int64_t Z, int64_t H, int64_t H_kv, int64_t n_q,
-                   int64_t D, int64_t prefix, int64_t block_m, int kernel, int device) {
+                   int64_t D, int64_t prefix, int64_t block_m, double scale, int kernel, int device) {
     if ((type != at::kHalf && type != at::kBFloat16) || (D != 64 && D != 128) ||
         (block_m != 32 && block_m != 64 && block_m != 128) || kernel == FST_KERNEL_SIMT || kernel == FST_KERNEL_MMA ||
         prefix <= 0)
         return {1, false};
     const int64_t cap = 65535 / std::max<int64_t>(Z, 1);
     const auto clamp = [&](int64_t v) { return int(std::max<int64_t>(1, std::min(v, cap))); };
+    if (kernel == FST_KERNEL_AUTO && scale <= 0.0 && prefix >= 256) {
+        const int64_t tiles = Z * H * ((n_q + 127) / 128);
+        const int runs = clamp(asked ? *asked : std::min(sm_count(device) / std::max<int64_t>(tiles, 1), prefix / 256));
+        return {runs, runs > 1};
+    }
     if (kernel == FST_KERNEL_TMA_UMMA || (kernel == FST_KERNEL_AUTO && fst::prefix_umma_pays(Z, H, H_kv, n_q, prefix, block_m, sm_count(device)))) {
         const fst::PrefixPlan plan = fst::prefix_plan(Z, H, H_kv, n_q, prefix, sm_count(device), true, asked ? clamp(*asked) : 0);
         return {plan.runs, plan.spread, true};
@@ -197,7 +204,7 @@ PyObject *launch(Call &c, const void *packed, size_t tree_stride, int64_t block_
                  const std::optional<long long> &kv_splits, void *status, void *stream) {
     const at::Device dev = c.q.device();
     const Splits sp = pick_splits(kv_splits, c.q.scalar_type(), c.Z, c.H, c.H_kv, c.n_q, c.D, c.n_kv - c.n_q, block_m,
-                                  kernel & FST_KERNEL_MASK, dev.index());
+                                  c.scale, kernel & FST_KERNEL_MASK, dev.index());
     at::Tensor ws;
     size_t ws_bytes = 0;
     if (sp.workspace) {
@@ -627,12 +634,13 @@ PyObject *attention_status(PyObject *const *a, Py_ssize_t n) {
     return THPVariable_Wrap(*status_of(at::Device(at::kCUDA, at::DeviceIndex(integer(a[0]))), true));
 }
 
-// splits(q, prefix, block_m, kernel, kv_splits) -> (runs, whether a workspace is needed)
+// splits(q, prefix, block_m, kernel, kv_splits, sm_scale) -> (runs, whether a workspace is needed, whether the tcgen05
+//   prefix kernel takes the call)
 PyObject *splits(PyObject *const *a, Py_ssize_t n) {
-    want_args(n, 5);
+    want_args(n, 6);
     const at::Tensor &q = tensor(a[0]);
     const Splits s = pick_splits(optional_int(a[4]), q.scalar_type(), q.size(0), q.size(1), q.size(1), q.size(2), q.size(3), integer(a[1]),
-                                 integer(a[2]), int(integer(a[3])), q.device().index());
+                                 integer(a[2]), real(a[5]), int(integer(a[3])), q.device().index());
     return Py_BuildValue("(iOO)", s.runs, s.workspace ? Py_True : Py_False, s.umma ? Py_True : Py_False);
 }
 

@@ -60,17 +60,17 @@ def _strides(t):
 
 
 def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[int] = None,
-                max_ancestors: int = 64) -> dict:
+                max_ancestors: int = 64, sm_scale: float = 1.0) -> dict:
     """Which kernels one ``fst_attention`` call on packed metadata launches for ``q`` (shape and
     dtype only), a shared prefix of ``prefix`` rows and the given block size, mirroring the
-    dispatch inside the library (for rows on 16-byte boundaries and a positive scale): ``{"kernels":
-    [...], "prefix_runs": r}``.  ``max_ancestors`` is the metadata's ancestor bound."""
-    splits, need_ws, umma = _lib.host().splits(q, prefix, block_m, _lib.KERNELS[kernel], kv_splits)
+    dispatch inside the library (for rows on 16-byte boundaries): ``{"kernels":
+    [...], "prefix_runs": r}``.  ``max_ancestors`` is the metadata's ancestor bound; of ``sm_scale`` the sign counts."""
+    splits, need_ws, umma = _lib.host().splits(q, prefix, block_m, _lib.KERNELS[kernel], kv_splits, sm_scale)
     tensor_core = q.dtype in (torch.float16, torch.bfloat16) and q.shape[-1] in (64, 128) \
         and block_m in (16, 32, 64, 128)
     tree = "attn_simt_kernel" if kernel == "simt" or not tensor_core else \
         "attn_mma_kernel" if kernel == "mma" or block_m == 16 else "attn_tma_kernel"
-    if tree == "attn_tma_kernel" and prefix == 0 and (kernel == "tree_umma" or (kernel == "auto" and _lib.lib().fst_attention_tree_kernel(
+    if tree == "attn_tma_kernel" and prefix == 0 and (kernel == "tree_umma" or (kernel == "auto" and sm_scale > 0 and _lib.lib().fst_attention_tree_kernel(
             q.shape[0], q.shape[1], q.shape[2], q.shape[3], block_m, max_ancestors) == _KERNELS["tree_umma"])):
         tree = "tree_umma_kernel"
     if kernel == "persist" and tree == "attn_tma_kernel" and prefix == 0 and block_m in (64, 128):

@@ -288,3 +288,16 @@ int main() {
     subprocess.run([cxx, "-O1", "-std=c++17", "-I", os.path.join(ROOT, "fstattention_b200", "csrc"), str(src), "-o", str(exe)], check=True)
     res = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert res.returncode == 0 and "plans" in res.stdout, (res.returncode, res.stdout[-500:])
+
+
+@pytest.mark.parametrize("H,n,prefix", [(8, 127, 4096), (32, 127, 4096), (4, 127, 16384), (1, 20, 600)])
+def test_a_scale_that_the_prefix_kernel_does_not_take_is_split(built_lib, H, n, prefix):
+    """Behind a long prefix a scale of zero or below goes to the tree kernel, which walks the prefix in runs."""
+    import fstattention_b200 as fst
+    q = torch.empty((1, H, n, 128), dtype=torch.float16)
+    assert fst.launch_plan(q, prefix, 64)["kernels"][0] == "prefix_umma_kernel"
+    for scale in (-0.1, 0.0):
+        plan = fst.launch_plan(q, prefix, 64, sm_scale=scale)
+        assert plan["kernels"] == ["attn_tma_kernel", "combine_splits_kernel"] and plan["prefix_runs"] > 1, plan
+        assert fst.launch_plan(q, prefix, 64, kv_splits=3, sm_scale=scale)["prefix_runs"] == 3
+        assert fst.launch_plan(q, 0, 64, sm_scale=scale) == {"kernels": ["attn_tma_kernel"], "prefix_runs": 1}
