@@ -634,12 +634,14 @@ PyObject *attention_status(PyObject *const *a, Py_ssize_t n) {
     return THPVariable_Wrap(*status_of(at::Device(at::kCUDA, at::DeviceIndex(integer(a[0]))), true));
 }
 
-// splits(q, prefix, block_m, kernel, kv_splits, sm_scale) -> (runs, whether a workspace is needed, whether the tcgen05
+// splits(q, prefix, block_m, kernel, kv_splits, sm_scale, kv_heads) -> (runs, whether a workspace is needed, whether the tcgen05
 //   prefix kernel takes the call)
 PyObject *splits(PyObject *const *a, Py_ssize_t n) {
-    want_args(n, 6);
+    want_args(n, 7);
     const at::Tensor &q = tensor(a[0]);
-    const Splits s = pick_splits(optional_int(a[4]), q.scalar_type(), q.size(0), q.size(1), q.size(1), q.size(2), q.size(3), integer(a[1]),
+    const int64_t H = q.size(1), H_kv = integer(a[6]);
+    if (H_kv < 1 || H % H_kv) raise(PyExc_ValueError, "the heads of q must be a multiple of kv_heads");
+    const Splits s = pick_splits(optional_int(a[4]), q.scalar_type(), q.size(0), H, H_kv, q.size(2), q.size(3), integer(a[1]),
                                  integer(a[2]), real(a[5]), int(integer(a[3])), q.device().index());
     return Py_BuildValue("(iOO)", s.runs, s.workspace ? Py_True : Py_False, s.umma ? Py_True : Py_False);
 }

@@ -60,12 +60,14 @@ def _strides(t):
 
 
 def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[int] = None,
-                max_ancestors: int = 64, sm_scale: float = 1.0) -> dict:
+                max_ancestors: int = 64, sm_scale: float = 1.0, kv_heads: Optional[int] = None) -> dict:
     """Which kernels one ``fst_attention`` call on packed metadata launches for ``q`` (shape and
     dtype only), a shared prefix of ``prefix`` rows and the given block size, mirroring the
     dispatch inside the library (for rows on 16-byte boundaries): ``{"kernels":
-    [...], "prefix_runs": r}``.  ``max_ancestors`` is the metadata's ancestor bound; of ``sm_scale`` the sign counts."""
-    splits, need_ws, umma = _lib.host().splits(q, prefix, block_m, _lib.KERNELS[kernel], kv_splits, sm_scale)
+    [...], "prefix_runs": r}``.  ``max_ancestors`` is the metadata's ancestor bound; of ``sm_scale`` the sign counts,
+    and ``kv_heads`` are the heads of K and V where they are fewer than those of ``q``."""
+    splits, need_ws, umma = _lib.host().splits(q, prefix, block_m, _lib.KERNELS[kernel], kv_splits, sm_scale,
+                                               q.shape[1] if kv_heads is None else kv_heads)
     tensor_core = q.dtype in (torch.float16, torch.bfloat16) and q.shape[-1] in (64, 128) \
         and block_m in (16, 32, 64, 128)
     tree = "attn_simt_kernel" if kernel == "simt" or not tensor_core else \

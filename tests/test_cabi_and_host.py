@@ -301,3 +301,15 @@ def test_a_scale_that_the_prefix_kernel_does_not_take_is_split(built_lib, H, n, 
         assert plan["kernels"] == ["attn_tma_kernel", "combine_splits_kernel"] and plan["prefix_runs"] > 1, plan
         assert fst.launch_plan(q, prefix, 64, kv_splits=3, sm_scale=scale)["prefix_runs"] == 3
         assert fst.launch_plan(q, 0, 64, sm_scale=scale) == {"kernels": ["attn_tma_kernel"], "prefix_runs": 1}
+
+
+def test_launch_plan_of_grouped_queries(built_lib):
+    """Heads of a group share query tiles behind a prefix, so there are fewer tiles and more runs of each."""
+    import fstattention_b200 as fst
+    q = torch.empty((1, 32, 16, 128), dtype=torch.float16)      # eight heads of sixteen rows fill a query tile
+    own, grouped = (fst.launch_plan(q, 8192, 64, **kw) for kw in ({}, {"kv_heads": 4}))
+    assert own["prefix_runs"] == fst.launch_plan(q, 8192, 64, kv_heads=32)["prefix_runs"]
+    one_tile = fst.launch_plan(torch.empty((1, 4, 128, 128), dtype=torch.float16), 8192, 64)     # what a group amounts to
+    assert grouped["prefix_runs"] == one_tile["prefix_runs"] > own["prefix_runs"]
+    with pytest.raises(ValueError, match="multiple"):
+        fst.launch_plan(q, 8192, 64, kv_heads=5)
