@@ -102,13 +102,15 @@ attn_simt_kernel(const AttnArgs a) {
             s[u] = key[u] >= 0 ? dot * a.scale_log2 : -INFINITY;
             mn = fmaxf(mn, s[u]);
         }
-        if (mn == -INFINITY) return;                  // no key so far (uniform within the group)
-        const float alpha = exp2f(m - mn);
+        // No key so far, or none with a score above -inf: weights of zero - but a NaN score, which no maximum shows,
+        // is a NaN weight, and the row's result is NaN.
+        const float base = mn == -INFINITY ? 0.f : mn;
+        const float alpha = exp2f(m - base);
         l *= alpha;
         acc.x *= alpha; acc.y *= alpha; acc.z *= alpha; acc.w *= alpha;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const float p = exp2f(s[u] - mn);
+            const float p = exp2f(s[u] - base);
             l += p;
             acc.x = fmaf(p, vr[u].x, acc.x); acc.y = fmaf(p, vr[u].y, acc.y);
             acc.z = fmaf(p, vr[u].z, acc.z); acc.w = fmaf(p, vr[u].w, acc.w);
