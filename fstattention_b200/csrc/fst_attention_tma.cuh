@@ -657,15 +657,14 @@ combine_splits_kernel(const AttnArgs a) {
         float top = big;
 #pragma unroll
         for (int u = 0; u < U; ++u) top = fmaxf(top, ls[u]);
-        if (top == -INFINITY) continue;
-        const float keep = exp2f(big - top);
+        const float base = top == -INFINITY ? 0.f : top, keep = exp2f(big - base);
         sum.x *= keep; sum.y *= keep; sum.z *= keep; sum.w *= keep;
         wsum *= keep;
         big = top;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (ls[u] == -INFINITY) continue;            // an empty run: its O row is not meaningful
-            const float w = exp2f(ls[u] - big);
+            const float w = exp2f(ls[u] - base);
             sum.x = fmaf(w, v[u].x, sum.x); sum.y = fmaf(w, v[u].y, sum.y);
             sum.z = fmaf(w, v[u].z, sum.z); sum.w = fmaf(w, v[u].w, sum.w);
             wsum += w;

@@ -659,8 +659,8 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         const int node = row & ((1 << pa.pack_shift) - 1), gr = (first ? tile_a.q0 : tile_b.q0) + node;
         const int h = (first ? tile_a.h : tile_b.h) + ((row & 127) >> pa.pack_shift);
         if (node >= (first ? tile_a.rows : tile_b.rows)) continue;
-        const float inv = l > 0.f ? 1.f / l : 0.f;
-        const float lse = l > 0.f ? mu + log2f(l) : -INFINITY;
+        const float inv = l == 0.f ? 0.f : 1.f / l;       // (a NaN stays one: no maximum shows it, but the sum does)
+        const float lse = l == 0.f ? -INFINITY : mu + log2f(l);
         if (partial) {
             const size_t slot_row = ((size_t(run) * a.Z + z) * a.H + h) * n_q + gr;
             float4 *to = reinterpret_cast<float4 *>(a.part_o + slot_row * D);

@@ -128,3 +128,32 @@ def test_lineage_on_the_host_is_checked_there(fst):
     bad[5, level[5] - 1] = 7
     with pytest.raises(ValueError, match="malformed"):
         fst.create_fst_attention_kernel_inputs(bad, level, 64, 128)
+
+
+@pytest.mark.parametrize("D,H,H_kv", [(128, 2, 2), (64, 4, 2)])
+@pytest.mark.parametrize("prefix", [1, 129, 300, 2000])
+def test_nan_keys_reach_their_rows(fst, prefix, D, H, H_kv):
+    """A NaN key is seen by every row that attends to it and by no other: as the only key of a tile or of a run, in
+    the prefix and in the tree, with runs in a cluster and spread."""
+    n = 70
+    par = comb(n, 30)
+    attends = torch.zeros((n, prefix + n), dtype=torch.bool)
+    attends[:, :prefix] = True
+    for i in range(n):
+        x = i
+        while x >= 0:
+            attends[i, prefix + x] = True
+            x = par[x]
+    meta = fst.build_tree_metadata(par, 32, 64, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(prefix)
+    q = torch.randn((1, H, n, D), generator=g, device="cuda").half()
+    k, v = (torch.randn((1, H_kv, prefix + n, D), generator=g, device="cuda").half() for _ in range(2))
+    for x in (0, prefix - 1, prefix, prefix + 29, prefix + 50):
+        bad = k.clone()
+        bad[:, :, x, 3] = float("nan")
+        for splits in (None, 1, 2, 3, 12):
+            o, lse = fst.fst_attention(q, bad, v, meta, sm_scale=0.1, kernel="tma_umma", kv_splits=splits, return_lse=True)
+            for h in range(H):
+                assert torch.equal(o[0, h].isnan().all(-1).cpu(), attends[:, x]), (x, splits)
+                assert torch.equal(o[0, h].isnan().any(-1).cpu(), attends[:, x]), (x, splits)
+                assert torch.equal(lse[h].isnan().cpu(), attends[:, x]), (x, splits)
