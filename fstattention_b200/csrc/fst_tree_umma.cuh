@@ -14,10 +14,12 @@
 //            tile is narrow - BM / 2 columns for each block - when the lists end in its first half.
 //   S = Q K^T     M 128, N 128 (64), both operands in shared memory (128-byte swizzle)
 //   softmax       thread r of a group owns row r and looks only at its block's columns; 32-column
-//                 words in which no row of its warp has a mask bit are not even read; P (zeros
-//                 outside the block's columns) goes back over S in tensor memory
+//                 words in which no row of its warp has a mask bit are not even read; P goes back
+//                 over S in tensor memory
 //   O += P V      A = P from tensor memory, V from shared memory (MN-major); 16-column steps
-//                 beyond every block's list are left out
+//                 beyond every block's list are left out, and a step adds to the rows that have a column in it
+//                 and to no others (O starts as zeros): zero times a V that is not finite would be NaN in rows
+//                 that do not attend to it, 128 of them.  Nor need P then be cleared where a warp has no column
 //
 // Sixteen warps.  Warps 0-3 and 4-7 are two softmax groups: group g takes the CTA's items g, g + 2, ... and
 // owns an S/P buffer and an accumulator (TMEM: 2 x 128 columns each), so that one group's latencies hide
@@ -77,7 +79,8 @@ struct Geo {
     static constexpr int OFF_BAR = POOL * TILE;
     static constexpr int N_BAR = 2 * POSITIONS + POOL + TURNS + 2 * ITEMS + 6;
     static constexpr int OFF_INFO = OFF_BAR + (N_BAR + 1) / 2 * 16;   // ItemInfo per item in flight
-    static constexpr int OFF_WHERE = OFF_INFO + ITEMS * 32;           // which buffer a position's tile is in; then the TMEM address
+    static constexpr int OFF_ROWS = OFF_INFO + ITEMS * 32;            // [group][step][warp] rows with columns in a 16-column step
+    static constexpr int OFF_WHERE = OFF_ROWS + 2 * 8 * 16;           // which buffer a position's tile is in; then the TMEM address
     static constexpr int SMEM_BYTES = OFF_WHERE + 2 * POSITIONS + 16 + 1024;  // + slack to align the base to 1 KB
     static_assert(SMEM_BYTES <= 227 * 1024, "one CTA's shared memory");
 };
@@ -486,13 +489,14 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                     ++at;
                     const uint64_t dvs = (narrow ? dv_narrow : dv) + uint64_t(b * (TILE >> 4));
                     fence_after_sync();
-                    bool more = t > 0;
-#pragma unroll 1
-                    for (uint32_t rest = steps; rest != 0u; rest &= rest - 1) {
-                        const int ks = __ffs(rest) - 1;
-                        mma_f16_ts(o_col, s_col + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, more);
-                        more = true;
-                    }
+                    const uint4 *rows = reinterpret_cast<const uint4 *>(smem + G::OFF_ROWS) + g * 8;
+                    uint4 on[8];
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks) on[ks] = rows[ks];
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks)
+                        if ((steps >> ks) & 1u)
+                            mma_f16_ts_rows(o_col, s_col + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, on[ks]);
                     mma_commit(bar_empty + b * 8);
                     if (t + 1 == tiles) mma_commit(bar_o + g * 8);
                 }
@@ -563,6 +567,11 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             const int4 in = info[(n % ITEMS) * 2];
             const int tiles = in.x;
             float m_ref = -INFINITY, l = 0.f;
+            uint32_t zero[16];                            // my row of O, while S is on its way
+#pragma unroll
+            for (int c = 0; c < 16; ++c) zero[c] = 0u;
+#pragma unroll 1
+            for (int c0 = 0; c0 < D; c0 += 16) tmem_st16(tmem_o + c0, zero);
 #pragma unroll 1
             for (int t = 0; t < tiles; ++t, ++tile_no) {
                 uint32_t word[NW];
@@ -580,8 +589,18 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 fence_after_sync();
 
                 uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
+                {
+                    uint32_t on = 0;                      // lane k: rows of my warp with a column in step k of the tile
+                    const int k = lane - sub * segw * 2;
 #pragma unroll
-                for (int i = 0; i < NW; ++i) live |= uint32_t(__any_sync(0xffffffffu, word[i] != 0u)) << i;
+                    for (int i = 0; i < NW; ++i) {
+                        const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
+                        live |= uint32_t((lo | hi) != 0u) << i;
+                        if (k == 2 * i) on = lo;
+                        if (k == 2 * i + 1) on = hi;
+                    }
+                    if (lane < 8) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * 8 + lane) * 4 + (warp & 3)] = on;
+                }
                 float sum[2] = {0.f, 0.f}, mu = 0.f, mx = -INFINITY;
                 // My live words, WT to a turn.  First round: the row's maximum, then the reference point.  Second round (or
                 // at once, when one turn was all): probabilities, over S - word i of P covers columns 16 i .. of S,
@@ -660,15 +679,6 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                     }
                 }
                 l += sum[0] + sum[1];
-                {
-                    uint32_t zero[16];
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) zero[c] = 0u;
-                    const uint32_t mine = live << (sub * segw);
-#pragma unroll 1
-                    for (int i = 0; i < SUB * segw; ++i)
-                        if (!((mine >> i) & 1u)) tmem_st16(tmem_s + i * 16, zero);
-                }
                 tmem_st_wait();
                 fence_before_sync();
                 arrive(bar_p + g * 8);

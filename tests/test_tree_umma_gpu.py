@@ -92,6 +92,39 @@ def test_tree_umma_rounds_like_the_other_kernel(fst, D, bm, dtype):
     assert err["tree_umma"] <= 1.04 * err["tma"], err
 
 
+def reaches(par, lo, hi):
+    """Which nodes attend to one of the nodes lo .. hi - 1."""
+    hit = torch.zeros(len(par), dtype=torch.bool)
+    for i, p in enumerate(par):
+        hit[i] = lo <= i < hi or (p >= 0 and bool(hit[p]))
+    return hit
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bm", [32, 64, 128])
+@pytest.mark.parametrize("fill", [float("nan"), float("inf")])
+def test_tree_umma_values_that_are_not_finite(fst, D, bm, fill):
+    """A row of V that is not finite reaches the rows that attend to it, and else only rows that attend to another of
+    the sixteen columns of one step of the product - not the rest of the item, whose weights for it are zero."""
+    n = 300
+    par = [-1] + [(i - 1) // 3 for i in range(1, n)]
+    meta = fst.build_tree_metadata(par, bm, 256, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(bm)
+    q, k, v = (torch.randn((2, 3, n, D), generator=g, device="cuda").half() for _ in range(3))
+    clean = fst.fst_attention(q, k, v, meta, sm_scale=D ** -0.5, kernel="tree_umma")
+    for x in (299, 200, 137, 40, 5):
+        bad = v.clone()
+        bad[:, :, x] = fill
+        o = fst.fst_attention(q, k, bad, meta, sm_scale=D ** -0.5, kernel="tree_umma")
+        hit, near = reaches(par, x, x + 1).cuda(), reaches(par, x // 16 * 16, x // 16 * 16 + 16).cuda()
+        assert not torch.isfinite(o[:, :, hit]).any(), x
+        if not any(p == x for p in par):                  # nobody's ancestor: in its own item's tile only
+            assert torch.equal(o[:, :, ~near], clean[:, :, ~near]), x
+        block = x // 128 * 128                            # rows of earlier items do not attend to it at all
+        assert torch.equal(o[:, :, :block], clean[:, :, :block]), x
+    assert fst.last_status() == 0
+
+
 def test_tree_umma_behind_a_long_launch(fst):
     """A launch that becomes resident while the one ahead runs for longer than the bound of its waits: no role's
     bound starts before the launch ahead has ended.  (The launch ahead is one CTA that walks a long prefix.)"""
