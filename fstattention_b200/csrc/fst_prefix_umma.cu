@@ -4,7 +4,9 @@
 // row attends to every prefix row.  A CTA has one or two query tiles of 128 rows and a run of column tiles;
 // the column tiles of a query tile are the prefix in 128-row tiles, then the tree: one tile with the
 // query tile's own K/V rows and, behind it, tiles of gathered ancestors, in which every block of the query tile has
-// a segment of columns.  Tree tiles are masked by the rows' mask words and cost what a prefix tile costs.
+// a segment of columns.  Tree tiles are masked by the rows' mask words and cost what a prefix tile costs; a 16-column
+// step of their second product updates the rows that have a column in it and no others, so that a V that is not
+// finite stays with those (32 heads of 256 rows behind 4096: 30.1 us with and without).
 // Per query tile and column tile, a step:
 //     S = Q K^T             tcgen05.mma  M=128 N=128 K=16 x D/16, both operands K-major in shared memory
 //     P = softmax part      one thread per query row (TMEM lane = row, so no shuffles): a row of S in 128 registers,
@@ -64,9 +66,11 @@ struct Geo {
     static constexpr int TILES = D == 128 ? 7 : 12;
     static constexpr int MAX_RING = TILES - 1;
     static constexpr int OFF_BAR = TILES * TILE;
-    static constexpr int SMEM_BYTES = OFF_BAR + 384 + 1024;   // + barriers, TMEM address, 1 KB alignment slack
+    static constexpr int OFF_ROWS = OFF_BAR + 384;            // [tile parity][group][step][warp] rows with columns in a step of a tree tile
+    static constexpr int SMEM_BYTES = OFF_ROWS + 512 + 1024;  // + 1 KB alignment slack
     static constexpr int OFF_STATS = 2 * QM * D * 4;          // [256] (exponent, sum) of the groups' rows, [256] of the CTA's
 };
+static_assert(Geo<128>::SMEM_BYTES <= 227 * 1024 && Geo<64>::SMEM_BYTES <= 227 * 1024, "one CTA's shared memory");
 static_assert(Geo<128>::OFF_STATS + 4 * QM * 8 <= Geo<128>::OFF_BAR, "merge buffers fit");
 static_assert(Geo<64>::OFF_STATS + 4 * QM * 8 <= Geo<64>::OFF_BAR, "merge buffers fit");
 static_assert(1 + 3 * Geo<64>::MAX_RING + 9 <= 46, "barriers fit");
@@ -328,11 +332,11 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                             mbar_wait(bar_p + g * 8, (j >> 1) & 1, a.status, qt);       // the first half of P is in tensor memory
                     if (!alive) break;
                     fence_after_sync();
-                    // rows of a gathered tile past the lists' ends were never fetched, and those of a paged prefix's last
-                    // tile past the sequence's end are not its own
+                    // rows of a gathered tile past the lists' ends were never fetched, and those of the prefix's last
+                    // tile past its end are not its own
                     const int tile = T0 + (two ? j >> 1 : j);
                     uint32_t live = 0xffu;
-                    if (PAGED && tile + 1 == tp) {
+                    if (tile + 1 == tp) {
                         live = (1u << ((prefix - tile * KN + 15) >> 4)) - 1u;
                     } else if (tile > tp) {
                         const QueryTile me = query(two && !same ? g : 0);
@@ -345,16 +349,21 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                         }
                     }
                     const uint64_t dvs = dv + uint64_t(v_st * (TILE >> 4));
-                    bool more = j > 1;
+                    auto steps = [&](auto &&product) {            // 16 rows of V each
 #pragma unroll
-                    for (int ks = 0; ks < KN / 16; ++ks) {        // 16 rows per step
-                        if (ks == KN / 32) {                      // the rest of P
-                            alive = mbar_wait(bar_p + 16 + g * 8, (j >> 1) & 1, a.status, qt);
-                            fence_after_sync();
+                        for (int ks = 0; ks < KN / 16; ++ks) {
+                            if (ks == KN / 32) {                  // the rest of P
+                                alive = mbar_wait(bar_p + 16 + g * 8, (j >> 1) & 1, a.status, qt);
+                                fence_after_sync();
+                            }
+                            if ((live >> ks) & 1u) product(ks, dvs + uint64_t((ks * 16 * 128) >> 4));
                         }
-                        if (!((live >> ks) & 1u)) continue;
-                        mma_f16_ts(tmem_o, tmem_p + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, more);
-                        more = true;
+                    };
+                    if (tile < tp) {
+                        steps([&](int ks, uint64_t dvk) { mma_f16_ts(tmem_o, tmem_p + ks * 8, dvk, idesc_pv, true); });
+                    } else {
+                        const uint4 *rows = reinterpret_cast<const uint4 *>(smem + G::OFF_ROWS) + ((j >> 1 & 1) * 2 + g) * 8;
+                        steps([&](int ks, uint64_t dvk) { mma_f16_ts_rows(tmem_o, tmem_p + ks * 8, dvk, idesc_pv, rows[ks]); });
                     }
                     if (j >= 2 * shared || g == 1) {      // the last to read this V
                         mma_commit(bar_empty + v_st * 8);
@@ -490,6 +499,13 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(ext_words));
         }
 
+        {
+            uint32_t zero[16];                            // my row of O, while the first tiles are on their way
+#pragma unroll
+            for (int i = 0; i < 16; ++i) zero[i] = 0u;
+#pragma unroll 1
+            for (int c0 = 0; c0 < D; c0 += 16) tmem_st16(tmem_o + c0, zero);
+        }
         int n = 0;                                        // tiles my group has taken
 #pragma unroll 1
         for (int j = g; j < n_steps; j += 2, ++n) {
@@ -510,6 +526,14 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     word[i] = real && i >= at && i < at + nw && first + i - at < have ? __ldg(from + first + i - at) : 0u;
+                // rows of my warp with a column in a step.  (S of my previous tile has landed, so the products of the one
+                // before it, which read what is there, have been issued.)
+                uint32_t *rows = reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS) + ((n & 1) * 2 + g) * 32 + (warp & 3);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
+                    if (lane < 2) rows[(2 * i + lane) * 4] = lane == 0 ? lo : hi;
+                }
             }
             // (S landing says that O += P V of my previous tile is done as well: it was issued before)
             alive = mbar_wait(bar_s + g * 8, n & 1, a.status, qt) && alive;

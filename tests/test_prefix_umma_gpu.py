@@ -157,3 +157,43 @@ def test_nan_keys_reach_their_rows(fst, prefix, D, H, H_kv):
                 assert torch.equal(o[0, h].isnan().all(-1).cpu(), attends[:, x]), (x, splits)
                 assert torch.equal(o[0, h].isnan().any(-1).cpu(), attends[:, x]), (x, splits)
                 assert torch.equal(lse[h].isnan().cpu(), attends[:, x]), (x, splits)
+
+
+@pytest.mark.parametrize("n,H,H_kv,D,bm", [(300, 2, 2, 128, 64), (300, 2, 2, 64, 128), (60, 8, 2, 128, 32), (30, 8, 2, 64, 32)])
+@pytest.mark.parametrize("fill", [float("nan"), float("inf")])
+def test_tree_values_that_are_not_finite(fst, n, H, H_kv, D, bm, fill):
+    """A row of V in the tree that is not finite reaches the rows that attend to it, and else only rows that attend to
+    another of the sixteen columns of one step of the product; behind a contiguous prefix and a paged one."""
+    prefix, ps = 400, 16
+    par = [-1] + [(i - 1) // 3 for i in range(1, n)]
+
+    def reaches(lo, hi):
+        hit = torch.zeros(n, dtype=torch.bool)
+        for i, p in enumerate(par):
+            hit[i] = lo <= i < hi or (p >= 0 and bool(hit[p]))
+        return hit.cuda()
+
+    meta = fst.build_tree_metadata(par, bm, 128, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q = torch.randn((1, H, n, D), generator=g, device="cuda").half()
+    k, v = (torch.randn((1, H_kv, prefix + n, D), generator=g, device="cuda").half() for _ in range(2))
+    pools = [t[:, :, :prefix].transpose(1, 2).reshape(prefix // ps, ps, H_kv, D).contiguous() for t in (k, v)]
+    table = torch.arange(prefix // ps, dtype=torch.int32, device="cuda")[None]
+    lens = torch.tensor([prefix], dtype=torch.int32, device="cuda")
+    for splits in (1, 2, 12):
+        def call(v, paged):
+            if paged:
+                return fst.fst_attention_paged(q, k[:, :, prefix:], v[:, :, prefix:], meta, *pools, table, lens, 0.1,
+                                               max_prefix=prefix, kv_splits=splits)
+            return fst.fst_attention(q, k, v, meta, sm_scale=0.1, kernel="tma_umma", kv_splits=splits)
+        for paged in (False, True):
+            clean = call(v, paged)
+            for x in (n - 1, n * 2 // 3, n // 2 - 3, 20, 5):
+                bad = v.clone()
+                bad[:, :, prefix + x] = fill
+                o = call(bad, paged)
+                assert not torch.isfinite(o[:, :, reaches(x, x + 1)]).any(), (x, splits, paged)
+                if x not in par:
+                    near = reaches(x // 16 * 16, x // 16 * 16 + 16)
+                    assert torch.equal(o[:, :, ~near], clean[:, :, ~near]), (x, splits, paged)
+    assert fst.last_status() == 0
