@@ -21,6 +21,7 @@
 //
 // Also here: the converter from reference-format metadata tensors to the packed form.
 
+#include <algorithm>
 #include <atomic>
 #include <climits>
 
@@ -468,11 +469,11 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
         }
     } else {                                              // too many ancestors, or too wide a mask: climb again
         for (int j = tid; j < bm; j += WIDE_THREADS)
-            for (int x = row0 + j < n_nodes ? row0 + j : -1; x >= 0; x = par(x)) {
-                const int pos = slot_of(x);
-                if (pos < 0) continue;
-                if (pos < ma) bits[j * maw + (pos >> 5)] |= 1u << (pos & 31);
-                if (x >= row0) blkmask[j * bw + ((x - row0) >> 5)] |= 1u << ((x - row0) & 31);
+            for (int x = row0 + j < n_nodes ? row0 + j : -1; x >= 0;) {
+                const int next = par(x), pos = slot_of(x);    // the next load is under way meanwhile
+                if (pos >= 0 && pos < ma) bits[j * maw + (pos >> 5)] |= 1u << (pos & 31);
+                if (pos >= 0 && x >= row0) blkmask[j * bw + ((x - row0) >> 5)] |= 1u << ((x - row0) & 31);
+                x = next;
             }
         __syncthreads();
     }
@@ -712,26 +713,6 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
     int depth_cap = int((48 * 1024) / (size_t(bm) * 4));
     if (depth_cap > 1024) depth_cap = 1024;
     if (depth_cap < 1) depth_cap = 1;
-    // Large trees: when a block's share of the parent array outgrows what one pass of the CTA stages in the
-    // time a climb through L2 takes (see precompute_wide_kernel).
-    const int slot = current_device_slot();
-    if (slot < 0) return cudaErrorInvalidDevice;
-    if (n_nodes > kWideNodes) {
-        const size_t Ww = (W + 32 * WIDE_WARPS - 1) / (32 * WIDE_WARPS) * (32 * WIDE_WARPS);
-        const bool inherit = ma <= 128;                   // masks of all slots: 2 KB, two words per thread
-        const size_t smem = wide_smem_words(Ww, bm, ma, inherit) * 4;
-        if (smem <= budget) {
-            if (smem > 48 * 1024 && smem > g_wide_smem_set[slot].load(std::memory_order_acquire)) {
-                cudaError_t e = cudaFuncSetAttribute(precompute_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-                if (e != cudaSuccess) return e;
-                g_wide_smem_set[slot].store(smem, std::memory_order_release);
-            }
-            precompute_wide_kernel<<<dim3(nb, n_trees), WIDE_THREADS, smem, stream>>>(
-                parent, n_nodes, bm, ma, inherit ? 1 : 0, anc_idx, anc_mask, leaf_idx, static_cast<unsigned char *>(packed),
-                packed_stride, status);
-            return cudaGetLastError();
-        }
-    }
     // Byte flags (one byte per node below the last row) while they leave room to stage a good
     // part of the parent array; beyond that the walkers set bitmap bits with atomics.
     bool byte_flags = base + W * 32 + size_t(depth_cap) * bm * 4 + 16 * 1024 <= budget;
@@ -740,10 +721,37 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
         depth_cap = depth_cap / 2;                         // (deeper rows are walked a second time)
         fixed = base + size_t(depth_cap) * bm * 4;
     }
-    if (fixed + 1024 > budget) return cudaErrorInvalidConfiguration;
-    const size_t cap = (budget - fixed) / 4;
+    const bool fits = fixed + 1024 <= budget;
+    const size_t cap = fits ? (budget - fixed) / 4 : 0;
     const int par_cap = int(cap < size_t(n_nodes) ? cap : size_t(n_nodes));
     const size_t smem = fixed + size_t(par_cap) * 4;
+    // Large trees: when a block's share of the parent array outgrows what one pass of the CTA stages in the
+    // time a climb through L2 takes (see precompute_wide_kernel).  A bound of more than 128 ancestors, and more
+    // than two to a row, is for deep trees, which that kernel climbs twice through L2 (its masks are not
+    // inherited): where the staging kernel needs a single wave it stays (9400 nodes, block_m 64: depth 100 25 us
+    // against 35, depth 500 118 against 130, parents drawn from the 256 nodes before 26 against 43; in two waves
+    // 46 against 35 and 229 against 129; with a bound of 128 a tree of depth 15 takes 17 against 12.6, of depth 64
+    // 21.2 against 22.8).
+    const int slot = current_device_slot();
+    if (slot < 0) return cudaErrorInvalidDevice;
+    const bool one_wave = fits && size_t(nb) * n_trees <= sm_count() * (228 * 1024 / (smem + 1024));
+    if (n_nodes > kWideNodes && !(one_wave && ma > std::max(128, 2 * bm))) {
+        const size_t Ww = (W + 32 * WIDE_WARPS - 1) / (32 * WIDE_WARPS) * (32 * WIDE_WARPS);
+        const bool inherit = ma <= 128;                   // masks of all slots: 2 KB, two words per thread
+        const size_t wide_smem = wide_smem_words(Ww, bm, ma, inherit) * 4;
+        if (wide_smem <= budget) {
+            if (wide_smem > 48 * 1024 && wide_smem > g_wide_smem_set[slot].load(std::memory_order_acquire)) {
+                cudaError_t e = cudaFuncSetAttribute(precompute_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wide_smem));
+                if (e != cudaSuccess) return e;
+                g_wide_smem_set[slot].store(wide_smem, std::memory_order_release);
+            }
+            precompute_wide_kernel<<<dim3(nb, n_trees), WIDE_THREADS, wide_smem, stream>>>(
+                parent, n_nodes, bm, ma, inherit ? 1 : 0, anc_idx, anc_mask, leaf_idx, static_cast<unsigned char *>(packed),
+                packed_stride, status);
+            return cudaGetLastError();
+        }
+    }
+    if (!fits) return cudaErrorInvalidConfiguration;
     auto kernel = byte_flags ? precompute_kernel<true> : precompute_kernel<false>;
     std::atomic<size_t> &enabled = g_pre_smem_set[byte_flags ? 1 : 0][slot];
     if (smem > 48 * 1024 && smem > enabled.load(std::memory_order_acquire)) {

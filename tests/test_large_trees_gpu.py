@@ -161,3 +161,19 @@ def test_captured_builds_are_kernels_only(fst):
     err, nodes, count = runtime.cudaGraphGetNodes(raw, count)
     kinds = [runtime.cudaGraphNodeGetType(n)[1] for n in nodes]
     assert len(kinds) == 4 and set(kinds) == {runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel}, kinds
+
+
+@pytest.mark.parametrize("n,bm,ma", [(8193, 64, 192), (9000, 64, 1000), (9001, 24, 136), (16384, 128, 320), (18945, 128, 320)])
+def test_one_tree_and_many_are_built_alike(fst, n, bm, ma):
+    """A deep tree alone may take one kernel and a batch of it another: the same metadata, bit for bit."""
+    rng = np.random.default_rng(n)
+    i = np.arange(n)
+    par = np.where(i < 60, i - 1, np.where(i % 8 == 0, rng.integers(30, 60, n), i - 1))      # chains of eight behind a trunk
+    par = torch.tensor(par, dtype=torch.int32, device="cuda")
+    one = fst.build_tree_metadata(par, bm, ma)
+    many = fst.build_tree_metadata(par.expand(6, n).contiguous(), bm, ma)
+    for a, b in zip(one, many):
+        assert all(torch.equal(a, b[t]) for t in range(6))
+    from helpers import decode_packed_raw                 # (the bytes between its parts are nobody's)
+    parts = [decode_packed_raw(x.cpu().numpy(), one.n_blocks, bm, ma) for x in (one.packed[0], *many.packed)]
+    assert all(np.array_equal(a, b) for other in parts[1:] for a, b in zip(parts[0], other))
