@@ -361,6 +361,9 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
         }
     }
     const c10::cuda::CUDAGuard guard(dev);
+    if (max_prefix <= 0)                                  // no prefix anywhere: plain tree attention
+        return launch(c, tensor(a[4]).data_ptr(), n_trees > 1 ? size_t(integer(a[5])) : 0, bm, ma, FST_KERNEL_AUTO, std::nullopt,
+                      status_of(dev, true)->data_ptr(), c10::cuda::getCurrentCUDAStream(dev.index()).stream());
     const at::Tensor lens = given_lens.contiguous();      // the kernel reads length z at word z
     at::Tensor ws;
     size_t ws_bytes = 0;

@@ -204,8 +204,6 @@ def fst_attention_paged(q, k_tree, v_tree, meta: TreeMetadata, k_pool, v_pool, b
         raise ValueError("pool_layout must be 'NHD' or 'HND'")
     if max_prefix is None:
         max_prefix = int(prefix_lens.max().item())
-    if max_prefix <= 0:                                   # no prefix anywhere: plain tree attention
-        return fst_attention(q, k_tree, v_tree, meta, sm_scale=sm_scale, out=out, return_lse=return_lse)
     host = _lib._host or _lib.host()
     return host.attention_paged(q, k_tree, v_tree, out, meta.packed, meta.tree_stride, meta.n_trees, meta.n_blocks,
                                 meta.block_m, meta.max_ancestors, k_pool, v_pool, pool_layout == "NHD", block_table,

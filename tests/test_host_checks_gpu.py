@@ -92,3 +92,21 @@ def test_block_size_of_the_metadata_tensors(fst):
                 fst.fst_attention(q, k, v, *three, sm_scale=0.1, BLOCK_M=bm, MAX_ANCESTORS=ma, scatter=scatter)
     want = fst.fst_attention(q, k, v, *three, sm_scale=0.1, BLOCK_M=32, MAX_ANCESTORS=64)
     assert torch.equal(fst.fst_attention(q, k, v, *three, sm_scale=0.1, BLOCK_M=32, MAX_ANCESTORS=64, scatter=to), want)
+
+
+def test_paged_without_a_prefix(fst):
+    """Plain tree attention, and the same checks as with a prefix."""
+    Z, H, n, D, ps = 2, 4, 20, 128, 16
+    meta = fst.build_tree_metadata([-1] + [0] * (n - 1), 32, 32, reference_format=False)
+    q, k, v = qkv(Z, H, n, D)
+    pool = torch.zeros((4, ps, H, D), dtype=torch.float16, device="cuda")
+    table, lens = torch.zeros((Z, 2), dtype=torch.int32, device="cuda"), torch.zeros(Z, dtype=torch.int32, device="cuda")
+    want, want_lse = fst.fst_attention(q, k, v, meta, sm_scale=-0.1, return_lse=True)
+    for max_prefix in (None, 0, -1):
+        got, lse = fst.fst_attention_paged(q, k, v, meta, pool, pool, table, lens, -0.1, max_prefix=max_prefix, return_lse=True)
+        assert torch.equal(got, want) and torch.equal(lse, want_lse)
+        for bad, error in (((pool.cpu(), pool, table, lens), RuntimeError), ((pool, pool.float(), table, lens), TypeError),
+                           ((pool[:, :, :2], pool[:, :, :2], table, lens), ValueError), ((pool, pool, table.long(), lens), ValueError),
+                           ((pool, pool, table, lens[:1]), ValueError), ((pool, pool, table[:1], lens), ValueError)):
+            with pytest.raises(error):
+                fst.fst_attention_paged(q, k, v, meta, *bad, 0.1, max_prefix=max_prefix)
