@@ -66,6 +66,7 @@ def launch_plan(q, prefix, block_m, kernel: str = "auto", kv_splits: Optional[in
     dispatch inside the library (for rows on 16-byte boundaries): ``{"kernels":
     [...], "prefix_runs": r}``.  ``max_ancestors`` is the metadata's ancestor bound; of ``sm_scale`` the sign counts,
     and ``kv_heads`` are the heads of K and V where they are fewer than those of ``q``."""
+    kv_splits = None if kv_splits is None else int(kv_splits)
     splits, need_ws, umma = _lib.host().splits(q, prefix, block_m, _lib.KERNELS[kernel], kv_splits, sm_scale,
                                                q.shape[1] if kv_heads is None else kv_heads)
     tensor_core = q.dtype in (torch.float16, torch.bfloat16) and q.shape[-1] in (64, 128) \
@@ -118,6 +119,8 @@ def fst_attention(q, k, v, ancestor_idx, ancestor_mask=None, leaf_idx=None, sm_s
     if scatter is not None:
         tensors = (ancestor_idx, ancestor_mask, leaf_idx, BLOCK_M, MAX_ANCESTORS)
         return _scattered(q, k, v, meta, tensors, sm_scale, kern, scatter, out, return_lse)
+    if kv_splits is not None:
+        kv_splits = int(kv_splits)
     host = _lib._host or _lib.host()
     if meta is None:
         # the reference's three tensors (fstattention.py:153), which the call packs first

@@ -313,3 +313,12 @@ def test_launch_plan_of_grouped_queries(built_lib):
     assert grouped["prefix_runs"] == one_tile["prefix_runs"] > own["prefix_runs"]
     with pytest.raises(ValueError, match="multiple"):
         fst.launch_plan(q, 8192, 64, kv_heads=5)
+
+
+def test_a_number_of_splits_of_any_type(built_lib):
+    import fstattention_b200 as fst
+    q = torch.empty((1, 8, 127, 128), dtype=torch.float16)
+    want = fst.launch_plan(q, 4096, 64, kv_splits=3)
+    assert want["prefix_runs"] == 3
+    for splits in (3.0, np.int64(3), np.float32(3), torch.tensor(3)):
+        assert fst.launch_plan(q, 4096, 64, kv_splits=splits) == want

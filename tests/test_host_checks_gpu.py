@@ -110,3 +110,16 @@ def test_paged_without_a_prefix(fst):
                            ((pool, pool, table, lens[:1]), ValueError), ((pool, pool, table[:1], lens), ValueError)):
             with pytest.raises(error):
                 fst.fst_attention_paged(q, k, v, meta, *bad, 0.1, max_prefix=max_prefix)
+
+
+def test_a_number_of_splits_of_any_type(fst):
+    n, prefix = 20, 600
+    meta = fst.build_tree_metadata([-1] + [0] * (n - 1), 32, 32)
+    q, k, v = qkv(1, 2, n, 64, prefix + n)
+    want = fst.fst_attention(q, k, v, meta, sm_scale=0.1, kv_splits=2)
+    for splits in (2.0, torch.tensor(2)):
+        assert torch.equal(fst.fst_attention(q, k, v, meta, sm_scale=0.1, kv_splits=splits), want)
+        idx, mask, leaf = (t.clone() for t in meta)
+        idx += prefix
+        leaf += prefix
+        assert torch.equal(fst.fst_attention(q, k, v, idx, mask, leaf, 0.1, BLOCK_M=32, MAX_ANCESTORS=32, kv_splits=splits), want)
