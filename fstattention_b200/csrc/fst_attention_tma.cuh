@@ -746,15 +746,17 @@ inline MapSlot *map_table() {
     return table.get();
 }
 
-// a map from the calling thread's table, encoded with `encode` when it is not there yet
-template <typename F>
-inline bool kept_map(CUtensorMap *map, const MapKey &key, F &&encode) {
+// rank-4 map (columns, rows, heads, batch) with 64-column x box_rows boxes, 128-byte swizzle: from the calling thread's
+// table, encoded when it is not there yet
+inline bool make_map(CUtensorMap *map, const void *base, bool bf16, int D, int rows, int H, int Z,
+                     int64_t stride_n, int64_t stride_h, int64_t stride_z, int box_rows = 32) {
+    const MapKey key{base, stride_n, stride_h, stride_z, rows, H, Z, D, bf16 ? 1 : 0, box_rows};
     MapSlot *table = map_table();
     MapSlot *slot = nullptr;
     if (table != nullptr) {
-        uint64_t hsh = reinterpret_cast<uintptr_t>(key.base) >> 4;
-        hsh = (hsh ^ (hsh >> 17) ^ uint64_t(key.rows) * 0x9E3779B97F4A7C15ull ^ uint64_t(key.stride_n) * 0xC2B2AE3D27D4EB4Full ^
-               uint64_t(key.H) << 20 ^ uint64_t(key.Z) << 40 ^ uint64_t(uint32_t(key.box_rows)) << 7) * 0xFF51AFD7ED558CCDull;
+        uint64_t hsh = reinterpret_cast<uintptr_t>(base) >> 4;
+        hsh = (hsh ^ (hsh >> 17) ^ uint64_t(rows) * 0x9E3779B97F4A7C15ull ^ uint64_t(stride_n) * 0xC2B2AE3D27D4EB4Full ^
+               uint64_t(H) << 20 ^ uint64_t(Z) << 40 ^ uint64_t(box_rows) << 7) * 0xFF51AFD7ED558CCDull;
         slot = &table[(hsh >> 40) % kMapSlots];
         if (slot->used && slot->key == key) {
             *map = slot->map;
@@ -762,28 +764,22 @@ inline bool kept_map(CUtensorMap *map, const MapKey &key, F &&encode) {
         }
     }
     EncodeTiledFn fn = encode_tiled_fn();
-    if (fn == nullptr || !encode(fn)) return false;
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[4] = {cuuint64_t(D), cuuint64_t(rows), cuuint64_t(H), cuuint64_t(Z)};
+    const cuuint64_t strides[3] = {cuuint64_t(stride_n) * 2, cuuint64_t(stride_h) * 2, cuuint64_t(stride_z) * 2};
+    const cuuint32_t box[4] = {64, cuuint32_t(box_rows), 1, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    if (fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+           const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
     if (slot != nullptr) {
         slot->map = *map;
         slot->key = key;
         slot->used = true;
     }
     return true;
-}
-
-// rank-4 map (columns, rows, heads, batch) with 64-column x box_rows boxes, 128-byte swizzle
-inline bool make_map(CUtensorMap *map, const void *base, bool bf16, int D, int rows, int H, int Z,
-                     int64_t stride_n, int64_t stride_h, int64_t stride_z, int box_rows = 32) {
-    return kept_map(map, MapKey{base, stride_n, stride_h, stride_z, rows, H, Z, D, bf16 ? 1 : 0, box_rows}, [&](EncodeTiledFn fn) {
-        const cuuint64_t dims[4] = {cuuint64_t(D), cuuint64_t(rows), cuuint64_t(H), cuuint64_t(Z)};
-        const cuuint64_t strides[3] = {cuuint64_t(stride_n) * 2, cuuint64_t(stride_h) * 2, cuuint64_t(stride_z) * 2};
-        const cuuint32_t box[4] = {64, cuuint32_t(box_rows), 1, 1};
-        const cuuint32_t estr[4] = {1, 1, 1, 1};
-        return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-                  const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    });
 }
 
 template <typename T, int D, int BM, int TN, bool PFX, int NOUT>

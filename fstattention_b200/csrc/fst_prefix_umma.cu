@@ -705,12 +705,6 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     cluster_sync();                                       // nobody leaves while its rows are being read
 }
 
-// rank-4 map with 64-column x 128-row boxes (kept in the calling thread's table of maps)
-static bool make_map_rows128(CUtensorMap *map, const void *base, bool bf16, int D, int rows, int H, int Z,
-                             int64_t stride_n, int64_t stride_h, int64_t stride_z) {
-    return make_map(map, base, bf16, D, rows, H, Z, stride_n, stride_h, stride_z, 128);
-}
-
 // rank-4 map over a page pool (columns, rows of a page, K/V heads, pages) with 64-column x page boxes
 static bool make_map_pool(CUtensorMap *map, bool bf16, int D, const PagedArgs &pg, int H_kv, const void *pool) {
     EncodeTiledFn fn = encode_tiled_fn();
@@ -733,8 +727,8 @@ static cudaError_t launch_prefix_t(const AttnArgs &a, const PagedArgs *pg, int n
     alignas(64) CUtensorMap tq, tk, tv, tkt, tvt;
     const int pack = prefix_heads_per_tile(a.H, H_kv, a.n_q);
     if (!make_map(&tq, a.q, bf16, D, a.n_q, a.H, a.Z, a.qs_n, a.qs_h, a.qs_z, umma::QM / pack) ||
-        !make_map_rows128(&tkt, a.k, bf16, D, a.n_kv, H_kv, a.Z, a.ks_n, a.ks_h, a.ks_z) ||
-        !make_map_rows128(&tvt, a.v, bf16, D, a.n_kv, H_kv, a.Z, a.vs_n, a.vs_h, a.vs_z))
+        !make_map(&tkt, a.k, bf16, D, a.n_kv, H_kv, a.Z, a.ks_n, a.ks_h, a.ks_z, umma::KN) ||
+        !make_map(&tvt, a.v, bf16, D, a.n_kv, H_kv, a.Z, a.vs_n, a.vs_h, a.vs_z, umma::KN))
         return cudaErrorNotSupported;
     if (!PAGED) {
         tk = tkt;
