@@ -73,16 +73,17 @@ inline bool prefix_umma_pays(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, in
     return prefix >= (sparse ? 256 : bm >= 128 ? 96 : 192);
 }
 
-// When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, six kinds of trees, from 64
-// items (128 query rows of one head) up, ratios of old to new time:
-//   D 128, block_m 128   1.27 - 1.72 from 256 items, up to 2.40 at 5184; 0.82 - 1.12 below 100
-//   D 128, block_m 64    1.10 from 256 items with an ancestor bound of two or three blocks, 1.28 - 1.32 from 1024 with
-//                        two or more (0.98 - 1.06 at 256 with long lists), 1.00 - 1.21 with one; 0.63 - 0.75 below 100
-//   D 128, block_m 32    1.19 - 1.83 at 256 items, 1.08 - 1.26 above; 0.89 - 0.97 above with long lists
-//   D 64, block_m 128    1.01 - 1.36 at 256 items, 1.12 - 1.65 above; 0.69 - 0.90 below 100
-//   D 64, block_m 64     1.03 - 1.31 from 4096 items, 1.04 - 1.16 from 1024 with a bound of two or three blocks;
-//                        0.92 - 1.09 otherwise, 0.56 - 0.95 up to 300
-//   D 64, block_m 32     1.01 - 1.43 from 1024 items; 0.64 - 0.85 with long lists, 0.61 - 0.97 up to 300
+// When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, five kinds of trees, 64 to 6144
+// items (128 query rows of one head), ratios of the mma.sync kernel's time to the other's; "bound" is the ancestor
+// bound in blocks:
+//   D 128, block_m 128   1.19 - 1.54 at 200 to 600 items, 1.54 - 2.39 above; 0.81 - 1.12 up to 160
+//   D 128, block_m 64    bound 1: 0.96 - 1.04, 1.05 - 1.19 at 300 to 600; bound 2 and 3: 0.97 - 1.06 at 256, 0.96 - 1.29 above;
+//                        bound 4 and up: 0.88 - 1.23 up to 600, 1.02 - 1.28 from 1000; all 0.61 - 0.95 below 200
+//   D 128, block_m 32    1.02 - 1.65 at 200 to 300 (0.97 - 1.33 with a bound of 8 and up), 0.92 - 1.03 at 300 to 600, 0.97 - 1.16
+//                        above; 0.71 - 1.05 from 300 on with a bound of 8 and up
+//   D 64, block_m 128    1.00 - 1.37 at 250 to 600, 1.18 - 1.56 above; 0.64 - 0.97 below 200
+//   D 64, block_m 64     1.10 - 1.45 at 4096 (1.03 with long lists), 1.05 - 1.42 at 1000 to 2000; 0.77 - 1.18 below
+//   D 64, block_m 32     0.98 - 1.33 from 1000, 0.69 - 1.01 with a bound of 8 and up; 0.54 - 1.04 below
 // Small grids are bound by one CTA's latency, which is longer here.  With one short tile of ancestors per 64 rows at
 // D 128 both kernels wait for the same HBM bytes and are within a few per cent of one another.
 inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int ma) {
@@ -91,7 +92,7 @@ inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int
     if (D == 128) {
         if (bm == 128) return items >= 200;
         if (bm == 64) return bound >= 4 ? items >= 1000 : bound >= 2 && items >= 256;
-        return items >= 200 && (bound < 8 || items <= 400);
+        return items >= 200 && (items <= 300 || (bound < 8 && items >= 600));
     }
     if (bm == 128) return items >= 250;
     if (bm == 64) return items >= (bound == 2 || bound == 3 ? 1000 : 2000);

@@ -322,3 +322,13 @@ def test_a_number_of_splits_of_any_type(built_lib):
     assert want["prefix_runs"] == 3
     for splits in (3.0, np.int64(3), np.float32(3), torch.tensor(3)):
         assert fst.launch_plan(q, 4096, 64, kv_splits=splits) == want
+
+
+def test_tree_kernel_of_short_blocks_with_long_lists(built_lib):
+    """block_m 32 at D 128: the tcgen05 kernel where an SM has one or two items, and on large grids where the ancestor
+    lists are short (three trees of 512 nodes with 320 ancestors, 32 heads: 28 us against 39)."""
+    from fstattention_b200 import _lib
+    kernel = lambda items, ma: _lib.lib().fst_attention_tree_kernel(1, items, 128, 128, 32, ma)
+    umma, tma = _lib.KERNELS["tree_umma"], _lib.KERNELS["tma"]
+    assert [kernel(n, 320) for n in (100, 256, 384, 1024, 4096)] == [tma, umma, tma, tma, tma]
+    assert [kernel(n, 64) for n in (100, 256, 384, 1024, 4096)] == [tma, umma, tma, umma, umma]
