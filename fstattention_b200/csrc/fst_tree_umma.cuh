@@ -32,9 +32,8 @@
 // tile's K and V in one buffer) - as they come free, in whatever order that is, so that the next items'
 // 96 KB are on their way while these are used up; O leaves through its item's Q buffer.
 //
-// Five roles share an instruction cache: waits loop out of line and long loops are kept rolled.  At 96 KB
-// of code instead of fifty the 64-tree forest took 199 us instead of 125 (ncu: no_instruction 3.6 of 11
-// stalled cycles per issue).
+// Five roles share an instruction cache: waits loop out of line and long loops are kept rolled, but for the
+// issue of products.  At 96 KB of code instead of fifty the 64-tree forest took 199 us instead of 125.
 //
 // All hand-offs are mbarriers with bounded waits; whoever times out records FST_DEV_TIMEOUT and stops.
 // A parity wait can tell a phase only from its neighbours, so no waiter may be two phases off: every group's
@@ -48,11 +47,11 @@
 // When S(t) has landed every earlier product of the group has too (one thread issues them in order), so
 // the group may rescale O without asking.
 //
-// Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 83 -> 71 (3.8 TB/s
-// over Q, K, V and O); 64 x 300-node dynamic trees, D 128, block_m 128 331 -> 170; 16 x 1000-node deep
-// trees, D 64 116 -> 86; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2180 -> 1978.
-// What bounds it is the chain of a group's tile - product, softmax, product - of some 5000 cycles per item
-// at D 64, and at D 128 the pool: a 96 KB item in use, one on its way, and the last one's O.
+// Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 85 -> 67.5 (4.0 TB/s
+// over Q, K, V and O); 64 x 300-node dynamic trees, D 128, block_m 128 380 -> 159; 16 x 1000-node deep
+// trees, D 64 120 -> 83; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2189 -> 1834.
+// What bounds it is the chain of a group's tile - product, softmax, rescale, product - of some 9000 cycles per item
+// of two tiles at D 64, and at D 128 the pool: a 96 KB item in use, one on its way, and the last one's O.
 // tree_umma_pays (fst_plan.h) has the line between the two kernels.
 #pragma once
 

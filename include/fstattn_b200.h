@@ -62,8 +62,9 @@ enum fst_kernel {
                                    /* shared-memory ring ahead of the arithmetic: block_m 64 or  */
                                    /* 128, no prefix.  Slower than FST_KERNEL_TMA on every shape */
                                    /* measured, so never the automatic choice                    */
-    FST_KERNEL_TREE_UMMA = 8       /* persistent tcgen05 kernel, 128-row items, TMA gathers: D 64/ */
-                                   /* 128, block_m 32/64/128, no prefix, positive sm_scale         */
+    FST_KERNEL_TREE_UMMA = 8       /* persistent tcgen05 kernel, 128-row items, ancestors gathered */
+                                   /* by cp.async: D 64/128, block_m 32/64/128, no prefix, positive */
+                                   /* sm_scale                                                      */
 };
 
 /*
@@ -302,10 +303,10 @@ int fst_attention_fwd_gqa(const void *q, const void *k, const void *v, void *o, 
  * k_pool / v_pool: element (page, row, head, d) at page * pool_stride_page + row * pool_stride_row
  * + head * pool_stride_head + d (element strides, multiples of 8).  page_size 16, 32, 64 or 128;
  * head_dim 64 or 128; fp16 / bf16.  max_prefix >= every prefix_lens[z] (it sizes the grid; lengths
- * above it are cut; rows of a page past a
- * sequence's length may hold anything).  Prefix and tree go to the tcgen05 kernel in kv_splits runs, partial results
- * of more than one run through `workspace`
- * (fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits) bytes).  A page number
+ * above it are cut; rows of a page past a sequence's length may hold anything).  Prefix and tree go to
+ * the tcgen05 kernel in kv_splits runs, which merge in a cluster or, where that leaves SMs idle and there
+ * is a `workspace` (fst_attention_split_workspace_bytes(Z, H, n_q, head_dim, kv_splits) bytes; may be
+ * NULL, and then at most eight runs are made), leave partial results there for a second kernel.  A page number
  * outside [0, n_pages) reads as zeros and sets FST_DEV_INDEX_RANGE.  block_table and prefix_lens
  * are device pointers.  sm_scale must be positive here (the tcgen05 prefix kernel takes Q as it
  * lies in shared memory and cannot fold a sign into it): FST_ERR_INVALID_ARG otherwise.

@@ -345,8 +345,7 @@ def test_prefix_tcgen05_moving_maximum(fst, prefix, runs, n, dtype):
 
 
 def test_prefix_tcgen05_in_a_cuda_graph(fst):
-    """The prefix path forks its tree kernel onto a second stream; captured into a CUDA graph and
-    replayed on new data it gives what the eager call gives."""
+    """The prefix path captured into a CUDA graph and replayed on new data gives what the eager call gives."""
     from fstattention_b200 import configs
     par = configs.left_weighted_tree()
     n, H, D, prefix = 256, 4, 128, 1024
@@ -494,8 +493,8 @@ def test_paged_prefix_with_an_empty_sequence(fst):
 
 
 def test_prefix_path_from_two_threads_on_their_own_streams(fst):
-    """The forked prefix path keeps its helper stream per host thread: two threads, each on its
-    own stream, calling it at the same time get what a single call gets."""
+    """The prefix path from two host threads at the same time, each on its own stream (tensor maps are kept per
+    thread, launch set-up per device): both get what a single call gets."""
     import threading
     from fstattention_b200 import configs
     par = configs.left_weighted_tree()

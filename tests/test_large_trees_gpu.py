@@ -96,7 +96,8 @@ def test_sorted_levels_with_random_scores_and_ties(fst, depth, topk, lwf):
 
 
 def test_a_captured_build_keeps_its_status_record(fst):
-    """A graph writes the record it was captured with; eager calls on other streams take records of their own."""
+    """A graph writes the record it was captured with, which lives on when an eager build takes one of its own (what a
+    replay reports there is the next test's)."""
     par = torch.tensor([-1] + [i // 2 for i in range(255)], dtype=torch.int32, device="cuda")
     meta = fst.build_tree_metadata(par, 64, 128, reference_format=False)
     side = torch.cuda.Stream()
