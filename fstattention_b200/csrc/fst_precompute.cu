@@ -296,6 +296,12 @@ precompute_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int bm, i
 //     parent's;
 // so that a CTA's time is one climb and its shared memory lets seven share an SM.  131068 nodes, block_m 128, with
 // the reference-format tensors: 161 us with precompute_kernel.
+//
+// With seven CTAs to an SM what counts is how many instructions a block takes, and a bitmap of 131068 nodes
+// is 4096 words to clear and to walk twice for some seventy ancestors (28.7 us; its list took 5.6 us of a CTA's 20, one lane
+// writing the neighbours that share a word).  Blocks and bounds of at most 128 therefore keep their ancestors in
+// a hash set (precompute_set): 16.4 us, of which the climb, one dependent L2 read for each of fifteen levels, is the
+// largest part.  A block with more ancestors than the bound is left to the bitmap, which counts them.
 constexpr int WIDE_THREADS = 256, WIDE_WARPS = WIDE_THREADS / 32;
 
 // 32-bit words of shared memory: bitmap and 16-bit ranks of Wp words, masks of slots or rows, block masks,
@@ -303,6 +309,165 @@ constexpr int WIDE_THREADS = 256, WIDE_WARPS = WIDE_THREADS / 32;
 __host__ __device__ inline size_t wide_smem_words(size_t Wp, int bm, int ma, bool inherit) {
     const size_t maw = (ma + 31) / 32, bw = (bm + 31) / 32;
     return Wp + Wp / 2 + size_t(inherit && ma > bm ? ma : bm) * maw + size_t(bm) * bw + size_t(bm) * 2 + (inherit ? size_t(ma) * 2 : 0);
+}
+
+// four bits as four bool bytes
+__device__ __forceinline__ uint32_t bool_bytes(uint32_t bits) { return ((bits & 0xfu) * 0x00204081u) & 0x01010101u; }
+
+constexpr int SET_MOST = 128;          // rows of a block, and its ancestors
+constexpr int SET_SLOTS = 1024;        // the set gives up beyond SET_MOST; the climbs under way then add one node each
+struct AncestorSet {
+    uint4 bits[SET_MOST];              // masks of the slots
+    uint4 row[SET_MOST];               // and of the block's rows
+    int key[SET_SLOTS];                // node at a place of the hash table, -1: none
+    int node[SET_MOST];                // in the order they were met, INT_MAX behind the last
+    int sorted[SET_MOST];              // by slot
+    uint32_t blk[SET_MOST * (SET_MOST / 32)];
+    int16_t up[SET_SLOTS];             // place of the parent, -1: a root
+    int16_t slot[SET_SLOTS];           // slot of the node at that place
+    int16_t place[SET_MOST];           // places in the order they were met
+    int16_t jump[SET_MOST], self[SET_MOST];    // of a slot: an ancestor's slot; of a row: its own slot, -1: nobody's ancestor
+    int n;
+};
+
+// One block's metadata by way of a hash set of its ancestors; false, with nothing written, when there are more than max_ancestors.
+//   * a row climbs until it meets a node that is in the set, and links every node to its parent's place on the way;
+//   * a node's slot is the number of smaller ones: everybody compares;
+//   * the slots' masks, a uint4 each, by pointer doubling over the links; a row's mask is its parent's.
+template <typename Parent>
+__device__ __forceinline__ bool precompute_set(AncestorSet &set, const Parent &par, int b, int n_nodes, int bm, int ma,
+                                               unsigned char *blob, const PackedLayout &L, int64_t *o_idx, uint8_t *o_mask, int64_t *o_leaf) {
+    const int tid = threadIdx.x, row0 = b * bm, maw = L.maw, bw = L.bw;
+    for (int i = tid; i < SET_SLOTS / 4; i += WIDE_THREADS) reinterpret_cast<int4 *>(set.key)[i] = make_int4(-1, -1, -1, -1);
+    if (tid < SET_MOST) {
+        set.node[tid] = INT_MAX;
+        set.self[tid] = -1;
+        reinterpret_cast<uint4 *>(set.blk)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (tid == 0) set.n = 0;
+    __syncthreads();
+
+    int first = -1;                                       // place of my row's parent
+    if (tid < bm) {
+        int x = row0 + tid < n_nodes ? par(row0 + tid) : -1, below = -1;
+        while (x >= 0) {
+            const int next = par(x);                      // under way while x is looked up
+            int at = int((uint32_t(x) * 0x9E3779B1u) >> 22), was;
+            while ((was = atomicCAS(&set.key[at], -1, x)) != -1 && was != x) at = (at + 1) & (SET_SLOTS - 1);
+            if (below < 0) first = at;
+            else set.up[below] = int16_t(at);
+            if (was == x) break;                          // somebody else goes on from here
+            const int k = atomicAdd(&set.n, 1);
+            if (k >= ma) break;                           // too many
+            set.place[k] = int16_t(at);
+            set.node[k] = x;
+            if (next < 0) set.up[at] = -1;
+            below = at;
+            x = next;
+        }
+    }
+    __syncthreads();
+    const int n = set.n;
+    if (n > ma) return false;
+
+    // slots: thread pairs share a node, half of the comparisons each
+    const int k = tid >> 1, mine = set.node[k];
+    int rank = 0;
+#pragma unroll 4
+    for (int i = tid & 1; i < (n + 3) >> 2; i += 2) {
+        const int4 v = reinterpret_cast<const int4 *>(set.node)[i];
+        rank += int(v.x < mine) + int(v.y < mine) + int(v.z < mine) + int(v.w < mine);
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    const bool have = (tid & 1) == 0 && k < n;
+    const int at = have ? set.place[k] : 0;
+    if (have) {
+        set.slot[at] = int16_t(rank);
+        set.sorted[rank] = mine;
+        if (mine >= row0) set.self[mine - row0] = int16_t(rank);
+    }
+    const int n_ext = __syncthreads_count(have && mine < row0);
+    if (have) {
+        const int p = set.up[at];
+        set.jump[rank] = p < 0 ? int16_t(-1) : set.slot[p];
+        const uint32_t bit = 1u << (rank & 31);
+        const int w = rank >> 5;
+        set.bits[rank] = make_uint4(w == 0 ? bit : 0u, w == 1 ? bit : 0u, w == 2 ? bit : 0u, w == 3 ? bit : 0u);
+    }
+    const int above = first < 0 ? -1 : set.slot[first];   // slot of my row's parent
+    if (tid < ma) {
+        const int node = tid < n ? set.sorted[tid] : -1;
+        if (o_idx) o_idx[tid] = node;
+        if (blob) reinterpret_cast<int32_t *>(blob + L.off_idx)[size_t(b) * ma + tid] = tid < n_ext ? node : -1;
+    }
+    if (tid == 0 && blob) reinterpret_cast<int32_t *>(blob + L.off_count)[b] = n_ext;
+    __syncthreads();
+    for (;;) {
+        uint4 got = make_uint4(0u, 0u, 0u, 0u);
+        int to = tid < n ? set.jump[tid] : -1;
+        const bool any = to >= 0;
+        if (any) {
+            got = set.bits[to];
+            to = set.jump[to];
+        }
+        if (!__syncthreads_or(any)) break;
+        if (any) {
+            uint4 m = set.bits[tid];
+            m.x |= got.x; m.y |= got.y; m.z |= got.z; m.w |= got.w;
+            set.bits[tid] = m;
+            set.jump[tid] = int16_t(to);
+        }
+        __syncthreads();
+    }
+    if (tid < bm) {
+        const int j = tid, self = set.self[j];
+        uint4 m = above >= 0 ? set.bits[above] : make_uint4(0u, 0u, 0u, 0u);
+        if (self >= 0) {
+            const uint32_t bit = 1u << (self & 31);
+            m.x |= self >> 5 == 0 ? bit : 0u; m.y |= self >> 5 == 1 ? bit : 0u; m.z |= self >> 5 == 2 ? bit : 0u; m.w |= self >> 5 == 3 ? bit : 0u;
+        }
+        set.row[j] = m;
+        uint32_t *blk = set.blk + j * bw;
+        blk[j >> 5] = 1u << (j & 31);                     // every row attends to itself, and to its ancestors in the block
+        const uint32_t word[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const int below = n_ext - w * 32;             // slots of this word that are outside
+            for (uint32_t in = below >= 32 ? 0u : below > 0 ? word[w] & ~((1u << below) - 1u) : word[w]; in != 0u; in &= in - 1u) {
+                const int c = set.sorted[w * 32 + __ffs(in) - 1] - row0;
+                blk[c >> 5] |= 1u << (c & 31);
+            }
+        }
+        if (o_leaf) o_leaf[j] = self >= 0 ? int64_t(-1) : int64_t(row0 + j);
+    }
+    __syncthreads();
+    const uint32_t *row = reinterpret_cast<const uint32_t *>(set.row);
+    if (blob) {
+        uint32_t *p_emask = reinterpret_cast<uint32_t *>(blob + L.off_emask) + size_t(b) * bm * maw;
+        uint32_t *p_bmask = reinterpret_cast<uint32_t *>(blob + L.off_bmask) + size_t(b) * bm * bw;
+        for (int i = tid; i < bm * maw; i += WIDE_THREADS) {
+            const int j = maw == 4 ? i >> 2 : i / maw, w = i - j * maw, outside = n_ext - w * 32;
+            p_emask[i] = row[j * 4 + w] & (outside >= 32 ? 0xffffffffu : outside > 0 ? (1u << outside) - 1u : 0u);
+        }
+        for (int i = tid; i < bm * bw; i += WIDE_THREADS) p_bmask[i] = set.blk[i];
+    }
+    if (o_mask) {
+        if ((ma & 15) == 0 && (reinterpret_cast<uintptr_t>(o_mask) & 15) == 0) {     // sixteen bool bytes per store
+            const int pieces = ma / 16, step = WIDE_THREADS / pieces, j0 = tid / pieces, at16 = (tid - j0 * pieces) * 16;
+            if (j0 < step)
+                for (int j = j0; j < bm; j += step) {
+                    const uint32_t half = row[j * 4 + (at16 >> 5)] >> (at16 & 31);
+                    reinterpret_cast<uint4 *>(o_mask)[j * pieces + (at16 >> 4)] =
+                        make_uint4(bool_bytes(half), bool_bytes(half >> 4), bool_bytes(half >> 8), bool_bytes(half >> 12));
+                }
+        } else {
+            for (int i = tid; i < bm * ma; i += WIDE_THREADS) {
+                const int j = i / ma, c = i - j * ma;
+                o_mask[i] = (row[j * 4 + (c >> 5)] >> (c & 31)) & 1u;
+            }
+        }
+    }
+    return true;
 }
 
 __global__ void __launch_bounds__(WIDE_THREADS, 7)
@@ -335,6 +500,15 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
         }
         return p;
     };
+    const PackedLayout L = packed_layout(nb, bm, ma);
+    unsigned char *blob = packed_all ? packed_all + size_t(tree) * packed_stride : nullptr;
+    const size_t blk = size_t(tree) * nb + b;
+    int64_t *o_idx = anc_idx_all ? anc_idx_all + blk * ma : nullptr, *o_leaf = leaf_idx_all ? leaf_idx_all + blk * bm : nullptr;
+    uint8_t *o_mask = anc_mask_all ? anc_mask_all + blk * size_t(bm) * ma : nullptr;
+    if (ma <= SET_MOST && bm <= SET_MOST) {
+        if (precompute_set(*reinterpret_cast<AncestorSet *>(smem_raw), par, b, n_nodes, bm, ma, blob, L, o_idx, o_mask, o_leaf)) return;
+        __syncthreads();                                  // the bitmap takes the set's place
+    }
     for (int i = tid; i < W / 4; i += WIDE_THREADS) reinterpret_cast<uint4 *>(bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
     for (int i = tid; i < bm * bw; i += WIDE_THREADS) blkmask[i] = 0u;
     __syncthreads();
@@ -369,11 +543,7 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
     const bool inherit = inherit_ok && n_anc <= ma;
     if (n_anc > ma && tid == 0) report(status, FST_DEV_ANCESTOR_OVERFLOW, tree * 65536 + b, n_anc);
 
-    const PackedLayout L = packed_layout(nb, bm, ma);
-    unsigned char *blob = packed_all ? packed_all + size_t(tree) * packed_stride : nullptr;
     int32_t *p_idx = blob ? reinterpret_cast<int32_t *>(blob + L.off_idx) + size_t(b) * ma : nullptr;
-    const size_t blk = size_t(tree) * nb + b;
-    int64_t *o_idx = anc_idx_all ? anc_idx_all + blk * ma : nullptr;
 
     // 3. ascending ancestor list, a lane per word
     int ext = 0;                                          // listed nodes below the block
@@ -500,18 +670,13 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
             p_emask[i] = row_word(j, w) & keep;
         }
     }
-    if (anc_mask_all) {
-        uint8_t *o_mask = anc_mask_all + blk * size_t(bm) * ma;
+    if (o_mask) {
         if ((ma & 15) == 0 && (reinterpret_cast<uintptr_t>(o_mask) & 15) == 0) {   // sixteen bool bytes per store
             const int pieces = ma / 16;
             for (int i = tid; i < bm * pieces; i += WIDE_THREADS) {
                 const int j = i / pieces, at = (i - j * pieces) * 16;
                 const uint32_t half = row_word(j, at >> 5) >> (at & 31);
-                auto four = [&](int k) {                  // bits 4 k .. 4 k + 3 as bytes
-                    const uint32_t nib = (half >> (4 * k)) & 0xfu;
-                    return (nib & 1u) | ((nib & 2u) << 7) | ((nib & 4u) << 14) | ((nib & 8u) << 21);
-                };
-                reinterpret_cast<uint4 *>(o_mask)[i] = make_uint4(four(0), four(1), four(2), four(3));
+                reinterpret_cast<uint4 *>(o_mask)[i] = make_uint4(bool_bytes(half), bool_bytes(half >> 4), bool_bytes(half >> 8), bool_bytes(half >> 12));
             }
         } else {
             for (int i = tid; i < bm * ma; i += WIDE_THREADS) {
@@ -521,10 +686,10 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
         }
     }
     // 5. leaves: block rows that are not in the ancestor set (rows past the last node too)
-    if (leaf_idx_all)
+    if (o_leaf)
         for (int j = tid; j < bm; j += WIDE_THREADS) {
             const int k = row0 + j;
-            leaf_idx_all[blk * bm + j] = ((bitmap[k >> 5] >> (k & 31)) & 1u) ? int64_t(-1) : int64_t(k);
+            o_leaf[j] = ((bitmap[k >> 5] >> (k & 31)) & 1u) ? int64_t(-1) : int64_t(k);
         }
     __syncthreads();
     if (blob) {
@@ -738,7 +903,7 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
     if (n_nodes > kWideNodes && !(one_wave && ma > std::max(128, 2 * bm))) {
         const size_t Ww = (W + 32 * WIDE_WARPS - 1) / (32 * WIDE_WARPS) * (32 * WIDE_WARPS);
         const bool inherit = ma <= 128;                   // masks of all slots: 2 KB, two words per thread
-        const size_t wide_smem = wide_smem_words(Ww, bm, ma, inherit) * 4;
+        const size_t wide_smem = std::max(wide_smem_words(Ww, bm, ma, inherit) * 4, ma <= SET_MOST && bm <= SET_MOST ? sizeof(AncestorSet) : 0);
         if (wide_smem <= budget) {
             if (wide_smem > 48 * 1024 && wide_smem > g_wide_smem_set[slot].load(std::memory_order_acquire)) {
                 cudaError_t e = cudaFuncSetAttribute(precompute_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wide_smem));

@@ -61,6 +61,38 @@ def test_wide_precompute(fst, n, bm, ma, kind):
         assert count[b] == sum(1 for x in anc if x < lo)
 
 
+@pytest.mark.parametrize("bm,ma", [(128, 128), (128, 127), (64, 128), (100, 31), (32, 33), (16, 16), (1, 5)])
+@pytest.mark.parametrize("apart", [1, 37, 1024])
+def test_ancestor_set_and_bitmap_agree(fst, bm, ma, apart):
+    """Bounds of up to 128 keep a block's ancestors in a hash set, larger ones in a bitmap: the same metadata, up to a
+    block whose list is full, and an error for one ancestor more.  Hubs 1024 apart crowd the hash table's places."""
+    n = 131072 if apart == 1024 and bm >= 32 else 9001
+    apart = min(apart, (n - 1) // ma)
+    for hubs in (1, ma):
+        hub = np.arange(hubs) * apart
+        i = np.arange(n)
+        earlier = np.maximum(np.searchsorted(hub, i), 1)  # hubs below node i, at least one
+        par = np.where(i > 0, hub[(i * 7919) % earlier], -1)
+        if bm * (hubs > 1) >= ma:
+            par[hub] = np.where(np.arange(hubs) > 0, hub[(np.arange(hubs) - 1) // 3], -1)
+        else:                                             # fewer rows than ancestors: the hubs are a chain
+            par[hub[1:]] = hub[:-1]
+            par[0] = -1
+        par = torch.tensor(par, dtype=torch.int32, device="cuda")
+        got = fst.build_tree_metadata(par, bm, ma)
+        want = fst.build_tree_metadata(par, bm, 160)
+        assert torch.equal(got.ancestor_idx, want.ancestor_idx[:, :ma])
+        assert torch.equal(got.ancestor_mask, want.ancestor_mask[..., :ma])
+        assert torch.equal(got.leaf_idx, want.leaf_idx)
+        from helpers import decode_packed_raw
+        a, b = (decode_packed_raw(m.packed[0].cpu().numpy(), m.n_blocks, bm, w) for m, w in ((got, ma), (want, 160)))
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1][:, :ma]) and np.array_equal(a[2], b[2][..., :ma])
+        assert np.array_equal(a[3], b[3])
+    if int((got.ancestor_idx >= 0).sum(1).max()) == ma:
+        with pytest.raises(RuntimeError, match=f"{ma} unique ancestors"):
+            fst.build_tree_metadata(par, bm, ma - 1)
+
+
 def test_wide_precompute_reports(fst):
     n = 10000
     star = torch.tensor([-1] * 200 + [i % 200 for i in range(200, n)], dtype=torch.int32)
