@@ -31,6 +31,10 @@
 // buffers (seven at D 128): warp 10 hands them out in item order - K, V, Q, gathered tiles (a narrow
 // tile's K and V in one buffer) - as they come free, in whatever order that is, so that the next items'
 // 96 KB are on their way while these are used up; O leaves through its item's Q buffer.
+// A gathering lane's copies arrive on the tile's barrier by themselves (cp.async.mbarrier.arrive.noinc; the product thread
+// then fences for the tensor core's proxy).  Waited for by the warp, they were announced when the next tile's were
+// under way or could not start, some 3000 cycles after they were asked for (64 x 256 nodes, block_m 64: 121 -> 115.8 us,
+// 1024-node dynamic tree 19.5 -> 18.4, 4096-node deep tree 64.6 -> 63.0).
 //
 // Five roles share an instruction cache: waits loop out of line and long loops are kept rolled, but for the
 // issue of products.  At 96 KB of code instead of fifty the 64-tree forest took 199 us instead of 125.
@@ -66,7 +70,7 @@ namespace tree_umma {
 constexpr int ROWS = 128;              // query rows per item, K/V rows per tile
 constexpr int GATHER = 4;              // gathering warps
 constexpr int THREADS = (12 + GATHER) * 32;
-constexpr int FULL_COUNT = GATHER + 1; // arrivals that complete a K or V tile
+constexpr int FULL_COUNT = GATHER * 32;   // arrivals that complete a K or V tile: the gathering lanes', or one for all of them
 constexpr int POSITIONS = 16;          // load positions of a group with a barrier of their own
 constexpr int TURNS = 16;              // hand-overs to the gathering warps that may be outstanding
 constexpr int ITEMS = 16;              // items whose Q or O may be outstanding (the pool holds fewer)
@@ -120,6 +124,12 @@ __device__ __forceinline__ uint32_t live_steps(int t, int seg, const int (&count
 __device__ __forceinline__ void arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
+// arrives when the calling thread's cp.async copies so far have landed
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+// what cp.async has written, for the tensor core to read through the async proxy
+__device__ __forceinline__ void fence_copied() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void arrive_n(uint32_t bar, int n) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(n) : "memory");
 }
@@ -377,16 +387,6 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
         constexpr int CH = D / 8, RPP = 32 / CH;          // 16-byte chunks per row, rows per pass of a warp
         const int lr = lane / CH, lc = lane % CH;
         int turn = 0;                                     // tiles handed to us so far
-        uint32_t pending = 0;                             // barrier of copies not yet announced
-        auto announce = [&](bool all) {
-            if (pending == 0) return;
-            if (all) cp_async_wait<0>();
-            else cp_async_wait<1>();
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // the tensor core reads through the async proxy
-            __syncwarp();
-            if (lane == 0) arrive_n(pending, gw == 0 ? FULL_COUNT - GATHER + 1 : 1);
-            pending = 0;
-        };
         bool alive = true, have = false;
 #pragma unroll 1
         for (bool more = true; more || have;) {           // index lists are fetched one tile ahead
@@ -403,12 +403,10 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             const T *kp = static_cast<const T *>(a.k) + cur.z * a.ks_z + cur.hk * a.ks_h + a.prefix * a.ks_n + lc * 8;
             const T *vp = static_cast<const T *>(a.v) + cur.z * a.vs_z + cur.hk * a.vs_h + a.prefix * a.vs_n + lc * 8;
             const int half = cur.narrow ? HALF / 2 : HALF;
-            auto claim = [&](int at) {                    // never block on a slot while copies wait to be announced
+            auto claim = [&](int at) {
                 const uint32_t bar = bar_go + (turn % TURNS) * 8, parity = (turn / TURNS) & 1;
                 ++turn;
-                if (__all_sync(0xffffffffu, over(bar, parity))) return;
-                announce(true);
-                alive = __all_sync(0xffffffffu, wait_slow(bar, parity, a.status, at));
+                alive = __all_sync(0xffffffffu, wait(bar, parity, a.status, at));
             };
 #pragma unroll 1
             for (int kv = 0; kv < 2 && alive; ++kv) {
@@ -430,15 +428,12 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                     }
                 }
                 if (kv == 0 && cur.narrow) continue;
-                cp_async_commit();                        // under way: announce the ones before
-                announce(false);
-                pending = full_of(cur.g, at);
+                cp_async_arrive(full_of(cur.g, at));      // by every lane, once its copies have landed
             }
             if (!alive) break;
             cur = nxt;
         }
-        announce(true);
-        cp_async_wait<0>();
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
     } else if (warp == 8 || warp == 9) {
         // ================================ products ================================
         const int g = warp - 8;
@@ -471,6 +466,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                     int b = buf_of(g, at);
                     const uint64_t dqs = dk + uint64_t(in.w * (TILE >> 4)), dks = dk + uint64_t(b * (TILE >> 4)),
                                    half16 = (narrow ? HALF / 2 : HALF) >> 4;
+                    if (t > 0) fence_copied();
                     fence_after_sync();
 #pragma unroll
                     for (int ks = 0; ks < D / 16; ++ks)
@@ -487,6 +483,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                     b = buf_of(g, at);
                     ++at;
                     const uint64_t dvs = (narrow ? dv_narrow : dv) + uint64_t(b * (TILE >> 4));
+                    if (t > 0) fence_copied();
                     fence_after_sync();
                     const uint4 *rows = reinterpret_cast<const uint4 *>(smem + G::OFF_ROWS) + g * 8;
                     uint4 on[8];
