@@ -12,6 +12,7 @@
 //            the item's own rows (contiguous, TMA boxes); tile t > 0 holds ancestor slots
 //            [(t-1) BM, t BM) of every block (gathered row by row; padding slots are zeros).  The last
 //            tile is narrow - BM / 2 columns for each block - when the lists end in its first half.
+//   round    the tiles that one softmax takes: one, or - MERGED - the own tile and the first gathered one (see Cut)
 //   S = Q K^T     M 128, N 128 (64), both operands in shared memory (128-byte swizzle)
 //   softmax       thread r of a group owns row r and looks only at its block's columns; 32-column
 //                 words in which no row of its warp has a mask bit are not even read; P goes back
@@ -22,7 +23,7 @@
 //                 that do not attend to it, 128 of them.  Nor need P then be cleared where a warp has no column
 //
 // Sixteen warps.  Warps 0-3 and 4-7 are two softmax groups: group g takes the CTA's items g, g + 2, ... and
-// owns an S/P buffer and an accumulator (TMEM: 2 x 128 columns each), so that one group's latencies hide
+// owns an S/P buffer and an accumulator (TMEM: 128 or 192 columns, and D), so that one group's latencies hide
 // behind the other's work (one group with a tile of lookahead in the products was bound by its own
 // instruction stream: 7000 cycles per 128 rows at D 64).  One lane of warp 8 + g issues the products of
 // group g.  Warp 10 loads Q and the own tiles, warps 11-14 gather (cp.async, 16 bytes a lane; TMA's gather4
@@ -31,10 +32,6 @@
 // buffers (seven at D 128): warp 10 hands them out in item order - K, V, Q, gathered tiles (a narrow
 // tile's K and V in one buffer) - as they come free, in whatever order that is, so that the next items'
 // 96 KB are on their way while these are used up; O leaves through its item's Q buffer.
-// A gathering lane's copies arrive on the tile's barrier by themselves (cp.async.mbarrier.arrive.noinc; the product thread
-// then fences for the tensor core's proxy).  Waited for by the warp, they were announced when the next tile's were
-// under way or could not start, some 3000 cycles after they were asked for (64 x 256 nodes, block_m 64: 121 -> 115.8 us,
-// 1024-node dynamic tree 19.5 -> 18.4, 4096-node deep tree 64.6 -> 63.0).
 //
 // Five roles share an instruction cache: waits loop out of line and long loops are kept rolled, but for the
 // issue of products.  At 96 KB of code instead of fifty the 64-tree forest took 199 us instead of 125.
@@ -51,11 +48,19 @@
 // When S(t) has landed every earlier product of the group has too (one thread issues them in order), so
 // the group may rescale O without asking.
 //
-// Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 85 -> 67.5 (4.0 TB/s
+// Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 82 -> 62 (4.3 TB/s
 // over Q, K, V and O); 64 x 300-node dynamic trees, D 128, block_m 128 380 -> 159; 16 x 1000-node deep
-// trees, D 64 120 -> 83; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2189 -> 1834.
-// What bounds it is the chain of a group's tile - product, softmax, rescale, product - of some 9000 cycles per item
-// of two tiles at D 64, and at D 128 the pool: a 96 KB item in use, one on its way, and the last one's O.
+// trees, D 64 120 -> 83; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2189 -> 1550.
+// What bounds it is the chain of a group's round - product, softmax, (rescale,) product - and at D 128 the pool: a 96 KB item
+// in use, one on its way, and the last one's O.  Items of one tile run at HBM's rate (D 128: 83 us where 64 trees of
+// 256 nodes take 112; D 64: 1165 where the forest takes 1550), so a second round is what the rest pays for.
+//
+// MERGED: the own tile and the first gathered one in one round, so that an item of two tiles goes once through the chain
+// and rescales nothing.  S has room for it because every block's product writes the same columns, each into the
+// lanes of its own block (disable-output-lane): 64 + 64 of 128 columns at D 128, block_m 64 (2 x N 64 cost 102 cycles
+// where N 128 costs 64), 128 + 64 of 192 at D 64, block_m 128.  Apart / merged: forest of 65532 nodes 1752 / 1615 us;
+// 4096-node deep tree 63.0 / 61.9; 64 x 256 nodes, D 128 115.8 / 112.  Not where it lost: long lists at D 128, block_m 64
+// (dynamic trees of 1024 nodes 54.4 / 56.0), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118).
 // tree_umma_pays (fst_plan.h) has the line between the two kernels.
 #pragma once
 
@@ -79,13 +84,31 @@ template <int D>
 struct Geo {
     static constexpr int TILE = ROWS * D * 2;
     static constexpr int POOL = D == 128 ? 7 : 14;            // tile buffers
+    static constexpr int COLS = 256 - D;                      // columns of S: 2 x (COLS + D) are all of tensor memory
     static constexpr int OFF_BAR = POOL * TILE;
     static constexpr int N_BAR = 2 * POSITIONS + POOL + TURNS + 2 * ITEMS + 6;
     static constexpr int OFF_INFO = OFF_BAR + (N_BAR + 1) / 2 * 16;   // ItemInfo per item in flight
-    static constexpr int OFF_ROWS = OFF_INFO + ITEMS * 32;            // [group][step][warp] rows with columns in a 16-column step
-    static constexpr int OFF_WHERE = OFF_ROWS + 2 * 8 * 16;           // which buffer a position's tile is in; then the TMEM address
+    static constexpr int OFF_ROWS = OFF_INFO + ITEMS * 32;            // [group][16 columns of S][warp] rows with a column there
+    static constexpr int OFF_WHERE = OFF_ROWS + 2 * COLS;             // which buffer a position's tile is in; then the TMEM address
     static constexpr int SMEM_BYTES = OFF_WHERE + 2 * POSITIONS + 16 + 1024;  // + slack to align the base to 1 KB
     static_assert(SMEM_BYTES <= 227 * 1024, "one CTA's shared memory");
+};
+
+// How a row's columns are cut into rounds of a product, a softmax and another product.  Apart: a round is a tile of 128
+// columns, in which every block has its own.  MERGED: all blocks use the same columns of S - each product writes the
+// lanes of its block only - so that a row's own BM columns and, behind them, the slots of the first FIRST gathered
+// tiles are one round, and MORE gathered tiles each of the later ones.
+template <int D, int BM, bool MERGED>
+struct Cut {
+    static constexpr int COLS = Geo<D>::COLS;
+    static constexpr bool PACKED = MERGED && BM == 128;       // K and V rows of a gathered tile share a buffer (64 slots)
+    static constexpr int GS = PACKED ? BM / 2 : BM;           // ancestor slots of a block in a gathered tile
+    static constexpr int FIRST = MERGED ? 1 : 0, MORE = MERGED ? 2 : 1;
+    static constexpr int NW = BM / 32;                        // mask words of a row: its own block's,
+    static constexpr int EW0 = FIRST * GS / 32, EW = MORE * GS / 32;   // the first round's slots', a later round's
+    static constexpr int WORDS = NW + EW0 > EW ? NW + EW0 : EW;
+    static constexpr bool LONE = PACKED;                      // look for words with a column a row (see the softmax)
+    static_assert(EW >= EW0 && (!MERGED || (BM + FIRST * GS <= COLS && MORE * GS <= COLS)), "a round's columns");
 };
 
 // what the loading warp tells a group and its issuing thread about their next item
@@ -97,28 +120,24 @@ struct ItemInfo {
     int q_buf;                         // buffer of Q, later of O
 };
 
-// column tiles of an item whose longest ancestor list has `longest` entries, and whether the last is narrow
-template <int BM>
-__device__ __forceinline__ int tiles_of(int longest, bool *narrow) {
-    const int tiles = 1 + (longest + BM - 1) / BM;
-    *narrow = BM > 32 && tiles > 1 && longest - (tiles - 2) * BM <= BM / 2;
-    return tiles;
-}
-
-// 16-column steps of tile t that hold columns of some block (bit ks: columns 16 ks ..); seg: columns per block
-template <int BM>
-__device__ __forceinline__ uint32_t live_steps(int t, int seg, const int (&count)[ROWS / BM], int own_rows) {
+// 16-column steps of gathered tile t that hold slots of some block (bit ks: rows 16 ks .. of the buffer); seg: slots per block
+template <int BM, int GS>
+__device__ __forceinline__ uint32_t live_steps(int t, int seg, const int (&count)[ROWS / BM]) {
     uint32_t steps = 0;
-    if (t == 0) {
-        const int n = min((own_rows + 15) >> 4, ROWS / 16);
-        return (1u << n) - 1u;
-    }
 #pragma unroll
     for (int s = 0; s < ROWS / BM; ++s) {
-        const int left = min(count[s] - (t - 1) * BM, seg), n = left > 0 ? (left + 15) >> 4 : 0;
+        const int left = min(count[s] - (t - 1) * GS, seg), n = left > 0 ? (left + 15) >> 4 : 0;
         steps |= ((1u << n) - 1u) << (s * seg >> 4);
     }
     return steps;
+}
+
+// column tiles of an item whose longest ancestor list has `longest` entries, and whether the last is narrow
+template <int BM, int GS>
+__device__ __forceinline__ int tiles_of(int longest, bool *narrow) {
+    const int tiles = 1 + (longest + GS - 1) / GS;
+    *narrow = BM > 32 && GS == BM && tiles > 1 && longest - (tiles - 2) * GS <= BM / 2;
+    return tiles;
 }
 
 __device__ __forceinline__ void arrive(uint32_t bar) {
@@ -142,7 +161,7 @@ struct TreeUmmaArgs {
     int heads_first;                   // item order: heads fastest and the last rows first
 };
 
-template <typename T, int D, int BM>
+template <typename T, int D, int BM, bool MERGED>
 __global__ void __launch_bounds__(tree_umma::THREADS, 1)
 tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -153,8 +172,9 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
     using G = Geo<D>;
     constexpr bool BF16 = !std::is_same<T, __half>::value;
     constexpr int DH = D / 64, TILE = G::TILE, POOL = G::POOL;
+    using C = Cut<D, BM, MERGED>;
     constexpr int SUB = ROWS / BM;                        // blocks per item
-    constexpr int NW = BM / 32;                           // mask words per row and tile
+    constexpr int GS = C::GS, NW = C::NW;
 
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     extern __shared__ unsigned char smem_raw[];
@@ -182,7 +202,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;                // S/P of group g at g * 128, O at 256 + g * 128
+    const uint32_t tmem_base = *tmem_slot;                // S/P of group g at g * COLS, O at 2 * COLS + g * D
 
     const PackedLayout L = packed_layout(a.nb, BM, a.ma);
     const int maw = L.maw, stride = gridDim.x;
@@ -281,9 +301,10 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             const int p = tile_of(w), h = head_of(w), hk = h / a.kv_group;
             int cnt[SUB];
             bool narrow;
-            const int tiles = tiles_of<BM>(spread(cnt_lane, cnt), &narrow);
+            const int tiles = tiles_of<BM, GS>(spread(cnt_lane, cnt), &narrow);
             cnt_lane = count_of(next);                    // one item ahead
             const int g = n & 1, pos = g ? ahead[1] : ahead[0];
+            const int end = pos + (C::PACKED ? tiles + 1 : 2 * tiles - int(narrow));   // positions: two for a tile, one where K and V share a buffer
 #pragma unroll 1
             for (int kv = 0; kv < 3; ++kv) {              // own K, own V, Q
                 const int b = take();
@@ -308,7 +329,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 __syncwarp();
             }
 #pragma unroll 1
-            for (int at = pos + 2; alive && at < pos + 2 * tiles - int(narrow); ++at) {
+            for (int at = pos + 2; alive && at < end; ++at) {
                 const int b = take();
                 if (!alive) break;
                 if (elect_one()) {
@@ -318,7 +339,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 ++turn;
                 __syncwarp();
             }
-            (g ? ahead[1] : ahead[0]) = pos + 2 * tiles - int(narrow);
+            (g ? ahead[1] : ahead[0]) = end;
             w = next;
         }
     } else if (warp >= 11 && warp < 11 + GATHER) {
@@ -333,7 +354,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
         int cnt_lane = count_of(next);
         struct Tile {
             int g, pos, z, hk, row_a, row_b, node, b, slot;  // row_a, row_b: first tile row of my steps, -1: none
-            bool narrow;
+            bool one;                                     // K and V share a buffer
         };
         auto advance = [&](Tile &x) -> bool {             // the next gathered tile of my CTA
             while (++t >= tiles) {
@@ -346,13 +367,13 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 next = plus(w, step);
                 const int longest = spread(cnt_lane, cnt);
                 cnt_lane = count_of(next);
-                tiles = tiles_of<BM>(longest, &narrow);
+                tiles = tiles_of<BM, GS>(longest, &narrow);
                 pos += 2;                                 // the own tile's slots
                 t = 0;
             }
-            x.narrow = narrow && t + 1 == tiles;
-            const int seg = x.narrow ? BM / 2 : BM;
-            uint32_t steps = live_steps<BM>(t, seg, cnt, 0);
+            x.one = C::PACKED || (narrow && t + 1 == tiles);
+            const int seg = x.one ? BM / 2 : BM;
+            uint32_t steps = live_steps<BM, GS>(t, seg, cnt);
             x.row_a = x.row_b = -1;
             for (int i = 0; steps != 0; ++i) {
                 const int row = (__ffs(steps) - 1) * 16;
@@ -366,7 +387,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             if (mine >= 0) {
                 const int s = mine / seg;
                 x.b = tile_of(w) * SUB + s;
-                x.slot = (t - 1) * BM + mine - s * seg + (lane & 15);
+                x.slot = (t - 1) * GS + mine - s * seg + (lane & 15);
                 int c = 0;
 #pragma unroll
                 for (int i = 0; i < SUB; ++i)
@@ -379,7 +400,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             x.hk = head_of(w) / a.kv_group;
             x.g = n & 1;
             x.pos = pos;
-            pos += x.narrow ? 1 : 2;
+            pos += x.one ? 1 : 2;
             return true;
         };
         Tile cur{}, nxt{};
@@ -402,7 +423,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             if (unsigned(node) >= unsigned(a.n_q)) node = -1;         // padding: zeros
             const T *kp = static_cast<const T *>(a.k) + cur.z * a.ks_z + cur.hk * a.ks_h + a.prefix * a.ks_n + lc * 8;
             const T *vp = static_cast<const T *>(a.v) + cur.z * a.vs_z + cur.hk * a.vs_h + a.prefix * a.vs_n + lc * 8;
-            const int half = cur.narrow ? HALF / 2 : HALF;
+            const int half = cur.one ? HALF / 2 : HALF;
             auto claim = [&](int at) {
                 const uint32_t bar = bar_go + (turn % TURNS) * 8, parity = (turn / TURNS) & 1;
                 ++turn;
@@ -410,10 +431,10 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             };
 #pragma unroll 1
             for (int kv = 0; kv < 2 && alive; ++kv) {
-                const int at = cur.pos + (cur.narrow ? 0 : kv);
-                if (kv == 0 || !cur.narrow) claim(at);
+                const int at = cur.pos + (cur.one ? 0 : kv);
+                if (kv == 0 || !cur.one) claim(at);
                 if (!alive) break;
-                const uint32_t d0 = s_base + buf_of(cur.g, at) * TILE + (kv && cur.narrow ? TILE / 2 : 0) + (lc >> 3) * half;
+                const uint32_t d0 = s_base + buf_of(cur.g, at) * TILE + (kv && cur.one ? TILE / 2 : 0) + (lc >> 3) * half;
                 const T *src = kv ? vp : kp;
                 const int64_t row_stride = kv ? a.vs_n : a.ks_n;
 #pragma unroll 1
@@ -427,7 +448,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                         cp_async16(d0 + row * 128 + (((lc & 7) ^ (row & 7)) << 4), src + (nd < 0 ? 0 : nd) * row_stride, nd >= 0);
                     }
                 }
-                if (kv == 0 && cur.narrow) continue;
+                if (kv == 0 && cur.one) continue;
                 cp_async_arrive(full_of(cur.g, at));      // by every lane, once its copies have landed
             }
             if (!alive) break;
@@ -440,10 +461,11 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
         // (as every role does before its first bounded wait: the grid ahead may run longer than the bound)
         if (a.meta_stable) asm volatile("griddepcontrol.wait;\n" ::: "memory");
         if (elect_one()) {
-            const uint64_t dk = smem_desc(s_base, 16), dv = smem_desc(s_base, HALF), dv_narrow = smem_desc(s_base + TILE / 2, HALF / 2);
-            const uint32_t idesc_pv = instr_desc(BF16, true, D), s_col = tmem_base + g * 128, o_col = s_col + 256;
+            const uint64_t dk = smem_desc(s_base, 16), dv = smem_desc(s_base, HALF), dv_one = smem_desc(s_base + TILE / 2, HALF / 2);
+            const uint32_t idesc_pv = instr_desc(BF16, true, D), s_col = tmem_base + g * C::COLS, o_col = tmem_base + 2 * C::COLS + g * D;
+            const uint4 *rows = reinterpret_cast<const uint4 *>(smem + G::OFF_ROWS) + g * (C::COLS / 16);
             bool alive = true;
-            int tile_no = 0, n = g;
+            int round = 0, n = g;
             Where w = first;
 #pragma unroll 1
             for (int item = blockIdx.x + g * stride; item < ta.n_items && alive; item += 2 * stride, n += 2, w = plus(w, step)) {
@@ -452,49 +474,139 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 if (!alive) break;
                 const int4 in = info[(n % ITEMS) * 2], counts = info[(n % ITEMS) * 2 + 1];
                 const int tiles = in.x, four[4] = {counts.x, counts.y, counts.z, counts.w};
+                const uint64_t dqs = dk + uint64_t(in.w * (TILE >> 4));
                 int cnt[SUB];
 #pragma unroll
                 for (int s = 0; s < SUB; ++s) cnt[s] = four[s];
-                int at = in.y;                            // position of the tile's K rows
+                if constexpr (MERGED) {
+                    auto one_buffer = [&](int t) { return t > 0 && (C::PACKED || (in.z != 0 && t + 1 == tiles)); };
+                    auto live = [&](int t, int s, int seg) -> int {   // 16-column steps of block s in tile t
+                        const int left = t == 0 ? min(own_rows - s * BM, BM) : min(cnt[s] - (t - 1) * GS, seg);
+                        return left > 0 ? (left + 15) >> 4 : 0;
+                    };
+                    // Every block's rows against its own columns, all blocks into the same columns of S (each its own lanes).
+                    // SEG: columns per block, BM or, where K and V share a buffer, BM / 2
+                    auto scores = [&](auto seg_c, int t, uint32_t to, uint64_t dks) {
+                        constexpr int SEG = decltype(seg_c)::value;
+#pragma unroll
+                        for (int s = 0; s < SUB; ++s) {
+                            const int steps = live(t, s, SEG);
+                            if (steps == 0) continue;
+                            const uint32_t idesc_s = instr_desc(BF16, false, 16 * steps);
+#pragma unroll
+                            for (int ks = 0; ks < D / 16; ++ks)
+                                mma_f16_block<BM>(to, dqs + uint64_t(((ks >> 2) * HALF + (ks & 3) * 32) >> 4),
+                                                  dks + uint64_t(((ks >> 2) * (SUB * SEG * 128) + (ks & 3) * 32 + s * SEG * 128) >> 4),
+                                                  idesc_s, ks > 0, s);
+                        }
+                    };
+                    auto output = [&](auto seg_c, int t, int col, uint64_t dvs) {
+                        constexpr int SEG = decltype(seg_c)::value;
+                        uint4 off[SEG / 16];
+#pragma unroll
+                        for (int ks = 0; ks < SEG / 16; ++ks) off[ks] = rows[(col >> 4) + ks];
+#pragma unroll
+                        for (int s = 0; s < SUB; ++s) {
+                            const int steps = live(t, s, SEG);
+#pragma unroll
+                            for (int ks = 0; ks < SEG / 16; ++ks)
+                                if (ks < steps)
+                                    mma_f16_ts_but(o_col, s_col + (col >> 1) + ks * 8, dvs + uint64_t(((s * SEG + ks * 16) * 128) >> 4), idesc_pv,
+                                                   not_block_rows<BM>(off[ks], s));
+                        }
+                    };
+                    using Full = std::integral_constant<int, BM>;
+                    using Part = std::integral_constant<int, BM / 2 < 32 ? BM : BM / 2>;   // (never one buffer with blocks of 32)
+                    int at = in.y;                            // position of the round's first tile
 #pragma unroll 1
-                for (int t = 0; t < tiles; ++t, ++tile_no) {
-                    const bool narrow = in.z != 0 && t + 1 == tiles;
-                    const uint32_t steps = live_steps<BM>(t, narrow ? BM / 2 : BM, cnt, own_rows);
-                    const uint32_t idesc_s = instr_desc(BF16, false, 16 * (32 - __clz(steps)));
-                    alive = wait(full_of(g, at), full_parity(at), a.status, item);
-                    if (!alive) break;
-                    int b = buf_of(g, at);
-                    const uint64_t dqs = dk + uint64_t(in.w * (TILE >> 4)), dks = dk + uint64_t(b * (TILE >> 4)),
-                                   half16 = (narrow ? HALF / 2 : HALF) >> 4;
-                    if (t > 0) fence_copied();
-                    fence_after_sync();
-#pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks)
-                        mma_f16(s_col, dqs + uint64_t(((ks >> 2) * HALF + (ks & 3) * 32) >> 4),
-                                dks + (ks >> 2) * half16 + (ks & 3) * 2, idesc_s, ks > 0);
-                    mma_commit(bar_s + g * 8);
-                    if (!narrow) {
-                        mma_commit(bar_empty + b * 8);
-                        ++at;
+                    for (int t0 = 0; t0 < tiles; ++round) {
+                        const int t1 = min(tiles, t0 == 0 ? 1 + C::FIRST : t0 + C::MORE);
+                        int p = at, col = 0;
+#pragma unroll 1
+                        for (int t = t0; t < t1; ++t) {
+                            alive = wait(full_of(g, p), full_parity(p), a.status, item);
+                            if (!alive) break;
+                            const int b = buf_of(g, p);
+                            const uint64_t dks = dk + uint64_t(b * (TILE >> 4));
+                            if (t > 0) fence_copied();
+                            fence_after_sync();
+                            const bool one = one_buffer(t);
+                            if (one) scores(Part{}, t, s_col + col, dks);
+                            else scores(Full{}, t, s_col + col, dks);
+                            if (t + 1 == t1) mma_commit(bar_s + g * 8);
+                            if (!one) mma_commit(bar_empty + b * 8);
+                            p += one ? 1 : 2;
+                            col += t == 0 ? BM : GS;
+                        }
+                        if (!alive) break;
+                        // (the first V tile is usually there long before P)
+                        alive = (one_buffer(t0) || wait(full_of(g, at + 1), full_parity(at + 1), a.status, item)) &&
+                                wait(bar_p + g * 8, round & 1, a.status, item);
+                        col = 0;
+#pragma unroll 1
+                        for (int t = t0; t < t1 && alive; ++t) {
+                            const bool one = one_buffer(t);
+                            at += one ? 0 : 1;
+                            alive = one || t == t0 || wait(full_of(g, at), full_parity(at), a.status, item);
+                            if (!alive) break;
+                            const int b = buf_of(g, at);
+                            ++at;
+                            if (t > 0) fence_copied();
+                            fence_after_sync();
+                            if (one) output(Part{}, t, col, dv_one + uint64_t(b * (TILE >> 4)));
+                            else output(Full{}, t, col, dv + uint64_t(b * (TILE >> 4)));
+                            mma_commit(bar_empty + b * 8);
+                            col += t == 0 ? BM : GS;
+                        }
+                        if (!alive) break;
+                        t0 = t1;
+                        if (t0 == tiles) mma_commit(bar_o + g * 8);
                     }
-                    alive = (narrow || wait(full_of(g, at), full_parity(at), a.status, item)) &&
-                            wait(bar_p + g * 8, tile_no & 1, a.status, item);
-                    if (!alive) break;
-                    b = buf_of(g, at);
-                    ++at;
-                    const uint64_t dvs = (narrow ? dv_narrow : dv) + uint64_t(b * (TILE >> 4));
-                    if (t > 0) fence_copied();
-                    fence_after_sync();
-                    const uint4 *rows = reinterpret_cast<const uint4 *>(smem + G::OFF_ROWS) + g * 8;
-                    uint4 on[8];
+                } else {
+                    // 16-column steps of tile t that some block has (bit ks: rows 16 ks .. of the buffer)
+                    auto steps_of = [&](int t, int seg) -> uint32_t {
+                        return t == 0 ? (1u << min((own_rows + 15) >> 4, ROWS / 16)) - 1u : live_steps<BM, GS>(t, seg, cnt);
+                    };
+                    int at = in.y;                            // position of the tile's K rows
+#pragma unroll 1
+                    for (int t = 0; t < tiles; ++t, ++round) {
+                        const bool narrow = in.z != 0 && t + 1 == tiles;
+                        const uint32_t steps = steps_of(t, narrow ? BM / 2 : BM);
+                        const uint32_t idesc_s = instr_desc(BF16, false, 16 * (32 - __clz(steps)));
+                        alive = wait(full_of(g, at), full_parity(at), a.status, item);
+                        if (!alive) break;
+                        int b = buf_of(g, at);
+                        const uint64_t dks = dk + uint64_t(b * (TILE >> 4)),
+                                       half16 = (narrow ? HALF / 2 : HALF) >> 4;
+                        if (t > 0) fence_copied();
+                        fence_after_sync();
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) on[ks] = rows[ks];
+                        for (int ks = 0; ks < D / 16; ++ks)
+                            mma_f16(s_col, dqs + uint64_t(((ks >> 2) * HALF + (ks & 3) * 32) >> 4),
+                                    dks + (ks >> 2) * half16 + (ks & 3) * 2, idesc_s, ks > 0);
+                        mma_commit(bar_s + g * 8);
+                        if (!narrow) {
+                            mma_commit(bar_empty + b * 8);
+                            ++at;
+                        }
+                        alive = (narrow || wait(full_of(g, at), full_parity(at), a.status, item)) &&
+                                wait(bar_p + g * 8, round & 1, a.status, item);
+                        if (!alive) break;
+                        b = buf_of(g, at);
+                        ++at;
+                        const uint64_t dvs = (narrow ? dv_one : dv) + uint64_t(b * (TILE >> 4));
+                        if (t > 0) fence_copied();
+                        fence_after_sync();
+                        uint4 on[8];
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks)
-                        if ((steps >> ks) & 1u)
-                            mma_f16_ts_rows(o_col, s_col + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, on[ks]);
-                    mma_commit(bar_empty + b * 8);
-                    if (t + 1 == tiles) mma_commit(bar_o + g * 8);
+                        for (int ks = 0; ks < 8; ++ks) on[ks] = rows[ks];
+#pragma unroll
+                        for (int ks = 0; ks < 8; ++ks)
+                            if ((steps >> ks) & 1u)
+                                mma_f16_ts_rows(o_col, s_col + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, on[ks]);
+                        mma_commit(bar_empty + b * 8);
+                        if (t + 1 == tiles) mma_commit(bar_o + g * 8);
+                    }
                 }
             }
         }
@@ -520,10 +632,10 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
         // ================================ softmax ================================
         const int g = warp >> 2, r = tid & 127;           // my group and query row of its items
         const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
-        const uint32_t tmem_s = tmem_base + g * 128 + lane_base, tmem_o = tmem_s + 256;
+        const uint32_t tmem_s = tmem_base + g * C::COLS + lane_base, tmem_o = tmem_base + 2 * C::COLS + g * D + lane_base;
         const int sub = r / BM, j = r % BM;               // my block and row in it (sub is uniform in a warp)
         const float c2 = a.scale_log2;
-        // mask words of my row: its own block's, and those of gathered tile t (item and block may not exist)
+        // mask words of my row: its own block's, and those from word w0 of its ancestor slots on (item and block may not exist)
         const uint32_t *mask = reinterpret_cast<const uint32_t *>(a.packed);
         const uint32_t blob_words = uint32_t(a.meta_stride >> 2), own0 = uint32_t(L.off_bmask >> 2) + j * NW,
                        ext0 = uint32_t(L.off_emask >> 2) + j * maw;
@@ -541,20 +653,20 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 w[0] = ok ? __ldg(from) : 0u;
             }
         };
-        auto ext_words = [&](const Where &at, int t, uint32_t (&w)[NW]) {
-            const int b = tile_of(at) * SUB + sub, w0 = (t - 1) * NW, left = at.z < a.Z && b < a.nb ? maw - w0 : 0;
+        auto ext_words = [&](const Where &at, int w0, uint32_t (&w)[C::EW]) {
+            const int b = tile_of(at) * SUB + sub, left = at.z < a.Z && b < a.nb ? maw - w0 : 0;
             const uint32_t *from = mask + (uint32_t(at.z) * blob_words + ext0 + uint32_t(b) * uint32_t(BM * maw) + uint32_t(w0));
 #pragma unroll
-            for (int i = 0; i < NW; ++i) w[i] = i < left ? __ldg(from + i) : 0u;
+            for (int i = 0; i < C::EW; ++i) w[i] = i < left ? __ldg(from + i) : 0u;
         };
-        uint32_t own[NW], ext[NW];
+        uint32_t own[NW], ext[C::EW];
         Where at = first;
         own_words(at, own);
-        ext_words(at, 1, ext);
+        ext_words(at, 0, ext);
         if (a.meta_stable) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
         bool alive = true;
-        int tile_no = 0, n = g;
+        int round = 0, n = g;
 #pragma unroll 1
         for (int item = blockIdx.x + g * stride; item < ta.n_items; item += 2 * stride, n += 2) {
             const Where at_next = plus(at, step);
@@ -568,116 +680,252 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             for (int c = 0; c < 16; ++c) zero[c] = 0u;
 #pragma unroll 1
             for (int c0 = 0; c0 < D; c0 += 16) tmem_st16(tmem_o + c0, zero);
+            if constexpr (MERGED) {
 #pragma unroll 1
-            for (int t = 0; t < tiles; ++t, ++tile_no) {
-                uint32_t word[NW];
+                for (int t = 0; t < tiles; ++round) {         // t: the round's first tile
+                    const bool first_round = t == 0;
+                    uint32_t word[C::WORDS];                  // the round's columns that my row attends to
 #pragma unroll
-                for (int i = 0; i < NW; ++i) word[i] = t == 0 ? own[i] : ext[i];
-                // the words of the tile after next go out now: a loaded L2 answers late
-                const bool last_tile = t + 1 == tiles;
-                if (t == 0) own_words(at_next, own);
-                if (t > 0 || last_tile) ext_words(last_tile ? at_next : at, last_tile ? 1 : t + 1, ext);
-                const bool narrow = in.z != 0 && last_tile;
-                const int segw = narrow ? NW / 2 : NW;    // my block's words in this tile; words past them are empty
-                const uint32_t tmem_my = tmem_s + sub * segw * 32;
-                alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, tile_no & 1, a.status, item));
-                if (!alive) break;
-                fence_after_sync();
+                    for (int i = 0; i < C::WORDS; ++i) {
+                        const uint32_t mine = i < NW ? own[i % NW] : i < NW + C::EW0 ? ext[(i - NW) % C::EW] : 0u;
+                        word[i] = first_round ? mine : i < C::EW ? ext[i % C::EW] : 0u;
+                    }
+                    t = first_round ? 1 + C::FIRST : t + C::MORE;
+                    // the words of the round after go out now: a loaded L2 answers late
+                    if (first_round) own_words(at_next, own);
+                    if (t >= tiles) ext_words(at_next, 0, ext);
+                    else ext_words(at, (t - 1) * (GS / 32), ext);
+                    alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, round & 1, a.status, item));
+                    if (!alive) break;
+                    fence_after_sync();
 
-                uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
-                {
-                    uint32_t on = 0;                      // lane k: rows of my warp with a column in step k of the tile
-                    const int k = lane - sub * segw * 2;
+                    uint32_t live = 0, lone_words = 0;        // bit i: some row of my warp has a bit in word i; no row has two
+                    {
+                        uint32_t on = 0;                      // lane k: rows of my warp with a column in 16 k ..
 #pragma unroll
-                    for (int i = 0; i < NW; ++i) {
-                        const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
-                        live |= uint32_t((lo | hi) != 0u) << i;
-                        if (k == 2 * i) on = lo;
-                        if (k == 2 * i + 1) on = hi;
+                        for (int i = 0; i < C::WORDS; ++i) {
+                            const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
+                            live |= uint32_t((lo | hi) != 0u) << i;
+                            if (C::LONE && i < NW && first_round && (lo | hi) != 0u && __ballot_sync(0xffffffffu, (word[i] & (word[i] - 1u)) != 0u) == 0u) lone_words |= 1u << i;
+                            if (lane == 2 * i) on = lo;
+                            if (lane == 2 * i + 1) on = hi;
+                        }
+                        if (lane < 2 * C::WORDS) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (C::COLS / 16) + lane) * 4 + (warp & 3)] = ~on;
                     }
-                    if (lane < 8) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * 8 + lane) * 4 + (warp & 3)] = on;
-                }
-                float sum[2] = {0.f, 0.f}, mu = 0.f, mx = -INFINITY;
-                // My live words, WT to a turn.  First round: the row's maximum, then the reference point.  Second round (or
-                // at once, when one turn was all): probabilities, over S - word i of P covers columns 16 i .. of S,
-                // below the words still to be read; words nobody uses are zeros.  One loop and one copy of its
-                // code: what runs once per tile and does not stay in the instruction cache costs more than it saves
-                // (two words to a turn at block_m 128: 1760 -> 1892 us on the forest of 65532 nodes; both words of
-                // a row in one turn at block_m 64: 69.0 -> 67.5 us on the deep tree).
-                constexpr int WT = NW == 2 ? 2 : 1;
-                bool second = false;
-#pragma unroll 1
-                for (uint32_t rest = live; rest != 0u;) {
-                    uint32_t s[WT][32];
-                    int wi[WT];                           // the words' numbers; NW: none
+                    float mu = 0.f, mx = -INFINITY;
+                    uint64_t sum2 = 0;
+                    // A word in which every row has one column at most - a block's own word where the tree is numbered breadth first and
+                    // a row attends to nobody in its block but itself - needs no 32 exponentials: the score is picked out (forest of 65532
+                    // nodes 1615 -> 1550 us).  At D 128, block_m 64 the lists are the longer part: deep tree 61.6 -> 64.8, not there.
+                    int lone = -1, lone_at = -1;              // that word, my row's column in it
+                    if (C::LONE && lone_words != 0u) {
+                        lone = __ffs(lone_words) - 1;
+                        live &= ~(1u << lone);
+                        uint32_t v[32], w = word[0];
 #pragma unroll
-                    for (int k = 0; k < WT; ++k) {
-                        wi[k] = WT == 1 || rest != 0u ? __ffs(rest) - 1 : NW;
+                        for (int i = 1; i < NW; ++i) w = lone == i ? word[i] : w;
+                        tmem_ld32(v, tmem_s + lone * 32);
+                        lone_at = __ffs(w) - 1;
+                        tmem_ld_wait(v);
+#pragma unroll
+                        for (int half = 16; half > 0; half /= 2)
+#pragma unroll
+                            for (int c = 0; c < half; ++c) v[c] = (lone_at & half) != 0 ? v[c + half] : v[c];
+                        mx = lone_at < 0 ? -INFINITY : __uint_as_float(v[0]);
+                    }
+                    const float lone_score = mx;
+                    // My live words, one to a turn (two spill: there are words of two kinds to keep).  First time through: the row's maximum, then the
+                    // reference point.  Second time (or at once, when one turn was all): probabilities, over S - word i of P
+                    // covers columns 16 i .. of S, below the words still to be read.
+                    bool second = false;
+#pragma unroll 1
+                    for (uint32_t rest = live; (C::LONE && !second) || rest != 0u;) {
+                        uint32_t s[32];
+                        const int wi = __ffs(rest) - 1;       // the word's number, -1: none but the lone one
                         rest &= rest - 1;
-                        if (WT == 1 || wi[k] < NW) tmem_ld32(s[k], tmem_my + wi[k] * 32);
-                    }
-                    float m = -INFINITY;
+                        if (!C::LONE || wi >= 0) {
+                            uint32_t w = word[0];
+                            tmem_ld32(s, tmem_s + wi * 32);
 #pragma unroll
-                    for (int k = 0; k < WT; ++k) {
-                        if (WT > 1 && wi[k] >= NW) continue;
-                        uint32_t w = word[0];
+                            for (int i = 1; i < C::WORDS; ++i) w = wi == i ? word[i] : w;
+                            tmem_ld_wait(s);
+                            float m2[2] = {mx, -INFINITY};
 #pragma unroll
-                        for (int i = 1; i < NW; ++i) w = wi[k] == i ? word[i] : w;
-                        tmem_ld_wait(s[k]);
-                        float m2[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-                        for (int c = 0; c < 32; c += 2) {
-                            s[k][c] = (w & (1u << c)) != 0u ? s[k][c] : 0xff800000u;
-                            s[k][c + 1] = (w & (2u << c)) != 0u ? s[k][c + 1] : 0xff800000u;
-                            m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[k][c]), __uint_as_float(s[k][c + 1])));
-                        }
-                        m = fmaxf(m, fmaxf(m2[0], m2[1]));
-                    }
-                    if (!second) {
-                        mx = fmaxf(mx, m);
-                        if (rest != 0u) continue;
-                        const bool up = mx > m_ref;
-                        if (__any_sync(0xffffffffu, up)) {
-                            if (t > 0) {                  // rescale my row of O (the stores are awaited with P's)
-                                const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
-#pragma unroll 1
-                                for (int c0 = 0; c0 < D; c0 += 16) {
-                                    uint32_t o[16];
-                                    tmem_ld16(o, tmem_o + c0);
-#pragma unroll
-                                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                                    tmem_st16(tmem_o + c0, o);
-                                }
-                                l *= alpha;
+                            for (int c = 0; c < 32; c += 2) {
+                                s[c] = (w & (1u << c)) != 0u ? s[c] : 0xff800000u;
+                                s[c + 1] = (w & (2u << c)) != 0u ? s[c + 1] : 0xff800000u;
+                                m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[c]), __uint_as_float(s[c + 1])));
                             }
-                            if (up) m_ref = mx;
+                            mx = fmaxf(m2[0], m2[1]);
                         }
-                        mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
-                        second = true;
-                        if (WT < NW && __popc(live) > WT) {       // more than a turn: once again from the first
-                            rest = live;
-                            continue;
+                        if (!second) {
+                            if (rest != 0u) continue;
+                            const bool up = mx > m_ref;
+                            if (__any_sync(0xffffffffu, up)) {
+                                if (!first_round) {           // rescale my row of O (the stores are awaited with P's)
+                                    const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
+#pragma unroll 1
+                                    for (int c0 = 0; c0 < D; c0 += 16) {
+                                        uint32_t o[16];
+                                        tmem_ld16(o, tmem_o + c0);
+#pragma unroll
+                                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                                        tmem_st16(tmem_o + c0, o);
+                                    }
+                                    l *= alpha;
+                                }
+                                if (up) m_ref = mx;
+                            }
+                            mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
+                            second = true;
+                            if ((live & (live - 1u)) != 0u) { // more than a turn: once again from the first
+                                rest = live;
+                                continue;
+                            }
+                        }
+                        if (!C::LONE || wi >= 0) {
+                            const uint64_t scale2 = pair(c2, c2), shift2 = pair(-mu, -mu);
+                            uint32_t pk[16];
+#pragma unroll
+                            for (int c = 0; c < 32; c += 2) {
+                                float p0, p1;
+                                unpair(fma2(pair(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), scale2, shift2), p0, p1);
+                                p0 = fast_exp2(p0);
+                                p1 = fast_exp2(p1);
+                                sum2 = add2(sum2, pair(p0, p1));
+                                pk[c >> 1] = MT::pack(p0, p1);
+                            }
+                            tmem_st16(tmem_s + wi * 16, pk);
                         }
                     }
-#pragma unroll
-                    for (int k = 0; k < WT; ++k) {
-                        if (WT > 1 && wi[k] >= NW) continue;
+                    if (C::LONE && lone >= 0) {
+                        const float p = fast_exp2(fmaf(lone_score, c2, -mu));
+                        const uint32_t v = (lone_at & 1) != 0 ? MT::pack(0.f, p) : MT::pack(p, 0.f);
                         uint32_t pk[16];
 #pragma unroll
-                        for (int c = 0; c < 32; c += 2) {
-                            const float p0 = fast_exp2(fmaf(__uint_as_float(s[k][c]), c2, -mu));
-                            const float p1 = fast_exp2(fmaf(__uint_as_float(s[k][c + 1]), c2, -mu));
-                            sum[0] += p0;
-                            sum[1] += p1;
-                            pk[c >> 1] = MT::pack(p0, p1);
-                        }
-                        tmem_st16(tmem_s + (sub * segw + wi[k]) * 16, pk);
+                        for (int i = 0; i < 16; ++i) pk[i] = lone_at >> 1 == i ? v : 0u;
+                        tmem_st16(tmem_s + lone * 16, pk);
+                        l += p;
                     }
+                    float sum[2];
+                    unpair(sum2, sum[0], sum[1]);
+                    l += sum[0] + sum[1];
+                    tmem_st_wait();
+                    fence_before_sync();
+                    arrive(bar_p + g * 8);
                 }
-                l += sum[0] + sum[1];
-                tmem_st_wait();
-                fence_before_sync();
-                arrive(bar_p + g * 8);
+            } else {
+#pragma unroll 1
+                for (int t = 0; t < tiles; ++t, ++round) {
+                    uint32_t word[NW];
+#pragma unroll
+                    for (int i = 0; i < NW; ++i) word[i] = t == 0 ? own[i] : ext[i];
+                    // the words of the tile after next go out now: a loaded L2 answers late
+                    const bool last_tile = t + 1 == tiles;
+                    if (t == 0) own_words(at_next, own);
+                    if (t > 0 || last_tile) ext_words(last_tile ? at_next : at, last_tile ? 0 : t * NW, ext);
+                    const bool narrow = in.z != 0 && last_tile;
+                    const int segw = narrow ? NW / 2 : NW;    // my block's words in this tile; words past them are empty
+                    const uint32_t tmem_my = tmem_s + sub * segw * 32;
+                    alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, round & 1, a.status, item));
+                    if (!alive) break;
+                    fence_after_sync();
+
+                    uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
+                    {
+                        uint32_t on = 0;                      // lane k: rows of my warp with a column in step k of the tile
+                        const int k = lane - sub * segw * 2;
+#pragma unroll
+                        for (int i = 0; i < NW; ++i) {
+                            const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
+                            live |= uint32_t((lo | hi) != 0u) << i;
+                            if (k == 2 * i) on = lo;
+                            if (k == 2 * i + 1) on = hi;
+                        }
+                        if (lane < 8) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (C::COLS / 16) + lane) * 4 + (warp & 3)] = on;
+                    }
+                    float sum[2] = {0.f, 0.f}, mu = 0.f, mx = -INFINITY;
+                    // My live words, WT to a turn.  First round: the row's maximum, then the reference point.  Second round (or
+                    // at once, when one turn was all): probabilities, over S - word i of P covers columns 16 i .. of S,
+                    // below the words still to be read; words nobody uses are zeros.  One loop and one copy of its
+                    // code: what runs once per tile and does not stay in the instruction cache costs more than it saves
+                    // (two words to a turn at block_m 128: 1760 -> 1892 us on the forest of 65532 nodes; both words of
+                    // a row in one turn at block_m 64: 69.0 -> 67.5 us on the deep tree).
+                    constexpr int WT = NW == 2 ? 2 : 1;
+                    bool second = false;
+#pragma unroll 1
+                    for (uint32_t rest = live; rest != 0u;) {
+                        uint32_t s[WT][32];
+                        int wi[WT];                           // the words' numbers; NW: none
+#pragma unroll
+                        for (int k = 0; k < WT; ++k) {
+                            wi[k] = WT == 1 || rest != 0u ? __ffs(rest) - 1 : NW;
+                            rest &= rest - 1;
+                            if (WT == 1 || wi[k] < NW) tmem_ld32(s[k], tmem_my + wi[k] * 32);
+                        }
+                        float m = -INFINITY;
+#pragma unroll
+                        for (int k = 0; k < WT; ++k) {
+                            if (WT > 1 && wi[k] >= NW) continue;
+                            uint32_t w = word[0];
+#pragma unroll
+                            for (int i = 1; i < NW; ++i) w = wi[k] == i ? word[i] : w;
+                            tmem_ld_wait(s[k]);
+                            float m2[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+                            for (int c = 0; c < 32; c += 2) {
+                                s[k][c] = (w & (1u << c)) != 0u ? s[k][c] : 0xff800000u;
+                                s[k][c + 1] = (w & (2u << c)) != 0u ? s[k][c + 1] : 0xff800000u;
+                                m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[k][c]), __uint_as_float(s[k][c + 1])));
+                            }
+                            m = fmaxf(m, fmaxf(m2[0], m2[1]));
+                        }
+                        if (!second) {
+                            mx = fmaxf(mx, m);
+                            if (rest != 0u) continue;
+                            const bool up = mx > m_ref;
+                            if (__any_sync(0xffffffffu, up)) {
+                                if (t > 0) {                  // rescale my row of O (the stores are awaited with P's)
+                                    const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
+#pragma unroll 1
+                                    for (int c0 = 0; c0 < D; c0 += 16) {
+                                        uint32_t o[16];
+                                        tmem_ld16(o, tmem_o + c0);
+#pragma unroll
+                                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                                        tmem_st16(tmem_o + c0, o);
+                                    }
+                                    l *= alpha;
+                                }
+                                if (up) m_ref = mx;
+                            }
+                            mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
+                            second = true;
+                            if (WT < NW && __popc(live) > WT) {       // more than a turn: once again from the first
+                                rest = live;
+                                continue;
+                            }
+                        }
+#pragma unroll
+                        for (int k = 0; k < WT; ++k) {
+                            if (WT > 1 && wi[k] >= NW) continue;
+                            uint32_t pk[16];
+#pragma unroll
+                            for (int c = 0; c < 32; c += 2) {
+                                const float p0 = fast_exp2(fmaf(__uint_as_float(s[k][c]), c2, -mu));
+                                const float p1 = fast_exp2(fmaf(__uint_as_float(s[k][c + 1]), c2, -mu));
+                                sum[0] += p0;
+                                sum[1] += p1;
+                                pk[c >> 1] = MT::pack(p0, p1);
+                            }
+                            tmem_st16(tmem_s + (sub * segw + wi[k]) * 16, pk);
+                        }
+                    }
+                    l += sum[0] + sum[1];
+                    tmem_st_wait();
+                    fence_before_sync();
+                    arrive(bar_p + g * 8);
+                }
             }
             if (!alive) break;
 
@@ -720,7 +968,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
 
 // ---- host side ---------------------------------------------------------------------------------
 
-template <typename T, int D, int BM>
+template <typename T, int D, int BM, bool MERGED>
 cudaError_t launch_tree_umma_t(const AttnArgs &a, cudaStream_t stream) {
     using G = tree_umma::Geo<D>;
     constexpr bool bf16 = !std::is_same<T, __half>::value;
@@ -733,7 +981,7 @@ cudaError_t launch_tree_umma_t(const AttnArgs &a, cudaStream_t stream) {
         return cudaErrorNotSupported;
     static DeviceOnce configured;
     const cudaError_t ce = configured.run([&] {
-        return cudaFuncSetAttribute(tree_umma_kernel<T, D, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES);
+        return cudaFuncSetAttribute(tree_umma_kernel<T, D, BM, MERGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES);
     });
     if (ce != cudaSuccess) return ce;
     TreeUmmaArgs ta = {};
@@ -754,15 +1002,17 @@ cudaError_t launch_tree_umma_t(const AttnArgs &a, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, tree_umma_kernel<T, D, BM>, a, ta, tq, tk, tv, to);
+    return cudaLaunchKernelEx(&cfg, tree_umma_kernel<T, D, BM, MERGED>, a, ta, tq, tk, tv, to);
 }
 
 template <typename T, int D>
 cudaError_t launch_tree_umma_d(const AttnArgs &a, cudaStream_t stream) {
     switch (a.bm) {
-        case 32: return launch_tree_umma_t<T, D, 32>(a, stream);
-        case 64: return launch_tree_umma_t<T, D, 64>(a, stream);
-        case 128: return launch_tree_umma_t<T, D, 128>(a, stream);
+        case 32: return launch_tree_umma_t<T, D, 32, false>(a, stream);
+        case 64:
+            if (D == 128 && a.ma <= 128) return launch_tree_umma_t<T, D, 64, D == 128>(a, stream);
+            return launch_tree_umma_t<T, D, 64, false>(a, stream);
+        case 128: return launch_tree_umma_t<T, D, 128, D == 64>(a, stream);
     }
     return cudaErrorNotSupported;
 }

@@ -59,6 +59,38 @@ def test_tree_umma_many_items_strided(fst, D, bm):
     assert fst.last_status() == 0
 
 
+@pytest.mark.parametrize("D,bm", [(64, 128), (128, 64)])
+@pytest.mark.parametrize("own", ["alone", "chained", "across"])
+@pytest.mark.parametrize("n,teeth", [(77, 1), (129, 20), (300, 32), (300, 33), (640, 64), (640, 65), (300, 96), (640, 97), (650, 128)])
+def test_tree_umma_merged_rounds(fst, D, bm, own, n, teeth):
+    """The own tile and the first gathered one in one softmax (bounds of up to 128 at D 128): lists that end in either half
+    of the first gathered tile, fill it, or need a second round; rows that attend to nobody in their block but
+    themselves, to their neighbours, and to a column in another 32-column word that nobody else uses.  A value that
+    is not finite stays with the rows that attend to it or to one of its fifteen neighbours."""
+    par = comb(n, teeth)
+    for i in range(teeth, n):
+        if own == "chained" and i % 3 and i > teeth or own == "across" and i % 32 == 0 and i > teeth:
+            par[i] = i - 1
+    try:
+        meta = fst.build_tree_metadata(par, bm, 128, reference_format=False)
+    except RuntimeError:                                  # with those inside the block there are more
+        meta = fst.build_tree_metadata(par, bm, 128 + bm, reference_format=False)
+    longest = int(meta.packed[0, : meta.n_blocks * 4].view(torch.int32).max())
+    assert longest <= teeth + 2 and (longest >= teeth or own == "chained" or n < 2 * bm)
+    g = torch.Generator().manual_seed(n + teeth)
+    q, k, v = (torch.randn((3, 60, n, D), generator=g).half().cuda() for _ in range(3))     # several items a CTA
+    o, lse = fst.fst_attention(q, k, v, meta, sm_scale=D ** -0.5, kernel="tree_umma", return_lse=True)
+    want, ref = fst.fst_attention(q.float(), k.float(), v.float(), meta, sm_scale=D ** -0.5, kernel="simt", return_lse=True)
+    assert (o.float() - want).abs().max().item() <= TOL[torch.float16] and (lse - ref).abs().max().item() <= 1e-3
+    x = n - 5
+    bad = v.clone()
+    bad[:, :, x] = float("nan")
+    got = fst.fst_attention(q, k, bad, meta, sm_scale=D ** -0.5, kernel="tree_umma")
+    near = reaches(par, x // 16 * 16, x // 16 * 16 + 16).cuda()
+    assert torch.isnan(got[:, :, reaches(par, x, x + 1).cuda()]).all() and torch.equal(got[:, :, ~near], o[:, :, ~near])
+    assert fst.last_status() == 0
+
+
 def test_tree_umma_moving_maximum(fst):
     """A late ancestor whose score dwarfs the row's own tile: the accumulator is rescaled."""
     n, D = 400, 128
