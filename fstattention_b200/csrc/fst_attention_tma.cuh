@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "fst_attention_mma.cuh"
+#include "fst_plan.h"
 
 namespace fst {
 
@@ -852,13 +853,12 @@ cudaError_t launch_tma_inst(const AttnArgs &a, cudaStream_t stream) {
                         : launch_tma_pfx<T, D, BM, TN, false, 1>(a, stream);
 }
 
-// tile_cols: 32, 64, or 0 = by grid size: 64-column tiles up to about eight CTAs per SM (measured:
-// 128 and 512 CTAs are faster with 64, 4096 CTAs equal, 8192 CTAs 20 % faster with 32)
+// tile_cols: 32, 64, or 0 = by grid and lists (tma_tile_cols)
 template <typename T, int D>
 cudaError_t launch_tma_d(const AttnArgs &a, int tile_cols, cudaStream_t stream) {
     if (tile_cols == 0) {
         const long long ctas = (long long)a.nb * a.H * a.Z * a.n_splits;
-        tile_cols = ctas <= 8LL * sm_count() ? 64 : 32;
+        tile_cols = a.prefix > 0 ? (ctas <= 8LL * sm_count() ? 64 : 32) : tma_tile_cols(ctas, D, a.bm, a.ma, sm_count());
     }
     if (tile_cols == 64) {
         switch (a.bm) {

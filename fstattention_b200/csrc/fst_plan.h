@@ -73,30 +73,53 @@ inline bool prefix_umma_pays(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, in
     return prefix >= (sparse ? 256 : bm >= 128 ? 96 : 192);
 }
 
-// When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, five kinds of trees, 64 to 6144
-// items (128 query rows of one head), ratios of the mma.sync kernel's time to the other's; "bound" is the ancestor
-// bound in blocks:
-//   D 128, block_m 128   1.19 - 1.54 at 200 to 600 items, 1.54 - 2.39 above; 0.81 - 1.12 up to 160
-//   D 128, block_m 64    bound 1: 0.96 - 1.04, 1.05 - 1.19 at 300 to 600; bound 2 and 3: 0.97 - 1.06 at 256, 0.96 - 1.29 above;
-//                        bound 4 and up: 0.88 - 1.23 up to 600, 1.02 - 1.28 from 1000; all 0.61 - 0.95 below 200
-//   D 128, block_m 32    1.02 - 1.65 at 200 to 300 (0.97 - 1.33 with a bound of 8 and up), 0.92 - 1.03 at 300 to 600, 0.97 - 1.16
-//                        above; 0.71 - 1.05 from 300 on with a bound of 8 and up
-//   D 64, block_m 128    1.00 - 1.37 at 250 to 600, 1.18 - 1.56 above; 0.64 - 0.97 below 200
-//   D 64, block_m 64     1.10 - 1.45 at 4096 (1.03 with long lists), 1.05 - 1.42 at 1000 to 2000; 0.77 - 1.18 below
-//   D 64, block_m 32     0.98 - 1.33 from 1000, 0.69 - 1.01 with a bound of 8 and up; 0.54 - 1.04 below
+// Columns of a column tile of the TMA tree kernel, 32 or 64.  64 halve the rounds of softmax that a warp runs one after the
+// other, but leave room for fewer CTAs on an SM: two instead of three (one instead of two at block_m 128, D 64; one either
+// way at D 128).  So what counts is whether 32 need fewer waves, and how many gathered tiles there can be.  Us per
+// call, 32 / 64 columns, by CTAs; "bound": ancestors allowed for, in blocks:
+//   block_m 64, bound 1    D 128: 384 8.2 / 10.6, 512 13.1 / 12.0, 768 15.8 / 17.2, 1024 18.9 / 21.8; D 64: 384 5.7 / 7.5, 512 9.6 / 8.4, 768 10.9 / 12.0
+//   block_m 64, bound 2    384 11.2 / 13.0, 512 17.5 / 14.3, 1024 27.4 / 26.3; bound 5: 384 19.6 / 19.0, 512 27.4 / 23.9
+//   block_m 32, 64 slots   D 128: 48 3.8 / 5.0, 512 6.0 / 10.1, 1024 10.6 / 19.2; D 64: 48 2.9 / 3.7, 1024 7.4 / 8.4
+//   block_m 32, longer     D 128: 256 12.5 / 11.3, 512 13.6 / 18.7, 2048 45.7 / 72.5; D 64: 512 9.7 / 8.8, 2048 32.4 / 29.9, 8192 66.3 / 62.8
+//   block_m 128, bound 1   D 64: 128 6.6 / 5.3, 256 8.6 / 9.7, 384 15.2 / 15.1, 512 15.8 / 19.3; D 128: 192 13.8 / 13.1
+//   block_m 128, bound 2   D 64: 192 10.1 / 11.3, 256 10.6 / 12.0; bound 3: 192 19.8 / 16.3
+// Above eight CTAs per SM 32 win (64 batched trees of 256 nodes: 112 / 143).
+inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
+    if (bm == 32) return ma > 64 && (D == 64 || ctas <= 2LL * sms) ? 64 : 32;
+    if (ctas > 8LL * sms) return 32;
+    if (bm == 128 && D == 128) return 64;
+    const int64_t fit = (bm == 64 ? 2LL : 1LL) * sms;     // CTAs at once with 64 columns; with 32 one more per SM
+    if (ctas <= fit) return 64;
+    if (ctas <= fit + sms) return ma <= 2 * bm ? 32 : 64;
+    return ma > bm || (ctas + fit - 1) / fit <= (ctas + fit + sms - 1) / (fit + sms) ? 64 : 32;
+}
+
+// When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, five kinds of trees, 64 to 8192
+// items (128 query rows of one head), ratios of the mma.sync kernel's time (with the better of its tiles) to the other's; "bound"
+// is the ancestor bound in blocks:
+//   D 128, block_m 128   1.13 - 1.34 at 160 to 200 items, 1.17 - 1.90 above; 0.77 - 1.08 up to one item per SM
+//   D 128, block_m 64    bound 1: 0.93 - 1.04 up to 1300, 1.00 - 1.03 above; bound 2 and 3: 0.90 - 1.00 at 160 to 200, 1.00 - 1.25 from 256;
+//                        bound 4 and up: 1.03 - 1.24 from 300 where the tree has 700 nodes and more (0.97 - 1.11 at 220 to 256), 0.85 - 0.95 up
+//                        to 512 with 512 nodes, 1.12 above
+//   D 128, block_m 32    0.88 - 1.00 up to 1000, 1.02 - 1.10 from 2000; 0.75 - 0.88 with a bound of 8 and up (the line is where it was
+//                        with 64-column tiles in the other kernel up to 300 items, 1.02 - 1.65 then: below 2000 either will do)
+//   D 64, block_m 128    bound 1: 0.88 - 1.04 up to 256, 1.14 - 1.59 above; bound 2 and up: 1.01 - 1.18 from 160; 0.63 - 0.83 up to one per SM
+//   D 64, block_m 64     bound 1: 0.85 - 0.97 up to 1000, 1.03 - 1.11 above; bound 2 and 3: 1.05 - 1.28 from 512, 0.92 at 256; bound 4 and
+//                        up: 1.09 - 1.23 from 768, 0.92 - 1.07 below
+//   D 64, block_m 32     64 slots: 1.04 - 1.31 from 960; longer lists 1.00 - 1.05 at 2048, 0.82 - 0.95 below; 0.75 - 0.88 with a bound of 8 and up
 // Small grids are bound by one CTA's latency, which is longer here.  With one short tile of ancestors per 64 rows at
 // D 128 both kernels wait for the same HBM bytes and are within a few per cent of one another.
 inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int ma) {
     const int64_t items = (n_q + 127) / 128 * H * Z;
     const int bound = ma / bm;                        // tiles of ancestors the caller allows for
     if (D == 128) {
-        if (bm == 128) return items >= 200;
-        if (bm == 64) return bound >= 4 ? items >= 1000 : bound >= 2 && items >= 256;
+        if (bm == 128) return items >= 150;
+        if (bm == 64) return items >= (bound >= 4 ? (n_q >= 700 ? 300 : 800) : bound >= 2 ? 250 : 2000);
         return items >= 200 && (items <= 300 || (bound < 8 && items >= 600));
     }
-    if (bm == 128) return items >= 250;
-    if (bm == 64) return items >= (bound == 2 || bound == 3 ? 1000 : 2000);
-    return bound < 8 && items >= 1000;
+    if (bm == 128) return items >= (bound >= 2 ? 150 : 300);
+    if (bm == 64) return items >= (bound >= 4 ? 700 : bound >= 2 ? 450 : 1200);
+    return bound < 8 && items >= (bound >= 4 ? 2000 : 900);
 }
 
 }  // namespace fst

@@ -53,7 +53,7 @@ enum fst_kernel {
     FST_KERNEL_SIMT = 1,           /* fp32 arithmetic, any dtype / head_dim in {16,32,64,128}   */
     FST_KERNEL_MMA = 2,            /* tensor-core kernel, cp.async gathers: fp16/bf16, D 64/128  */
     FST_KERNEL_TMA = 3,            /* same arithmetic, TMA tile loads + mbarriers, swizzled smem; */
-                                   /* 32- or 64-column tiles chosen by grid size                 */
+                                   /* 32- or 64-column tiles chosen by grid and ancestor bound    */
     FST_KERNEL_TMA_T32 = 4,        /* ... forced 32-column tiles (three CTAs per SM)             */
     FST_KERNEL_TMA_T64 = 5,        /* ... forced 64-column tiles (fewest softmax rounds)         */
     FST_KERNEL_TMA_UMMA = 6,       /* shared prefix and tree by one tcgen05 kernel (head_dim 64  */
