@@ -397,6 +397,14 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
 // new_metadata(parent, block_m, max_ancestors, reference_format)
 //   -> (n_trees, n_nodes, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx, whether the call was
 //   captured into a graph), buffers made here.
+// Record i of a block of them: a tensor over the block's storage, made without the dispatcher (narrow takes a microsecond).
+at::Tensor record_of(const at::Tensor &words, int64_t i) {
+    auto impl = c10::make_intrusive<c10::TensorImpl>(c10::Storage(words.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA), words.dtype());
+    impl->set_sizes_contiguous({4});
+    impl->set_storage_offset(4 * i);
+    return at::Tensor(std::move(impl));
+}
+
 // A cleared status record.  Clearing one per call is a launch (about a microsecond in front of a five
 // microsecond kernel), so a thread takes them from a block that it cleared in one go on the same stream;
 // a new block is made for another stream or device and when one is used up (256 records, 4 KB,
@@ -430,7 +438,7 @@ at::Tensor clear_record(const at::Device &dev, cudaStream_t stream, const at::Te
             check_status(FST_ERR_CUDA, what);
         }
     }
-    return block->words.narrow(0, 4 * block->next++, 4);
+    return record_of(block->words, block->next++);
 }
 
 void run_precompute(const at::Tensor &par, int64_t n_trees, int64_t n_nodes, int64_t bm, int64_t ma, const at::Tensor &packed,
@@ -473,36 +481,44 @@ PyObject *wrap_or_none(const at::Tensor &t) {
     Py_RETURN_NONE;
 }
 
+// buffers for the metadata of n_trees trees of n_nodes nodes, and the build launched into them
+struct Built {
+    at::Tensor packed, status, ai, am, li;
+    size_t stride;
+    bool captured = false;
+};
+Built build_metadata(const at::Tensor &par, bool batched, int64_t n_trees, int64_t n_nodes, int64_t bm, int64_t ma, bool reference_format) {
+    if (bm <= 0 || ma <= 0) raise(PyExc_ValueError, "block_m and max_ancestors must be positive");
+    const int64_t nb = (n_nodes + bm - 1) / bm;
+    const at::Device dev = par.device();
+    Built m;
+    m.stride = fst_packed_meta_bytes(int(nb), int(bm), int(ma));
+    m.packed = empty({n_trees, int64_t(m.stride)}, at::kByte, dev);
+    m.status = clear_record(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), at::Tensor(), "fst_precompute", &m.captured);
+    if (reference_format) {
+        if (batched) {
+            m.ai = empty({n_trees, nb, ma}, at::kLong, dev);
+            m.am = empty({n_trees, nb, bm, ma}, at::kBool, dev);
+            m.li = empty({n_trees, nb, bm}, at::kLong, dev);
+        } else {
+            m.ai = empty({nb, ma}, at::kLong, dev);
+            m.am = empty({nb, bm, ma}, at::kBool, dev);
+            m.li = empty({nb, bm}, at::kLong, dev);
+        }
+    }
+    run_precompute(par, n_trees, n_nodes, bm, ma, m.packed, m.stride, m.status, m.ai, m.am, m.li);
+    return m;
+}
+
 PyObject *new_metadata(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 4);
     const at::Tensor &par = parent_arg(a[0]);
-    const int64_t bm = integer(a[1]), ma = integer(a[2]);
     const int64_t n_trees = par.dim() == 2 ? par.size(0) : 1, n_nodes = par.size(-1);
-    if (bm <= 0 || ma <= 0) raise(PyExc_ValueError, "block_m and max_ancestors must be positive");
-    const int64_t nb = (n_nodes + bm - 1) / bm;
-    const size_t stride = fst_packed_meta_bytes(int(nb), int(bm), int(ma));
-    const at::Device dev = par.device();
-    const c10::cuda::CUDAGuard guard(dev);
-    bool captured = false;
-    const at::Tensor packed = empty({n_trees, int64_t(stride)}, at::kByte, dev),
-                     status = clear_record(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), at::Tensor(), "fst_precompute",
-                                           &captured);
-    at::Tensor ai, am, li;
-    if (a[3] == Py_True) {
-        if (par.dim() == 2) {
-            ai = empty({n_trees, nb, ma}, at::kLong, dev);
-            am = empty({n_trees, nb, bm, ma}, at::kBool, dev);
-            li = empty({n_trees, nb, bm}, at::kLong, dev);
-        } else {
-            ai = empty({nb, ma}, at::kLong, dev);
-            am = empty({nb, bm, ma}, at::kBool, dev);
-            li = empty({nb, bm}, at::kLong, dev);
-        }
-    }
-    run_precompute(par, n_trees, n_nodes, bm, ma, packed, stride, status, ai, am, li);
-    return Py_BuildValue("(LLNnNNNNO)", (long long)n_trees, (long long)n_nodes, THPVariable_Wrap(packed), Py_ssize_t(stride),
-                         THPVariable_Wrap(status), wrap_or_none(ai), wrap_or_none(am), wrap_or_none(li),
-                         captured ? Py_True : Py_False);
+    const c10::cuda::CUDAGuard guard(par.device());
+    const Built m = build_metadata(par, par.dim() == 2, n_trees, n_nodes, integer(a[1]), integer(a[2]), a[3] == Py_True);
+    return Py_BuildValue("(LLNnNNNNO)", (long long)n_trees, (long long)n_nodes, THPVariable_Wrap(m.packed), Py_ssize_t(m.stride),
+                         THPVariable_Wrap(m.status), wrap_or_none(m.ai), wrap_or_none(m.am), wrap_or_none(m.li),
+                         m.captured ? Py_True : Py_False);
 }
 
 // dfs_order(parent) -> (order, new_parent, status)
@@ -521,13 +537,18 @@ PyObject *dfs_order(PyObject *const *a, Py_ssize_t n) {
     return Py_BuildValue("(NNN)", THPVariable_Wrap(order), THPVariable_Wrap(npar), THPVariable_Wrap(status));
 }
 
-// build_tree_topk(scores, depth, topk, left_weight_factor, n, return_choice, return_scores)
+// build_tree_topk(scores, depth, topk, left_weight_factor, n or None for as many as the forest has, return_choice, return_scores)
 //   -> (parent, choice or None, node scores or None)
 PyObject *build_tree_topk(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 7);
+    const long long total = fst_tree_topk_nodes(int(integer(a[1])), int(integer(a[2])), real(a[3]));
+    if (total < 0)
+        raise(PyExc_ValueError, "forest shape beyond the kernel's limits (a level above 4096 nodes, or more than 32 levels)");
+    const int64_t nodes = a[4] == Py_None ? total : integer(a[4]);
+    if (nodes <= 0) raise(PyExc_ValueError, "max_nodes must be positive");
     const at::Tensor sc = tensor(a[0]).contiguous();
     const bool batched = sc.dim() == 3;
-    const int64_t n_trees = batched ? sc.size(0) : 1, nodes = integer(a[4]);
+    const int64_t n_trees = batched ? sc.size(0) : 1;
     const at::Device dev = sc.device();
     const c10::cuda::CUDAGuard guard(dev);
     const auto made = [&](at::ScalarType t) { return batched ? empty({n_trees, nodes}, t, dev) : empty({nodes}, t, dev); };
@@ -560,14 +581,9 @@ PyObject *parents_of_lineage(PyObject *const *a, Py_ssize_t n) {
     return THPVariable_Wrap(parent);
 }
 
-// check_tree(parent, block_m, max_ancestors): what the device status record of a metadata build would say, from a
-// parent array on the host (int32, contiguous), so that the caller need not wait for the device to learn it.
-// Every node is marked once per block: the marks of a block are its ancestors.
-PyObject *check_tree(PyObject *const *a, Py_ssize_t n) {
-    want_args(n, 3);
-    const at::Tensor &par = tensor(a[0]);
-    const int64_t N = par.size(0), bm = integer(a[1]), ma = integer(a[2]);
-    const int32_t *P = static_cast<const int32_t *>(par.data_ptr());
+// What the device status record of a metadata build would say, from a parent array on the host, so that the caller need
+// not wait for the device to learn it.  Every node is marked once per block: the marks of a block are its ancestors.
+void check_parents(const int32_t *P, int64_t N, int64_t bm, int64_t ma) {
     for (int64_t k = 0; k < N; ++k)
         if (P[k] >= k || P[k] < -1) {
             PyErr_Format(PyExc_ValueError, "malformed tree: parent[%lld]=%d must be -1 or an earlier node", (long long)k, int(P[k]));
@@ -584,7 +600,45 @@ PyObject *check_tree(PyObject *const *a, Py_ssize_t n) {
             throw PyError{};
         }
     }
+}
+// check_tree(parent, block_m, max_ancestors), parent on the host (int32, contiguous)
+PyObject *check_tree(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 3);
+    const at::Tensor &par = tensor(a[0]);
+    check_parents(static_cast<const int32_t *>(par.data_ptr()), par.size(0), integer(a[1]), integer(a[2]));
     Py_RETURN_NONE;
+}
+
+// metadata_of_lineage(lineage, level_lookup, block_m, max_ancestors) -> (packed, tree_stride, ancestor_idx, ancestor_mask, leaf_idx), checked, for
+// int64 CPU tensors; None where the call is for the general path: more parents than the driver takes from pageable
+// memory at once (it would wait for the stream), or a stream that is being captured (a replay would read
+// memory that is gone).  The driver has copied the parents when cudaMemcpyAsync returns, so neither a pinned buffer nor an event of
+// torch's pool is needed: 16 us from the parents on the host to the launch, 8 without them.
+PyObject *metadata_of_lineage(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 4);
+    constexpr int64_t kInline = 8192;                     // parents: 32 KB, the driver stages up to 64
+    const at::Tensor &lin = tensor(a[0]), &lvl = tensor(a[1]);
+    const int64_t N = lin.size(0), W = lin.size(1), s0 = lin.stride(0), s1 = lin.stride(1), t0 = lvl.stride(0);
+    const int64_t bm = integer(a[2]), ma = integer(a[3]);
+    if (N == 0 || N > kInline) Py_RETURN_NONE;
+    const int64_t *Lp = static_cast<const int64_t *>(lin.data_ptr()), *V = static_cast<const int64_t *>(lvl.data_ptr());
+    std::vector<int32_t> P(N);
+    for (int64_t k = 0; k < N; ++k) {
+        const int64_t lv = V[k * t0];
+        if (lv > W) raise(PyExc_IndexError, "level_lookup points past the lineage columns");
+        P[k] = lv > 0 ? int32_t(Lp[k * s0 + (lv - 1) * s1]) : -1;
+    }
+    const at::Tensor par = empty({N}, at::kInt, at::Device(at::kCUDA, c10::cuda::current_device()));
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(par.device().index()).stream();
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) check_status(FST_ERR_CUDA, "fst_precompute");
+    if (capturing != cudaStreamCaptureStatusNone) Py_RETURN_NONE;
+    if (cudaMemcpyAsync(par.data_ptr(), P.data(), size_t(N) * 4, cudaMemcpyHostToDevice, stream) != cudaSuccess)
+        check_status(FST_ERR_CUDA, "fst_precompute");
+    const Built m = build_metadata(par, false, 1, N, bm, ma, true);
+    check_parents(P.data(), N, bm, ma);
+    return Py_BuildValue("(NnNNN)", THPVariable_Wrap(m.packed), Py_ssize_t(m.stride), THPVariable_Wrap(m.ai), THPVariable_Wrap(m.am),
+                         THPVariable_Wrap(m.li));
 }
 
 // write_self(lineage, level_lookup): lineage[k, level[k]] = k (utils.py:124-125), int64 CPU tensors
@@ -653,7 +707,7 @@ PyObject *splits(PyObject *const *a, Py_ssize_t n) {
 PyMethodDef methods[] = {
     FST_METHOD(attention),      FST_METHOD(attention_ref), FST_METHOD(attention_paged), FST_METHOD(pack),
     FST_METHOD(precompute),     FST_METHOD(new_metadata),  FST_METHOD(dfs_order),
-    FST_METHOD(build_tree_topk), FST_METHOD(parents_of_lineage), FST_METHOD(write_self), FST_METHOD(check_tree), FST_METHOD(read_status), FST_METHOD(status_record), FST_METHOD(attention_status),
+    FST_METHOD(build_tree_topk), FST_METHOD(parents_of_lineage), FST_METHOD(write_self), FST_METHOD(check_tree), FST_METHOD(metadata_of_lineage), FST_METHOD(read_status), FST_METHOD(status_record), FST_METHOD(attention_status),
     FST_METHOD(splits),         {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fst_host", "tensor-level calls into libfstattn_b200.so", -1, methods};
 

@@ -45,7 +45,7 @@ class TreeMetadata:
         # second one on, the launch ahead of the call in the stream cannot be the writer
         self.reads_since_build = 0
         self._captured_status = []                        # records that graphs write at their replays
-        self._twin = None if ancestor_idx is None else _PackedTwin(self)
+        self._twin = None if ancestor_idx is None else _PackedTwin.of(self)
 
     def _rebuilt(self) -> None:
         """The buffers have just been written (again)."""
@@ -64,7 +64,7 @@ class TreeMetadata:
 
     def __setstate__(self, state):
         self.__dict__.update(state)
-        self._twin = None if self.ancestor_idx is None else _PackedTwin(self)
+        self._twin = None if self.ancestor_idx is None else _PackedTwin.of(self)
         if not state["_twin"]:
             self._twin.versions = None
         elif self._twin is not None:
@@ -108,8 +108,9 @@ class TreeMetadata:
         return self.packed.device
 
 
-def _versions(tensors):
-    return tuple(t._version for t in tensors)
+def _versions(three):
+    a, b, c = three
+    return a._version, b._version, c._version
 
 
 # The three tensors handed out by the precompute remember the packed form they came with, so that
@@ -125,14 +126,19 @@ class _PackedTwin:
     __slots__ = ("n_trees", "n_blocks", "block_m", "max_ancestors", "packed", "tree_stride", "reads_since_build",
                  "versions", "tensors")
 
-    def __init__(self, meta: TreeMetadata):
-        three = (meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx)
-        self.n_trees, self.n_blocks = meta.n_trees, meta.n_blocks
-        self.block_m, self.max_ancestors = meta.block_m, meta.max_ancestors
-        self.packed, self.tree_stride = meta.packed, meta.tree_stride
+    def __init__(self, n_trees, n_blocks, block_m, max_ancestors, packed, tree_stride, three):
+        self.n_trees, self.n_blocks = n_trees, n_blocks
+        self.block_m, self.max_ancestors = block_m, max_ancestors
+        self.packed, self.tree_stride = packed, tree_stride
         self.reads_since_build = 0
-        self.versions = _versions(three)
-        self.tensors = tuple(weakref.ref(t) for t in three)
+        a, b, c = three
+        self.versions = a._version, b._version, c._version
+        self.tensors = weakref.ref(a), weakref.ref(b), weakref.ref(c)
+
+    @classmethod
+    def of(cls, meta: TreeMetadata):
+        return cls(meta.n_trees, meta.n_blocks, meta.block_m, meta.max_ancestors, meta.packed, meta.tree_stride,
+                   (meta.ancestor_idx, meta.ancestor_mask, meta.leaf_idx))
 
     def __reduce__(self):                                 # a tensor saved or copied on its own is a plain one
         return type(None), ()
@@ -141,8 +147,11 @@ class _PackedTwin:
 def metadata_of(ancestor_idx, ancestor_mask, leaf_idx) -> Optional[_PackedTwin]:
     """The packed form of three tensors handed out together, while nobody has changed them."""
     twin = getattr(ancestor_idx, _ORIGIN_ATTR, None)
-    three = (ancestor_idx, ancestor_mask, leaf_idx)
-    if twin is not None and all(r() is t for r, t in zip(twin.tensors, three)) and twin.versions == _versions(three):
+    if twin is None:
+        return None
+    a, b, c = twin.tensors
+    if a() is ancestor_idx and b() is ancestor_mask and c() is leaf_idx \
+            and twin.versions == _versions((ancestor_idx, ancestor_mask, leaf_idx)):
         return twin
     return None
 
@@ -236,12 +245,9 @@ def build_tree_topk(scores: torch.Tensor, depth: Optional[int] = None, topk: Opt
     topk = k if topk is None else topk
     if (depth + 1, topk) != (levels, k):
         raise ValueError("scores must have depth + 1 rows of topk entries")
-    total = tree_topk_nodes(depth, topk, left_weight_factor)
-    n = total if max_nodes is None else int(max_nodes)
-    if n <= 0:
-        raise ValueError("max_nodes must be positive")
     parent, choice, nscore = (_lib._host or _lib.host()).build_tree_topk(
-        scores, depth, topk, float(left_weight_factor), n, bool(return_choice), bool(return_scores))
+        scores, depth, topk, float(left_weight_factor), None if max_nodes is None else int(max_nodes), bool(return_choice),
+        bool(return_scores))
     extra = tuple(t for t in (choice, nscore) if t is not None)
     return (parent,) + extra if extra else parent
 
@@ -271,6 +277,13 @@ def create_fst_attention_kernel_inputs(lineage: torch.Tensor, level_lookup: torc
     """
     native = _on_host(lineage, 2) and _on_host(level_lookup, 1) and lineage.shape[0] == level_lookup.shape[0]
     host = _lib._host or _lib.host()
+    built = host.metadata_of_lineage(lineage, level_lookup, block_m, max_ancestors) if native else None
+    if built is not None:                                 # the whole of it in one call, for trees of ordinary size
+        packed, stride, idx, mask, leaf = built
+        setattr(idx, _ORIGIN_ATTR, _PackedTwin(1, idx.shape[0], block_m, max_ancestors, packed, stride, (idx, mask, leaf)))
+        if mutate_lineage:
+            host.write_self(lineage, level_lookup)
+        return idx, mask, leaf
     parent = host.parents_of_lineage(lineage, level_lookup) if native else parent_from_lineage(lineage, level_lookup)
     meta = build_tree_metadata(parent, block_m, max_ancestors, reference_format=True, check=not native)
     if native:

@@ -328,3 +328,26 @@ def test_device_built_tree_follows_the_scores(fst):
         assert torch.equal(a.cpu(), b)
     with pytest.raises(ValueError, match="limits"):
         fst.tree_topk_nodes(14, 4, 0.5)                  # a level of 32768 nodes
+
+
+@pytest.mark.parametrize("depth", [0, 7, 10, 11])
+@pytest.mark.parametrize("mutate", [True, False])
+def test_inputs_of_a_lineage_small_and_large(fst, depth, mutate):
+    """Up to 8192 parents go to the device by value, more through pinned memory: the same tensors, side effect and
+    errors, on a stream of the caller's too."""
+    lineage, level = fst.create_tree(depth)
+    n, before = lineage.shape[0], lineage.clone()
+    want = fst.build_tree_metadata(fst.parent_from_lineage(lineage, level).to(torch.int32), 64, 128)
+    side = torch.cuda.Stream()
+    for stream in (torch.cuda.current_stream(), side):
+        lin = before.clone()
+        with torch.cuda.stream(stream):
+            got = fst.create_fst_attention_kernel_inputs(lin, level, block_m=64, max_ancestors=128, mutate_lineage=mutate)
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+        rows = torch.arange(n)
+        assert torch.equal(lin[rows, level], rows if mutate else before[rows, level])
+    if depth >= 7:
+        with pytest.raises(RuntimeError, match="unique ancestors"):
+            fst.create_fst_attention_kernel_inputs(before.clone(), level, block_m=64, max_ancestors=8)
+    q, k, v = (torch.randn((1, 2, n, 64), device="cuda").half() for _ in range(3))
+    assert torch.equal(fst.fst_attention(q, k, v, *got, 0.1, BLOCK_M=64, MAX_ANCESTORS=128), fst.fst_attention(q, k, v, want, sm_scale=0.1))
