@@ -32,11 +32,199 @@ namespace fst {
 constexpr int PRE_THREADS = 256;
 constexpr int PRE_WARPS = PRE_THREADS / 32;
 
+// four bits as four bool bytes
+__device__ __forceinline__ uint32_t bool_bytes(uint32_t bits) { return ((bits & 0xfu) * 0x00204081u) & 0x01010101u; }
+
+constexpr int kWideNodes = 8192;       // larger trees are not staged
+constexpr int SET_MOST = 128;          // rows of a block, and its ancestors
+constexpr int SET_SLOTS = 1024;
+struct AncestorSet {
+    uint4 bits[SET_MOST];              // masks of the slots
+    uint4 row[SET_MOST];               // and of the block's rows
+    int key[SET_SLOTS];                // node at a place of the hash table, -1: none
+    int node[SET_MOST];                // in the order of their places, INT_MAX behind the last
+    int sorted[SET_MOST];              // by slot
+    uint32_t blk[SET_MOST * (SET_MOST / 32)];
+    int16_t up[SET_SLOTS];             // place of the parent, -1: a root
+    int16_t slot[SET_SLOTS];           // slot of the node at that place
+    int16_t place[SET_MOST];           // their places
+    int16_t jump[SET_MOST], self[SET_MOST];    // of a slot: an ancestor's slot; of a row: its own slot, -1: nobody's ancestor
+    int warp[PRE_WARPS];               // taken places of a warp's share
+    int full;                          // too many nodes for the table
+};
+
+// One block's metadata by way of a hash set of its ancestors; false, with nothing written, when there are more than max_ancestors.
+//   * a row climbs until it meets a node that is in the set, and links every node to its parent's place on the way;
+//   * a node's slot is the number of smaller ones: everybody compares;
+//   * the slots' masks, a uint4 each, by pointer doubling over the links; a row's mask is its parent's.
+template <typename Parent>
+__device__ __forceinline__ bool precompute_set(AncestorSet &set, const Parent &par, int b, int n_nodes, int bm, int ma,
+                                               unsigned char *blob, const PackedLayout &L, int64_t *o_idx, uint8_t *o_mask, int64_t *o_leaf) {
+    const int tid = threadIdx.x, row0 = b * bm, maw = L.maw, bw = L.bw;
+    for (int i = tid; i < SET_SLOTS / 4; i += PRE_THREADS) reinterpret_cast<int4 *>(set.key)[i] = make_int4(-1, -1, -1, -1);
+    if (tid < SET_MOST) {
+        set.node[tid] = INT_MAX;
+        set.self[tid] = -1;
+        reinterpret_cast<uint4 *>(set.blk)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (tid == 0) set.full = 0;
+    __syncthreads();
+
+    int first = -1;                                       // place of my row's parent
+    if (tid < bm) {
+        int x = row0 + tid < n_nodes ? par(row0 + tid) : -1, below = -1;
+        while (x >= 0) {
+            const int next = par(x);                      // under way while x is looked up
+            int at = int((uint32_t(x) * 0x9E3779B1u) >> 22), was, tries = 0;
+            while ((was = atomicCAS(&set.key[at], -1, x)) != -1 && was != x && ++tries < 2 * SET_MOST) at = (at + 1) & (SET_SLOTS - 1);
+            if (tries >= 2 * SET_MOST) {                  // no set of SET_MOST nodes has such a run of taken places
+                set.full = 1;
+                break;
+            }
+            if (below < 0) first = at;
+            else set.up[below] = int16_t(at);
+            if (was == x) break;                          // somebody else goes on from here
+            if (next < 0) set.up[at] = -1;
+            below = at;
+            x = next;
+        }
+    }
+    __syncthreads();
+    // the nodes and their places, in the order of the places: four to a thread (counting them in the climb would make the
+    // counter a link of a deep tree's chain)
+    static_assert(SET_SLOTS == 4 * PRE_THREADS, "four places to a thread");
+    const int4 mine4 = reinterpret_cast<const int4 *>(set.key)[tid];
+    const int own = int(mine4.x >= 0) + int(mine4.y >= 0) + int(mine4.z >= 0) + int(mine4.w >= 0);
+    int before = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, before, o);
+        if ((tid & 31) >= o) before += v;
+    }
+    if ((tid & 31) == 31) set.warp[tid >> 5] = before;
+    __syncthreads();
+    int n = 0;
+    before -= own;
+#pragma unroll
+    for (int w = 0; w < PRE_WARPS; ++w) {
+        before += w < tid >> 5 ? set.warp[w] : 0;
+        n += set.warp[w];
+    }
+    if (n > ma || set.full) return false;
+    const int four[4] = {mine4.x, mine4.y, mine4.z, mine4.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (four[i] >= 0) {
+            set.place[before] = int16_t(tid * 4 + i);
+            set.node[before++] = four[i];
+        }
+    __syncthreads();
+
+    // slots: thread pairs share a node, half of the comparisons each
+    const int k = tid >> 1, mine = set.node[k];
+    int rank = 0;
+#pragma unroll 4
+    for (int i = tid & 1; i < (n + 3) >> 2; i += 2) {
+        const int4 v = reinterpret_cast<const int4 *>(set.node)[i];
+        rank += int(v.x < mine) + int(v.y < mine) + int(v.z < mine) + int(v.w < mine);
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    const bool have = (tid & 1) == 0 && k < n;
+    const int at = have ? set.place[k] : 0;
+    if (have) {
+        set.slot[at] = int16_t(rank);
+        set.sorted[rank] = mine;
+        if (mine >= row0) set.self[mine - row0] = int16_t(rank);
+    }
+    const int n_ext = __syncthreads_count(have && mine < row0);
+    if (have) {
+        const int p = set.up[at];
+        set.jump[rank] = p < 0 ? int16_t(-1) : set.slot[p];
+        const uint32_t bit = 1u << (rank & 31);
+        const int w = rank >> 5;
+        set.bits[rank] = make_uint4(w == 0 ? bit : 0u, w == 1 ? bit : 0u, w == 2 ? bit : 0u, w == 3 ? bit : 0u);
+    }
+    const int above = first < 0 ? -1 : set.slot[first];   // slot of my row's parent
+    if (tid < ma) {
+        const int node = tid < n ? set.sorted[tid] : -1;
+        if (o_idx) o_idx[tid] = node;
+        if (blob) reinterpret_cast<int32_t *>(blob + L.off_idx)[size_t(b) * ma + tid] = tid < n_ext ? node : -1;
+    }
+    if (tid == 0 && blob) reinterpret_cast<int32_t *>(blob + L.off_count)[b] = n_ext;
+    __syncthreads();
+    for (;;) {
+        uint4 got = make_uint4(0u, 0u, 0u, 0u);
+        int to = tid < n ? set.jump[tid] : -1;
+        const bool any = to >= 0;
+        if (any) {
+            got = set.bits[to];
+            to = set.jump[to];
+        }
+        if (!__syncthreads_or(any)) break;
+        if (any) {
+            uint4 m = set.bits[tid];
+            m.x |= got.x; m.y |= got.y; m.z |= got.z; m.w |= got.w;
+            set.bits[tid] = m;
+            set.jump[tid] = int16_t(to);
+        }
+        __syncthreads();
+    }
+    if (tid < bm) {
+        const int j = tid, self = set.self[j];
+        uint4 m = above >= 0 ? set.bits[above] : make_uint4(0u, 0u, 0u, 0u);
+        if (self >= 0) {
+            const uint32_t bit = 1u << (self & 31);
+            m.x |= self >> 5 == 0 ? bit : 0u; m.y |= self >> 5 == 1 ? bit : 0u; m.z |= self >> 5 == 2 ? bit : 0u; m.w |= self >> 5 == 3 ? bit : 0u;
+        }
+        set.row[j] = m;
+        uint32_t *blk = set.blk + j * bw;
+        blk[j >> 5] = 1u << (j & 31);                     // every row attends to itself, and to its ancestors in the block
+        const uint32_t word[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const int below = n_ext - w * 32;             // slots of this word that are outside
+            for (uint32_t in = below >= 32 ? 0u : below > 0 ? word[w] & ~((1u << below) - 1u) : word[w]; in != 0u; in &= in - 1u) {
+                const int c = set.sorted[w * 32 + __ffs(in) - 1] - row0;
+                blk[c >> 5] |= 1u << (c & 31);
+            }
+        }
+        if (o_leaf) o_leaf[j] = self >= 0 ? int64_t(-1) : int64_t(row0 + j);
+    }
+    __syncthreads();
+    const uint32_t *row = reinterpret_cast<const uint32_t *>(set.row);
+    if (blob) {
+        uint32_t *p_emask = reinterpret_cast<uint32_t *>(blob + L.off_emask) + size_t(b) * bm * maw;
+        uint32_t *p_bmask = reinterpret_cast<uint32_t *>(blob + L.off_bmask) + size_t(b) * bm * bw;
+        for (int i = tid; i < bm * maw; i += PRE_THREADS) {
+            const int j = maw == 4 ? i >> 2 : i / maw, w = i - j * maw, outside = n_ext - w * 32;
+            p_emask[i] = row[j * 4 + w] & (outside >= 32 ? 0xffffffffu : outside > 0 ? (1u << outside) - 1u : 0u);
+        }
+        for (int i = tid; i < bm * bw; i += PRE_THREADS) p_bmask[i] = set.blk[i];
+    }
+    if (o_mask) {
+        if ((ma & 15) == 0 && (reinterpret_cast<uintptr_t>(o_mask) & 15) == 0) {     // sixteen bool bytes per store
+            const int pieces = ma / 16, step = PRE_THREADS / pieces, j0 = tid / pieces, at16 = (tid - j0 * pieces) * 16;
+            if (j0 < step)
+                for (int j = j0; j < bm; j += step) {
+                    const uint32_t half = row[j * 4 + (at16 >> 5)] >> (at16 & 31);
+                    reinterpret_cast<uint4 *>(o_mask)[j * pieces + (at16 >> 4)] =
+                        make_uint4(bool_bytes(half), bool_bytes(half >> 4), bool_bytes(half >> 8), bool_bytes(half >> 12));
+                }
+        } else {
+            for (int i = tid; i < bm * ma; i += PRE_THREADS) {
+                const int j = i / ma, c = i - j * ma;
+                o_mask[i] = (row[j * 4 + (c >> 5)] >> (c & 31)) & 1u;
+            }
+        }
+    }
+    return true;
+}
+
 // BYTE_FLAGS: ancestors are first marked as one byte per node and packed into the bitmap by
 // ballots (the fast path: plain stores never serialise).  Without it the walkers set bitmap bits
 // with atomicOr directly; that needs 1/9 of the shared memory and is what lets trees of a
 // hundred thousand nodes and more fit (a CTA keeps a bitmap of every node below its last row).
-template <bool BYTE_FLAGS>
+template <bool BYTE_FLAGS, bool SET>
 __global__ void __launch_bounds__(PRE_THREADS)
 precompute_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int bm, int ma, int par_cap, int depth_cap,
                   int64_t *__restrict__ anc_idx_all, uint8_t *__restrict__ anc_mask_all,
@@ -60,7 +248,8 @@ precompute_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int bm, i
     unsigned char *flag = reinterpret_cast<unsigned char *>(warp_tot + 40);   // [W*32] node is an ancestor
     int *chain = reinterpret_cast<int *>(flag + (BYTE_FLAGS ? size_t(W) * 32 : 0));   // [depth_cap][bm] ancestors of row j
     int *depth = chain + size_t(depth_cap) * bm;                      // [bm] recorded chain length
-    int *s_par = depth + bm;
+    // SET: the parents of all nodes below the block's end, then the set; everything above takes their place if it does not do
+    int *s_par = SET ? reinterpret_cast<int *>(smem_raw) : depth + bm;
 
     const int32_t *parent = parent_all + size_t(tree) * n_nodes;
     const int cap = min(par_cap, n_here);
@@ -85,6 +274,20 @@ precompute_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int bm, i
             const int i = i0 + u * PRE_THREADS;
             if (i < cap) s_par[i] = checked(i, v[u]);
         }
+    }
+    if constexpr (SET) {
+        AncestorSet &set = *reinterpret_cast<AncestorSet *>(smem_raw + ((size_t(cap) * 4 + 15) & ~size_t(15)));
+        const PackedLayout L = packed_layout(nb, bm, ma);
+        const size_t blk = size_t(tree) * nb + b;
+        __syncthreads();
+        if (precompute_set(set, [&](int x) { return s_par[x]; }, b, n_nodes, bm, ma, packed_all ? packed_all + size_t(tree) * packed_stride : nullptr, L,
+                           anc_idx_all ? anc_idx_all + blk * ma : nullptr, anc_mask_all ? anc_mask_all + blk * size_t(bm) * ma : nullptr,
+                           leaf_idx_all ? leaf_idx_all + blk * bm : nullptr))
+            return;
+        // more ancestors than the bound: again, with room for as many as there are
+        s_par = depth + bm;
+        __syncthreads();
+        for (int i = tid; i < cap; i += PRE_THREADS) s_par[i] = checked(i, __ldg(parent + i));
     }
     if (BYTE_FLAGS) {
         for (int i = tid; i < W * 8; i += PRE_THREADS) reinterpret_cast<uint32_t *>(flag)[i] = 0u;
@@ -302,172 +505,13 @@ precompute_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int bm, i
 // writing the neighbours that share a word).  Blocks and bounds of at most 128 therefore keep their ancestors in
 // a hash set (precompute_set): 16.4 us, of which the climb, one dependent L2 read for each of fifteen levels, is the
 // largest part.  A block with more ancestors than the bound is left to the bitmap, which counts them.
-constexpr int WIDE_THREADS = 256, WIDE_WARPS = WIDE_THREADS / 32;
+constexpr int WIDE_THREADS = PRE_THREADS, WIDE_WARPS = WIDE_THREADS / 32;
 
 // 32-bit words of shared memory: bitmap and 16-bit ranks of Wp words, masks of slots or rows, block masks,
 // parent and own slot of every row, and of every slot its node and parent slot
 __host__ __device__ inline size_t wide_smem_words(size_t Wp, int bm, int ma, bool inherit) {
     const size_t maw = (ma + 31) / 32, bw = (bm + 31) / 32;
     return Wp + Wp / 2 + size_t(inherit && ma > bm ? ma : bm) * maw + size_t(bm) * bw + size_t(bm) * 2 + (inherit ? size_t(ma) * 2 : 0);
-}
-
-// four bits as four bool bytes
-__device__ __forceinline__ uint32_t bool_bytes(uint32_t bits) { return ((bits & 0xfu) * 0x00204081u) & 0x01010101u; }
-
-constexpr int SET_MOST = 128;          // rows of a block, and its ancestors
-constexpr int SET_SLOTS = 1024;        // the set gives up beyond SET_MOST; the climbs under way then add one node each
-struct AncestorSet {
-    uint4 bits[SET_MOST];              // masks of the slots
-    uint4 row[SET_MOST];               // and of the block's rows
-    int key[SET_SLOTS];                // node at a place of the hash table, -1: none
-    int node[SET_MOST];                // in the order they were met, INT_MAX behind the last
-    int sorted[SET_MOST];              // by slot
-    uint32_t blk[SET_MOST * (SET_MOST / 32)];
-    int16_t up[SET_SLOTS];             // place of the parent, -1: a root
-    int16_t slot[SET_SLOTS];           // slot of the node at that place
-    int16_t place[SET_MOST];           // places in the order they were met
-    int16_t jump[SET_MOST], self[SET_MOST];    // of a slot: an ancestor's slot; of a row: its own slot, -1: nobody's ancestor
-    int n;
-};
-
-// One block's metadata by way of a hash set of its ancestors; false, with nothing written, when there are more than max_ancestors.
-//   * a row climbs until it meets a node that is in the set, and links every node to its parent's place on the way;
-//   * a node's slot is the number of smaller ones: everybody compares;
-//   * the slots' masks, a uint4 each, by pointer doubling over the links; a row's mask is its parent's.
-template <typename Parent>
-__device__ __forceinline__ bool precompute_set(AncestorSet &set, const Parent &par, int b, int n_nodes, int bm, int ma,
-                                               unsigned char *blob, const PackedLayout &L, int64_t *o_idx, uint8_t *o_mask, int64_t *o_leaf) {
-    const int tid = threadIdx.x, row0 = b * bm, maw = L.maw, bw = L.bw;
-    for (int i = tid; i < SET_SLOTS / 4; i += WIDE_THREADS) reinterpret_cast<int4 *>(set.key)[i] = make_int4(-1, -1, -1, -1);
-    if (tid < SET_MOST) {
-        set.node[tid] = INT_MAX;
-        set.self[tid] = -1;
-        reinterpret_cast<uint4 *>(set.blk)[tid] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    if (tid == 0) set.n = 0;
-    __syncthreads();
-
-    int first = -1;                                       // place of my row's parent
-    if (tid < bm) {
-        int x = row0 + tid < n_nodes ? par(row0 + tid) : -1, below = -1;
-        while (x >= 0) {
-            const int next = par(x);                      // under way while x is looked up
-            int at = int((uint32_t(x) * 0x9E3779B1u) >> 22), was;
-            while ((was = atomicCAS(&set.key[at], -1, x)) != -1 && was != x) at = (at + 1) & (SET_SLOTS - 1);
-            if (below < 0) first = at;
-            else set.up[below] = int16_t(at);
-            if (was == x) break;                          // somebody else goes on from here
-            const int k = atomicAdd(&set.n, 1);
-            if (k >= ma) break;                           // too many
-            set.place[k] = int16_t(at);
-            set.node[k] = x;
-            if (next < 0) set.up[at] = -1;
-            below = at;
-            x = next;
-        }
-    }
-    __syncthreads();
-    const int n = set.n;
-    if (n > ma) return false;
-
-    // slots: thread pairs share a node, half of the comparisons each
-    const int k = tid >> 1, mine = set.node[k];
-    int rank = 0;
-#pragma unroll 4
-    for (int i = tid & 1; i < (n + 3) >> 2; i += 2) {
-        const int4 v = reinterpret_cast<const int4 *>(set.node)[i];
-        rank += int(v.x < mine) + int(v.y < mine) + int(v.z < mine) + int(v.w < mine);
-    }
-    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
-    const bool have = (tid & 1) == 0 && k < n;
-    const int at = have ? set.place[k] : 0;
-    if (have) {
-        set.slot[at] = int16_t(rank);
-        set.sorted[rank] = mine;
-        if (mine >= row0) set.self[mine - row0] = int16_t(rank);
-    }
-    const int n_ext = __syncthreads_count(have && mine < row0);
-    if (have) {
-        const int p = set.up[at];
-        set.jump[rank] = p < 0 ? int16_t(-1) : set.slot[p];
-        const uint32_t bit = 1u << (rank & 31);
-        const int w = rank >> 5;
-        set.bits[rank] = make_uint4(w == 0 ? bit : 0u, w == 1 ? bit : 0u, w == 2 ? bit : 0u, w == 3 ? bit : 0u);
-    }
-    const int above = first < 0 ? -1 : set.slot[first];   // slot of my row's parent
-    if (tid < ma) {
-        const int node = tid < n ? set.sorted[tid] : -1;
-        if (o_idx) o_idx[tid] = node;
-        if (blob) reinterpret_cast<int32_t *>(blob + L.off_idx)[size_t(b) * ma + tid] = tid < n_ext ? node : -1;
-    }
-    if (tid == 0 && blob) reinterpret_cast<int32_t *>(blob + L.off_count)[b] = n_ext;
-    __syncthreads();
-    for (;;) {
-        uint4 got = make_uint4(0u, 0u, 0u, 0u);
-        int to = tid < n ? set.jump[tid] : -1;
-        const bool any = to >= 0;
-        if (any) {
-            got = set.bits[to];
-            to = set.jump[to];
-        }
-        if (!__syncthreads_or(any)) break;
-        if (any) {
-            uint4 m = set.bits[tid];
-            m.x |= got.x; m.y |= got.y; m.z |= got.z; m.w |= got.w;
-            set.bits[tid] = m;
-            set.jump[tid] = int16_t(to);
-        }
-        __syncthreads();
-    }
-    if (tid < bm) {
-        const int j = tid, self = set.self[j];
-        uint4 m = above >= 0 ? set.bits[above] : make_uint4(0u, 0u, 0u, 0u);
-        if (self >= 0) {
-            const uint32_t bit = 1u << (self & 31);
-            m.x |= self >> 5 == 0 ? bit : 0u; m.y |= self >> 5 == 1 ? bit : 0u; m.z |= self >> 5 == 2 ? bit : 0u; m.w |= self >> 5 == 3 ? bit : 0u;
-        }
-        set.row[j] = m;
-        uint32_t *blk = set.blk + j * bw;
-        blk[j >> 5] = 1u << (j & 31);                     // every row attends to itself, and to its ancestors in the block
-        const uint32_t word[4] = {m.x, m.y, m.z, m.w};
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const int below = n_ext - w * 32;             // slots of this word that are outside
-            for (uint32_t in = below >= 32 ? 0u : below > 0 ? word[w] & ~((1u << below) - 1u) : word[w]; in != 0u; in &= in - 1u) {
-                const int c = set.sorted[w * 32 + __ffs(in) - 1] - row0;
-                blk[c >> 5] |= 1u << (c & 31);
-            }
-        }
-        if (o_leaf) o_leaf[j] = self >= 0 ? int64_t(-1) : int64_t(row0 + j);
-    }
-    __syncthreads();
-    const uint32_t *row = reinterpret_cast<const uint32_t *>(set.row);
-    if (blob) {
-        uint32_t *p_emask = reinterpret_cast<uint32_t *>(blob + L.off_emask) + size_t(b) * bm * maw;
-        uint32_t *p_bmask = reinterpret_cast<uint32_t *>(blob + L.off_bmask) + size_t(b) * bm * bw;
-        for (int i = tid; i < bm * maw; i += WIDE_THREADS) {
-            const int j = maw == 4 ? i >> 2 : i / maw, w = i - j * maw, outside = n_ext - w * 32;
-            p_emask[i] = row[j * 4 + w] & (outside >= 32 ? 0xffffffffu : outside > 0 ? (1u << outside) - 1u : 0u);
-        }
-        for (int i = tid; i < bm * bw; i += WIDE_THREADS) p_bmask[i] = set.blk[i];
-    }
-    if (o_mask) {
-        if ((ma & 15) == 0 && (reinterpret_cast<uintptr_t>(o_mask) & 15) == 0) {     // sixteen bool bytes per store
-            const int pieces = ma / 16, step = WIDE_THREADS / pieces, j0 = tid / pieces, at16 = (tid - j0 * pieces) * 16;
-            if (j0 < step)
-                for (int j = j0; j < bm; j += step) {
-                    const uint32_t half = row[j * 4 + (at16 >> 5)] >> (at16 & 31);
-                    reinterpret_cast<uint4 *>(o_mask)[j * pieces + (at16 >> 4)] =
-                        make_uint4(bool_bytes(half), bool_bytes(half >> 4), bool_bytes(half >> 8), bool_bytes(half >> 12));
-                }
-        } else {
-            for (int i = tid; i < bm * ma; i += WIDE_THREADS) {
-                const int j = i / ma, c = i - j * ma;
-                o_mask[i] = (row[j * 4 + (c >> 5)] >> (c & 31)) & 1u;
-            }
-        }
-    }
-    return true;
 }
 
 __global__ void __launch_bounds__(WIDE_THREADS, 7)
@@ -859,10 +903,9 @@ pack_kernel(const int64_t *__restrict__ anc_idx_all, const uint8_t *__restrict__
 }
 
 // largest dynamic shared memory enabled so far, per device and kernel variant
-static std::atomic<size_t> g_pre_smem_set[2][kMaxDevices];
+static std::atomic<size_t> g_pre_smem_set[3][kMaxDevices];
 static std::atomic<size_t> g_pack_smem_set[kMaxDevices];
 static std::atomic<size_t> g_wide_smem_set[kMaxDevices];
-constexpr int kWideNodes = 8192;
 
 cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, int bm, int ma,
                               int64_t *anc_idx, uint8_t *anc_mask, int64_t *leaf_idx,
@@ -877,7 +920,12 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
     // recording space for the rows' chains: as deep as 48 KB allows, at most 1024 levels
     int depth_cap = int((48 * 1024) / (size_t(bm) * 4));
     if (depth_cap > 1024) depth_cap = 1024;
-    if (depth_cap < 1) depth_cap = 1;
+    // Blocks and bounds of up to 128 start with the ancestor set; what is left to the flags then is a tree that is
+    // refused, which need not be quick: its rows are climbed twice, and the space goes to more CTAs on an SM.
+    // Us per build, flags / set, with the reference-format tensors: 256 nodes 6.5 / 5.7, 1020 7.5 / 6.0, 64 of them 17.1 / 12.4,
+    // 16 x 8192 61.6 / 28.9, 4096 deep ones (depth 96) 15.3 / 14.5, four of 8000 32.6 / 18.7.
+    const bool set = bm <= SET_MOST && ma <= SET_MOST && n_nodes <= kWideNodes;
+    if (depth_cap < 1 || set) depth_cap = 1;
     // Byte flags (one byte per node below the last row) while they leave room to stage a good
     // part of the parent array; beyond that the walkers set bitmap bits with atomics.
     bool byte_flags = base + W * 32 + size_t(depth_cap) * bm * 4 + 16 * 1024 <= budget;
@@ -889,7 +937,7 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
     const bool fits = fixed + 1024 <= budget;
     const size_t cap = fits ? (budget - fixed) / 4 : 0;
     const int par_cap = int(cap < size_t(n_nodes) ? cap : size_t(n_nodes));
-    const size_t smem = fixed + size_t(par_cap) * 4;
+    const size_t smem = std::max(fixed + size_t(par_cap) * 4, set ? ((size_t(n_nodes) * 4 + 15) & ~size_t(15)) + sizeof(AncestorSet) : 0);
     // Large trees: when a block's share of the parent array outgrows what one pass of the CTA stages in the
     // time a climb through L2 takes (see precompute_wide_kernel).  A bound of more than 128 ancestors, and more
     // than two to a row, is for deep trees, which that kernel climbs twice through L2 (its masks are not
@@ -917,8 +965,8 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
         }
     }
     if (!fits) return cudaErrorInvalidConfiguration;
-    auto kernel = byte_flags ? precompute_kernel<true> : precompute_kernel<false>;
-    std::atomic<size_t> &enabled = g_pre_smem_set[byte_flags ? 1 : 0][slot];
+    auto kernel = set ? precompute_kernel<true, true> : byte_flags ? precompute_kernel<true, false> : precompute_kernel<false, false>;
+    std::atomic<size_t> &enabled = g_pre_smem_set[set ? 2 : byte_flags ? 1 : 0][slot];
     if (smem > 48 * 1024 && smem > enabled.load(std::memory_order_acquire)) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;

@@ -63,10 +63,12 @@ def test_wide_precompute(fst, n, bm, ma, kind):
 
 @pytest.mark.parametrize("bm,ma", [(128, 128), (128, 127), (64, 128), (100, 31), (32, 33), (16, 16), (1, 5)])
 @pytest.mark.parametrize("apart", [1, 37, 1024])
-def test_ancestor_set_and_bitmap_agree(fst, bm, ma, apart):
+@pytest.mark.parametrize("staged", [False, True])
+def test_ancestor_set_and_bitmap_agree(fst, bm, ma, apart, staged):
     """Bounds of up to 128 keep a block's ancestors in a hash set, larger ones in a bitmap: the same metadata, up to a
-    block whose list is full, and an error for one ancestor more.  Hubs 1024 apart crowd the hash table's places."""
-    n = 131072 if apart == 1024 and bm >= 32 else 9001
+    block whose list is full, and an error for one ancestor more.  Hubs 1024 apart crowd the hash table's places;
+    staged: a tree whose parents fit shared memory."""
+    n = (8192 if apart == 37 else 2500) if staged else 131072 if apart == 1024 and bm >= 32 else 9001
     apart = min(apart, (n - 1) // ma)
     for hubs in (1, ma):
         hub = np.arange(hubs) * apart
