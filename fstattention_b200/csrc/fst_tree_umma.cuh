@@ -305,38 +305,45 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             cnt_lane = count_of(next);                    // one item ahead
             const int g = n & 1, pos = g ? ahead[1] : ahead[0];
             const int end = pos + (C::PACKED ? tiles + 1 : 2 * tiles - int(narrow));   // positions: two for a tile, one where K and V share a buffer
+            // Own K and Q, (merged: the first gathered tile,) own V, the (other) gathered tiles: as the round needs them, for
+            // buffers come free one by one, some 1000 cycles apart where the pool is what bounds the kernel (with V second
+            // and Q third: 64 x 256 nodes D 128 112.2 -> 106.4 us, block_m 128 103.6 -> 99.5, block_m 32 104.5 -> 92.7, 4096-node
+            // deep tree 62.0 -> 58.0).  PACKED keeps Q last: its pool has room, and this order took 1485 -> 1500 us.
+            const int gathered = end - pos - 2, q_at = C::PACKED ? 2 : 1,
+                      v_at = C::PACKED ? 1 : 2 + (MERGED ? min(gathered, narrow && tiles == 2 ? 1 : 2) : 0);
+            int at = pos + 2;
 #pragma unroll 1
-            for (int kv = 0; kv < 3; ++kv) {              // own K, own V, Q
+            for (int i = 0; i < 3 + gathered; ++i) {
                 const int b = take();
                 if (!alive) break;
-                if (elect_one()) {
-                    const uint32_t bar = kv < 2 ? full_of(g, pos + kv) : q_of(n);
-                    if (kv < 2) {
-                        buf_of(g, pos + kv) = (unsigned char)b;
-                        arrive_n(bar, FULL_COUNT - 1);
-                    } else {
-                        info[(n % ITEMS) * 2] = make_int4(tiles, pos, narrow, b);
-                        info[(n % ITEMS) * 2 + 1] =
-                            make_int4(cnt[0], SUB > 1 ? cnt[1 % SUB] : 0, SUB > 2 ? cnt[2 % SUB] : 0, SUB > 2 ? cnt[3 % SUB] : 0);
-                    }
-                    mbar_arrive_expect_tx(bar, TILE);
-                    const CUtensorMap *map = kv == 0 ? &tm_k : kv == 1 ? &tm_v : &tm_q;
-                    const int row = (kv < 2 ? a.prefix : 0) + p * ROWS, head = kv < 2 ? hk : h;
+                if (i == 0 || i == q_at || i == v_at) {
+                    if (elect_one()) {
+                        const bool q = i == q_at;
+                        const int own = i == 0 ? pos : pos + 1;
+                        const uint32_t bar = q ? q_of(n) : full_of(g, own);
+                        if (!q) {
+                            buf_of(g, own) = (unsigned char)b;
+                            arrive_n(bar, FULL_COUNT - 1);
+                        } else {
+                            info[(n % ITEMS) * 2] = make_int4(tiles, pos, narrow, b);
+                            info[(n % ITEMS) * 2 + 1] =
+                                make_int4(cnt[0], SUB > 1 ? cnt[1 % SUB] : 0, SUB > 2 ? cnt[2 % SUB] : 0, SUB > 2 ? cnt[3 % SUB] : 0);
+                        }
+                        mbar_arrive_expect_tx(bar, TILE);
+                        const CUtensorMap *map = q ? &tm_q : i == 0 ? &tm_k : &tm_v;
+                        const int row = (q ? 0 : a.prefix) + p * ROWS, head = q ? h : hk;
 #pragma unroll
-                    for (int hf = 0; hf < DH; ++hf)
-                        tma_load_4d(s_base + b * TILE + hf * HALF, map, hf * 64, row, head, w.z, bar);
+                        for (int hf = 0; hf < DH; ++hf)
+                            tma_load_4d(s_base + b * TILE + hf * HALF, map, hf * 64, row, head, w.z, bar);
+                    }
+                } else {
+                    if (elect_one()) {
+                        buf_of(g, at) = (unsigned char)b;
+                        arrive(bar_go + (turn % TURNS) * 8);
+                    }
+                    ++at;
+                    ++turn;
                 }
-                __syncwarp();
-            }
-#pragma unroll 1
-            for (int at = pos + 2; alive && at < end; ++at) {
-                const int b = take();
-                if (!alive) break;
-                if (elect_one()) {
-                    buf_of(g, at) = (unsigned char)b;
-                    arrive(bar_go + (turn % TURNS) * 8);
-                }
-                ++turn;
                 __syncwarp();
             }
             (g ? ahead[1] : ahead[0]) = end;
