@@ -160,6 +160,13 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     const bool wraps = n0 + 1 == pa.q_tiles;              // the second one is the next heads' first
     auto query = [&](int g) { return QueryTile(a, pa, g && wraps ? h0 + pa.pack : h0, g ? (wraps ? 0 : n0 + 1) * QM : n0 * QM); };
     const int ring = G::TILES - (two ? 2 : 1);
+    // Order of the loads.  skew: K of the next unit ahead of V.  K is done with after the first product and V a softmax later, so in
+    // the order of use K waited for a stage behind an earlier V, was requested some 2500 cycles before its product and
+    // came late for every fourth tile of a query tile by itself at D 128 (six stages; 32 heads of 256 rows behind
+    // 4096: 27.0 -> 26.2 us).  Two query tiles, the longer ring of D 64 and runs spread over the GPU lose 1 to 3 % by it.
+    const bool skew = !PAGED && D == 128 && !two && pa.cluster > 1;
+    auto k_item = [&](int u) { return skew ? max(2 * u - 1, 0) : 2 * u; };
+    auto v_item = [&](int u) { return 2 * u + (skew ? 2 : 1); };
     const uint32_t s_ring = s_base + (two ? 2 : 1) * TILE;
 
     // barriers: Q, full / empty / go (a gathered tile may be written) of every stage, S (landed), P (written), O (all
@@ -224,7 +231,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
     const int nt_all = warp == 8 ? 0 : count_tiles();     // (the loading warp asks when it has nothing else to do)
 
     if (warp == 8) {
-        // ====== loads: unit u is items 2u (K) and 2u + 1 (V) of the ring.  The whole warp for a paged prefix, one lane
+        // ====== loads: K and V of unit u are items k_item(u) and v_item(u) of the ring.  The whole warp for a paged prefix, one lane
         // otherwise.  Paged: a tile is KN / page_size pages, one pair of boxes each, and lane j takes page j - it
         // reads that page's number from the block table a tile before it requests the boxes, so the
         // table's latency is off the path, and a single thread is not left to issue sixteen copies one after
@@ -237,41 +244,69 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             auto my_page = [&](int tile) -> int {
                 return PAGED && lane < npt && tile < tp ? __ldg(table + min(tile * KN / ps + lane, last_page)) : 0;
             };
-            int page = my_page(T0);
+            int page = my_page(T0), page_v = 0;           // of the next K's tile, of the next V's
             bool known = false, alive = true;
             int nt = nt_sure, st = 0;
             uint32_t use = 0;                             // fills of the current stage before this one
             const int shared = n_shared(nt_sure);         // the same for the final count: see above
-            int n_units = (two ? 2 : 1) * nt - shared;
+            int n_units = (two ? 2 : 1) * nt - shared, i0 = 0;
+            auto unit_of = [&](int i) { return skew ? (i & 1 ? (i + 1) >> 1 : max(i - 2, 0) >> 1) : i >> 1; };
+            auto v_next = [&](int i) { return skew ? i > 0 && (i & 1) == 0 : (i & 1) != 0; };
+            auto load_q = [&]() {
+                mbar_arrive_expect_tx(bar_q, (two ? 2 : 1) * TILE);
 #pragma unroll 1
-            for (int u = 0; alive; ++u) {
-                if (u >= n_units) {                       // only now ask how many gathered tiles there are
-                    if (known) break;
+                for (int g = 0; g < (two ? 2 : 1); ++g) {
+                    const QueryTile me = query(g);
+#pragma unroll 1
+                    for (int k = 0; k < pa.pack; ++k)
+#pragma unroll
+                        for (int hf = 0; hf < DH; ++hf)
+                            tma_load_4d(s_base + g * TILE + hf * HALF + (k << pa.pack_shift) * 128, &tm_q, hf * 64, me.q0, me.h + k, z, bar_q);
+                }
+            };
+            const int head_start = (two ? 2 : 4) + int(skew);         // everybody's first steps go ahead of the rest
+            if constexpr (!PAGED && D == 128) {
+                // Whole prefix tiles by themselves: with everything that the others need decided for every item one took some
+                // 770 cycles, and a query tile's K and V together 1540 of the 1700 that its softmax takes.
+                const int n_plain = min(max(tp - T0, 0), nt), limit = n_plain == 0 ? 0 : 2 * n_plain - int(skew);
+                if (n_plain > 0) load_q();
+#pragma unroll 1
+                for (; i0 < limit; ++i0) {
+                    const bool v = v_next(i0);
+                    const uint32_t bar = bar_full + st * 8, dst = s_ring + st * TILE;
+                    if (i0 == head_start) alive = mbar_wait(bar_full, 0, a.status, qt);
+                    if (use > 0) alive = alive && wait(bar_empty + st * 8, (use - 1) & 1, a.status, qt);
+                    if (!alive) break;
+                    mbar_arrive_expect_tx(bar, TILE);
+#pragma unroll
+                    for (int hf = 0; hf < DH; ++hf) tma_load_4d(dst + hf * HALF, v ? &tm_vt : &tm_kt, hf * 64, (T0 + unit_of(i0)) * KN, hk, z, bar);
+                    if (++st == ring) {
+                        st = 0;
+                        ++use;
+                    }
+                }
+            }
+#pragma unroll 1
+            for (int i = i0; alive; ++i) {
+                const bool is_v = v_next(i);
+                const int u = unit_of(i);
+                if (u >= n_units && !known) {             // only now ask how many gathered tiles there are
                     known = true;
                     nt = count_tiles();
                     n_units = (two ? 2 : 1) * nt - n_shared(nt);
-                    if (u >= n_units) break;
                 }
-                if (lead && u == 0) {                     // Q, when there is anything to do: nobody would wait for it otherwise
-                    mbar_arrive_expect_tx(bar_q, (two ? 2 : 1) * TILE);
-#pragma unroll 1
-                    for (int g = 0; g < (two ? 2 : 1); ++g) {
-                        const QueryTile me = query(g);
-#pragma unroll 1
-                        for (int i = 0; i < pa.pack; ++i)
-#pragma unroll
-                            for (int hf = 0; hf < DH; ++hf)
-                                tma_load_4d(s_base + g * TILE + hf * HALF + (i << pa.pack_shift) * 128, &tm_q, hf * 64, me.q0, me.h + i, z, bar_q);
+                if (u >= n_units && (is_v || !skew)) break;
+                if (u < n_units) {
+                    if (lead && i == 0) load_q();         // when there is anything to do: nobody would wait for it otherwise
+                    const int x = u - shared, g = two && !same && x >= 0 ? x & 1 : 0;
+                    const int tile = T0 + (two && !same && x >= 0 ? shared + (x >> 1) : u);
+                    if (PAGED && !is_v) {
+                        page_v = page;
+                        if (tile + 1 < tp) page = my_page(tile + 1);
                     }
-                }
-                const int x = u - shared, g = two && !same && x >= 0 ? x & 1 : 0;
-                const int tile = T0 + (two && !same && x >= 0 ? shared + (x >> 1) : u);
-                const int here = page;
-                if (tile + 1 < tp) page = my_page(tile + 1);
-#pragma unroll 1
-                for (int kv = 0; kv < 2; ++kv) {
-                    const uint32_t dst = s_ring + st * TILE, bar = tail && kv && tile + 1 == tp ? bar_tail : bar_full + st * 8;
-                    if (u == (two ? 1 : 2) && kv == 0 && T0 <= tp) {  // everybody's first steps ahead of the rest
+                    const int here = page_v;
+                    const uint32_t dst = s_ring + st * TILE, bar = tail && is_v && tile + 1 == tp ? bar_tail : bar_full + st * 8;
+                    if (i == head_start && T0 <= tp) {
                         if (lead) alive = mbar_wait(bar_full, 0, a.status, qt);
                         if (PAGED) alive = __all_sync(0xffffffffu, alive);
                         if (!alive) break;
@@ -287,7 +322,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                         if (lead) mbar_arrive_expect_tx(bar, TILE);
                         if (PAGED) __syncwarp();
                         const bool pool = PAGED && tile < tp;
-                        const CUtensorMap *map = pool ? (kv ? &tm_v : &tm_k) : (kv ? &tm_vt : &tm_kt);
+                        const CUtensorMap *map = pool ? (is_v ? &tm_v : &tm_k) : (is_v ? &tm_vt : &tm_kt);
                         if (pool ? lane < npt : lead) {
                             if (pool && unsigned(here) >= unsigned(pa.n_pages))   // the boxes then read as zeros
                                 report(a.status, FST_DEV_INDEX_RANGE, z, tile * KN / ps + lane);
@@ -297,10 +332,10 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                             for (int hf = 0; hf < DH; ++hf) tma_load_4d(to + hf * HALF, map, hf * 64, row, hk, pool ? here : z, bar);
                         }
                     }
-                    if (++st == ring) {
-                        st = 0;
-                        ++use;
-                    }
+                }
+                if (++st == ring) {                       // (the place of a K that does not exist stays empty)
+                    st = 0;
+                    ++use;
                 }
             }
         }
@@ -313,10 +348,10 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             const uint32_t idesc_s = instr_desc(BF16, false, KN), idesc_pv = instr_desc(BF16, true, D);
             // descriptors of the tiles' first 16-wide step; a step further on adds its byte offset / 16
             const uint64_t dq = smem_desc(s_base, 16), dk = smem_desc(s_ring, 16), dv = smem_desc(s_ring, HALF);
-            int k_st = 0, v_st = 1;                       // stages of the next K and the next V tile
+            int k_st = 0, v_st = v_item(0), k_by = k_item(1);     // stages of the next K and the next V tile, items to the K after
             uint32_t k_ph = 0, v_ph = 0;
-            auto next = [&](int &st, uint32_t &ph) {
-                st += 2;
+            auto next = [&](int &st, uint32_t &ph, int by) {
+                st += by;
                 if (st >= ring) {
                     st -= ring;
                     ph ^= 1u;
@@ -367,7 +402,7 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                     }
                     if (j >= 2 * shared || g == 1) {      // the last to read this V
                         mma_commit(bar_empty + v_st * 8);
-                        next(v_st, v_ph);
+                        next(v_st, v_ph, 2);
                     }
                 }
                 const int j2 = j + 2;
@@ -387,7 +422,8 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                 mma_commit(bar_s + g * 8);
                 if (j2 >= 2 * shared || g == 1) {         // the last to read this K
                     mma_commit(bar_empty + k_st * 8);
-                    next(k_st, k_ph);
+                    next(k_st, k_ph, k_by);
+                    k_by = 2;
                 }
             }
         }
@@ -401,15 +437,21 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         constexpr int CH = D / 8, RPP = 32 / CH;          // 16-byte chunks per row, rows per pass of the warp
         const int lr = lane / CH, lc = lane % CH;
         src += (PAGED ? 0 : a.prefix) * row_stride + lc * 8;
-        int st = (2 * u0 + (warp - 10)) % ring, turn = warp - 10;     // stage; items since the first gathered one, mod ring
-        uint32_t go_ph = 0;
+        auto item_of = [&](int u) { return warp == 10 ? k_item(u) : v_item(u); };
+        // parity of a stage's turns so far: its earlier items that were gathered
+        auto turn_of = [&](int item) -> uint32_t {
+            uint32_t odd = 0;
+#pragma unroll 1
+            for (int i = item - ring; i >= k_item(u0); i -= ring) odd ^= uint32_t(!skew || (i & 1) || i == 0 || i >= v_item(u0));
+            return odd;
+        };
         // The first pass, while the tensor cores are at the prefix, only asks for the rows to be brought into L2: a
         // unit's count, indices and rows are three memory latencies one after the other.
         const bool early = u0 > 0;
 #pragma unroll 1
         for (int v = early ? 2 * u0 - n_units : u0; v <= n_units; ++v) {
             if (PAGED && v == u0 && tail && warp == 11) { // ahead of the gathered tiles: rows behind the prefix's end
-                const int left = prefix - (tp - 1) * KN, rows = -left & 15, at = (2 * (tp - 1 - T0) + 1) % ring;
+                const int left = prefix - (tp - 1) * KN, rows = -left & 15, at = v_item(tp - 1 - T0) % ring;
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_tail, 0, a.status, qt))) break;
                 for (int i = lane; i < rows * DH * 8; i += 32)
                     asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n"
@@ -446,7 +488,8 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(src - lc * 8 + node[k] * row_stride + hf * 64));
                 continue;
             }
-            if (!__all_sync(0xffffffffu, mbar_wait(bar_go + st * 8, go_ph, a.status, qt))) break;
+            const int st = item_of(u) % ring;
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_go + st * 8, turn_of(item_of(u)), a.status, qt))) break;
             const uint32_t dst = s_ring + st * TILE + (lc >> 3) * HALF;
 #pragma unroll 1
             for (int step = 0; step < QM / 16; ++step) {
@@ -465,13 +508,6 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_full + st * 8) : "memory");
-            st += 2;
-            if (st >= ring) st -= ring;
-            turn += 2;
-            if (turn >= ring) {
-                turn -= ring;
-                go_ph ^= 1u;
-            }
         }
     } else {
         // ====== softmax: two groups of 128 threads, one thread per query row ======

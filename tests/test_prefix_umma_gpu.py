@@ -38,6 +38,23 @@ def test_prefix_and_tree_in_one(fst, n, teeth, prefix, splits, D, bm):
     assert fst.last_status() == 0
 
 
+@pytest.mark.parametrize("splits", [2, 3, 4, 8])
+@pytest.mark.parametrize("prefix,n,teeth", [(128, 60, 1), (257, 60, 20), (640, 100, 70), (1100, 128, 128), (1500, 90, 200), (2304, 128, 300)])
+def test_one_query_tile_in_clustered_runs(fst, prefix, n, teeth, splits):
+    """One query tile to a K/V head at D 128, in a cluster: K is loaded a tile ahead of V.  Runs of no, one and more tiles,
+    of the tree's tiles only, with up to three gathered ones, that go round the ring of six stages and do not."""
+    n = max(n, teeth + 20)
+    par = comb(n, teeth)
+    meta = fst.build_tree_metadata(par, 128, 512, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(prefix + splits)
+    q = torch.randn((3, 25, n, 128), generator=g, device="cuda").half()       # more query tiles than idle SMs: nothing is spread
+    k, v = (torch.randn((3, 25, prefix + n, 128), generator=g, device="cuda").half() for _ in range(2))
+    o, lse = fst.fst_attention(q, k, v, meta, sm_scale=128 ** -0.5, kernel="tma_umma", kv_splits=splits, return_lse=True)
+    want, ref = fst.fst_attention(q.float(), k.float(), v.float(), meta, sm_scale=128 ** -0.5, kernel="simt", return_lse=True)
+    assert (o.float() - want).abs().max().item() <= 2e-3 and (lse - ref).abs().max().item() <= 1e-3
+    assert fst.last_status() == 0
+
+
 @pytest.mark.parametrize("rows", [slice(40, 50), slice(700, 710), slice(1100, 1110)])     # prefix, prefix, tree
 def test_prefix_moving_maximum(fst, rows):
     """Rows whose scores dwarf the first reference point: the accumulators are rescaled."""
