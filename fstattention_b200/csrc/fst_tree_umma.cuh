@@ -12,7 +12,7 @@
 //            the item's own rows (contiguous, TMA boxes); tile t > 0 holds ancestor slots
 //            [(t-1) BM, t BM) of every block (gathered row by row; padding slots are zeros).  The last
 //            tile is narrow - BM / 2 columns for each block - when the lists end in its first half.
-//   round    the tiles that one softmax takes: one, or - MERGED - the own tile and the first gathered one (see Cut)
+//   round    the tiles that one softmax takes (see Round)
 //   S = Q K^T     M 128, N 128 (64), both operands in shared memory (128-byte swizzle)
 //   softmax       thread r of a group owns row r and looks only at its block's columns; 32-column
 //                 words in which no row of its warp has a mask bit are not even read; P goes back
@@ -55,12 +55,12 @@
 // in use, one on its way, and the last one's O.  Items of one tile run at HBM's rate (D 128: 83 us where 64 trees of
 // 256 nodes take 112; D 64: 1165 where the forest takes 1550), so a second round is what the rest pays for.
 //
-// MERGED: the own tile and the first gathered one in one round, so that an item of two tiles goes once through the chain
-// and rescales nothing.  S has room for it because every block's product writes the same columns, each into the
-// lanes of its own block (disable-output-lane): 64 + 64 of 128 columns at D 128, block_m 64 (2 x N 64 cost 102 cycles
-// where N 128 costs 64), 128 + 64 of 192 at D 64, block_m 128.  Apart / merged: forest of 65532 nodes 1752 / 1615 us;
-// 4096-node deep tree 63.0 / 61.9; 64 x 256 nodes, D 128 115.8 / 112.  Not where it lost: long lists at D 128, block_m 64
-// (dynamic trees of 1024 nodes 54.4 / 56.0), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118).
+// Both tiles of an item in one round (Round::BOTH and SHARED): once through the chain, and nothing to rescale.  BOTH, for
+// bounds of up to 64: forest of 65532 nodes 1752 -> 1340 us, of 8188 and 16380 43 -> 35 and 227 -> 173.  SHARED, for bounds of up to 128, as
+// calls follow one another in a program: 64 x 256 nodes 110.2 -> 105.8, 4096-node deep tree 63.8 -> 61.8 (in graphs of one call they
+// are within 3 % of one another; two products of N 64 cost 102 cycles of tensor core where one of N 128 costs 64).  Not where
+// it lost: longer lists (dynamic trees of 1024 nodes, D 128 54.4 / 56.0; D 64, block_m 128, further rounds of 64 or 128
+// slots: 24.4 / 27.1 and 68 / 79), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118).
 // tree_umma_pays (fst_plan.h) has the line between the two kernels.
 #pragma once
 
@@ -94,22 +94,11 @@ struct Geo {
     static_assert(SMEM_BYTES <= 227 * 1024, "one CTA's shared memory");
 };
 
-// How a row's columns are cut into rounds of a product, a softmax and another product.  Apart: a round is a tile of 128
-// columns, in which every block has its own.  MERGED: all blocks use the same columns of S - each product writes the
-// lanes of its block only - so that a row's own BM columns and, behind them, the slots of the first FIRST gathered
-// tiles are one round, and MORE gathered tiles each of the later ones.
-template <int D, int BM, bool MERGED>
-struct Cut {
-    static constexpr int COLS = Geo<D>::COLS;
-    static constexpr bool PACKED = MERGED && BM == 128;       // K and V rows of a gathered tile share a buffer (64 slots)
-    static constexpr int GS = PACKED ? BM / 2 : BM;           // ancestor slots of a block in a gathered tile
-    static constexpr int FIRST = MERGED ? 1 : 0, MORE = MERGED ? 2 : 1;
-    static constexpr int NW = BM / 32;                        // mask words of a row: its own block's,
-    static constexpr int EW0 = FIRST * GS / 32, EW = MORE * GS / 32;   // the first round's slots', a later round's
-    static constexpr int WORDS = NW + EW0 > EW ? NW + EW0 : EW;
-    static constexpr bool LONE = PACKED;                      // look for words with a column a row (see the softmax)
-    static_assert(EW >= EW0 && (!MERGED || (BM + FIRST * GS <= COLS && MORE * GS <= COLS)), "a round's columns");
-};
+// What one softmax takes.  TILE: a column tile.  BOTH: the two tiles of an item whose lists end in the first half of a
+// gathered tile (D 64, block_m 128: 128 + 64 of S's 192 columns).  SHARED: the own tile and the first gathered one, then
+// two gathered ones at a time, where the item's two blocks use the same columns of S, each product writing the lanes of its
+// block (D 128, block_m 64: 64 + 64 of 128 columns).
+enum class Round { TILE, BOTH, SHARED };
 
 // what the loading warp tells a group and its issuing thread about their next item
 struct ItemInfo {
@@ -121,22 +110,22 @@ struct ItemInfo {
 };
 
 // 16-column steps of gathered tile t that hold slots of some block (bit ks: rows 16 ks .. of the buffer); seg: slots per block
-template <int BM, int GS>
+template <int BM>
 __device__ __forceinline__ uint32_t live_steps(int t, int seg, const int (&count)[ROWS / BM]) {
     uint32_t steps = 0;
 #pragma unroll
     for (int s = 0; s < ROWS / BM; ++s) {
-        const int left = min(count[s] - (t - 1) * GS, seg), n = left > 0 ? (left + 15) >> 4 : 0;
+        const int left = min(count[s] - (t - 1) * BM, seg), n = left > 0 ? (left + 15) >> 4 : 0;
         steps |= ((1u << n) - 1u) << (s * seg >> 4);
     }
     return steps;
 }
 
 // column tiles of an item whose longest ancestor list has `longest` entries, and whether the last is narrow
-template <int BM, int GS>
+template <int BM>
 __device__ __forceinline__ int tiles_of(int longest, bool *narrow) {
-    const int tiles = 1 + (longest + GS - 1) / GS;
-    *narrow = BM > 32 && GS == BM && tiles > 1 && longest - (tiles - 2) * GS <= BM / 2;
+    const int tiles = 1 + (longest + BM - 1) / BM;
+    *narrow = BM > 32 && tiles > 1 && longest - (tiles - 2) * BM <= BM / 2;
     return tiles;
 }
 
@@ -161,7 +150,7 @@ struct TreeUmmaArgs {
     int heads_first;                   // item order: heads fastest and the last rows first
 };
 
-template <typename T, int D, int BM, bool MERGED>
+template <typename T, int D, int BM, tree_umma::Round ROUND>
 __global__ void __launch_bounds__(tree_umma::THREADS, 1)
 tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -172,9 +161,11 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
     using G = Geo<D>;
     constexpr bool BF16 = !std::is_same<T, __half>::value;
     constexpr int DH = D / 64, TILE = G::TILE, POOL = G::POOL;
-    using C = Cut<D, BM, MERGED>;
+    constexpr bool BOTH = ROUND == Round::BOTH, SHARED = ROUND == Round::SHARED;
+    static_assert((!BOTH || (BM == 128 && D == 64)) && (!SHARED || (BM == 64 && D == 128)), "room in tensor memory for the columns of both tiles");
     constexpr int SUB = ROWS / BM;                        // blocks per item
-    constexpr int GS = C::GS, NW = C::NW;
+    constexpr int NW = BM / 32;                           // mask words per row and tile
+    constexpr int EW = BOTH ? 2 : SHARED ? 2 * NW : NW;   // of them in the gathered tiles of a round
 
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     extern __shared__ unsigned char smem_raw[];
@@ -301,16 +292,16 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             const int p = tile_of(w), h = head_of(w), hk = h / a.kv_group;
             int cnt[SUB];
             bool narrow;
-            const int tiles = tiles_of<BM, GS>(spread(cnt_lane, cnt), &narrow);
+            const int tiles = tiles_of<BM>(spread(cnt_lane, cnt), &narrow);
             cnt_lane = count_of(next);                    // one item ahead
             const int g = n & 1, pos = g ? ahead[1] : ahead[0];
-            const int end = pos + (C::PACKED ? tiles + 1 : 2 * tiles - int(narrow));   // positions: two for a tile, one where K and V share a buffer
-            // Own K and Q, (merged: the first gathered tile,) own V, the (other) gathered tiles: as the round needs them, for
-            // buffers come free one by one, some 1000 cycles apart where the pool is what bounds the kernel (with V second
-            // and Q third: 64 x 256 nodes D 128 112.2 -> 106.4 us, block_m 128 103.6 -> 99.5, block_m 32 104.5 -> 92.7, 4096-node
-            // deep tree 62.0 -> 58.0).  PACKED keeps Q last: its pool has room, and this order took 1485 -> 1500 us.
-            const int gathered = end - pos - 2, q_at = C::PACKED ? 2 : 1,
-                      v_at = C::PACKED ? 1 : 2 + (MERGED ? min(gathered, narrow && tiles == 2 ? 1 : 2) : 0);
+            const int end = pos + 2 * tiles - int(narrow);    // positions: two for a tile, one where K and V share a buffer
+            // Own K, Q, the first gathered tile, own V, the other gathered ones: buffers come free one by one, some 1000
+            // cycles apart where the pool is what bounds the kernel, the first product needs Q and the first gathered tile
+            // takes longest to come (with V second and Q third: 64 x 256 nodes D 128 115.8 -> 106.5 us, block_m 128 103.6 ->
+            // 99.5, block_m 32 104.5 -> 92.7, 4096-node deep tree 63.0 -> 58.0).  BOTH keeps Q last: its pool has room,
+            // and this order took 1485 -> 1500 us.
+            const int gathered = end - pos - 2, q_at = BOTH ? 2 : 1, v_at = BOTH ? 1 : 2 + min(gathered, narrow && tiles == 2 ? 1 : 2);
             int at = pos + 2;
 #pragma unroll 1
             for (int i = 0; i < 3 + gathered; ++i) {
@@ -374,13 +365,13 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 next = plus(w, step);
                 const int longest = spread(cnt_lane, cnt);
                 cnt_lane = count_of(next);
-                tiles = tiles_of<BM, GS>(longest, &narrow);
+                tiles = tiles_of<BM>(longest, &narrow);
                 pos += 2;                                 // the own tile's slots
                 t = 0;
             }
-            x.one = C::PACKED || (narrow && t + 1 == tiles);
+            x.one = narrow && t + 1 == tiles;
             const int seg = x.one ? BM / 2 : BM;
-            uint32_t steps = live_steps<BM, GS>(t, seg, cnt);
+            uint32_t steps = live_steps<BM>(t, seg, cnt);
             x.row_a = x.row_b = -1;
             for (int i = 0; steps != 0; ++i) {
                 const int row = (__ffs(steps) - 1) * 16;
@@ -394,7 +385,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             if (mine >= 0) {
                 const int s = mine / seg;
                 x.b = tile_of(w) * SUB + s;
-                x.slot = (t - 1) * GS + mine - s * seg + (lane & 15);
+                x.slot = (t - 1) * BM + mine - s * seg + (lane & 15);
                 int c = 0;
 #pragma unroll
                 for (int i = 0; i < SUB; ++i)
@@ -469,8 +460,8 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
         if (a.meta_stable) asm volatile("griddepcontrol.wait;\n" ::: "memory");
         if (elect_one()) {
             const uint64_t dk = smem_desc(s_base, 16), dv = smem_desc(s_base, HALF), dv_one = smem_desc(s_base + TILE / 2, HALF / 2);
-            const uint32_t idesc_pv = instr_desc(BF16, true, D), s_col = tmem_base + g * C::COLS, o_col = tmem_base + 2 * C::COLS + g * D;
-            const uint4 *rows = reinterpret_cast<const uint4 *>(smem + G::OFF_ROWS) + g * (C::COLS / 16);
+            const uint32_t idesc_pv = instr_desc(BF16, true, D), s_col = tmem_base + g * G::COLS, o_col = tmem_base + 2 * G::COLS + g * D;
+            const uint4 *rows = reinterpret_cast<const uint4 *>(smem + G::OFF_ROWS) + g * (G::COLS / 16);
             bool alive = true;
             int round = 0, n = g;
             Where w = first;
@@ -485,10 +476,55 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 int cnt[SUB];
 #pragma unroll
                 for (int s = 0; s < SUB; ++s) cnt[s] = four[s];
-                if constexpr (MERGED) {
-                    auto one_buffer = [&](int t) { return t > 0 && (C::PACKED || (in.z != 0 && t + 1 == tiles)); };
+                if constexpr (BOTH) {
+                    // the own tile and, when there are ancestors, one narrow tile: both products of S, the softmax, both of O
+                    const int at = in.y, steps0 = min((own_rows + 15) >> 4, ROWS / 16), steps1 = (cnt[0] + 15) >> 4;
+                    alive = wait(full_of(g, at), full_parity(at), a.status, item);
+                    if (!alive) break;
+                    int b = buf_of(g, at);
+                    auto scores = [&](uint32_t to, uint64_t dks, int steps) {
+                        const uint32_t idesc_s = instr_desc(BF16, false, 16 * steps);
+                        fence_after_sync();
+#pragma unroll
+                        for (int ks = 0; ks < D / 16; ++ks) mma_f16(to, dqs + ks * 2, dks + ks * 2, idesc_s, ks > 0);
+                    };
+                    scores(s_col, dk + uint64_t(b * (TILE >> 4)), steps0);
+                    int b1 = 0;
+                    if (tiles > 1) {
+                        alive = wait(full_of(g, at + 2), full_parity(at + 2), a.status, item);
+                        if (!alive) break;
+                        b1 = buf_of(g, at + 2);
+                        fence_copied();
+                        scores(s_col + BM, dk + uint64_t(b1 * (TILE >> 4)), steps1);
+                    }
+                    mma_commit(bar_s + g * 8);
+                    mma_commit(bar_empty + b * 8);
+                    // (V is usually there long before P)
+                    alive = wait(full_of(g, at + 1), full_parity(at + 1), a.status, item) && wait(bar_p + g * 8, round & 1, a.status, item);
+                    if (!alive) break;
+                    ++round;
+                    b = buf_of(g, at + 1);
+                    fence_after_sync();
+                    auto output = [&](auto most, int col, uint64_t dvs, int steps) {
+                        constexpr int MOST = decltype(most)::value;
+                        uint4 off[MOST];
+#pragma unroll
+                        for (int ks = 0; ks < MOST; ++ks) off[ks] = rows[(col >> 4) + ks];
+#pragma unroll
+                        for (int ks = 0; ks < MOST; ++ks)
+                            if (ks < steps) mma_f16_ts_but(o_col, s_col + (col >> 1) + ks * 8, dvs + uint64_t((ks * 16 * 128) >> 4), idesc_pv, off[ks]);
+                    };
+                    output(std::integral_constant<int, 8>{}, 0, dv + uint64_t(b * (TILE >> 4)), steps0);
+                    mma_commit(bar_empty + b * 8);
+                    if (tiles > 1) {
+                        output(std::integral_constant<int, 4>{}, BM, dv_one + uint64_t(b1 * (TILE >> 4)), steps1);
+                        mma_commit(bar_empty + b1 * 8);
+                    }
+                    mma_commit(bar_o + g * 8);
+                } else if constexpr (SHARED) {
+                    auto one_buffer = [&](int t) { return in.z != 0 && t > 0 && t + 1 == tiles; };
                     auto live = [&](int t, int s, int seg) -> int {   // 16-column steps of block s in tile t
-                        const int left = t == 0 ? min(own_rows - s * BM, BM) : min(cnt[s] - (t - 1) * GS, seg);
+                        const int left = t == 0 ? min(own_rows - s * BM, BM) : min(cnt[s] - (t - 1) * BM, seg);
                         return left > 0 ? (left + 15) >> 4 : 0;
                     };
                     // Every block's rows against its own columns, all blocks into the same columns of S (each its own lanes).
@@ -523,11 +559,11 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                         }
                     };
                     using Full = std::integral_constant<int, BM>;
-                    using Part = std::integral_constant<int, BM / 2 < 32 ? BM : BM / 2>;   // (never one buffer with blocks of 32)
+                    using Part = std::integral_constant<int, BM / 2>;
                     int at = in.y;                            // position of the round's first tile
 #pragma unroll 1
                     for (int t0 = 0; t0 < tiles; ++round) {
-                        const int t1 = min(tiles, t0 == 0 ? 1 + C::FIRST : t0 + C::MORE);
+                        const int t1 = min(tiles, t0 == 0 ? 2 : t0 + 2);
                         int p = at, col = 0;
 #pragma unroll 1
                         for (int t = t0; t < t1; ++t) {
@@ -543,7 +579,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                             if (t + 1 == t1) mma_commit(bar_s + g * 8);
                             if (!one) mma_commit(bar_empty + b * 8);
                             p += one ? 1 : 2;
-                            col += t == 0 ? BM : GS;
+                            col += BM;
                         }
                         if (!alive) break;
                         // (the first V tile is usually there long before P)
@@ -563,7 +599,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                             if (one) output(Part{}, t, col, dv_one + uint64_t(b * (TILE >> 4)));
                             else output(Full{}, t, col, dv + uint64_t(b * (TILE >> 4)));
                             mma_commit(bar_empty + b * 8);
-                            col += t == 0 ? BM : GS;
+                            col += BM;
                         }
                         if (!alive) break;
                         t0 = t1;
@@ -572,7 +608,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 } else {
                     // 16-column steps of tile t that some block has (bit ks: rows 16 ks .. of the buffer)
                     auto steps_of = [&](int t, int seg) -> uint32_t {
-                        return t == 0 ? (1u << min((own_rows + 15) >> 4, ROWS / 16)) - 1u : live_steps<BM, GS>(t, seg, cnt);
+                        return t == 0 ? (1u << min((own_rows + 15) >> 4, ROWS / 16)) - 1u : live_steps<BM>(t, seg, cnt);
                     };
                     int at = in.y;                            // position of the tile's K rows
 #pragma unroll 1
@@ -639,7 +675,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
         // ================================ softmax ================================
         const int g = warp >> 2, r = tid & 127;           // my group and query row of its items
         const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
-        const uint32_t tmem_s = tmem_base + g * C::COLS + lane_base, tmem_o = tmem_base + 2 * C::COLS + g * D + lane_base;
+        const uint32_t tmem_s = tmem_base + g * G::COLS + lane_base, tmem_o = tmem_base + 2 * G::COLS + g * D + lane_base;
         const int sub = r / BM, j = r % BM;               // my block and row in it (sub is uniform in a warp)
         const float c2 = a.scale_log2;
         // mask words of my row: its own block's, and those from word w0 of its ancestor slots on (item and block may not exist)
@@ -660,13 +696,13 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 w[0] = ok ? __ldg(from) : 0u;
             }
         };
-        auto ext_words = [&](const Where &at, int w0, uint32_t (&w)[C::EW]) {
+        auto ext_words = [&](const Where &at, int w0, uint32_t (&w)[EW]) {
             const int b = tile_of(at) * SUB + sub, left = at.z < a.Z && b < a.nb ? maw - w0 : 0;
             const uint32_t *from = mask + (uint32_t(at.z) * blob_words + ext0 + uint32_t(b) * uint32_t(BM * maw) + uint32_t(w0));
 #pragma unroll
-            for (int i = 0; i < C::EW; ++i) w[i] = i < left ? __ldg(from + i) : 0u;
+            for (int i = 0; i < EW; ++i) w[i] = i < left ? __ldg(from + i) : 0u;
         };
-        uint32_t own[NW], ext[C::EW];
+        uint32_t own[NW], ext[EW];
         Where at = first;
         own_words(at, own);
         ext_words(at, 0, ext);
@@ -687,84 +723,170 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             for (int c = 0; c < 16; ++c) zero[c] = 0u;
 #pragma unroll 1
             for (int c0 = 0; c0 < D; c0 += 16) tmem_st16(tmem_o + c0, zero);
-            if constexpr (MERGED) {
+            if constexpr (BOTH) {
+                constexpr int WORDS = NW + EW;
+                uint32_t word[WORDS];                     // the columns that my row attends to: its own block's, its ancestors'
+#pragma unroll
+                for (int i = 0; i < WORDS; ++i) word[i] = i < NW ? own[i % NW] : ext[(i - NW) % EW];
+                own_words(at_next, own);                  // the next item's go out now: a loaded L2 answers late
+                ext_words(at_next, 0, ext);
+                alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, round & 1, a.status, item));
+                if (!alive) break;
+                ++round;
+                fence_after_sync();
+
+                uint32_t live = 0, lone_words = 0;        // bit i: some row of my warp has a bit in word i; no row has two
+                {
+                    uint32_t on = 0;                      // lane k: rows of my warp with a column in 16 k ..
+#pragma unroll
+                    for (int i = 0; i < WORDS; ++i) {
+                        const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
+                        live |= uint32_t((lo | hi) != 0u) << i;
+                        if (i < NW && (lo | hi) != 0u && __ballot_sync(0xffffffffu, (word[i] & (word[i] - 1u)) != 0u) == 0u) lone_words |= 1u << i;
+                        if (lane == 2 * i) on = lo;
+                        if (lane == 2 * i + 1) on = hi;
+                    }
+                    if (lane < 2 * WORDS) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (G::COLS / 16) + lane) * 4 + (warp & 3)] = ~on;
+                }
+                float mu = 0.f, mx = -INFINITY;
+                uint64_t sum2 = 0;
+                // A word in which every row has one column at most - a block's own word where the tree is numbered breadth first and
+                // a row attends to nobody in its block but itself - needs no 32 exponentials: the score is picked out (forest of 65532
+                // nodes 1615 -> 1550 us).
+                int lone = -1, lone_at = -1;              // that word, my row's column in it
+                if (lone_words != 0u) {
+                    lone = __ffs(lone_words) - 1;
+                    live &= ~(1u << lone);
+                    uint32_t v[32], w = word[0];
+#pragma unroll
+                    for (int i = 1; i < NW; ++i) w = lone == i ? word[i] : w;
+                    tmem_ld32(v, tmem_s + lone * 32);
+                    lone_at = __ffs(w) - 1;
+                    tmem_ld_wait(v);
+#pragma unroll
+                    for (int half = 16; half > 0; half /= 2)
+#pragma unroll
+                        for (int c = 0; c < half; ++c) v[c] = (lone_at & half) != 0 ? v[c + half] : v[c];
+                    mx = lone_at < 0 ? -INFINITY : __uint_as_float(v[0]);
+                }
+                const float lone_score = mx;
+                // My live words, one to a turn (two spill).  First time through: the row's maximum, which is the reference
+                // point.  Second time (or at once, when one turn was all): probabilities, over S - word i of P covers
+                // columns 16 i .. of S, below the words still to be read.
+                bool second = false;
+#pragma unroll 1
+                for (uint32_t rest = live; !second || rest != 0u;) {
+                    uint32_t s[32];
+                    const int wi = __ffs(rest) - 1;       // the word's number, -1: none but the lone one
+                    rest &= rest - 1;
+                    if (wi >= 0) {
+                        uint32_t w = word[0];
+                        tmem_ld32(s, tmem_s + wi * 32);
+#pragma unroll
+                        for (int i = 1; i < WORDS; ++i) w = wi == i ? word[i] : w;
+                        tmem_ld_wait(s);
+                        float m2[2] = {mx, -INFINITY};
+#pragma unroll
+                        for (int c = 0; c < 32; c += 2) {
+                            s[c] = (w & (1u << c)) != 0u ? s[c] : 0xff800000u;
+                            s[c + 1] = (w & (2u << c)) != 0u ? s[c + 1] : 0xff800000u;
+                            m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[c]), __uint_as_float(s[c + 1])));
+                        }
+                        mx = fmaxf(m2[0], m2[1]);
+                    }
+                    if (!second) {
+                        if (rest != 0u) continue;
+                        m_ref = mx;
+                        mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
+                        second = true;
+                        if ((live & (live - 1u)) != 0u) { // more than a turn: once again from the first
+                            rest = live;
+                            continue;
+                        }
+                    }
+                    if (wi >= 0) {
+                        const uint64_t scale2 = pair(c2, c2), shift2 = pair(-mu, -mu);
+                        uint32_t pk[16];
+#pragma unroll
+                        for (int c = 0; c < 32; c += 2) {
+                            float p0, p1;
+                            unpair(fma2(pair(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), scale2, shift2), p0, p1);
+                            p0 = fast_exp2(p0);
+                            p1 = fast_exp2(p1);
+                            sum2 = add2(sum2, pair(p0, p1));
+                            pk[c >> 1] = MT::pack(p0, p1);
+                        }
+                        tmem_st16(tmem_s + wi * 16, pk);
+                    }
+                }
+                if (lone >= 0) {
+                    const float p = fast_exp2(fmaf(lone_score, c2, -mu));
+                    const uint32_t v = (lone_at & 1) != 0 ? MT::pack(0.f, p) : MT::pack(p, 0.f);
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) pk[i] = lone_at >> 1 == i ? v : 0u;
+                    tmem_st16(tmem_s + lone * 16, pk);
+                    l += p;
+                }
+                float sum[2];
+                unpair(sum2, sum[0], sum[1]);
+                l += sum[0] + sum[1];
+                tmem_st_wait();
+                fence_before_sync();
+                arrive(bar_p + g * 8);
+            } else if constexpr (SHARED) {
 #pragma unroll 1
                 for (int t = 0; t < tiles; ++round) {         // t: the round's first tile
                     const bool first_round = t == 0;
-                    uint32_t word[C::WORDS];                  // the round's columns that my row attends to
+                    constexpr int WORDS = 2 * NW;
+                    uint32_t word[WORDS];                     // the round's columns that my row attends to
 #pragma unroll
-                    for (int i = 0; i < C::WORDS; ++i) {
-                        const uint32_t mine = i < NW ? own[i % NW] : i < NW + C::EW0 ? ext[(i - NW) % C::EW] : 0u;
-                        word[i] = first_round ? mine : i < C::EW ? ext[i % C::EW] : 0u;
+                    for (int i = 0; i < WORDS; ++i) {
+                        word[i] = !first_round ? ext[i % EW] : i < NW ? own[i % NW] : ext[(i - NW) % EW];
                     }
-                    t = first_round ? 1 + C::FIRST : t + C::MORE;
+                    t += 2;
                     // the words of the round after go out now: a loaded L2 answers late
                     if (first_round) own_words(at_next, own);
                     if (t >= tiles) ext_words(at_next, 0, ext);
-                    else ext_words(at, (t - 1) * (GS / 32), ext);
+                    else ext_words(at, (t - 1) * NW, ext);
                     alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, round & 1, a.status, item));
                     if (!alive) break;
                     fence_after_sync();
 
-                    uint32_t live = 0, lone_words = 0;        // bit i: some row of my warp has a bit in word i; no row has two
+                    uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
                     {
                         uint32_t on = 0;                      // lane k: rows of my warp with a column in 16 k ..
 #pragma unroll
-                        for (int i = 0; i < C::WORDS; ++i) {
+                        for (int i = 0; i < WORDS; ++i) {
                             const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
                             live |= uint32_t((lo | hi) != 0u) << i;
-                            if (C::LONE && i < NW && first_round && (lo | hi) != 0u && __ballot_sync(0xffffffffu, (word[i] & (word[i] - 1u)) != 0u) == 0u) lone_words |= 1u << i;
                             if (lane == 2 * i) on = lo;
                             if (lane == 2 * i + 1) on = hi;
                         }
-                        if (lane < 2 * C::WORDS) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (C::COLS / 16) + lane) * 4 + (warp & 3)] = ~on;
+                        if (lane < 2 * WORDS) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (G::COLS / 16) + lane) * 4 + (warp & 3)] = ~on;
                     }
                     float mu = 0.f, mx = -INFINITY;
                     uint64_t sum2 = 0;
-                    // A word in which every row has one column at most - a block's own word where the tree is numbered breadth first and
-                    // a row attends to nobody in its block but itself - needs no 32 exponentials: the score is picked out (forest of 65532
-                    // nodes 1615 -> 1550 us).  At D 128, block_m 64 the lists are the longer part: deep tree 61.6 -> 64.8, not there.
-                    int lone = -1, lone_at = -1;              // that word, my row's column in it
-                    if (C::LONE && lone_words != 0u) {
-                        lone = __ffs(lone_words) - 1;
-                        live &= ~(1u << lone);
-                        uint32_t v[32], w = word[0];
-#pragma unroll
-                        for (int i = 1; i < NW; ++i) w = lone == i ? word[i] : w;
-                        tmem_ld32(v, tmem_s + lone * 32);
-                        lone_at = __ffs(w) - 1;
-                        tmem_ld_wait(v);
-#pragma unroll
-                        for (int half = 16; half > 0; half /= 2)
-#pragma unroll
-                            for (int c = 0; c < half; ++c) v[c] = (lone_at & half) != 0 ? v[c + half] : v[c];
-                        mx = lone_at < 0 ? -INFINITY : __uint_as_float(v[0]);
-                    }
-                    const float lone_score = mx;
-                    // My live words, one to a turn (two spill: there are words of two kinds to keep).  First time through: the row's maximum, then the
-                    // reference point.  Second time (or at once, when one turn was all): probabilities, over S - word i of P
-                    // covers columns 16 i .. of S, below the words still to be read.
+                    // As above, but the reference point may move from round to round.
                     bool second = false;
 #pragma unroll 1
-                    for (uint32_t rest = live; (C::LONE && !second) || rest != 0u;) {
+                    for (uint32_t rest = live; rest != 0u;) {
                         uint32_t s[32];
-                        const int wi = __ffs(rest) - 1;       // the word's number, -1: none but the lone one
+                        const int wi = __ffs(rest) - 1;       // the word's number
                         rest &= rest - 1;
-                        if (!C::LONE || wi >= 0) {
-                            uint32_t w = word[0];
-                            tmem_ld32(s, tmem_s + wi * 32);
+                        uint32_t w = word[0];
+                        tmem_ld32(s, tmem_s + wi * 32);
 #pragma unroll
-                            for (int i = 1; i < C::WORDS; ++i) w = wi == i ? word[i] : w;
-                            tmem_ld_wait(s);
-                            float m2[2] = {mx, -INFINITY};
+                        for (int i = 1; i < WORDS; ++i) w = wi == i ? word[i] : w;
+                        tmem_ld_wait(s);
+                        float m2[2] = {mx, -INFINITY};
 #pragma unroll
-                            for (int c = 0; c < 32; c += 2) {
-                                s[c] = (w & (1u << c)) != 0u ? s[c] : 0xff800000u;
-                                s[c + 1] = (w & (2u << c)) != 0u ? s[c + 1] : 0xff800000u;
-                                m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[c]), __uint_as_float(s[c + 1])));
-                            }
-                            mx = fmaxf(m2[0], m2[1]);
+                        for (int c = 0; c < 32; c += 2) {
+                            s[c] = (w & (1u << c)) != 0u ? s[c] : 0xff800000u;
+                            s[c + 1] = (w & (2u << c)) != 0u ? s[c + 1] : 0xff800000u;
+                            m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[c]), __uint_as_float(s[c + 1])));
                         }
+                        mx = fmaxf(m2[0], m2[1]);
                         if (!second) {
                             if (rest != 0u) continue;
                             const bool up = mx > m_ref;
@@ -790,29 +912,18 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                                 continue;
                             }
                         }
-                        if (!C::LONE || wi >= 0) {
-                            const uint64_t scale2 = pair(c2, c2), shift2 = pair(-mu, -mu);
-                            uint32_t pk[16];
-#pragma unroll
-                            for (int c = 0; c < 32; c += 2) {
-                                float p0, p1;
-                                unpair(fma2(pair(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), scale2, shift2), p0, p1);
-                                p0 = fast_exp2(p0);
-                                p1 = fast_exp2(p1);
-                                sum2 = add2(sum2, pair(p0, p1));
-                                pk[c >> 1] = MT::pack(p0, p1);
-                            }
-                            tmem_st16(tmem_s + wi * 16, pk);
-                        }
-                    }
-                    if (C::LONE && lone >= 0) {
-                        const float p = fast_exp2(fmaf(lone_score, c2, -mu));
-                        const uint32_t v = (lone_at & 1) != 0 ? MT::pack(0.f, p) : MT::pack(p, 0.f);
+                        const uint64_t scale2 = pair(c2, c2), shift2 = pair(-mu, -mu);
                         uint32_t pk[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) pk[i] = lone_at >> 1 == i ? v : 0u;
-                        tmem_st16(tmem_s + lone * 16, pk);
-                        l += p;
+                        for (int c = 0; c < 32; c += 2) {
+                            float p0, p1;
+                            unpair(fma2(pair(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), scale2, shift2), p0, p1);
+                            p0 = fast_exp2(p0);
+                            p1 = fast_exp2(p1);
+                            sum2 = add2(sum2, pair(p0, p1));
+                            pk[c >> 1] = MT::pack(p0, p1);
+                        }
+                        tmem_st16(tmem_s + wi * 16, pk);
                     }
                     float sum[2];
                     unpair(sum2, sum[0], sum[1]);
@@ -849,7 +960,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                             if (k == 2 * i) on = lo;
                             if (k == 2 * i + 1) on = hi;
                         }
-                        if (lane < 8) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (C::COLS / 16) + lane) * 4 + (warp & 3)] = on;
+                        if (lane < 8) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (G::COLS / 16) + lane) * 4 + (warp & 3)] = on;
                     }
                     float sum[2] = {0.f, 0.f}, mu = 0.f, mx = -INFINITY;
                     // My live words, WT to a turn.  First round: the row's maximum, then the reference point.  Second round (or
@@ -975,7 +1086,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
 
 // ---- host side ---------------------------------------------------------------------------------
 
-template <typename T, int D, int BM, bool MERGED>
+template <typename T, int D, int BM, tree_umma::Round ROUND>
 cudaError_t launch_tree_umma_t(const AttnArgs &a, cudaStream_t stream) {
     using G = tree_umma::Geo<D>;
     constexpr bool bf16 = !std::is_same<T, __half>::value;
@@ -988,7 +1099,7 @@ cudaError_t launch_tree_umma_t(const AttnArgs &a, cudaStream_t stream) {
         return cudaErrorNotSupported;
     static DeviceOnce configured;
     const cudaError_t ce = configured.run([&] {
-        return cudaFuncSetAttribute(tree_umma_kernel<T, D, BM, MERGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES);
+        return cudaFuncSetAttribute(tree_umma_kernel<T, D, BM, ROUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES);
     });
     if (ce != cudaSuccess) return ce;
     TreeUmmaArgs ta = {};
@@ -1009,17 +1120,22 @@ cudaError_t launch_tree_umma_t(const AttnArgs &a, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, tree_umma_kernel<T, D, BM, MERGED>, a, ta, tq, tk, tv, to);
+    return cudaLaunchKernelEx(&cfg, tree_umma_kernel<T, D, BM, ROUND>, a, ta, tq, tk, tv, to);
 }
 
 template <typename T, int D>
 cudaError_t launch_tree_umma_d(const AttnArgs &a, cudaStream_t stream) {
+    using tree_umma::Round;
     switch (a.bm) {
-        case 32: return launch_tree_umma_t<T, D, 32, false>(a, stream);
+        case 32: return launch_tree_umma_t<T, D, 32, Round::TILE>(a, stream);
         case 64:
-            if (D == 128 && a.ma <= 128) return launch_tree_umma_t<T, D, 64, D == 128>(a, stream);
-            return launch_tree_umma_t<T, D, 64, false>(a, stream);
-        case 128: return launch_tree_umma_t<T, D, 128, D == 64>(a, stream);
+            if constexpr (D == 128)
+                if (a.ma <= 128) return launch_tree_umma_t<T, D, 64, Round::SHARED>(a, stream);
+            return launch_tree_umma_t<T, D, 64, Round::TILE>(a, stream);
+        case 128:
+            if constexpr (D == 64)
+                if (a.ma <= 64) return launch_tree_umma_t<T, D, 128, Round::BOTH>(a, stream);
+            return launch_tree_umma_t<T, D, 128, Round::TILE>(a, stream);
     }
     return cudaErrorNotSupported;
 }

@@ -61,20 +61,22 @@ def test_tree_umma_many_items_strided(fst, D, bm):
 
 @pytest.mark.parametrize("D,bm", [(64, 128), (128, 64)])
 @pytest.mark.parametrize("own", ["alone", "chained", "across"])
-@pytest.mark.parametrize("n,teeth", [(77, 1), (129, 20), (300, 32), (300, 33), (640, 64), (640, 65), (300, 96), (640, 97), (650, 128)])
-def test_tree_umma_merged_rounds(fst, D, bm, own, n, teeth):
-    """The own tile and the first gathered one in one softmax (bounds of up to 128 at D 128): lists that end in either half
-    of the first gathered tile, fill it, or need a second round; rows that attend to nobody in their block but
+@pytest.mark.parametrize("n,teeth", [(77, 1), (129, 20), (300, 16), (640, 17), (300, 32), (300, 33), (640, 64), (640, 65), (640, 97), (650, 128)])
+def test_tree_umma_merged_round(fst, D, bm, own, n, teeth):
+    """Both tiles of an item in one softmax (D 64, block_m 128, bounds of up to 64; D 128, block_m 64, bounds of up to 128;
+    longer bounds take the same trees tile by tile): lists that end in any 16-column step or fill the tile; rows that attend to nobody in their block but
     themselves, to their neighbours, and to a column in another 32-column word that nobody else uses.  A value that
     is not finite stays with the rows that attend to it or to one of its fifteen neighbours."""
     par = comb(n, teeth)
     for i in range(teeth, n):
         if own == "chained" and i % 3 and i > teeth or own == "across" and i % 32 == 0 and i > teeth:
             par[i] = i - 1
-    try:
-        meta = fst.build_tree_metadata(par, bm, 128, reference_format=False)
-    except RuntimeError:                                  # with those inside the block there are more
-        meta = fst.build_tree_metadata(par, bm, 128 + bm, reference_format=False)
+    for bound in (64, 128, 128 + bm):
+        try:
+            meta = fst.build_tree_metadata(par, bm, bound, reference_format=False)
+            break
+        except RuntimeError:                              # with those inside the block there are more
+            assert bound < 128 + bm
     longest = int(meta.packed[0, : meta.n_blocks * 4].view(torch.int32).max())
     assert longest <= teeth + 2 and (longest >= teeth or own == "chained" or n < 2 * bm)
     g = torch.Generator().manual_seed(n + teeth)
