@@ -438,11 +438,15 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
         const int lr = lane / CH, lc = lane % CH;
         src += (PAGED ? 0 : a.prefix) * row_stride + lc * 8;
         auto item_of = [&](int u) { return warp == 10 ? k_item(u) : v_item(u); };
-        // parity of a stage's turns so far: its earlier items that were gathered
+        // (stage and parity go along where the order is the plain one: 177 rows of 42 heads and 4 trees behind 401, where
+        // they are on the path, 43.4 -> 42.9 us against a division and a count for each tile)
+        int st = (2 * u0 + (warp - 10)) % ring, turn = warp - 10;     // stage; items since the first gathered one, mod ring
+        uint32_t go_ph = 0;
+        // skew: parity of a stage's turns so far, its earlier items that were gathered
         auto turn_of = [&](int item) -> uint32_t {
             uint32_t odd = 0;
 #pragma unroll 1
-            for (int i = item - ring; i >= k_item(u0); i -= ring) odd ^= uint32_t(!skew || (i & 1) || i == 0 || i >= v_item(u0));
+            for (int i = item - ring; i >= k_item(u0); i -= ring) odd ^= uint32_t((i & 1) || i == 0 || i >= v_item(u0));
             return odd;
         };
         // The first pass, while the tensor cores are at the prefix, only asks for the rows to be brought into L2: a
@@ -488,8 +492,11 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
                             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(src - lc * 8 + node[k] * row_stride + hf * 64));
                 continue;
             }
-            const int st = item_of(u) % ring;
-            if (!__all_sync(0xffffffffu, mbar_wait(bar_go + st * 8, turn_of(item_of(u)), a.status, qt))) break;
+            if (skew) {
+                st = item_of(u) % ring;
+                go_ph = turn_of(item_of(u));
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_go + st * 8, go_ph, a.status, qt))) break;
             const uint32_t dst = s_ring + st * TILE + (lc >> 3) * HALF;
 #pragma unroll 1
             for (int step = 0; step < QM / 16; ++step) {
@@ -508,6 +515,13 @@ prefix_umma_kernel(const AttnArgs a, const PrefixArgs pa, const __grid_constant_
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_full + st * 8) : "memory");
+            st += 2;
+            if (st >= ring) st -= ring;
+            turn += 2;
+            if (turn >= ring) {
+                turn -= ring;
+                go_ph ^= 1u;
+            }
         }
     } else {
         // ====== softmax: two groups of 128 threads, one thread per query row ======
