@@ -98,15 +98,15 @@ inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
 // items (128 query rows of one head), ratios of the mma.sync kernel's time (with the better of its tiles) to the other's; "bound"
 // is the ancestor bound in blocks:
 //   D 128, block_m 128   1.15 - 1.45 at 160 to 200 items, 1.19 - 2.03 above; 0.81 - 1.12 up to one item per SM
-//   D 128, block_m 64    bound 1: 0.91 - 1.09 up to 800, 1.04 - 1.10 above; bound 2 and 3: 0.91 - 0.96 at 160 to 200, 1.05 - 1.34 from 256;
-//                        bound 4 and up: 1.03 - 1.24 from 300 where the tree has 700 nodes and more (0.97 - 1.15 at 190 to 256, but 0.97
-//                        inside a decode step), 0.88 - 0.99 up to 512 with 512 nodes, 1.07 - 1.20 above
-//   D 128, block_m 32    64 slots: 0.90 - 0.99 up to 512, 1.02 - 1.25 above; longer lists 0.95 - 0.99 up to 1800, 1.01 from 2000; 0.73 - 0.88 with
-//                        a bound of 8 and up (the line at 200 to 300 items is where it was when the other kernel had 64-column
-//                        tiles there, 1.02 - 1.65)
+//   D 128, block_m 64    bound 1: 0.91 - 1.00 up to 512, 1.05 from 700; bound 2 and 3: 0.91 - 0.96 at 160 to 200, 1.02 - 1.40 from 256;
+//                        bound 4 and up: 1.03 - 1.41 from 300 where the tree has 700 nodes and more (0.97 - 1.15 at 190 to 256, but 0.97
+//                        inside a decode step), 0.88 - 1.00 up to 512 with 512 nodes, 1.10 - 1.25 above
+//   D 128, block_m 32    64 slots: 0.87 - 1.00 up to 512, 1.05 - 1.25 above; lists of 128: 0.94 at 320, 1.00 - 1.08 at 512, 1.04 - 1.18
+//                        above; 0.74 - 0.90 with 320 slots and up (the line at 200 to 300 items is where it was when the
+//                        other kernel had 64-column tiles there, 1.02 - 1.65)
 //   D 64, block_m 128    bound 1: 0.89 - 0.92 up to 256, 1.05 - 1.26 above; bound 2 and up: 0.98 - 1.18 from 160; 0.64 - 0.84 up to one per SM
-//   D 64, block_m 64     bound 1: 0.88 - 1.05 up to 1000, 1.06 - 1.11 above; bound 2 and 3: 1.07 - 1.38 from 512, 0.94 at 256; bound 4 and
-//                        up: 1.07 - 1.23 from 768, 0.88 - 1.07 below
+//   D 64, block_m 64     bound 1: 0.88 - 0.99 up to 700, 1.05 - 1.11 from 1000; bound 2 and 3: 1.07 - 1.38 from 512, 0.94 at 256; bound 4 and
+//                        up: 1.20 at 512 with 1024 nodes; with 512 nodes 0.90 there, 1.07 - 1.23 from 640
 //   D 64, block_m 32     64 slots: 1.08 - 1.32 from 700, 1.02 at 512; longer lists 1.00 at 2048, 0.91 - 0.95 below; 0.59 - 0.82 with a bound of 8 and up
 // Small grids are bound by one CTA's latency, which is longer here.  With one short tile of ancestors per 64 rows at
 // D 128 both kernels wait for the same HBM bytes and are within a few per cent of one another.
@@ -115,11 +115,11 @@ inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int
     const int bound = ma / bm;                        // tiles of ancestors the caller allows for
     if (D == 128) {
         if (bm == 128) return items >= 150;
-        if (bm == 64) return items >= (bound >= 4 ? (n_q >= 700 ? 300 : 800) : bound >= 2 ? 250 : 900);
-        return items >= 200 && (items <= 300 || (bound < 8 && items >= (bound >= 4 ? 2000 : 600)));
+        if (bm == 64) return items >= (bound >= 4 ? (n_q >= 700 ? 300 : 600) : bound >= 2 ? 250 : 650);
+        return items >= 200 && (items <= 300 || (bound < 8 && items >= (bound >= 4 ? 500 : 600)));
     }
     if (bm == 128) return items >= (bound >= 2 ? 150 : 300);
-    if (bm == 64) return items >= (bound >= 4 ? 700 : bound >= 2 ? 450 : 1200);
+    if (bm == 64) return items >= (bound >= 4 ? (n_q >= 700 ? 450 : 600) : bound >= 2 ? 450 : 1000);
     return bound < 8 && items >= (bound >= 4 ? 2000 : 700);
 }
 

@@ -29,7 +29,7 @@
 // group g.  Warp 10 loads Q and the own tiles, warps 11-14 gather (cp.async, 16 bytes a lane; TMA's gather4
 // fills the same layout but takes the engine about 100 cycles for its four rows, 6500 per item of 64
 // trees against the 5700 that its HBM bytes take), warp 15 stores O.  All tiles share one pool of 128-row
-// buffers (seven at D 128): warp 10 hands them out in item order - K, V, Q, gathered tiles (a narrow
+// buffers (seven at D 128): warp 10 hands them out in item order - K, Q, a gathered tile, V, the others (a narrow
 // tile's K and V in one buffer) - as they come free, in whatever order that is, so that the next items'
 // 96 KB are on their way while these are used up; O leaves through its item's Q buffer.
 //
@@ -50,17 +50,18 @@
 //
 // Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 82 -> 62 (4.3 TB/s
 // over Q, K, V and O); 64 x 300-node dynamic trees, D 128, block_m 128 380 -> 159; 16 x 1000-node deep
-// trees, D 64 120 -> 83; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2189 -> 1550.
+// trees, D 64 120 -> 83; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2189 -> 1340.
 // What bounds it is the chain of a group's round - product, softmax, (rescale,) product - and at D 128 the pool: a 96 KB item
 // in use, one on its way, and the last one's O.  Items of one tile run at HBM's rate (D 128: 83 us where 64 trees of
-// 256 nodes take 112; D 64: 1165 where the forest takes 1550), so a second round is what the rest pays for.
+// 256 nodes take 106; D 64: 1165 where the forest takes 1340), so the ancestors are what the rest pays for.
 //
-// Both tiles of an item in one round (Round::BOTH and SHARED): once through the chain, and nothing to rescale.  BOTH, for
-// bounds of up to 64: forest of 65532 nodes 1752 -> 1340 us, of 8188 and 16380 43 -> 35 and 227 -> 173.  SHARED, for bounds of up to 128, as
-// calls follow one another in a program: 64 x 256 nodes 110.2 -> 105.8, 4096-node deep tree 63.8 -> 61.8 (in graphs of one call they
-// are within 3 % of one another; two products of N 64 cost 102 cycles of tensor core where one of N 128 costs 64).  Not where
-// it lost: longer lists (dynamic trees of 1024 nodes, D 128 54.4 / 56.0; D 64, block_m 128, further rounds of 64 or 128
-// slots: 24.4 / 27.1 and 68 / 79), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118).
+// Both tiles of an item in one round (Round::BOTH and SHARED): once through the chain.  BOTH, for bounds of up to 64,
+// has nothing to rescale: forest of 65532 nodes 1752 -> 1340 us, of 8188 and 16380 43 -> 35 and 227 -> 173.  SHARED,
+// for bounds of up to 128, as calls follow one another in a program: 64 x 256 nodes 110.2 -> 105.8, 4096-node deep
+// tree 63.8 -> 61.8 (in graphs of one call they are within 3 % of one another; two products of N 64 cost 102 cycles of
+// tensor core where one of N 128 costs 64).  Not where it lost: longer lists (dynamic trees of 1024 nodes, D 128
+// 54.4 / 56.0; D 64, block_m 128, further rounds of 64 or 128 slots: 24.4 / 27.1 and 68 / 79), block_m 64 at D 64
+// (140 / 155), block_m 32 (104 / 118).
 // tree_umma_pays (fst_plan.h) has the line between the two kernels.
 #pragma once
 

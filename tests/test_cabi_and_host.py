@@ -332,3 +332,15 @@ def test_tree_kernel_of_short_blocks_with_long_lists(built_lib):
     umma, tma = _lib.KERNELS["tree_umma"], _lib.KERNELS["tma"]
     assert [kernel(n, 320) for n in (100, 256, 384, 1024, 4096)] == [tma, umma, tma, tma, tma]
     assert [kernel(n, 64) for n in (100, 256, 384, 1024, 4096)] == [tma, umma, tma, umma, umma]
+
+
+@pytest.mark.parametrize("D,bm,ma,n_q,line", [(128, 32, 128, 128, 500), (128, 64, 64, 256, 650), (128, 64, 320, 512, 600), (128, 64, 256, 1024, 300),
+                                              (64, 64, 64, 256, 1000), (64, 64, 256, 1024, 450), (64, 64, 320, 512, 600)])
+def test_tree_kernel_lines(built_lib, D, bm, ma, n_q, line):
+    """The tcgen05 kernel from the grid on where it was measured to be the faster one, whatever makes up the grid."""
+    from fstattention_b200 import _lib
+    per = n_q // 128
+    for heads in (-(-line // per), -(-line // per) - 1):
+        want = _lib.KERNELS["tree_umma" if heads * per >= line else "tma"]
+        assert _lib.lib().fst_attention_tree_kernel(1, heads, n_q, D, bm, ma) == want
+        assert _lib.lib().fst_attention_tree_kernel(heads, 1, n_q, D, bm, ma) == want
