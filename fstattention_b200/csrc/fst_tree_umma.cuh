@@ -48,20 +48,19 @@
 // When S(t) has landed every earlier product of the group has too (one thread issues them in order), so
 // the group may rescale O without asking.
 //
-// Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 82 -> 62 (4.3 TB/s
+// Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 84 -> 60 (4.5 TB/s
 // over Q, K, V and O); 64 x 300-node dynamic trees, D 128, block_m 128 380 -> 159; 16 x 1000-node deep
 // trees, D 64 120 -> 83; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2189 -> 1340.
 // What bounds it is the chain of a group's round - product, softmax, (rescale,) product - and at D 128 the pool: a 96 KB item
 // in use, one on its way, and the last one's O.  Items of one tile run at HBM's rate (D 128: 83 us where 64 trees of
-// 256 nodes take 106; D 64: 1165 where the forest takes 1340), so the ancestors are what the rest pays for.
+// 256 nodes take 92 to 113; D 64: 1165 where the forest takes 1340), so the ancestors are what the rest pays for.
 //
-// Both tiles of an item in one round (Round::BOTH and SHARED): once through the chain.  BOTH, for bounds of up to 64,
-// has nothing to rescale: forest of 65532 nodes 1752 -> 1340 us, of 8188 and 16380 43 -> 35 and 227 -> 173.  SHARED,
-// for bounds of up to 128, as calls follow one another in a program: 64 x 256 nodes 110.2 -> 105.8, 4096-node deep
-// tree 63.8 -> 61.8 (in graphs of one call they are within 3 % of one another; two products of N 64 cost 102 cycles of
-// tensor core where one of N 128 costs 64).  Not where it lost: longer lists (dynamic trees of 1024 nodes, D 128
-// 54.4 / 56.0; D 64, block_m 128, further rounds of 64 or 128 slots: 24.4 / 27.1 and 68 / 79), block_m 64 at D 64
-// (140 / 155), block_m 32 (104 / 118).
+// Both tiles of an item in one round (Round::BOTH), for bounds of up to 64 at D 64 and block_m 128: once through the
+// chain, and nothing to rescale: forest of 65532 nodes 1752 -> 1340 us, of 8188 and 16380 43 -> 35 and 227 -> 173.
+// Not where it lost: longer lists (dynamic trees of 1024 nodes, D 128 54.4 / 56.0; further rounds of 64 or 128 slots
+// 24.4 / 27.1 and 68 / 79), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118), nor at D 128 with block_m 64, where the
+// blocks of an item would share the columns of S (within 3 % of one another in graphs of one call, 1 to 3 % in a program): there
+// all weights of an item against one reference point cost 1.5 to 2.8 % in error.
 // tree_umma_pays (fst_plan.h) has the line between the two kernels.
 #pragma once
 
@@ -96,10 +95,8 @@ struct Geo {
 };
 
 // What one softmax takes.  TILE: a column tile.  BOTH: the two tiles of an item whose lists end in the first half of a
-// gathered tile (D 64, block_m 128: 128 + 64 of S's 192 columns).  SHARED: the own tile and the first gathered one, then
-// two gathered ones at a time, where the item's two blocks use the same columns of S, each product writing the lanes of its
-// block (D 128, block_m 64: 64 + 64 of 128 columns).
-enum class Round { TILE, BOTH, SHARED };
+// gathered tile (D 64, block_m 128: 128 + 64 of S's 192 columns).
+enum class Round { TILE, BOTH };
 
 // what the loading warp tells a group and its issuing thread about their next item
 struct ItemInfo {
@@ -162,11 +159,11 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
     using G = Geo<D>;
     constexpr bool BF16 = !std::is_same<T, __half>::value;
     constexpr int DH = D / 64, TILE = G::TILE, POOL = G::POOL;
-    constexpr bool BOTH = ROUND == Round::BOTH, SHARED = ROUND == Round::SHARED;
-    static_assert((!BOTH || (BM == 128 && D == 64)) && (!SHARED || (BM == 64 && D == 128)), "room in tensor memory for the columns of both tiles");
+    constexpr bool BOTH = ROUND == Round::BOTH;
+    static_assert(!BOTH || (BM == 128 && D == 64), "room in tensor memory for the columns of both tiles");
     constexpr int SUB = ROWS / BM;                        // blocks per item
     constexpr int NW = BM / 32;                           // mask words per row and tile
-    constexpr int EW = BOTH ? 2 : SHARED ? 2 * NW : NW;   // of them in the gathered tiles of a round
+    constexpr int EW = BOTH ? 2 : NW;                     // of them in a gathered tile
 
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     extern __shared__ unsigned char smem_raw[];
@@ -522,90 +519,6 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                         mma_commit(bar_empty + b1 * 8);
                     }
                     mma_commit(bar_o + g * 8);
-                } else if constexpr (SHARED) {
-                    auto one_buffer = [&](int t) { return in.z != 0 && t > 0 && t + 1 == tiles; };
-                    auto live = [&](int t, int s, int seg) -> int {   // 16-column steps of block s in tile t
-                        const int left = t == 0 ? min(own_rows - s * BM, BM) : min(cnt[s] - (t - 1) * BM, seg);
-                        return left > 0 ? (left + 15) >> 4 : 0;
-                    };
-                    // Every block's rows against its own columns, all blocks into the same columns of S (each its own lanes).
-                    // SEG: columns per block, BM or, where K and V share a buffer, BM / 2
-                    auto scores = [&](auto seg_c, int t, uint32_t to, uint64_t dks) {
-                        constexpr int SEG = decltype(seg_c)::value;
-#pragma unroll
-                        for (int s = 0; s < SUB; ++s) {
-                            const int steps = live(t, s, SEG);
-                            if (steps == 0) continue;
-                            const uint32_t idesc_s = instr_desc(BF16, false, 16 * steps);
-#pragma unroll
-                            for (int ks = 0; ks < D / 16; ++ks)
-                                mma_f16_block<BM>(to, dqs + uint64_t(((ks >> 2) * HALF + (ks & 3) * 32) >> 4),
-                                                  dks + uint64_t(((ks >> 2) * (SUB * SEG * 128) + (ks & 3) * 32 + s * SEG * 128) >> 4),
-                                                  idesc_s, ks > 0, s);
-                        }
-                    };
-                    auto output = [&](auto seg_c, int t, int col, uint64_t dvs) {
-                        constexpr int SEG = decltype(seg_c)::value;
-                        uint4 off[SEG / 16];
-#pragma unroll
-                        for (int ks = 0; ks < SEG / 16; ++ks) off[ks] = rows[(col >> 4) + ks];
-#pragma unroll
-                        for (int s = 0; s < SUB; ++s) {
-                            const int steps = live(t, s, SEG);
-#pragma unroll
-                            for (int ks = 0; ks < SEG / 16; ++ks)
-                                if (ks < steps)
-                                    mma_f16_ts_but(o_col, s_col + (col >> 1) + ks * 8, dvs + uint64_t(((s * SEG + ks * 16) * 128) >> 4), idesc_pv,
-                                                   not_block_rows<BM>(off[ks], s));
-                        }
-                    };
-                    using Full = std::integral_constant<int, BM>;
-                    using Part = std::integral_constant<int, BM / 2>;
-                    int at = in.y;                            // position of the round's first tile
-#pragma unroll 1
-                    for (int t0 = 0; t0 < tiles; ++round) {
-                        const int t1 = min(tiles, t0 == 0 ? 2 : t0 + 2);
-                        int p = at, col = 0;
-#pragma unroll 1
-                        for (int t = t0; t < t1; ++t) {
-                            alive = wait(full_of(g, p), full_parity(p), a.status, item);
-                            if (!alive) break;
-                            const int b = buf_of(g, p);
-                            const uint64_t dks = dk + uint64_t(b * (TILE >> 4));
-                            if (t > 0) fence_copied();
-                            fence_after_sync();
-                            const bool one = one_buffer(t);
-                            if (one) scores(Part{}, t, s_col + col, dks);
-                            else scores(Full{}, t, s_col + col, dks);
-                            if (t + 1 == t1) mma_commit(bar_s + g * 8);
-                            if (!one) mma_commit(bar_empty + b * 8);
-                            p += one ? 1 : 2;
-                            col += BM;
-                        }
-                        if (!alive) break;
-                        // (the first V tile is usually there long before P)
-                        alive = (one_buffer(t0) || wait(full_of(g, at + 1), full_parity(at + 1), a.status, item)) &&
-                                wait(bar_p + g * 8, round & 1, a.status, item);
-                        col = 0;
-#pragma unroll 1
-                        for (int t = t0; t < t1 && alive; ++t) {
-                            const bool one = one_buffer(t);
-                            at += one ? 0 : 1;
-                            alive = one || t == t0 || wait(full_of(g, at), full_parity(at), a.status, item);
-                            if (!alive) break;
-                            const int b = buf_of(g, at);
-                            ++at;
-                            if (t > 0) fence_copied();
-                            fence_after_sync();
-                            if (one) output(Part{}, t, col, dv_one + uint64_t(b * (TILE >> 4)));
-                            else output(Full{}, t, col, dv + uint64_t(b * (TILE >> 4)));
-                            mma_commit(bar_empty + b * 8);
-                            col += BM;
-                        }
-                        if (!alive) break;
-                        t0 = t1;
-                        if (t0 == tiles) mma_commit(bar_o + g * 8);
-                    }
                 } else {
                     // 16-column steps of tile t that some block has (bit ks: rows 16 ks .. of the buffer)
                     auto steps_of = [&](int t, int seg) -> uint32_t {
@@ -835,104 +748,6 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 tmem_st_wait();
                 fence_before_sync();
                 arrive(bar_p + g * 8);
-            } else if constexpr (SHARED) {
-#pragma unroll 1
-                for (int t = 0; t < tiles; ++round) {         // t: the round's first tile
-                    const bool first_round = t == 0;
-                    constexpr int WORDS = 2 * NW;
-                    uint32_t word[WORDS];                     // the round's columns that my row attends to
-#pragma unroll
-                    for (int i = 0; i < WORDS; ++i) {
-                        word[i] = !first_round ? ext[i % EW] : i < NW ? own[i % NW] : ext[(i - NW) % EW];
-                    }
-                    t += 2;
-                    // the words of the round after go out now: a loaded L2 answers late
-                    if (first_round) own_words(at_next, own);
-                    if (t >= tiles) ext_words(at_next, 0, ext);
-                    else ext_words(at, (t - 1) * NW, ext);
-                    alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, round & 1, a.status, item));
-                    if (!alive) break;
-                    fence_after_sync();
-
-                    uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
-                    {
-                        uint32_t on = 0;                      // lane k: rows of my warp with a column in 16 k ..
-#pragma unroll
-                        for (int i = 0; i < WORDS; ++i) {
-                            const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
-                            live |= uint32_t((lo | hi) != 0u) << i;
-                            if (lane == 2 * i) on = lo;
-                            if (lane == 2 * i + 1) on = hi;
-                        }
-                        if (lane < 2 * WORDS) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (G::COLS / 16) + lane) * 4 + (warp & 3)] = ~on;
-                    }
-                    float mu = 0.f, mx = -INFINITY;
-                    uint64_t sum2 = 0;
-                    // As above, but the reference point may move from round to round.
-                    bool second = false;
-#pragma unroll 1
-                    for (uint32_t rest = live; rest != 0u;) {
-                        uint32_t s[32];
-                        const int wi = __ffs(rest) - 1;       // the word's number
-                        rest &= rest - 1;
-                        uint32_t w = word[0];
-                        tmem_ld32(s, tmem_s + wi * 32);
-#pragma unroll
-                        for (int i = 1; i < WORDS; ++i) w = wi == i ? word[i] : w;
-                        tmem_ld_wait(s);
-                        float m2[2] = {mx, -INFINITY};
-#pragma unroll
-                        for (int c = 0; c < 32; c += 2) {
-                            s[c] = (w & (1u << c)) != 0u ? s[c] : 0xff800000u;
-                            s[c + 1] = (w & (2u << c)) != 0u ? s[c + 1] : 0xff800000u;
-                            m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[c]), __uint_as_float(s[c + 1])));
-                        }
-                        mx = fmaxf(m2[0], m2[1]);
-                        if (!second) {
-                            if (rest != 0u) continue;
-                            const bool up = mx > m_ref;
-                            if (__any_sync(0xffffffffu, up)) {
-                                if (!first_round) {           // rescale my row of O (the stores are awaited with P's)
-                                    const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
-#pragma unroll 1
-                                    for (int c0 = 0; c0 < D; c0 += 16) {
-                                        uint32_t o[16];
-                                        tmem_ld16(o, tmem_o + c0);
-#pragma unroll
-                                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                                        tmem_st16(tmem_o + c0, o);
-                                    }
-                                    l *= alpha;
-                                }
-                                if (up) m_ref = mx;
-                            }
-                            mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
-                            second = true;
-                            if ((live & (live - 1u)) != 0u) { // more than a turn: once again from the first
-                                rest = live;
-                                continue;
-                            }
-                        }
-                        const uint64_t scale2 = pair(c2, c2), shift2 = pair(-mu, -mu);
-                        uint32_t pk[16];
-#pragma unroll
-                        for (int c = 0; c < 32; c += 2) {
-                            float p0, p1;
-                            unpair(fma2(pair(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), scale2, shift2), p0, p1);
-                            p0 = fast_exp2(p0);
-                            p1 = fast_exp2(p1);
-                            sum2 = add2(sum2, pair(p0, p1));
-                            pk[c >> 1] = MT::pack(p0, p1);
-                        }
-                        tmem_st16(tmem_s + wi * 16, pk);
-                    }
-                    float sum[2];
-                    unpair(sum2, sum[0], sum[1]);
-                    l += sum[0] + sum[1];
-                    tmem_st_wait();
-                    fence_before_sync();
-                    arrive(bar_p + g * 8);
-                }
             } else {
 #pragma unroll 1
                 for (int t = 0; t < tiles; ++t, ++round) {
@@ -1129,10 +944,7 @@ cudaError_t launch_tree_umma_d(const AttnArgs &a, cudaStream_t stream) {
     using tree_umma::Round;
     switch (a.bm) {
         case 32: return launch_tree_umma_t<T, D, 32, Round::TILE>(a, stream);
-        case 64:
-            if constexpr (D == 128)
-                if (a.ma <= 128) return launch_tree_umma_t<T, D, 64, Round::SHARED>(a, stream);
-            return launch_tree_umma_t<T, D, 64, Round::TILE>(a, stream);
+        case 64: return launch_tree_umma_t<T, D, 64, Round::TILE>(a, stream);
         case 128:
             if constexpr (D == 64)
                 if (a.ma <= 64) return launch_tree_umma_t<T, D, 128, Round::BOTH>(a, stream);

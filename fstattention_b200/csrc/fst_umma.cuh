@@ -56,33 +56,11 @@ __device__ __forceinline__ void mma_f16_ts_rows(uint32_t d_tmem, uint32_t a_tmem
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%4, %5, %6, %7}, p;\n\t}\n"
                  ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(~rows.x), "r"(~rows.y), "r"(~rows.z), "r"(~rows.w) : "memory");
 }
-// rows of block `s` of a tile that has 128 / BM blocks of BM rows
-template <int BM>
-__device__ __forceinline__ uint4 block_rows(uint4 rows, int s) {
-    return make_uint4(0 / BM == s ? rows.x : 0u, 32 / BM == s ? rows.y : 0u, 64 / BM == s ? rows.z : 0u, 96 / BM == s ? rows.w : 0u);
-}
-// and all rows but those of `rows` that are block `s`'s
-template <int BM>
-__device__ __forceinline__ uint4 not_block_rows(uint4 off, int s) {
-    return make_uint4(0 / BM == s ? off.x : ~0u, 32 / BM == s ? off.y : ~0u, 64 / BM == s ? off.z : ~0u, 96 / BM == s ? off.w : ~0u);
-}
 // A from tensor memory; rows whose bit is set in `off` keep their D
 __device__ __forceinline__ void mma_f16_ts_but(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint4 off) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%4, %5, %6, %7}, p;\n\t}\n"
                  ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(off.x), "r"(off.y), "r"(off.z), "r"(off.w) : "memory");
-}
-// A from shared memory, into the lanes of block `s` only
-template <int BM>
-__device__ __forceinline__ void mma_f16_block(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate, int s) {
-    if constexpr (BM == 128) {
-        mma_f16(d_tmem, a_desc, b_desc, idesc, accumulate);
-    } else {
-        const uint4 rows = block_rows<BM>(make_uint4(~0u, ~0u, ~0u, ~0u), s);
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
-                     ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(uint32_t(accumulate)), "r"(~rows.x), "r"(~rows.y), "r"(~rows.z), "r"(~rows.w) : "memory");
-    }
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");

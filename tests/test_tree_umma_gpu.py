@@ -63,8 +63,8 @@ def test_tree_umma_many_items_strided(fst, D, bm):
 @pytest.mark.parametrize("own", ["alone", "chained", "across"])
 @pytest.mark.parametrize("n,teeth", [(77, 1), (129, 20), (300, 16), (640, 17), (300, 32), (300, 33), (640, 64), (640, 65), (640, 97), (650, 128)])
 def test_tree_umma_merged_round(fst, D, bm, own, n, teeth):
-    """Both tiles of an item in one softmax (D 64, block_m 128, bounds of up to 64; D 128, block_m 64, bounds of up to 128;
-    longer bounds take the same trees tile by tile): lists that end in any 16-column step or fill the tile; rows that attend to nobody in their block but
+    """Both tiles of an item in one softmax (D 64, block_m 128, bounds of up to 64; longer bounds, and D 128 with block_m 64, take
+    the same trees tile by tile): lists that end in any 16-column step or fill the tile; rows that attend to nobody in their block but
     themselves, to their neighbours, and to a column in another 32-column word that nobody else uses.  A value that
     is not finite stays with the rows that attend to it or to one of its fifteen neighbours."""
     par = comb(n, teeth)
@@ -124,6 +124,32 @@ def test_tree_umma_rounds_like_the_other_kernel(fst, D, bm, dtype):
         o = fst.fst_attention(q.cuda(), k.cuda(), v.cuda(), meta, sm_scale=D ** -0.5, kernel=kernel).cpu().double()
         err[kernel] = (o - want).norm().item() / want.norm().item()
     assert err["tree_umma"] <= 1.04 * err["tma"], err
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,bm", [(128, 64)])
+def test_tree_umma_bound_changes_no_bit(fst, D, bm, dtype):
+    """The bound says how long lists may be, not how they are rounded: the own tile's weights are against its own
+    largest score, an ancestor tile's against the largest so far, with short bounds as with long ones.  (All
+    weights of an item against one reference point were 1.2 to 2.8 % further from 64 bits.)"""
+    trees = [fst.parent_from_lineage(*fst.create_tree(7)).tolist(), comb(300, 20), comb(129, 1), comb(640, 60), comb(77, 33)]
+    trees.append([-1] + [(i - 1) // 3 if i % 5 else i - 1 for i in range(1, 500)])
+    compared = 0
+    for par in trees:
+        g = torch.Generator(device="cuda").manual_seed(len(par))
+        q, k, v = (torch.randn((2, 24, len(par), D), generator=g, device="cuda").to(dtype) for _ in range(3))
+        want = None
+        for bound in (256, 128, 64):
+            try:
+                meta = fst.build_tree_metadata(par, bm, bound, reference_format=False)
+            except RuntimeError:                          # the tree needs more
+                continue
+            got = fst.fst_attention(q, k, v, meta, sm_scale=D ** -0.5, kernel="tree_umma", return_lse=True)
+            if want is not None:
+                assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), (len(par), bound)
+                compared += bound == 64
+            want = want or got
+    assert compared >= 4 and fst.last_status() == 0
 
 
 def reaches(par, lo, hi):
