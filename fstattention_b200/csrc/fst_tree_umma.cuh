@@ -12,7 +12,7 @@
 //            the item's own rows (contiguous, TMA boxes); tile t > 0 holds ancestor slots
 //            [(t-1) BM, t BM) of every block (gathered row by row; padding slots are zeros).  The last
 //            tile is narrow - BM / 2 columns for each block - when the lists end in its first half.
-//   round    the tiles that one softmax takes (see Round)
+//   round    the tiles whose scores are computed at once (see Round)
 //   S = Q K^T     M 128, N 128 (64), both operands in shared memory (128-byte swizzle)
 //   softmax       thread r of a group owns row r and looks only at its block's columns; 32-column
 //                 words in which no row of its warp has a mask bit are not even read; P goes back
@@ -44,23 +44,25 @@
 // The exponent's reference point is the row's largest score so far; when a later tile has a larger one, O is
 // rescaled in tensor memory.  So the weight that dominates a row is exactly 1 and loses nothing when P is
 // rounded to 16 bits, as in attn_tma_kernel: errors against 64 bits over six kinds of trees are 1.000 of that
-// kernel's (0.991 - 1.008).  Moving it only past 2^8 saved 2 to 3 % of the time and cost 9 to 20 % in error.
+// kernel's (0.991 - 1.008; 1.002 - 1.006 where the scores of both tiles come at once).  Moving it only past 2^8 saved
+// 2 to 3 % of the time and cost 9 to 20 % in error.
 // When S(t) has landed every earlier product of the group has too (one thread issues them in order), so
-// the group may rescale O without asking.
+// the group may rescale O without asking; where S(1) comes with S(0) it asks bar_m.
 //
 // Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 84 -> 60 (4.5 TB/s
-// over Q, K, V and O); 64 x 300-node dynamic trees, D 128, block_m 128 380 -> 159; 16 x 1000-node deep
-// trees, D 64 120 -> 83; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2189 -> 1340.
+// over Q, K, V and O); 64 x 300-node dynamic trees, D 128, block_m 128 381 -> 146; 16 x 1000-node deep
+// trees, D 64 120 -> 82; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2190 -> 1403.
 // What bounds it is the chain of a group's round - product, softmax, (rescale,) product - and at D 128 the pool: a 96 KB item
 // in use, one on its way, and the last one's O.  Items of one tile run at HBM's rate (D 128: 83 us where 64 trees of
-// 256 nodes take 92 to 113; D 64: 1165 where the forest takes 1340), so the ancestors are what the rest pays for.
+// 256 nodes take 101; D 64: 1165 where the forest takes 1403), so the ancestors are what the rest pays for.
 //
-// Both tiles of an item in one round (Round::BOTH), for bounds of up to 64 at D 64 and block_m 128: once through the
-// chain, and nothing to rescale: forest of 65532 nodes 1752 -> 1340 us, of 8188 and 16380 43 -> 35 and 227 -> 173.
-// Not where it lost: longer lists (dynamic trees of 1024 nodes, D 128 54.4 / 56.0; further rounds of 64 or 128 slots
-// 24.4 / 27.1 and 68 / 79), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118), nor at D 128 with block_m 64, where the
-// blocks of an item would share the columns of S (within 3 % of one another in graphs of one call, 1 to 3 % in a program): there
-// all weights of an item against one reference point cost 1.5 to 2.8 % in error.
+// The scores of both tiles of an item at once (Round::BOTH), for bounds of up to 64 at D 64 and block_m 128: their columns
+// fit beside one another, so the second tile's are there when the softmax of the first is done, and the first's product
+// with V runs under the second's exponentials: forest of 65532 nodes 1745 -> 1403 us, of 8188 217 -> 179.  The
+// roundings are those of the tiles one by one.  One softmax over both (1332 us) rounded the own tile's largest weight too,
+// 1.2 to 2.8 % more error; with the second tile's output in columns of its own, scaled when O is read, it had the
+// error of now and the speed, but not the bits.  One softmax lost elsewhere: longer lists (dynamic trees of 1024 nodes, D 128
+// 54.4 / 56.0; further rounds of 64 or 128 slots 24.4 / 27.1 and 68 / 79), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118).
 // tree_umma_pays (fst_plan.h) has the line between the two kernels.
 #pragma once
 
@@ -86,7 +88,7 @@ struct Geo {
     static constexpr int POOL = D == 128 ? 7 : 14;            // tile buffers
     static constexpr int COLS = 256 - D;                      // columns of S: 2 x (COLS + D) are all of tensor memory
     static constexpr int OFF_BAR = POOL * TILE;
-    static constexpr int N_BAR = 2 * POSITIONS + POOL + TURNS + 2 * ITEMS + 6;
+    static constexpr int N_BAR = 2 * POSITIONS + POOL + TURNS + 2 * ITEMS + 8;
     static constexpr int OFF_INFO = OFF_BAR + (N_BAR + 1) / 2 * 16;   // ItemInfo per item in flight
     static constexpr int OFF_ROWS = OFF_INFO + ITEMS * 32;            // [group][16 columns of S][warp] rows with a column there
     static constexpr int OFF_WHERE = OFF_ROWS + 2 * COLS;             // which buffer a position's tile is in; then the TMEM address
@@ -94,7 +96,7 @@ struct Geo {
     static_assert(SMEM_BYTES <= 227 * 1024, "one CTA's shared memory");
 };
 
-// What one softmax takes.  TILE: a column tile.  BOTH: the two tiles of an item whose lists end in the first half of a
+// What one round of scores takes.  TILE: a column tile.  BOTH: the two tiles of an item whose lists end in the first half of a
 // gathered tile (D 64, block_m 128: 128 + 64 of S's 192 columns).
 enum class Round { TILE, BOTH };
 
@@ -171,7 +173,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
     unsigned char *smem = smem_raw + (s_base - smem_u32(smem_raw));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar_full = s_base + G::OFF_BAR, bar_empty = bar_full + 2 * POSITIONS * 8, bar_go = bar_empty + POOL * 8,
-                   bar_q = bar_go + TURNS * 8, bar_ob = bar_q + ITEMS * 8, bar_s = bar_ob + ITEMS * 8, bar_p = bar_s + 16, bar_o = bar_s + 32;
+                   bar_q = bar_go + TURNS * 8, bar_ob = bar_q + ITEMS * 8, bar_s = bar_ob + ITEMS * 8, bar_p = bar_s + 16, bar_o = bar_s + 32, bar_m = bar_s + 48;
     int4 *info = reinterpret_cast<int4 *>(smem + G::OFF_INFO);        // ItemInfo, read and written in two halves
     volatile unsigned char *buf_at = smem + G::OFF_WHERE;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + G::OFF_WHERE + 2 * POSITIONS);
@@ -184,6 +186,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             mbar_init(bar_s + i * 8, 1);
             mbar_init(bar_p + i * 8, ROWS);
             mbar_init(bar_o + i * 8, 1);
+            mbar_init(bar_m + i * 8, 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -475,7 +478,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
 #pragma unroll
                 for (int s = 0; s < SUB; ++s) cnt[s] = four[s];
                 if constexpr (BOTH) {
-                    // the own tile and, when there are ancestors, one narrow tile: both products of S, the softmax, both of O
+                    // the own tile and, when there are ancestors, one narrow tile: both products of S, then those of O as P comes
                     const int at = in.y, steps0 = min((own_rows + 15) >> 4, ROWS / 16), steps1 = (cnt[0] + 15) >> 4;
                     alive = wait(full_of(g, at), full_parity(at), a.status, item);
                     if (!alive) break;
@@ -515,6 +518,11 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                     output(std::integral_constant<int, 8>{}, 0, dv + uint64_t(b * (TILE >> 4)), steps0);
                     mma_commit(bar_empty + b * 8);
                     if (tiles > 1) {
+                        mma_commit(bar_m + g * 8);        // O may be rescaled
+                        alive = wait(bar_p + g * 8, round & 1, a.status, item);
+                        if (!alive) break;
+                        ++round;
+                        fence_after_sync();
                         output(std::integral_constant<int, 4>{}, BM, dv_one + uint64_t(b1 * (TILE >> 4)), steps1);
                         mma_commit(bar_empty + b1 * 8);
                     }
@@ -623,7 +631,7 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
         if (a.meta_stable) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
         bool alive = true;
-        int round = 0, n = g;
+        int round = 0, pairs = 0, n = g;                  // tiles, items with a second one (BOTH) so far; item number
 #pragma unroll 1
         for (int item = blockIdx.x + g * stride; item < ta.n_items; item += 2 * stride, n += 2) {
             const Where at_next = plus(at, step);
@@ -637,229 +645,160 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
             for (int c = 0; c < 16; ++c) zero[c] = 0u;
 #pragma unroll 1
             for (int c0 = 0; c0 < D; c0 += 16) tmem_st16(tmem_o + c0, zero);
-            if constexpr (BOTH) {
-                constexpr int WORDS = NW + EW;
-                uint32_t word[WORDS];                     // the columns that my row attends to: its own block's, its ancestors'
+#pragma unroll 1
+            for (int t = 0; t < tiles; ++t, ++round) {
+                uint32_t word[NW];
 #pragma unroll
-                for (int i = 0; i < WORDS; ++i) word[i] = i < NW ? own[i % NW] : ext[(i - NW) % EW];
-                own_words(at_next, own);                  // the next item's go out now: a loaded L2 answers late
-                ext_words(at_next, 0, ext);
-                alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, round & 1, a.status, item));
-                if (!alive) break;
-                ++round;
-                fence_after_sync();
+                for (int i = 0; i < NW; ++i) word[i] = t == 0 ? own[i] : i < EW ? ext[i % EW] : 0u;
+                // the words of the tile after next go out now: a loaded L2 answers late
+                const bool last_tile = t + 1 == tiles;
+                if (t == 0) own_words(at_next, own);
+                if (t > 0 || last_tile) ext_words(last_tile ? at_next : at, last_tile ? 0 : t * NW, ext);
+                const bool narrow = in.z != 0 && last_tile;
+                const int segw = narrow ? NW / 2 : NW;    // my block's words in this tile; words past them are empty
+                const int col_my = BOTH ? t * BM : sub * segw * 32;
+                const uint32_t tmem_my = tmem_s + col_my;
+                if (!BOTH || t == 0) {
+                    alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, (BOTH ? n >> 1 : round) & 1, a.status, item));
+                    if (!alive) break;
+                    fence_after_sync();
+                }
 
-                uint32_t live = 0, lone_words = 0;        // bit i: some row of my warp has a bit in word i; no row has two
+                uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
                 {
-                    uint32_t on = 0;                      // lane k: rows of my warp with a column in 16 k ..
+                    uint32_t on = 0;                      // lane k: rows of my warp with a column in step k of the tile
+                    const int k = BOTH ? lane : lane - (col_my >> 4);
 #pragma unroll
-                    for (int i = 0; i < WORDS; ++i) {
+                    for (int i = 0; i < NW; ++i) {
                         const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
                         live |= uint32_t((lo | hi) != 0u) << i;
-                        if (i < NW && (lo | hi) != 0u && __ballot_sync(0xffffffffu, (word[i] & (word[i] - 1u)) != 0u) == 0u) lone_words |= 1u << i;
-                        if (lane == 2 * i) on = lo;
-                        if (lane == 2 * i + 1) on = hi;
+                        if (k == 2 * i) on = lo;
+                        if (k == 2 * i + 1) on = hi;
                     }
-                    if (lane < 2 * WORDS) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (G::COLS / 16) + lane) * 4 + (warp & 3)] = ~on;
+                    if constexpr (BOTH) {
+                        if (lane < (t == 0 ? 8 : 4)) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (G::COLS / 16) + t * 8 + lane) * 4 + (warp & 3)] = ~on;
+                    } else if (lane < 8) {
+                        reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (G::COLS / 16) + lane) * 4 + (warp & 3)] = on;
+                    }
                 }
-                float mu = 0.f, mx = -INFINITY;
-                uint64_t sum2 = 0;
-                // A word in which every row has one column at most - a block's own word where the tree is numbered breadth first and
-                // a row attends to nobody in its block but itself - needs no 32 exponentials: the score is picked out (forest of 65532
-                // nodes 1615 -> 1550 us).
-                int lone = -1, lone_at = -1;              // that word, my row's column in it
-                if (lone_words != 0u) {
-                    lone = __ffs(lone_words) - 1;
-                    live &= ~(1u << lone);
-                    uint32_t v[32], w = word[0];
+                float sum[2] = {0.f, 0.f}, mu = 0.f, mx = -INFINITY;
+                // My live words, WT to a turn.  First round: the row's maximum, then the reference point.  Second round (or
+                // at once, when one turn was all): probabilities, over S - word i of P covers columns 16 i .. of S,
+                // below the words still to be read; words nobody uses are zeros.  One loop and one copy of its
+                // code: what runs once per tile and does not stay in the instruction cache costs more than it saves
+                // (two words to a turn at block_m 128: 1760 -> 1892 us on the forest of 65532 nodes; both words of
+                // a row in one turn at block_m 64: 69.0 -> 67.5 us on the deep tree).
+                constexpr int WT = NW == 2 ? 2 : 1;
+                bool second = false, settled = !BOTH || t == 0;       // the earlier products of O have landed
+                if constexpr (BOTH) {
+                    // A row that attends to nobody in its block but itself, as where the tree is numbered breadth first, needs no 32
+                    // exponentials: where one word is all that a warp has, and one column of it all that a row has, the score is
+                    // picked out (forest of 65532 nodes 1615 -> 1550 us).
+                    uint32_t w = word[0];
 #pragma unroll
-                    for (int i = 1; i < NW; ++i) w = lone == i ? word[i] : w;
-                    tmem_ld32(v, tmem_s + lone * 32);
-                    lone_at = __ffs(w) - 1;
-                    tmem_ld_wait(v);
+                    for (int i = 1; i < NW; ++i) w |= word[i];
+                    if (t == 0 && live != 0u && (live & (live - 1u)) == 0u && __ballot_sync(0xffffffffu, (w & (w - 1u)) != 0u) == 0u) {
+                        const int wi = __ffs(live) - 1, at_c = __ffs(w) - 1;
+                        uint32_t v[32], pk[16];
+                        tmem_ld32(v, tmem_my + wi * 32);
+                        tmem_ld_wait(v);
 #pragma unroll
-                    for (int half = 16; half > 0; half /= 2)
+                        for (int half = 16; half > 0; half /= 2)
 #pragma unroll
-                        for (int c = 0; c < half; ++c) v[c] = (lone_at & half) != 0 ? v[c + half] : v[c];
-                    mx = lone_at < 0 ? -INFINITY : __uint_as_float(v[0]);
+                            for (int c = 0; c < half; ++c) v[c] = (at_c & half) != 0 ? v[c + half] : v[c];
+                        const float score = at_c < 0 ? -INFINITY : __uint_as_float(v[0]);
+                        m_ref = fmaxf(m_ref, score);
+                        const float p = fast_exp2(fmaf(score, c2, m_ref == -INFINITY ? 0.f : -(m_ref * c2)));
+                        const uint32_t both = (at_c & 1) != 0 ? MT::pack(0.f, p) : MT::pack(p, 0.f);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) pk[i] = at_c >> 1 == i ? both : 0u;
+                        tmem_st16(tmem_my + wi * 16, pk);
+                        sum[0] = p;
+                        live = 0u;
+                    }
                 }
-                const float lone_score = mx;
-                // My live words, one to a turn (two spill).  First time through: the row's maximum, which is the reference
-                // point.  Second time (or at once, when one turn was all): probabilities, over S - word i of P covers
-                // columns 16 i .. of S, below the words still to be read.
-                bool second = false;
 #pragma unroll 1
-                for (uint32_t rest = live; !second || rest != 0u;) {
-                    uint32_t s[32];
-                    const int wi = __ffs(rest) - 1;       // the word's number, -1: none but the lone one
-                    rest &= rest - 1;
-                    if (wi >= 0) {
-                        uint32_t w = word[0];
-                        tmem_ld32(s, tmem_s + wi * 32);
+                for (uint32_t rest = live; rest != 0u;) {
+                    uint32_t s[WT][32];
+                    int wi[WT];                           // the words' numbers; NW: none
 #pragma unroll
-                        for (int i = 1; i < WORDS; ++i) w = wi == i ? word[i] : w;
-                        tmem_ld_wait(s);
-                        float m2[2] = {mx, -INFINITY};
+                    for (int k = 0; k < WT; ++k) {
+                        wi[k] = WT == 1 || rest != 0u ? __ffs(rest) - 1 : NW;
+                        rest &= rest - 1;
+                        if (WT == 1 || wi[k] < NW) tmem_ld32(s[k], tmem_my + wi[k] * 32);
+                    }
+                    float m = -INFINITY;
+#pragma unroll
+                    for (int k = 0; k < WT; ++k) {
+                        if (WT > 1 && wi[k] >= NW) continue;
+                        uint32_t w = word[0];
+#pragma unroll
+                        for (int i = 1; i < NW; ++i) w = wi[k] == i ? word[i] : w;
+                        tmem_ld_wait(s[k]);
+                        float m2[2] = {-INFINITY, -INFINITY};
 #pragma unroll
                         for (int c = 0; c < 32; c += 2) {
-                            s[c] = (w & (1u << c)) != 0u ? s[c] : 0xff800000u;
-                            s[c + 1] = (w & (2u << c)) != 0u ? s[c + 1] : 0xff800000u;
-                            m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[c]), __uint_as_float(s[c + 1])));
+                            s[k][c] = (w & (1u << c)) != 0u ? s[k][c] : 0xff800000u;
+                            s[k][c + 1] = (w & (2u << c)) != 0u ? s[k][c + 1] : 0xff800000u;
+                            m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[k][c]), __uint_as_float(s[k][c + 1])));
                         }
-                        mx = fmaxf(m2[0], m2[1]);
+                        m = fmaxf(m, fmaxf(m2[0], m2[1]));
                     }
                     if (!second) {
+                        mx = fmaxf(mx, m);
                         if (rest != 0u) continue;
-                        m_ref = mx;
+                        const bool up = mx > m_ref;
+                        if (!settled) {
+                            settled = true;
+                            alive = __all_sync(0xffffffffu, wait(bar_m + g * 8, pairs & 1, a.status, item));
+                            fence_after_sync();
+                        }
+                        if (__any_sync(0xffffffffu, up)) {
+                            if (t > 0) {                  // rescale my row of O (the stores are awaited with P's)
+                                const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
+#pragma unroll 1
+                                for (int c0 = 0; c0 < D; c0 += 16) {
+                                    uint32_t o[16];
+                                    tmem_ld16(o, tmem_o + c0);
+#pragma unroll
+                                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                                    tmem_st16(tmem_o + c0, o);
+                                }
+                                l *= alpha;
+                            }
+                            if (up) m_ref = mx;
+                        }
                         mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
                         second = true;
-                        if ((live & (live - 1u)) != 0u) { // more than a turn: once again from the first
+                        if (WT < NW && __popc(live) > WT) {       // more than a turn: once again from the first
                             rest = live;
                             continue;
                         }
                     }
-                    if (wi >= 0) {
-                        const uint64_t scale2 = pair(c2, c2), shift2 = pair(-mu, -mu);
+#pragma unroll
+                    for (int k = 0; k < WT; ++k) {
+                        if (WT > 1 && wi[k] >= NW) continue;
                         uint32_t pk[16];
 #pragma unroll
                         for (int c = 0; c < 32; c += 2) {
-                            float p0, p1;
-                            unpair(fma2(pair(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), scale2, shift2), p0, p1);
-                            p0 = fast_exp2(p0);
-                            p1 = fast_exp2(p1);
-                            sum2 = add2(sum2, pair(p0, p1));
+                            const float p0 = fast_exp2(fmaf(__uint_as_float(s[k][c]), c2, -mu));
+                            const float p1 = fast_exp2(fmaf(__uint_as_float(s[k][c + 1]), c2, -mu));
+                            sum[0] += p0;
+                            sum[1] += p1;
                             pk[c >> 1] = MT::pack(p0, p1);
                         }
-                        tmem_st16(tmem_s + wi * 16, pk);
+                        tmem_st16(tmem_s + (col_my >> 1) + wi[k] * 16, pk);
                     }
                 }
-                if (lone >= 0) {
-                    const float p = fast_exp2(fmaf(lone_score, c2, -mu));
-                    const uint32_t v = (lone_at & 1) != 0 ? MT::pack(0.f, p) : MT::pack(p, 0.f);
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) pk[i] = lone_at >> 1 == i ? v : 0u;
-                    tmem_st16(tmem_s + lone * 16, pk);
-                    l += p;
+                if (!settled) {                           // no row of my warp has ancestors, but it keeps step with the barrier
+                    alive = __all_sync(0xffffffffu, wait(bar_m + g * 8, pairs & 1, a.status, item));
                 }
-                float sum[2];
-                unpair(sum2, sum[0], sum[1]);
+                if (!alive) break;
+                pairs += int(BOTH && t > 0);
                 l += sum[0] + sum[1];
                 tmem_st_wait();
                 fence_before_sync();
                 arrive(bar_p + g * 8);
-            } else {
-#pragma unroll 1
-                for (int t = 0; t < tiles; ++t, ++round) {
-                    uint32_t word[NW];
-#pragma unroll
-                    for (int i = 0; i < NW; ++i) word[i] = t == 0 ? own[i] : ext[i];
-                    // the words of the tile after next go out now: a loaded L2 answers late
-                    const bool last_tile = t + 1 == tiles;
-                    if (t == 0) own_words(at_next, own);
-                    if (t > 0 || last_tile) ext_words(last_tile ? at_next : at, last_tile ? 0 : t * NW, ext);
-                    const bool narrow = in.z != 0 && last_tile;
-                    const int segw = narrow ? NW / 2 : NW;    // my block's words in this tile; words past them are empty
-                    const uint32_t tmem_my = tmem_s + sub * segw * 32;
-                    alive = __all_sync(0xffffffffu, wait(bar_s + g * 8, round & 1, a.status, item));
-                    if (!alive) break;
-                    fence_after_sync();
-
-                    uint32_t live = 0;                        // bit i: some row of my warp has a bit in word i
-                    {
-                        uint32_t on = 0;                      // lane k: rows of my warp with a column in step k of the tile
-                        const int k = lane - sub * segw * 2;
-#pragma unroll
-                        for (int i = 0; i < NW; ++i) {
-                            const uint32_t lo = __ballot_sync(0xffffffffu, (word[i] & 0xffffu) != 0u), hi = __ballot_sync(0xffffffffu, word[i] > 0xffffu);
-                            live |= uint32_t((lo | hi) != 0u) << i;
-                            if (k == 2 * i) on = lo;
-                            if (k == 2 * i + 1) on = hi;
-                        }
-                        if (lane < 8) reinterpret_cast<uint32_t *>(smem + G::OFF_ROWS)[(g * (G::COLS / 16) + lane) * 4 + (warp & 3)] = on;
-                    }
-                    float sum[2] = {0.f, 0.f}, mu = 0.f, mx = -INFINITY;
-                    // My live words, WT to a turn.  First round: the row's maximum, then the reference point.  Second round (or
-                    // at once, when one turn was all): probabilities, over S - word i of P covers columns 16 i .. of S,
-                    // below the words still to be read; words nobody uses are zeros.  One loop and one copy of its
-                    // code: what runs once per tile and does not stay in the instruction cache costs more than it saves
-                    // (two words to a turn at block_m 128: 1760 -> 1892 us on the forest of 65532 nodes; both words of
-                    // a row in one turn at block_m 64: 69.0 -> 67.5 us on the deep tree).
-                    constexpr int WT = NW == 2 ? 2 : 1;
-                    bool second = false;
-#pragma unroll 1
-                    for (uint32_t rest = live; rest != 0u;) {
-                        uint32_t s[WT][32];
-                        int wi[WT];                           // the words' numbers; NW: none
-#pragma unroll
-                        for (int k = 0; k < WT; ++k) {
-                            wi[k] = WT == 1 || rest != 0u ? __ffs(rest) - 1 : NW;
-                            rest &= rest - 1;
-                            if (WT == 1 || wi[k] < NW) tmem_ld32(s[k], tmem_my + wi[k] * 32);
-                        }
-                        float m = -INFINITY;
-#pragma unroll
-                        for (int k = 0; k < WT; ++k) {
-                            if (WT > 1 && wi[k] >= NW) continue;
-                            uint32_t w = word[0];
-#pragma unroll
-                            for (int i = 1; i < NW; ++i) w = wi[k] == i ? word[i] : w;
-                            tmem_ld_wait(s[k]);
-                            float m2[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-                            for (int c = 0; c < 32; c += 2) {
-                                s[k][c] = (w & (1u << c)) != 0u ? s[k][c] : 0xff800000u;
-                                s[k][c + 1] = (w & (2u << c)) != 0u ? s[k][c + 1] : 0xff800000u;
-                                m2[(c >> 1) & 1] = fmaxf(m2[(c >> 1) & 1], fmaxf(__uint_as_float(s[k][c]), __uint_as_float(s[k][c + 1])));
-                            }
-                            m = fmaxf(m, fmaxf(m2[0], m2[1]));
-                        }
-                        if (!second) {
-                            mx = fmaxf(mx, m);
-                            if (rest != 0u) continue;
-                            const bool up = mx > m_ref;
-                            if (__any_sync(0xffffffffu, up)) {
-                                if (t > 0) {                  // rescale my row of O (the stores are awaited with P's)
-                                    const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
-#pragma unroll 1
-                                    for (int c0 = 0; c0 < D; c0 += 16) {
-                                        uint32_t o[16];
-                                        tmem_ld16(o, tmem_o + c0);
-#pragma unroll
-                                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                                        tmem_st16(tmem_o + c0, o);
-                                    }
-                                    l *= alpha;
-                                }
-                                if (up) m_ref = mx;
-                            }
-                            mu = m_ref == -INFINITY ? 0.f : m_ref * c2;
-                            second = true;
-                            if (WT < NW && __popc(live) > WT) {       // more than a turn: once again from the first
-                                rest = live;
-                                continue;
-                            }
-                        }
-#pragma unroll
-                        for (int k = 0; k < WT; ++k) {
-                            if (WT > 1 && wi[k] >= NW) continue;
-                            uint32_t pk[16];
-#pragma unroll
-                            for (int c = 0; c < 32; c += 2) {
-                                const float p0 = fast_exp2(fmaf(__uint_as_float(s[k][c]), c2, -mu));
-                                const float p1 = fast_exp2(fmaf(__uint_as_float(s[k][c + 1]), c2, -mu));
-                                sum[0] += p0;
-                                sum[1] += p1;
-                                pk[c >> 1] = MT::pack(p0, p1);
-                            }
-                            tmem_st16(tmem_s + (sub * segw + wi[k]) * 16, pk);
-                        }
-                    }
-                    l += sum[0] + sum[1];
-                    tmem_st_wait();
-                    fence_before_sync();
-                    arrive(bar_p + g * 8);
-                }
             }
             if (!alive) break;
 

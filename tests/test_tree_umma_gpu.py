@@ -63,8 +63,8 @@ def test_tree_umma_many_items_strided(fst, D, bm):
 @pytest.mark.parametrize("own", ["alone", "chained", "across"])
 @pytest.mark.parametrize("n,teeth", [(77, 1), (129, 20), (300, 16), (640, 17), (300, 32), (300, 33), (640, 64), (640, 65), (640, 97), (650, 128)])
 def test_tree_umma_merged_round(fst, D, bm, own, n, teeth):
-    """Both tiles of an item in one softmax (D 64, block_m 128, bounds of up to 64; longer bounds, and D 128 with block_m 64, take
-    the same trees tile by tile): lists that end in any 16-column step or fill the tile; rows that attend to nobody in their block but
+    """The scores of both tiles of an item at once (D 64, block_m 128, bounds of up to 64; longer bounds, and D 128 with block_m 64,
+    take the same trees tile by tile): lists that end in any 16-column step or fill the tile; rows that attend to nobody in their block but
     themselves, to their neighbours, and to a column in another 32-column word that nobody else uses.  A value that
     is not finite stays with the rows that attend to it or to one of its fifteen neighbours."""
     par = comb(n, teeth)
@@ -127,7 +127,7 @@ def test_tree_umma_rounds_like_the_other_kernel(fst, D, bm, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("D,bm", [(128, 64)])
+@pytest.mark.parametrize("D,bm", [(128, 64), (64, 128)])
 def test_tree_umma_bound_changes_no_bit(fst, D, bm, dtype):
     """The bound says how long lists may be, not how they are rounded: the own tile's weights are against its own
     largest score, an ancestor tile's against the largest so far, with short bounds as with long ones.  (All
