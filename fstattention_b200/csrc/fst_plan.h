@@ -77,15 +77,23 @@ inline bool prefix_umma_pays(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, in
 // other, but leave room for fewer CTAs on an SM: two instead of three (one instead of two at block_m 128, D 64; one either
 // way at D 128).  So what counts is whether 32 need fewer waves, and how many gathered tiles there can be.  Us per
 // call, 32 / 64 columns, by CTAs; "bound": ancestors allowed for, in blocks:
-//   block_m 64, bound 1    D 128: 384 8.2 / 10.6, 512 13.1 / 12.0, 768 15.8 / 17.2, 1024 18.9 / 21.8; D 64: 384 5.7 / 7.5, 512 9.6 / 8.4, 768 10.9 / 12.0
-//   block_m 64, bound 2    384 11.2 / 13.0, 512 17.5 / 14.3, 1024 27.4 / 26.3; bound 5: 384 19.6 / 19.0, 512 27.4 / 23.9
-//   block_m 32, 64 slots   D 128: 48 3.8 / 5.0, 512 6.0 / 10.1, 1024 10.6 / 19.2; D 64: 48 2.9 / 3.7, 1024 7.4 / 8.4
-//   block_m 32, longer     D 128: 256 12.5 / 11.3, 512 13.6 / 18.7, 2048 45.7 / 72.5; D 64: 512 9.7 / 8.8, 2048 32.4 / 29.9, 8192 66.3 / 62.8
-//   block_m 128, bound 1   D 64: 128 6.6 / 5.3, 256 8.6 / 9.7, 384 15.2 / 15.1, 512 15.8 / 19.3; D 128: 192 13.8 / 13.1
-//   block_m 128, bound 2   D 64: 192 10.1 / 11.3, 256 10.6 / 12.0; bound 3: 192 19.8 / 16.3
-// Above eight CTAs per SM 32 win (64 batched trees of 256 nodes: 112 / 143).
+//   block_m 64, bound 1    D 128: 384 8.8 / 10.7, 512 12.9 / 12.1, 768 15.7 / 17.1, 1024 19.4 / 21.8; D 64: 384 6.1 / 7.5, 512 9.1 / 8.5, 768 10.5 / 12.0
+//   block_m 64, bound 2    D 128: 384 11.8 / 13.1, 512 18.1 / 14.5, 1024 28.1 / 26.2; bound 5: 384 19.9 / 19.0, 512 27.5 / 23.7
+//   block_m 32, 64 slots   D 128: 128 3.9 / 5.2, 512 6.3 / 10.1, 1024 11.1 / 18.9; D 64: 128 2.9 / 3.8, 512 4.6 / 4.5, 1024 7.8 / 8.6
+//   block_m 128, bound 1   D 64: 128 7.1 / 5.3, 256 8.8 / 10.1, 384 14.4 / 14.5, 512 15.6 / 18.8; D 128: 192 14.7 / 13.4
+//   block_m 128, bound 2   D 64: 192 10.3 / 11.4, 256 10.8 / 12.3; bound 3: 192 18.1 / 13.2
+// Above eight CTAs per SM 32 win at block_m 64 and 128 (64 batched trees of 256 nodes: 104 / 142).  Longer lists at block_m 32:
+//   D 128, 128 slots       scored trees 128 4.0 / 5.3, 256 5.6 / 5.5, 512 6.6 / 10.3; deep ones 5.5 / 5.7, 7.2 / 5.8, 8.2 / 11.1
+//   D 64, 128 slots        scored 128 3.2 / 3.8, 512 4.8 / 4.6, 1024 8.5 / 8.8, 1536 11.9 / 12.5, 4096 26.5 / 29.4; deep 4.1 / 4.1, 6.0 / 5.0,
+//                          10.7 / 9.6, 15.1 / 13.5, 34.1 / 31.7: they part above eight CTAs per SM, where scored (and Medusa)
+//                          trees lose 5 to 20 % by 64 columns and deep ones 3 to 12 % by 32
+//   D 64, 320 slots        window trees 512 9.9 / 8.7, 1024 17.7 / 14.8, 2048 30.5 / 28.5, 8192 101 / 100
 inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
-    if (bm == 32) return ma > 64 && (D == 64 || ctas <= 2LL * sms) ? 64 : 32;
+    if (bm == 32) {
+        if (D == 128) return ma > 64 && ctas <= 2LL * sms ? 64 : 32;
+        if (ma <= 64) return ctas > 3LL * sms && ctas <= 4LL * sms ? 64 : 32;     // two waves either way
+        return ma > 256 || ctas <= 8LL * sms ? 64 : 32;
+    }
     if (ctas > 8LL * sms) return 32;
     if (bm == 128 && D == 128) return 64;
     const int64_t fit = (bm == 64 ? 2LL : 1LL) * sms;     // CTAs at once with 64 columns; with 32 one more per SM
