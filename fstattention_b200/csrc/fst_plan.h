@@ -115,7 +115,11 @@ inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
 //   D 64, block_m 128    bound 1: 0.89 - 0.92 up to 256, 1.05 - 1.26 above; bound 2 and up: 0.98 - 1.18 from 160; 0.64 - 0.84 up to one per SM
 //   D 64, block_m 64     bound 1: 0.88 - 0.99 up to 700, 1.05 - 1.11 from 1000; bound 2 and 3: 1.07 - 1.38 from 512, 0.94 at 256; bound 4 and
 //                        up: 1.20 at 512 with 1024 nodes; with 512 nodes 0.90 there, 1.07 - 1.23 from 640
-//   D 64, block_m 32     64 slots: 1.08 - 1.32 from 700, 1.02 at 512; longer lists 1.00 at 2048, 0.91 - 0.95 below; 0.59 - 0.82 with a bound of 8 and up
+//   D 64, block_m 32     64 slots: 1.07 at 512, 1.08 - 1.32 above; bound 4 to 7: scored and Medusa trees 1.08 - 1.11 at 512, 1.12 - 1.32 above,
+//                        deep ones 0.91 - 0.95 up to 800 and 0.97 - 1.01 above (the line is where they lose nothing against the
+//                        columns that the others want); 0.75 - 1.01 with a bound of 8 and up (scored trees 1.04 - 1.25 from 500).
+//                        Rows of an item for which there is no node cost as much as the others here and nothing there: 64 nodes
+//                        0.64 - 0.70 at any size; 300 nodes 0.87 - 1.02 up to 770, 1.09 - 1.17 from 1000
 // Small grids are bound by one CTA's latency, which is longer here.  With one short tile of ancestors per 64 rows at
 // D 128 both kernels wait for the same HBM bytes and are within a few per cent of one another.
 inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int ma) {
@@ -128,7 +132,10 @@ inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int
     }
     if (bm == 128) return items >= (bound >= 2 ? 150 : 300);
     if (bm == 64) return items >= (bound >= 4 ? (n_q >= 700 ? 450 : 600) : bound >= 2 ? 450 : 1000);
-    return bound < 8 && items >= (bound >= 4 ? 2000 : 700);
+    const int64_t slots = (n_q + 127) / 128 * 128;
+    if (bound >= 8 || 4 * n_q < 3 * slots) return false;
+    if (5 * n_q < 4 * slots) return items >= 1000;
+    return items >= (bound < 4 ? 700 : n_q >= 700 ? 500 : 1000);
 }
 
 }  // namespace fst
