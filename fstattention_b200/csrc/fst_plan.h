@@ -109,33 +109,35 @@ inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
 //   D 128, block_m 64    bound 1: 0.91 - 1.00 up to 512, 1.05 from 700; bound 2 and 3: 0.91 - 0.96 at 160 to 200, 1.02 - 1.40 from 256;
 //                        bound 4 and up: 1.03 - 1.41 from 300 where the tree has 700 nodes and more (0.97 - 1.15 at 190 to 256, but 0.97
 //                        inside a decode step), 0.88 - 1.00 up to 512 with 512 nodes, 1.10 - 1.25 above
-//   D 128, block_m 32    64 slots: 0.87 - 1.00 up to 512, 1.05 - 1.25 above; lists of 128: 0.94 at 320, 1.00 - 1.08 at 512, 1.04 - 1.18
-//                        above; 0.74 - 0.90 with 320 slots and up (the line at 200 to 300 items is where it was when the
-//                        other kernel had 64-column tiles there, 1.02 - 1.65)
+//   D 128, block_m 32    64 slots: 0.85 - 0.99 up to 650, 1.03 - 1.24 from 770; bound 4 to 7: 0.85 - 1.00 up to 450, 0.99 - 1.07 at 512, 0.96 - 1.09
+//                        up to 770, 1.07 - 1.27 above (256-node deep trees 0.93 - 1.04); 0.63 - 0.99 with 320 slots.  64 nodes
+//                        0.58 - 0.75 at any size, 300 nodes 0.83 - 1.01 up to 770 and 1.04 - 1.13 from 1000
 //   D 64, block_m 128    bound 1: 0.89 - 0.92 up to 256, 1.05 - 1.26 above; bound 2 and up: 0.98 - 1.18 from 160; 0.64 - 0.84 up to one per SM
 //   D 64, block_m 64     bound 1: 0.88 - 0.99 up to 700, 1.05 - 1.11 from 1000; bound 2 and 3: 1.07 - 1.38 from 512, 0.94 at 256; bound 4 and
 //                        up: 1.20 at 512 with 1024 nodes; with 512 nodes 0.90 there, 1.07 - 1.23 from 640
 //   D 64, block_m 32     64 slots: 1.07 at 512, 1.08 - 1.32 above; bound 4 to 7: scored and Medusa trees 1.08 - 1.11 at 512, 1.12 - 1.32 above,
 //                        deep ones 0.91 - 0.95 up to 800 and 0.97 - 1.01 above (the line is where they lose nothing against the
 //                        columns that the others want); 0.75 - 1.01 with a bound of 8 and up (scored trees 1.04 - 1.25 from 500).
-//                        Rows of an item for which there is no node cost as much as the others here and nothing there: 64 nodes
-//                        0.64 - 0.70 at any size; 300 nodes 0.87 - 1.02 up to 770, 1.09 - 1.17 from 1000
+//                        64 nodes 0.64 - 0.70 at any size, 300 nodes 0.87 - 1.02 up to 770 and 1.09 - 1.17 from 1000
+// Rows of an item for which there is no node cost as much as the others here and nothing there.
 // Small grids are bound by one CTA's latency, which is longer here.  With one short tile of ancestors per 64 rows at
 // D 128 both kernels wait for the same HBM bytes and are within a few per cent of one another.
 inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int ma) {
     const int64_t items = (n_q + 127) / 128 * H * Z;
     const int bound = ma / bm;                        // tiles of ancestors the caller allows for
-    if (D == 128) {
+    if (D == 128 && bm != 32) {
         if (bm == 128) return items >= 150;
-        if (bm == 64) return items >= (bound >= 4 ? (n_q >= 700 ? 300 : 600) : bound >= 2 ? 250 : 650);
-        return items >= 200 && (items <= 300 || (bound < 8 && items >= (bound >= 4 ? 500 : 600)));
+        return items >= (bound >= 4 ? (n_q >= 700 ? 300 : 600) : bound >= 2 ? 250 : 650);
+    }
+    if (bm == 32) {
+        const int64_t slots = (n_q + 127) / 128 * 128;
+        if (bound >= 8 || 4 * n_q < 3 * slots) return false;
+        if (5 * n_q < 4 * slots) return items >= 1000;
+        if (D == 128) return items >= (bound >= 4 ? 500 : 600);
+        return items >= (bound < 4 ? 700 : n_q >= 700 ? 500 : 1000);
     }
     if (bm == 128) return items >= (bound >= 2 ? 150 : 300);
-    if (bm == 64) return items >= (bound >= 4 ? (n_q >= 700 ? 450 : 600) : bound >= 2 ? 450 : 1000);
-    const int64_t slots = (n_q + 127) / 128 * 128;
-    if (bound >= 8 || 4 * n_q < 3 * slots) return false;
-    if (5 * n_q < 4 * slots) return items >= 1000;
-    return items >= (bound < 4 ? 700 : n_q >= 700 ? 500 : 1000);
+    return items >= (bound >= 4 ? (n_q >= 700 ? 450 : 600) : bound >= 2 ? 450 : 1000);
 }
 
 }  // namespace fst

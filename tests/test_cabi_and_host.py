@@ -325,16 +325,6 @@ def test_a_number_of_splits_of_any_type(built_lib):
         assert fst.launch_plan(q, 4096, 64, kv_splits=splits) == want
 
 
-def test_tree_kernel_of_short_blocks_with_long_lists(built_lib):
-    """block_m 32 at D 128: the tcgen05 kernel where an SM has one or two items, and on large grids where the ancestor
-    lists are short (three trees of 512 nodes with 320 ancestors, 32 heads: 28 us against 39)."""
-    from fstattention_b200 import _lib
-    kernel = lambda items, ma: _lib.lib().fst_attention_tree_kernel(1, items, 128, 128, 32, ma)
-    umma, tma = _lib.KERNELS["tree_umma"], _lib.KERNELS["tma"]
-    assert [kernel(n, 320) for n in (100, 256, 384, 1024, 4096)] == [tma, umma, tma, tma, tma]
-    assert [kernel(n, 64) for n in (100, 256, 384, 1024, 4096)] == [tma, umma, tma, umma, umma]
-
-
 @pytest.mark.parametrize("D,bm,ma,n_q,line", [(128, 32, 128, 128, 500), (128, 64, 64, 256, 650), (128, 64, 320, 512, 600), (128, 64, 256, 1024, 300),
                                               (64, 64, 64, 256, 1000), (64, 64, 256, 1024, 450), (64, 64, 320, 512, 600)])
 def test_tree_kernel_lines(built_lib, D, bm, ma, n_q, line):
@@ -376,6 +366,22 @@ medusa 64 32 64 64 64 32     23.1 26.8 33.1
 medusa 64 32 64 256 12 32    19.2 22.7 17.7
 create 64 32 64 1020 3 32    19.8 23.3 17.7
 window 64 32 320 1024 8 32   101.0 99.6 132.0
+scored 128 32 128 1024 1 28  11.5 18.3 11.8
+scored 128 32 128 1024 1 32  12.0 20.1 12.4
+scored 128 32 128 1024 2 32  21.2 36.0 19.8
+scored 128 32 128 1024 16 32 123.8 269.9 98.4
+scored 128 32 128 300 6 28   16.6 29.1 17.9
+scored 128 32 128 300 43 32  101.0 220.1 89.1
+deep   128 32 128 1024 2 32  27.2 38.4 26.8
+deep   128 32 128 256 16 32  45.0 74.0 43.2
+medusa 128 32 64 256 1 32    5.2 5.4 8.0
+medusa 128 32 64 256 4 32    11.1 18.9 12.1
+medusa 128 32 64 256 16 32   33.3 67.3 30.5
+medusa 128 32 64 64 64 32    31.4 62.2 42.2
+window 128 32 320 512 2 28   21.5 25.3 26.7
+window 128 32 320 512 2 32   23.0 28.1 28.9
+window 128 32 320 512 3 24   24.2 31.9 26.5
+window 128 32 320 512 16 32  124.2 228.3 181.7
 """
 
 
