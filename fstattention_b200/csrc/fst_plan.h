@@ -106,8 +106,10 @@ inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
 // items (128 query rows of one head), ratios of the mma.sync kernel's time (with the better of its tiles) to the other's; "bound"
 // is the ancestor bound in blocks:
 //   D 128, block_m 128   1.15 - 1.45 at 160 to 200 items, 1.19 - 2.03 above; 0.81 - 1.12 up to one item per SM
-//   D 128, block_m 64    bound 1: 0.91 - 1.00 up to 512, 1.05 from 700; bound 2 and 3: 0.91 - 0.96 at 160 to 200, 1.02 - 1.40 from 256;
-//                        bound 4 and up: 1.03 - 1.41 from 300 where the tree has 700 nodes and more (0.97 - 1.15 at 190 to 256, but 0.97
+//   D 128, block_m 64    64 slots: 0.93 - 1.05 up to 1024, 1.04 - 1.13 above in graphs of calls, 1.01 in a program whose inputs come from HBM
+//                        (64 x 256 nodes 114.6 / 113.4 us), and errors against 64 bits of 1.003 of the other kernel's: not there.
+//                        Bound 2 and 3 (and 96 slots from 650): 0.91 - 0.96 at 160 to 200, 1.02 - 1.40 from 256; bound 4 and up:
+//                        1.03 - 1.41 from 300 where the tree has 700 nodes and more (0.97 - 1.15 at 190 to 256, but 0.97
 //                        inside a decode step), 0.88 - 1.00 up to 512 with 512 nodes, 1.10 - 1.25 above
 //   D 128, block_m 32    64 slots: 0.85 - 0.99 up to 650, 1.03 - 1.24 from 770; bound 4 to 7: 0.85 - 1.00 up to 450, 0.99 - 1.07 at 512, 0.96 - 1.09
 //                        up to 770, 1.07 - 1.27 above (256-node deep trees 0.93 - 1.04); 0.63 - 0.99 with 320 slots.  64 nodes
@@ -120,14 +122,13 @@ inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
 //                        columns that the others want); 0.75 - 1.01 with a bound of 8 and up (scored trees 1.04 - 1.25 from 500).
 //                        64 nodes 0.64 - 0.70 at any size, 300 nodes 0.87 - 1.02 up to 770 and 1.09 - 1.17 from 1000
 // Rows of an item for which there is no node cost as much as the others here and nothing there.
-// Small grids are bound by one CTA's latency, which is longer here.  With one short tile of ancestors per 64 rows at
-// D 128 both kernels wait for the same HBM bytes and are within a few per cent of one another.
+// Small grids are bound by one CTA's latency, which is longer here.
 inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int ma) {
     const int64_t items = (n_q + 127) / 128 * H * Z;
     const int bound = ma / bm;                        // tiles of ancestors the caller allows for
     if (D == 128 && bm != 32) {
         if (bm == 128) return items >= 150;
-        return items >= (bound >= 4 ? (n_q >= 700 ? 300 : 600) : bound >= 2 ? 250 : 650);
+        return ma > 64 && items >= (bound >= 4 ? (n_q >= 700 ? 300 : 600) : bound >= 2 ? 250 : 650);
     }
     if (bm == 32) {
         const int64_t slots = (n_q + 127) / 128 * 128;

@@ -325,7 +325,7 @@ def test_a_number_of_splits_of_any_type(built_lib):
         assert fst.launch_plan(q, 4096, 64, kv_splits=splits) == want
 
 
-@pytest.mark.parametrize("D,bm,ma,n_q,line", [(128, 32, 128, 128, 500), (128, 64, 64, 256, 650), (128, 64, 320, 512, 600), (128, 64, 256, 1024, 300),
+@pytest.mark.parametrize("D,bm,ma,n_q,line", [(128, 32, 128, 128, 500), (128, 64, 320, 512, 600), (128, 64, 256, 1024, 300),
                                               (64, 64, 64, 256, 1000), (64, 64, 256, 1024, 450), (64, 64, 320, 512, 600)])
 def test_tree_kernel_lines(built_lib, D, bm, ma, n_q, line):
     """The tcgen05 kernel from the grid on where it was measured to be the faster one, whatever makes up the grid."""

@@ -152,6 +152,19 @@ def test_tree_umma_bound_changes_no_bit(fst, D, bm, dtype):
     assert compared >= 4 and fst.last_status() == 0
 
 
+def test_forest_is_rounded_as_by_the_mma_kernel(fst):
+    """D 128, block_m 64, one short list to a block: both kernels wait for the same bytes, so the choice falls on the one that
+    is nearer to 64 bits (by 0.3 %), however large the forest."""
+    from fstattention_b200 import configs
+    trees = configs.jittered_forest(0, 24, 256)
+    trees = [t + [0] * (256 - len(t)) for t in trees]
+    meta = fst.build_tree_metadata(trees, 64, 64, reference_format=False)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn((24, 32, 256, 128), generator=g, device="cuda").half() for _ in range(3))
+    got, want = (fst.fst_attention(q, k, v, meta, sm_scale=128 ** -0.5, kernel=kernel) for kernel in ("auto", "tma"))
+    assert torch.equal(got, want)
+
+
 def reaches(par, lo, hi):
     """Which nodes attend to one of the nodes lo .. hi - 1."""
     hit = torch.zeros(len(par), dtype=torch.bool)
