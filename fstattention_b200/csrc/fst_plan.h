@@ -80,6 +80,8 @@ inline bool prefix_umma_pays(int64_t Z, int64_t H, int64_t H_kv, int64_t n_q, in
 //   block_m 64, bound 1    D 128: 384 8.8 / 10.7, 512 12.9 / 12.1, 768 15.7 / 17.1, 1024 19.4 / 21.8; D 64: 384 6.1 / 7.5, 512 9.1 / 8.5, 768 10.5 / 12.0
 //   block_m 64, bound 2    D 128: 384 11.8 / 13.1, 512 18.1 / 14.5, 1024 28.1 / 26.2; bound 5: 384 19.9 / 19.0, 512 27.5 / 23.7
 //   block_m 32, 64 slots   D 128: 128 3.9 / 5.2, 512 6.3 / 10.1, 1024 11.1 / 18.9; D 64: 128 2.9 / 3.8, 512 4.6 / 4.5, 1024 7.8 / 8.6
+//                          a few CTAs more than fit at once, 304: deep trees D 128 11.1 / 9.5, D 64 8.2 / 6.8, scored ones 9.6 / 9.6,
+//                          6.9 / 6.9; 320: deep 11.3 / 12.2, 8.2 / 8.7
 //   block_m 128, bound 1   D 64: 128 7.1 / 5.3, 256 8.8 / 10.1, 384 14.4 / 14.5, 512 15.6 / 18.8; D 128: 192 14.7 / 13.4
 //   block_m 128, bound 2   D 64: 192 10.3 / 11.4, 256 10.8 / 12.3; bound 3: 192 18.1 / 13.2
 // Above eight CTAs per SM 32 win at block_m 64 and 128 (64 batched trees of 256 nodes: 104 / 142).  Longer lists at block_m 32:
@@ -97,7 +99,7 @@ inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
     if (ctas > 8LL * sms) return 32;
     if (bm == 128 && D == 128) return 64;
     const int64_t fit = (bm == 64 ? 2LL : 1LL) * sms;     // CTAs at once with 64 columns; with 32 one more per SM
-    if (ctas <= fit) return 64;
+    if (ctas <= fit + (ma > bm ? sms / 16 : 0)) return 64;
     if (ctas <= fit + sms) return ma <= 2 * bm ? 32 : 64;
     return ma > bm || (ctas + fit - 1) / fit <= (ctas + fit + sms - 1) / (fit + sms) ? 64 : 32;
 }

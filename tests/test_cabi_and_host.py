@@ -382,6 +382,14 @@ window 128 32 320 512 2 28   21.5 25.3 26.7
 window 128 32 320 512 2 32   23.0 28.1 28.9
 window 128 32 320 512 3 24   24.2 31.9 26.5
 window 128 32 320 512 16 32  124.2 228.3 181.7
+deep   64 64 128 1024 1 19   8.2 6.8 9.4
+deep   64 64 128 256 3 25    8.2 6.3 9.4
+deep   64 64 128 4096 1 5    8.2 8.7 9.8
+scored 64 64 128 1024 1 19   6.9 6.9 9.2
+deep   128 64 128 1024 1 19  11.1 9.5 11.1
+deep   128 64 128 256 3 25   11.1 9.0 11.1
+scored 128 64 128 1024 1 19  9.6 9.6 10.7
+create 64 64 64 1020 1 19    5.8 6.6 8.8
 """
 
 
