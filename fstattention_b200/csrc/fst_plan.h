@@ -104,43 +104,44 @@ inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
     return ma > bm || (ctas + fit - 1) / fit <= (ctas + fit + sms - 1) / (fit + sms) ? 64 : 32;
 }
 
-// When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, five kinds of trees, 64 to 8192
-// items (128 query rows of one head), ratios of the mma.sync kernel's time (with the better of its tiles) to the other's; "bound"
-// is the ancestor bound in blocks:
-//   D 128, block_m 128   1.15 - 1.45 at 160 to 200 items, 1.19 - 2.03 above; 0.81 - 1.12 up to one item per SM
-//   D 128, block_m 64    64 slots: 0.93 - 1.05 up to 1024, 1.04 - 1.13 above in graphs of calls, 1.01 in a program whose inputs come from HBM
-//                        (64 x 256 nodes 114.6 / 113.4 us), and errors against 64 bits of 1.003 of the other kernel's: not there.
-//                        Bound 2 and 3 (and 96 slots from 650): 0.91 - 0.96 at 160 to 200, 1.02 - 1.40 from 256; bound 4 and up:
-//                        1.03 - 1.41 from 300 where the tree has 700 nodes and more (0.97 - 1.15 at 190 to 256, but 0.97
-//                        inside a decode step), 0.88 - 1.00 up to 512 with 512 nodes, 1.10 - 1.25 above
-//   D 128, block_m 32    64 slots: 0.85 - 0.99 up to 650, 1.03 - 1.24 from 770; bound 4 to 7: 0.85 - 1.00 up to 450, 0.99 - 1.07 at 512, 0.96 - 1.09
-//                        up to 770, 1.07 - 1.27 above (256-node deep trees 0.93 - 1.04); 0.63 - 0.99 with 320 slots.  64 nodes
-//                        0.58 - 0.75 at any size, 300 nodes 0.83 - 1.01 up to 770 and 1.04 - 1.13 from 1000
-//   D 64, block_m 128    bound 1: 0.89 - 0.92 up to 256, 1.05 - 1.26 above; bound 2 and up: 0.98 - 1.18 from 160; 0.64 - 0.84 up to one per SM
-//   D 64, block_m 64     bound 1: 0.88 - 0.99 up to 700, 1.05 - 1.11 from 1000; bound 2 and 3: 1.07 - 1.38 from 512, 0.94 at 256; bound 4 and
-//                        up: 1.20 at 512 with 1024 nodes; with 512 nodes 0.90 there, 1.07 - 1.23 from 640
-//   D 64, block_m 32     64 slots: 1.07 at 512, 1.08 - 1.32 above; bound 4 to 7: scored and Medusa trees 1.08 - 1.11 at 512, 1.12 - 1.32 above,
-//                        deep ones 0.91 - 0.95 up to 800 and 0.97 - 1.01 above (the line is where they lose nothing against the
-//                        columns that the others want); 0.75 - 1.01 with a bound of 8 and up (scored trees 1.04 - 1.25 from 500).
-//                        64 nodes 0.64 - 0.70 at any size, 300 nodes 0.87 - 1.02 up to 770 and 1.09 - 1.17 from 1000
+// When the tcgen05 tree kernel beats the mma.sync one.  Measured on B200, fp16, six kinds of trees of 64 to 4096 nodes, 30 to 4130
+// items (128 query rows of one head), in graphs of calls; ratios of the mma.sync kernel's time (with the better of its
+// tiles) to the other's; "bound" is the ancestor bound in blocks:
+//   D 128, block_m 128   0.69 - 1.15 up to one item per SM, 1.01 - 1.29 at 150 to 170, 1.06 - 1.67 up to 420, 1.32 - 2.28 above
+//   D 128, block_m 64    64 slots: 0.55 - 1.02 up to 900, 1.02 - 1.15 above, but 1.01 in a program whose inputs come from HBM (64 x 256
+//                        nodes 114.6 / 113.4 us), and errors against 64 bits of 1.003 of the other kernel's: not there.
+//                        96 slots: 0.84 - 1.02 up to 420, 0.97 - 1.08 at 500, 1.06 - 1.21 above.  Bound 2 and 3: 0.56 - 1.08 up to 224; deep trees
+//                        1.07 at 250 to 310, others 0.83 - 1.00; 0.86 - 1.16 up to 420, 0.93 - 1.21 at 500, 0.98 - 1.43 above.  Bound 4 and
+//                        up: 0.63 - 1.11 up to 224; with 700 nodes and more 1.02 - 1.18 at 250 to 310 (in a decode step of 1024 window
+//                        nodes, 256 items, 103.8 / 99.8), 0.98 - 1.22 up to 420 (scored trees 0.90 at 312), 1.01 - 1.44 above; with fewer
+//                        0.86 - 1.17 up to 420, 1.00 - 1.22 at 500, 1.05 - 1.39 above
+//   D 128, block_m 32    64 slots: 0.53 - 0.99 up to 530, 1.00 - 1.03 up to 900, 1.09 - 1.23 above; bound 4 to 7: 0.54 - 1.03 up to 420, 0.88 - 1.07 at 500,
+//                        0.96 - 1.10 up to 900, 0.98 - 1.27 above (256-node deep trees 0.93 - 1.04); 0.62 - 1.01 with 320 slots.  64 nodes
+//                        0.55 - 0.75 at any size, 300 nodes 0.54 - 1.00 up to 900 and 1.05 - 1.13 above
+//   D 64, block_m 128    bound 1: 0.58 - 1.04 up to 310, 1.04 - 1.47 above; bound 2: 0.69 - 0.80 up to one per SM, 0.96 - 1.05 up to 310, 1.08 - 1.39
+//                        above; bound 3: 0.85 - 1.00 up to 170, 1.03 - 1.67 above
+//   D 64, block_m 64     64 slots: 0.54 - 1.01 up to 900, 1.07 - 1.21 above (64 nodes 0.52 - 0.91); bound 2 and 3: 0.54 - 0.96 up to 310, 0.84 - 1.06 up to
+//                        420, 0.98 - 1.18 at 500 and 1.03 - 1.47 above (Medusa trees 0.92 - 1.00, 0.94 at 640, 1.02 - 1.18); bound 4 and up:
+//                        0.55 - 1.08 up to 420, 0.92 - 1.20 at 500, 1.04 - 1.46 above (512 window nodes 0.94 - 0.96 from 1200 on: four row tiles
+//                        to a head in a grid of 148, so that the longest lists fall to the same CTAs); 300 nodes in short lists
+//                        0.54 - 0.94 up to 900 and 1.01 - 1.09 above, in long ones 0.58 - 0.97 up to 700, 1.04 - 1.18 above
+//   D 64, block_m 32     64 slots: 0.47 - 0.99 up to 420, 0.93 - 1.07 at 500, 1.07 - 1.31 above; bound 4 to 7: scored and Medusa trees 0.49 - 1.05 up to 420,
+//                        0.96 - 1.12 at 500, 1.12 - 1.34 above, deep ones 0.81 - 0.92 at 250 to 900 and 0.92 - 1.00 above (the line is where
+//                        they lose next to nothing against the columns that the others want); 0.53 - 1.03 with a bound of 8 and
+//                        up (scored trees 1.07 - 1.25 from 500).  64 nodes 0.45 - 0.70 at any size, 300 nodes 0.50 - 1.02 up to
+//                        900 and 1.09 - 1.16 above
 // Rows of an item for which there is no node cost as much as the others here and nothing there.
 // Small grids are bound by one CTA's latency, which is longer here.
 inline bool tree_umma_pays(int64_t Z, int64_t H, int64_t n_q, int D, int bm, int ma) {
-    const int64_t items = (n_q + 127) / 128 * H * Z;
+    const int64_t slots = (n_q + 127) / 128 * 128, items = slots / 128 * H * Z;
     const int bound = ma / bm;                        // tiles of ancestors the caller allows for
-    if (D == 128 && bm != 32) {
-        if (bm == 128) return items >= 150;
-        return ma > 64 && items >= (bound >= 4 ? (n_q >= 700 ? 300 : 600) : bound >= 2 ? 250 : 650);
-    }
-    if (bm == 32) {
-        const int64_t slots = (n_q + 127) / 128 * 128;
-        if (bound >= 8 || 4 * n_q < 3 * slots) return false;
-        if (5 * n_q < 4 * slots) return items >= 1000;
-        if (D == 128) return items >= (bound >= 4 ? 500 : 600);
-        return items >= (bound < 4 ? 700 : n_q >= 700 ? 500 : 1000);
-    }
-    if (bm == 128) return items >= (bound >= 2 ? 150 : 300);
-    return items >= (bound >= 4 ? (n_q >= 700 ? 450 : 600) : bound >= 2 ? 450 : 1000);
+    if (bm == 128) return items >= (D == 128 || bound == 2 ? 150 : bound > 2 ? 166 : 300);
+    if (D == 128 && bm == 64) return ma > 64 && items >= (bound < 2 ? 650 : bound < 4 || n_q >= 700 ? 250 : 600);
+    if (4 * n_q < 3 * slots || (bm == 32 && bound >= 8)) return false;
+    if (5 * n_q < 4 * slots) return items >= (bm == 64 && bound >= 4 ? 700 : 1000);
+    if (D == 128) return items >= (bound >= 4 ? 500 : 600);
+    if (bm == 64) return items >= (bound >= 4 ? (n_q >= 700 ? 500 : 600) : bound >= 2 ? 450 : 1000);
+    return items >= (bound < 4 ? 700 : n_q >= 700 ? 500 : 1000);
 }
 
 }  // namespace fst

@@ -325,71 +325,107 @@ def test_a_number_of_splits_of_any_type(built_lib):
         assert fst.launch_plan(q, 4096, 64, kv_splits=splits) == want
 
 
-@pytest.mark.parametrize("D,bm,ma,n_q,line", [(128, 32, 128, 128, 500), (128, 64, 320, 512, 600), (128, 64, 256, 1024, 300),
-                                              (64, 64, 64, 256, 1000), (64, 64, 256, 1024, 450), (64, 64, 320, 512, 600)])
-def test_tree_kernel_lines(built_lib, D, bm, ma, n_q, line):
-    """The tcgen05 kernel from the grid on where it was measured to be the faster one, whatever makes up the grid."""
+def test_tree_kernel_of_a_grid(built_lib):
+    """What counts is how many items there are, not what makes them up; and each kernel has its grids."""
     from fstattention_b200 import _lib
-    per = n_q // 128
-    for heads in (-(-line // per), -(-line // per) - 1):
-        want = _lib.KERNELS["tree_umma" if heads * per >= line else "tma"]
-        assert _lib.lib().fst_attention_tree_kernel(1, heads, n_q, D, bm, ma) == want
-        assert _lib.lib().fst_attention_tree_kernel(heads, 1, n_q, D, bm, ma) == want
+    kernel = _lib.lib().fst_attention_tree_kernel
+    seen = {}
+    for D in (64, 128):
+        for bm in (32, 64, 128):
+            for ma in (64, 96, 128, 256, 320, 512):
+                for n in (20, 64, 130, 256, 300, 700, 1024, 5000):
+                    for many in (1, 24, 60, 148, 500, 3000):
+                        picks = {kernel(z, h, n, D, bm, ma) for z, h in ((1, many), (many, 1))}
+                        assert len(picks) == 1
+                        seen.setdefault((D, bm), set()).update(picks)
+    assert all(picks == {_lib.KERNELS["tma"], _lib.KERNELS["tree_umma"]} for picks in seen.values())
 
 
 # Tree kernels timed on a B200, us per call (fp16, graphs of calls on cold inputs): head_dim, block_m, ancestor bound, nodes, batch, heads;
 # the mma.sync kernel with 32 and with 64 columns to a tile, the tcgen05 kernel.
 MEASURED = """
-scored 64 32 128 1024 1 8    4.8 4.6 7.5
-scored 64 32 128 1024 1 32   8.5 8.8 9.4
+scored 64 32 128 1024 1 16   4.8 4.6 7.6
+scored 64 32 128 1024 1 32   8.6 8.7 9.4
 scored 64 32 128 1024 1 48   11.9 12.5 11.6
-scored 64 32 128 1024 3 27   18.4 20.1 15.7
-scored 64 32 128 1024 4 32   26.5 29.4 21.2
-scored 64 32 128 1024 16 32  95.0 111.8 70.4
-medusa 64 32 128 256 12 32   19.8 22.8 17.6
-medusa 64 32 128 256 24 32   36.1 42.5 29.7
-deep   64 32 128 1024 1 8    6.0 5.0 8.9
-deep   64 32 128 1024 1 32   10.7 9.6 11.6
-deep   64 32 128 1024 1 48   15.1 13.5 15.2
-deep   64 32 128 1024 4 32   34.1 31.7 31.5
-window 64 32 320 1024 1 16   9.9 8.7 13.4
-window 64 32 320 1024 2 32   30.5 28.5 37.7
-medusa 64 32 64 64 9 32      4.6 4.4 8.9
+scored 64 32 128 1024 3 27   18.4 20.1 15.8
+scored 64 32 128 1024 4 32   26.5 29.2 21.2
+scored 64 32 128 1024 16 32  95.0 112.2 72.1
+medusa 64 32 128 256 12 32   19.8 22.7 17.7
+medusa 64 32 128 256 24 32   36.1 42.7 29.6
+deep 64 32 128 1024 1 16     6.0 5.0 9.0
+deep 64 32 128 1024 1 32     10.7 9.6 11.7
+deep 64 32 128 1024 1 48     15.1 13.5 15.5
+deep 64 32 128 1024 4 32     33.9 31.7 32.4
+window 64 32 320 1024 1 16   9.9 8.8 13.6
+window 64 32 320 1024 2 32   30.5 28.5 38.7
+medusa 64 32 64 64 9 32      4.7 4.4 8.9
 medusa 64 32 64 256 1 16     2.9 3.8 6.1
 medusa 64 32 64 256 5 32     9.9 11.4 11.0
-scored 64 32 128 1024 2 32   15.1 16.4 13.6
-scored 64 32 128 300 8 32    17.6 19.7 17.2
-scored 64 32 128 300 16 32   31.4 35.9 28.4
-deep   64 32 128 1024 2 32   19.3 17.6 19.3
-medusa 64 32 64 64 24 32     10.2 11.2 16.1
-medusa 64 32 64 64 64 32     23.1 26.8 33.1
-medusa 64 32 64 256 12 32    19.2 22.7 17.7
-create 64 32 64 1020 3 32    19.8 23.3 17.7
-window 64 32 320 1024 8 32   101.0 99.6 132.0
-scored 128 32 128 1024 1 28  11.5 18.3 11.8
-scored 128 32 128 1024 1 32  12.0 20.1 12.4
-scored 128 32 128 1024 2 32  21.2 36.0 19.8
-scored 128 32 128 1024 16 32 123.8 269.9 98.4
-scored 128 32 128 300 6 28   16.6 29.1 17.9
-scored 128 32 128 300 43 32  101.0 220.1 89.1
-deep   128 32 128 1024 2 32  27.2 38.4 26.8
-deep   128 32 128 256 16 32  45.0 74.0 43.2
-medusa 128 32 64 256 1 32    5.2 5.4 8.0
-medusa 128 32 64 256 4 32    11.1 18.9 12.1
-medusa 128 32 64 256 16 32   33.3 67.3 30.5
-medusa 128 32 64 64 64 32    31.4 62.2 42.2
-window 128 32 320 512 2 28   21.5 25.3 26.7
-window 128 32 320 512 2 32   23.0 28.1 28.9
-window 128 32 320 512 3 24   24.2 31.9 26.5
-window 128 32 320 512 16 32  124.2 228.3 181.7
-deep   64 64 128 1024 1 19   8.2 6.8 9.4
-deep   64 64 128 256 3 25    8.2 6.3 9.4
-deep   64 64 128 4096 1 5    8.2 8.7 9.8
-scored 64 64 128 1024 1 19   6.9 6.9 9.2
-deep   128 64 128 1024 1 19  11.1 9.5 11.1
-deep   128 64 128 256 3 25   11.1 9.0 11.1
-scored 128 64 128 1024 1 19  9.6 9.6 10.7
+scored 64 32 128 1024 2 32   15.1 16.3 13.5
+scored 64 32 128 300 8 32    17.6 19.6 17.2
+scored 64 32 128 300 16 32   31.3 35.9 28.4
+deep 64 32 128 1024 2 32     19.2 17.6 19.7
+medusa 64 32 64 64 24 32     10.3 11.2 16.0
+medusa 64 32 64 64 64 32     23.0 26.9 32.8
+medusa 64 32 64 256 12 32    19.2 22.6 17.6
+create 64 32 64 1020 3 32    19.9 23.4 17.6
+window 64 32 320 1024 8 32   100.8 99.4 136.1
+deep 64 64 128 1024 1 19     8.1 6.8 9.5
+deep 64 64 128 256 3 25      8.2 6.3 9.4
+deep 64 64 128 4096 1 5      8.2 8.7 9.8
+scored 64 64 128 1024 1 19   6.8 6.9 9.2
 create 64 64 64 1020 1 19    5.8 6.6 8.8
+deep 64 64 128 256 4 32      11.8 9.7 10.4
+deep 64 64 128 256 8 32      18.6 17.1 15.3
+scored 64 64 128 300 5 30    11.8 12.4 13.7
+scored 64 64 128 300 16 32   31.0 35.6 30.4
+scored 64 64 128 1024 2 28   14.3 14.6 14.4
+scored 64 64 128 1024 4 32   27.7 30.0 23.5
+medusa 64 64 64 64 32 32     13.1 13.0 14.3
+medusa 64 64 64 256 8 32     13.7 15.1 13.9
+medusa 64 64 64 256 32 32    42.2 53.4 36.8
+window 64 64 320 700 3 25    25.7 21.3 23.3
+window 64 64 320 700 3 28    27.1 23.0 23.2
+window 64 64 320 512 5 32    32.1 30.6 28.7
+window 64 64 320 1024 2 32   31.9 28.0 26.3
+window 64 64 320 300 8 32    26.9 25.6 24.7
+window 64 128 384 512 1 38   17.6 10.7 12.6
+window 64 128 384 1024 1 19  19.4 11.0 12.5
+window 64 128 384 512 1 48   18.1 13.2 12.8
+deep 64 128 256 1024 1 24    10.4 11.3 10.2
+create 64 128 64 1020 1 32   8.7 10.2 9.6
+create 64 128 64 1020 1 40   13.2 14.0 11.7
+scored 128 32 128 1024 1 28  11.5 18.3 11.9
+scored 128 32 128 1024 1 32  12.1 20.1 12.4
+scored 128 32 128 1024 2 32  21.4 36.1 19.9
+scored 128 32 128 1024 16 32 123.6 270.2 98.3
+scored 128 32 128 300 6 28   16.6 29.1 17.9
+scored 128 32 128 300 43 32  101.1 219.7 89.1
+deep 128 32 128 1024 2 32    27.2 38.4 26.7
+deep 128 32 128 256 16 32    45.0 74.0 43.3
+medusa 128 32 64 256 1 32    5.3 5.5 8.0
+medusa 128 32 64 256 4 32    11.2 18.9 12.2
+medusa 128 32 64 256 16 32   33.3 67.3 30.4
+medusa 128 32 64 64 64 32    31.4 62.4 42.1
+window 128 32 320 512 2 28   21.5 25.4 26.7
+window 128 32 320 512 2 32   22.9 28.1 28.9
+window 128 32 320 512 3 24   24.4 31.9 26.2
+window 128 32 320 512 16 32  124.4 227.2 180.5
+deep 128 64 128 1024 1 19    11.1 9.4 11.9
+deep 128 64 128 256 3 25     11.1 9.0 11.7
+scored 128 64 128 1024 1 19  9.6 9.7 11.1
+scored 128 64 128 1024 1 32  15.2 13.1 13.4
+scored 128 64 96 1024 3 27   26.2 28.8 24.7
+scored 128 64 256 700 2 32   17.3 19.0 16.5
+deep 128 64 256 1024 1 28    14.6 14.3 13.1
+deep 128 64 128 1024 1 32    18.1 14.5 13.6
+window 128 64 320 1024 1 24  19.9 18.9 17.8
+window 128 64 320 1024 1 32  27.7 23.7 20.5
+window 128 64 320 512 2 32   24.3 18.7 20.3
+window 128 64 320 512 5 32   43.0 44.3 37.5
+medusa 128 128 128 256 2 32  8.9 7.6 9.7
+medusa 128 128 128 256 3 25  13.6 12.3 11.0
+deep 128 128 256 1024 1 32   18.8 17.3 13.6
 """
 
 
