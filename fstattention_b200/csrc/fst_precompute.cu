@@ -514,6 +514,8 @@ __host__ __device__ inline size_t wide_smem_words(size_t Wp, int bm, int ma, boo
     return Wp + Wp / 2 + size_t(inherit && ma > bm ? ma : bm) * maw + size_t(bm) * bw + size_t(bm) * 2 + (inherit ? size_t(ma) * 2 : 0);
 }
 
+// (apart by SET: the set's code beside the bitmap's took registers from it, 12 to 20 % of a build with a bound of 512)
+template <bool SET>
 __global__ void __launch_bounds__(WIDE_THREADS, 7)
 precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int bm, int ma, int inherit_ok,
                        int64_t *__restrict__ anc_idx_all, uint8_t *__restrict__ anc_mask_all,
@@ -544,14 +546,14 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
         }
         return p;
     };
-    const PackedLayout L = packed_layout(nb, bm, ma);
-    unsigned char *blob = packed_all ? packed_all + size_t(tree) * packed_stride : nullptr;
-    const size_t blk = size_t(tree) * nb + b;
-    int64_t *o_idx = anc_idx_all ? anc_idx_all + blk * ma : nullptr, *o_leaf = leaf_idx_all ? leaf_idx_all + blk * bm : nullptr;
-    uint8_t *o_mask = anc_mask_all ? anc_mask_all + blk * size_t(bm) * ma : nullptr;
-    if (ma <= SET_MOST && bm <= SET_MOST) {
-        if (precompute_set(*reinterpret_cast<AncestorSet *>(smem_raw), par, b, n_nodes, bm, ma, blob, L, o_idx, o_mask, o_leaf)) return;
-        __syncthreads();                                  // the bitmap takes the set's place
+    if constexpr (SET) {
+        const size_t blk = size_t(tree) * nb + b;
+        if (precompute_set(*reinterpret_cast<AncestorSet *>(smem_raw), par, b, n_nodes, bm, ma,
+                           packed_all ? packed_all + size_t(tree) * packed_stride : nullptr, packed_layout(nb, bm, ma),
+                           anc_idx_all ? anc_idx_all + blk * ma : nullptr, anc_mask_all ? anc_mask_all + blk * size_t(bm) * ma : nullptr,
+                           leaf_idx_all ? leaf_idx_all + blk * bm : nullptr))
+            return;
+        __syncthreads();                                  // more ancestors than the bound: the bitmap takes the set's place
     }
     for (int i = tid; i < W / 4; i += WIDE_THREADS) reinterpret_cast<uint4 *>(bitmap)[i] = make_uint4(0u, 0u, 0u, 0u);
     for (int i = tid; i < bm * bw; i += WIDE_THREADS) blkmask[i] = 0u;
@@ -587,6 +589,10 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
     const bool inherit = inherit_ok && n_anc <= ma;
     if (n_anc > ma && tid == 0) report(status, FST_DEV_ANCESTOR_OVERFLOW, tree * 65536 + b, n_anc);
 
+    const PackedLayout L = packed_layout(nb, bm, ma);
+    unsigned char *blob = packed_all ? packed_all + size_t(tree) * packed_stride : nullptr;
+    const size_t blk = size_t(tree) * nb + b;
+    int64_t *o_idx = anc_idx_all ? anc_idx_all + blk * ma : nullptr;
     int32_t *p_idx = blob ? reinterpret_cast<int32_t *>(blob + L.off_idx) + size_t(b) * ma : nullptr;
 
     // 3. ascending ancestor list, a lane per word
@@ -714,7 +720,8 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
             p_emask[i] = row_word(j, w) & keep;
         }
     }
-    if (o_mask) {
+    if (anc_mask_all) {
+        uint8_t *o_mask = anc_mask_all + blk * size_t(bm) * ma;
         if ((ma & 15) == 0 && (reinterpret_cast<uintptr_t>(o_mask) & 15) == 0) {   // sixteen bool bytes per store
             const int pieces = ma / 16;
             for (int i = tid; i < bm * pieces; i += WIDE_THREADS) {
@@ -730,10 +737,10 @@ precompute_wide_kernel(const int32_t *__restrict__ parent_all, int n_nodes, int 
         }
     }
     // 5. leaves: block rows that are not in the ancestor set (rows past the last node too)
-    if (o_leaf)
+    if (leaf_idx_all)
         for (int j = tid; j < bm; j += WIDE_THREADS) {
             const int k = row0 + j;
-            o_leaf[j] = ((bitmap[k >> 5] >> (k & 31)) & 1u) ? int64_t(-1) : int64_t(k);
+            leaf_idx_all[blk * bm + j] = ((bitmap[k >> 5] >> (k & 31)) & 1u) ? int64_t(-1) : int64_t(k);
         }
     __syncthreads();
     if (blob) {
@@ -905,7 +912,7 @@ pack_kernel(const int64_t *__restrict__ anc_idx_all, const uint8_t *__restrict__
 // largest dynamic shared memory enabled so far, per device and kernel variant
 static std::atomic<size_t> g_pre_smem_set[3][kMaxDevices];
 static std::atomic<size_t> g_pack_smem_set[kMaxDevices];
-static std::atomic<size_t> g_wide_smem_set[kMaxDevices];
+static std::atomic<size_t> g_wide_smem_set[2][kMaxDevices];
 
 cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, int bm, int ma,
                               int64_t *anc_idx, uint8_t *anc_mask, int64_t *leaf_idx,
@@ -924,7 +931,7 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
     // refused, which need not be quick: its rows are climbed twice, and the space goes to more CTAs on an SM.
     // Us per build, flags / set, with the reference-format tensors: 256 nodes 6.5 / 5.7, 1020 7.5 / 6.0, 64 of them 17.1 / 12.4,
     // 16 x 8192 61.6 / 28.9, 4096 deep ones (depth 96) 15.3 / 14.5, four of 8000 32.6 / 18.7.
-    const bool set = bm <= SET_MOST && ma <= SET_MOST && n_nodes <= kWideNodes;
+    const bool few = bm <= SET_MOST && ma <= SET_MOST, set = few && n_nodes <= kWideNodes;
     if (depth_cap < 1 || set) depth_cap = 1;
     // Byte flags (one byte per node below the last row) while they leave room to stage a good
     // part of the parent array; beyond that the walkers set bitmap bits with atomics.
@@ -950,15 +957,17 @@ cudaError_t launch_precompute(const int32_t *parent, int n_trees, int n_nodes, i
     const bool one_wave = fits && size_t(nb) * n_trees <= sm_count() * (228 * 1024 / (smem + 1024));
     if (n_nodes > kWideNodes && !(one_wave && ma > std::max(128, 2 * bm))) {
         const size_t Ww = (W + 32 * WIDE_WARPS - 1) / (32 * WIDE_WARPS) * (32 * WIDE_WARPS);
-        const bool inherit = ma <= 128;                   // masks of all slots: 2 KB, two words per thread
-        const size_t wide_smem = std::max(wide_smem_words(Ww, bm, ma, inherit) * 4, ma <= SET_MOST && bm <= SET_MOST ? sizeof(AncestorSet) : 0);
+        const bool inherit = ma <= 128 && !few;           // masks of all slots: 2 KB, two words per thread
+        const size_t wide_smem = std::max(wide_smem_words(Ww, bm, ma, inherit) * 4, few ? sizeof(AncestorSet) : 0);
         if (wide_smem <= budget) {
-            if (wide_smem > 48 * 1024 && wide_smem > g_wide_smem_set[slot].load(std::memory_order_acquire)) {
-                cudaError_t e = cudaFuncSetAttribute(precompute_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wide_smem));
+            auto kernel = few ? precompute_wide_kernel<true> : precompute_wide_kernel<false>;
+            std::atomic<size_t> &enabled = g_wide_smem_set[few ? 1 : 0][slot];
+            if (wide_smem > 48 * 1024 && wide_smem > enabled.load(std::memory_order_acquire)) {
+                cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wide_smem));
                 if (e != cudaSuccess) return e;
-                g_wide_smem_set[slot].store(wide_smem, std::memory_order_release);
+                enabled.store(wide_smem, std::memory_order_release);
             }
-            precompute_wide_kernel<<<dim3(nb, n_trees), WIDE_THREADS, wide_smem, stream>>>(
+            kernel<<<dim3(nb, n_trees), WIDE_THREADS, wide_smem, stream>>>(
                 parent, n_nodes, bm, ma, inherit ? 1 : 0, anc_idx, anc_mask, leaf_idx, static_cast<unsigned char *>(packed),
                 packed_stride, status);
             return cudaGetLastError();
