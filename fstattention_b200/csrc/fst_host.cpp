@@ -60,6 +60,12 @@ at::Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Device &de
     return at::detail::empty_cuda(size, type, dev, std::nullopt);
 }
 
+// Tensors that outlive the call and are written in place later - metadata, whose versions say whether anybody has, and status
+// records - are ordinary ones also when the call is made under torch.inference_mode().
+struct OrdinaryTensors {
+    c10::InferenceMode off{false};
+};
+
 // Attention launches on a device share one status record (the first problem seen stays until it
 // is cleared).  Records live as long as the process.
 at::Tensor *const *status_slots() {
@@ -72,8 +78,10 @@ at::Tensor *status_of(const at::Device &dev, bool create) {
     const int i = dev.index();
     if (i < 0 || i >= 64) raise(PyExc_RuntimeError, "device index out of range");
     std::lock_guard<std::mutex> lock(mutex);
-    if (slots[i] == nullptr && create)
+    if (slots[i] == nullptr && create) {
+        const OrdinaryTensors guard;
         slots[i] = new at::Tensor(at::zeros({4}, at::TensorOptions().dtype(at::kInt).device(dev)));
+    }
     return slots[i];
 }
 
@@ -414,6 +422,7 @@ at::Tensor record_of(const at::Tensor &words, int64_t i) {
 // 8.2 us with the memset, 5.2 with the fill).
 at::Tensor clear_record(const at::Device &dev, cudaStream_t stream, const at::Tensor &old, const char *what,
                         bool *captured = nullptr) {
+    const OrdinaryTensors guard;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) check_status(FST_ERR_CUDA, what);
     if (captured != nullptr) *captured = capturing != cudaStreamCaptureStatusNone;
@@ -491,6 +500,7 @@ Built build_metadata(const at::Tensor &par, bool batched, int64_t n_trees, int64
     if (bm <= 0 || ma <= 0) raise(PyExc_ValueError, "block_m and max_ancestors must be positive");
     const int64_t nb = (n_nodes + bm - 1) / bm;
     const at::Device dev = par.device();
+    const OrdinaryTensors guard;
     Built m;
     m.stride = fst_packed_meta_bytes(int(nb), int(bm), int(ma));
     m.packed = empty({n_trees, int64_t(m.stride)}, at::kByte, dev);

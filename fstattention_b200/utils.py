@@ -56,7 +56,7 @@ class TreeMetadata:
 
     def tensors_untouched(self) -> bool:
         """True while nobody has modified the three reference-format tensors in place."""
-        return self._twin is None or self._twin.versions == _versions((self.ancestor_idx, self.ancestor_mask, self.leaf_idx))
+        return self._twin is None or _unchanged(self._twin, (self.ancestor_idx, self.ancestor_mask, self.leaf_idx))
 
     # Saved or deep-copied metadata has tensors of its own, and a twin that belongs to them.
     def __getstate__(self):
@@ -109,8 +109,16 @@ class TreeMetadata:
 
 
 def _versions(three):
+    """None where nobody counts: tensors loaded or copied under ``torch.inference_mode()``."""
     a, b, c = three
-    return a._version, b._version, c._version
+    try:
+        return a._version, b._version, c._version
+    except RuntimeError:
+        return None
+
+
+def _unchanged(twin, three) -> bool:
+    return twin.versions is not None and twin.versions == _versions(three)
 
 
 # The three tensors handed out by the precompute remember the packed form they came with, so that
@@ -132,7 +140,7 @@ class _PackedTwin:
         self.packed, self.tree_stride = packed, tree_stride
         self.reads_since_build = 0
         a, b, c = three
-        self.versions = a._version, b._version, c._version
+        self.versions = _versions(three)
         self.tensors = weakref.ref(a), weakref.ref(b), weakref.ref(c)
 
     @classmethod
@@ -151,7 +159,7 @@ def metadata_of(ancestor_idx, ancestor_mask, leaf_idx) -> Optional[_PackedTwin]:
         return None
     a, b, c = twin.tensors
     if a() is ancestor_idx and b() is ancestor_mask and c() is leaf_idx \
-            and twin.versions == _versions((ancestor_idx, ancestor_mask, leaf_idx)):
+            and _unchanged(twin, (ancestor_idx, ancestor_mask, leaf_idx)):
         return twin
     return None
 

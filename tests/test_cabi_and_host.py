@@ -251,6 +251,27 @@ def test_metadata_and_its_tensors_can_be_copied_and_saved(built_lib):
     assert saved(plain).tensors_untouched() and saved(plain).ancestor_idx is None
 
 
+def test_metadata_of_tensors_without_versions(built_lib):
+    """Under inference mode nobody counts how often a tensor is written: its metadata has no packed form to rely on."""
+    import pickle
+
+    from fstattention_b200.utils import TreeMetadata, metadata_of
+    make = lambda: TreeMetadata(1, 8, 4, 4, torch.zeros(64, dtype=torch.uint8), 64, torch.zeros(4, dtype=torch.int32),
+                                torch.zeros((2, 4), dtype=torch.long), torch.zeros((2, 4, 4), dtype=torch.bool),
+                                torch.zeros((2, 4), dtype=torch.long))
+    counted = make()
+    with torch.inference_mode():
+        loaded = pickle.loads(pickle.dumps(counted))
+        for meta in (make(), loaded):
+            assert not meta.tensors_untouched() and metadata_of(*meta) is None
+            meta.ancestor_idx += 5
+            assert metadata_of(*meta) is None
+            meta._rebuilt()
+            assert metadata_of(*meta) is None
+        assert counted.tensors_untouched()
+    assert pickle.loads(pickle.dumps(loaded)).ancestor_idx is not None
+
+
 def test_prefix_plans_on_any_number_of_sms(tmp_path):
     """A slice of a GPU may have fewer SMs than a GPC: every plan is one that can be launched."""
     import shutil

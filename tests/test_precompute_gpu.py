@@ -1,5 +1,7 @@
 """GPU precompute kernel against the reference's own outputs (golden) and the CPU oracle."""
 import numpy as np
+import os
+
 import pytest
 import torch
 
@@ -351,3 +353,47 @@ def test_inputs_of_a_lineage_small_and_large(fst, depth, mutate):
             fst.create_fst_attention_kernel_inputs(before.clone(), level, block_m=64, max_ancestors=8)
     q, k, v = (torch.randn((1, 2, n, 64), device="cuda").half() for _ in range(3))
     assert torch.equal(fst.fst_attention(q, k, v, *got, 0.1, BLOCK_M=64, MAX_ANCESTORS=128), fst.fst_attention(q, k, v, want, sm_scale=0.1))
+
+
+INFERENCE = """
+import torch
+import fstattention_b200 as fst
+lineage, level = fst.create_tree(5)
+n, prefix = lineage.shape[0], 40
+q = torch.randn((1, 2, n, 64), device="cuda").half()
+k, v = (torch.randn((1, 2, prefix + n, 64), device="cuda").half() for _ in range(2))
+def sequence():
+    three = fst.create_fst_attention_kernel_inputs(lineage.clone(), level, block_m=64, max_ancestors=64)
+    three[0].add_(prefix); three[2].add_(prefix)
+    o = fst.fst_attention(q, k, v, *three, 0.1, BLOCK_M=64, MAX_ANCESTORS=64)
+    meta = fst.build_tree_metadata(fst.parent_from_lineage(lineage, level), 64, 64)
+    again = fst.fst_attention(q, k, v, *meta, 0.1, BLOCK_M=64, MAX_ANCESTORS=64)
+    return three, o, meta, again
+with torch.inference_mode():                       # the process's first calls
+    inside = sequence()
+    order = fst.dfs_order_device(inside[2].ancestor_idx.new_tensor([-1, 0, 0, 1]).int())
+assert fst.last_status() == 0
+fst.clear_status()
+outside = sequence()
+assert all(torch.equal(a, b) for a, b in zip(inside[0], outside[0])) and torch.equal(inside[1], outside[1])
+assert all(torch.equal(a, b) for a, b in zip(inside[2], outside[2]))
+assert torch.equal(inside[3], inside[1]) and torch.equal(outside[3], inside[1])
+meta = inside[2]
+fst.build_tree_metadata(fst.parent_from_lineage(lineage, level), 64, 64, out=meta)
+with torch.inference_mode():
+    fst.build_tree_metadata(fst.parent_from_lineage(lineage, level), 64, 64, out=meta)
+    assert meta.tensors_untouched()
+    meta.leaf_idx += 1                             # seen, inside as well as outside
+    assert not meta.tensors_untouched()
+print("ok")
+"""
+
+
+def test_calls_under_inference_mode(built_lib):
+    """The call sequence of the original package, and metadata in its format, in a program that decodes under
+    torch.inference_mode() from its first call on."""
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", INFERENCE], cwd=root, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0 and "ok" in run.stdout, run.stdout + run.stderr
