@@ -86,10 +86,15 @@ at::Tensor *status_of(const at::Device &dev, bool create) {
 }
 
 int sm_count(int device) {
+    constexpr int kB200 = 148;
     static std::atomic<int> cached[64];
+    if (device < 0) return kB200;                         // the tensor is on the host
     int n = cached[device & 63].load(std::memory_order_acquire);
     if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 148;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) {
+            cudaGetLastError();                           // or torch would report it after its next launch
+            n = kB200;
+        }
         cached[device & 63].store(n, std::memory_order_release);
     }
     return n;

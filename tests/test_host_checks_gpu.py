@@ -123,3 +123,11 @@ def test_a_number_of_splits_of_any_type(fst):
         idx += prefix
         leaf += prefix
         assert torch.equal(fst.fst_attention(q, k, v, idx, mask, leaf, 0.1, BLOCK_M=32, MAX_ANCESTORS=32, kv_splits=splits), want)
+
+
+def test_a_plan_for_a_host_tensor_leaves_no_error_behind(fst):
+    """launch_plan looks at shape and type; the next launch in the process must not be blamed for the host's device index."""
+    q = torch.empty((1, 8, 127, 128), dtype=torch.float16)
+    want = fst.launch_plan(q.cuda(), 4096, 64)
+    assert fst.launch_plan(q, 4096, 64) == want
+    assert torch.equal(torch.ones(8, device="cuda").clone(), torch.ones(8, device="cuda"))
