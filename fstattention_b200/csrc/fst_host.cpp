@@ -404,20 +404,6 @@ PyObject *attention_paged(PyObject *const *a, Py_ssize_t n) {
 }
 
 // ---- trees ---------------------------------------------------------------------------------------
-// precompute(parent, block_m, max_ancestors, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx)
-//   -> the status record of this build; parent is a contiguous int32 CUDA tensor [N] or [T, N], the buffers belong to the caller and
-//   the last three may be None.
-// new_metadata(parent, block_m, max_ancestors, reference_format)
-//   -> (n_trees, n_nodes, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx, whether the call was
-//   captured into a graph), buffers made here.
-// Record i of a block of them: a tensor over the block's storage, made without the dispatcher (narrow takes a microsecond).
-at::Tensor record_of(const at::Tensor &words, int64_t i) {
-    auto impl = c10::make_intrusive<c10::TensorImpl>(c10::Storage(words.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA), words.dtype());
-    impl->set_sizes_contiguous({4});
-    impl->set_storage_offset(4 * i);
-    return at::Tensor(std::move(impl));
-}
-
 // A cleared status record.  Clearing one per call is a launch (about a microsecond in front of a five
 // microsecond kernel), so a thread takes them from a block that it cleared in one go on the same stream;
 // a new block is made for another stream or device and when one is used up (256 records, 4 KB,
@@ -425,6 +411,13 @@ at::Tensor record_of(const at::Tensor &words, int64_t i) {
 // clears its record in the graph, for every replay: `old` if it is given.  That is a fill kernel: kernels
 // follow one another faster than a kernel follows a memset node (a 256-node build, 64 of them in a graph:
 // 8.2 us with the memset, 5.2 with the fill).
+// record_of: record i of a block, a tensor over the block's storage made without the dispatcher (narrow takes a microsecond).
+at::Tensor record_of(const at::Tensor &words, int64_t i) {
+    auto impl = c10::make_intrusive<c10::TensorImpl>(c10::Storage(words.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA), words.dtype());
+    impl->set_sizes_contiguous({4});
+    impl->set_storage_offset(4 * i);
+    return at::Tensor(std::move(impl));
+}
 at::Tensor clear_record(const at::Device &dev, cudaStream_t stream, const at::Tensor &old, const char *what,
                         bool *captured = nullptr) {
     const OrdinaryTensors guard;
@@ -479,6 +472,9 @@ const at::Tensor &parent_arg(PyObject *o) {
 }
 at::Tensor optional_tensor(PyObject *o) { return o == Py_None ? at::Tensor() : tensor(o); }
 
+// precompute(parent, block_m, max_ancestors, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx)
+//   -> the status record of this build; parent is a contiguous int32 CUDA tensor [N] or [T, N], the buffers belong to the caller and
+//   the last three may be None.
 PyObject *precompute(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 9);
     const at::Tensor &par = parent_arg(a[0]);
@@ -525,6 +521,9 @@ Built build_metadata(const at::Tensor &par, bool batched, int64_t n_trees, int64
     return m;
 }
 
+// new_metadata(parent, block_m, max_ancestors, reference_format)
+//   -> (n_trees, n_nodes, packed, tree_stride, status, ancestor_idx, ancestor_mask, leaf_idx, whether the call was
+//   captured into a graph), buffers made here.
 PyObject *new_metadata(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 4);
     const at::Tensor &par = parent_arg(a[0]);
@@ -578,32 +577,35 @@ PyObject *build_tree_topk(PyObject *const *a, Py_ssize_t n) {
     return Py_BuildValue("(NNN)", THPVariable_Wrap(parent), wrap_or_none(choice), wrap_or_none(score));
 }
 
-// parents_of_lineage(lineage, level_lookup, mutate) -> int32 parent array on the host (pinned), for int64 CPU
-// tensors: parent[k] = lineage[k, level[k] - 1], -1 on level 0 (utils.py:42-44 of the reference).  The
-// reference's side effect (utils.py:124-125) - every node written into its own lineage row - is a second call.
-PyObject *parents_of_lineage(PyObject *const *a, Py_ssize_t n) {
-    want_args(n, 2);
-    const at::Tensor &lin = tensor(a[0]), &lvl = tensor(a[1]);
+// parent[k] = lineage[k, level[k] - 1], -1 on level 0 (utils.py:42-44 of the reference), for int64 CPU tensors; an entry
+// is looked at before it is narrowed to 32 bits.
+void parents_from(const at::Tensor &lin, const at::Tensor &lvl, int32_t *P) {
     const int64_t N = lin.size(0), W = lin.size(1), s0 = lin.stride(0), s1 = lin.stride(1), t0 = lvl.stride(0);
     const int64_t *L = static_cast<const int64_t *>(lin.data_ptr()), *V = static_cast<const int64_t *>(lvl.data_ptr());
-    const at::Tensor parent = at::empty({N}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));   // torch's pinned pool
-    int32_t *P = static_cast<int32_t *>(parent.data_ptr());
     for (int64_t k = 0; k < N; ++k) {
         const int64_t lv = V[k * t0];
         if (lv > W) raise(PyExc_IndexError, "level_lookup points past the lineage columns");
-        P[k] = lv > 0 ? int32_t(L[k * s0 + (lv - 1) * s1]) : -1;
+        const int64_t p = lv > 0 ? L[k * s0 + (lv - 1) * s1] : -1;
+        if (p >= k || p < -1) {
+            PyErr_Format(PyExc_ValueError, "malformed tree: parent[%lld]=%lld must be -1 or an earlier node", (long long)k, (long long)p);
+            throw PyError{};
+        }
+        P[k] = int32_t(p);
     }
+}
+// parents_of_lineage(lineage, level_lookup) -> int32 parent array on the host (pinned).  The reference's side effect
+// (utils.py:124-125) - every node written into its own lineage row - is a second call.
+PyObject *parents_of_lineage(PyObject *const *a, Py_ssize_t n) {
+    want_args(n, 2);
+    const at::Tensor &lin = tensor(a[0]);
+    const at::Tensor parent = at::empty({lin.size(0)}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));   // torch's pinned pool
+    parents_from(lin, tensor(a[1]), static_cast<int32_t *>(parent.data_ptr()));
     return THPVariable_Wrap(parent);
 }
 
-// What the device status record of a metadata build would say, from a parent array on the host, so that the caller need
-// not wait for the device to learn it.  Every node is marked once per block: the marks of a block are its ancestors.
-void check_parents(const int32_t *P, int64_t N, int64_t bm, int64_t ma) {
-    for (int64_t k = 0; k < N; ++k)
-        if (P[k] >= k || P[k] < -1) {
-            PyErr_Format(PyExc_ValueError, "malformed tree: parent[%lld]=%d must be -1 or an earlier node", (long long)k, int(P[k]));
-            throw PyError{};
-        }
+// What the device status record of a metadata build would say of the ancestor bound, from parents_from's array on the host, so
+// that the caller need not wait for the device to learn it.  Every node is marked once per block: the marks of a block are its ancestors.
+void check_bound(const int32_t *P, int64_t N, int64_t bm, int64_t ma) {
     std::vector<int32_t> seen(N, -1);                     // last block that met the node
     for (int64_t b = 0; b * bm < N; ++b) {
         int64_t count = 0;
@@ -616,11 +618,11 @@ void check_parents(const int32_t *P, int64_t N, int64_t bm, int64_t ma) {
         }
     }
 }
-// check_tree(parent, block_m, max_ancestors), parent on the host (int32, contiguous)
+// check_tree(parent, block_m, max_ancestors), parent what parents_of_lineage has returned
 PyObject *check_tree(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 3);
     const at::Tensor &par = tensor(a[0]);
-    check_parents(static_cast<const int32_t *>(par.data_ptr()), par.size(0), integer(a[1]), integer(a[2]));
+    check_bound(static_cast<const int32_t *>(par.data_ptr()), par.size(0), integer(a[1]), integer(a[2]));
     Py_RETURN_NONE;
 }
 
@@ -633,16 +635,10 @@ PyObject *metadata_of_lineage(PyObject *const *a, Py_ssize_t n) {
     want_args(n, 4);
     constexpr int64_t kInline = 8192;                     // parents: 32 KB, the driver stages up to 64
     const at::Tensor &lin = tensor(a[0]), &lvl = tensor(a[1]);
-    const int64_t N = lin.size(0), W = lin.size(1), s0 = lin.stride(0), s1 = lin.stride(1), t0 = lvl.stride(0);
-    const int64_t bm = integer(a[2]), ma = integer(a[3]);
+    const int64_t N = lin.size(0), bm = integer(a[2]), ma = integer(a[3]);
     if (N == 0 || N > kInline) Py_RETURN_NONE;
-    const int64_t *Lp = static_cast<const int64_t *>(lin.data_ptr()), *V = static_cast<const int64_t *>(lvl.data_ptr());
     std::vector<int32_t> P(N);
-    for (int64_t k = 0; k < N; ++k) {
-        const int64_t lv = V[k * t0];
-        if (lv > W) raise(PyExc_IndexError, "level_lookup points past the lineage columns");
-        P[k] = lv > 0 ? int32_t(Lp[k * s0 + (lv - 1) * s1]) : -1;
-    }
+    parents_from(lin, lvl, P.data());
     const at::Tensor par = empty({N}, at::kInt, at::Device(at::kCUDA, c10::cuda::current_device()));
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(par.device().index()).stream();
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -651,7 +647,7 @@ PyObject *metadata_of_lineage(PyObject *const *a, Py_ssize_t n) {
     if (cudaMemcpyAsync(par.data_ptr(), P.data(), size_t(N) * 4, cudaMemcpyHostToDevice, stream) != cudaSuccess)
         check_status(FST_ERR_CUDA, "fst_precompute");
     const Built m = build_metadata(par, false, 1, N, bm, ma, true);
-    check_parents(P.data(), N, bm, ma);
+    check_bound(P.data(), N, bm, ma);
     return Py_BuildValue("(NnNNN)", THPVariable_Wrap(m.packed), Py_ssize_t(m.stride), THPVariable_Wrap(m.ai), THPVariable_Wrap(m.am),
                          THPVariable_Wrap(m.li));
 }

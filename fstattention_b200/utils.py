@@ -173,7 +173,14 @@ def _as_parent_tensor(parent: TreeLike, device) -> torch.Tensor:
         return parent
     if device is None:
         device = parent.device if parent.is_cuda else "cuda"
+    if parent.dtype == torch.long and not parent.is_cuda:
+        parent = _in_32_bits(parent)
     return parent.to(device=device, dtype=torch.int32, non_blocking=True).contiguous()
+
+
+def _in_32_bits(parent: torch.Tensor) -> torch.Tensor:
+    """What does not fit into 32 bits stays what it is, no node's number."""
+    return parent.clamp(-2, 2 ** 31 - 1)
 
 
 def packed_meta_bytes(n_blocks: int, block_m: int, max_ancestors: int) -> int:
@@ -293,6 +300,8 @@ def create_fst_attention_kernel_inputs(lineage: torch.Tensor, level_lookup: torc
             host.write_self(lineage, level_lookup)
         return idx, mask, leaf
     parent = host.parents_of_lineage(lineage, level_lookup) if native else parent_from_lineage(lineage, level_lookup)
+    if parent.dtype == torch.long and parent.is_cuda:
+        parent = _in_32_bits(parent)
     meta = build_tree_metadata(parent, block_m, max_ancestors, reference_format=True, check=not native)
     if native:
         # the parents are on the host: so is the check, and nobody waits for the device

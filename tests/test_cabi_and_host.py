@@ -251,6 +251,16 @@ def test_metadata_and_its_tensors_can_be_copied_and_saved(built_lib):
     assert saved(plain).tensors_untouched() and saved(plain).ancestor_idx is None
 
 
+@pytest.mark.parametrize("entry", [2 ** 32, 2 ** 32 + 3, -2 ** 33 - 1, 2 ** 63 - 1, 6, -2])
+def test_a_lineage_entry_that_is_no_earlier_node(built_lib, entry):
+    """Whatever its low 32 bits say, and before anything is launched."""
+    import fstattention_b200 as fst
+    lineage, level = fst.lineage_from_parent([-1, 0, 0, 1, 1, 2, 5, 6])
+    lineage[6, level[6] - 1] = entry
+    with pytest.raises(ValueError, match=rf"parent\[6\]={entry} "):
+        fst.create_fst_attention_kernel_inputs(lineage, level, block_m=4, max_ancestors=8)
+
+
 def test_metadata_of_tensors_without_versions(built_lib):
     """Under inference mode nobody counts how often a tensor is written: its metadata has no packed form to rely on."""
     import pickle

@@ -355,6 +355,22 @@ def test_inputs_of_a_lineage_small_and_large(fst, depth, mutate):
     assert torch.equal(fst.fst_attention(q, k, v, *got, 0.1, BLOCK_M=64, MAX_ANCESTORS=128), fst.fst_attention(q, k, v, want, sm_scale=0.1))
 
 
+@pytest.mark.parametrize("entry", [2 ** 32 + 3, -2 ** 33])
+def test_entries_beyond_32_bits(fst, entry):
+    """A lineage on the host or on the GPU, small or large, and a parent array on the host."""
+    for n in (100, 9000):
+        lineage, level = fst.lineage_from_parent([-1] + [i // 9 for i in range(n - 1)])
+        lineage[50, level[50] - 1] = entry
+        for lin in (lineage, lineage.cuda()):
+            with pytest.raises(ValueError, match=r"parent\[50\]"):
+                fst.create_fst_attention_kernel_inputs(lin.clone(), level, block_m=64, max_ancestors=128)
+        parent = fst.parent_from_lineage(lineage, level)
+        with pytest.raises(ValueError, match=r"parent\[50\]"):
+            fst.build_tree_metadata(parent, 64, 128)
+        with pytest.raises(ValueError, match=r"parent\[50\]"):
+            fst.build_tree_metadata(parent[None].repeat(2, 1), 64, 128, reference_format=False)
+
+
 INFERENCE = """
 import torch
 import fstattention_b200 as fst
