@@ -51,18 +51,19 @@
 //
 // Measured against attn_tma_kernel (us per call, fp16): 4096-node deep tree, 64 heads, D 128 84 -> 60 (4.5 TB/s
 // over Q, K, V and O); 64 x 300-node dynamic trees, D 128, block_m 128 381 -> 146; 16 x 1000-node deep
-// trees, D 64 120 -> 82; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2190 -> 1403.
+// trees, D 64 120 -> 82; the create_tree forest of 65532 nodes, 4 x 48 heads, D 64, block_m 128 2190 -> 1360.
 // What bounds it is the chain of a group's round - product, softmax, (rescale,) product - and at D 128 the pool: a 96 KB item
 // in use, one on its way, and the last one's O.  Items of one tile run at HBM's rate (D 128: 83 us where 64 trees of
-// 256 nodes take 101; D 64: 1165 where the forest takes 1403), so the ancestors are what the rest pays for.
+// 256 nodes take 101; D 64: 1165 where the forest takes 1360), so the ancestors are what the rest pays for.
 //
 // The scores of both tiles of an item at once (Round::BOTH), for bounds of up to 64 at D 64 and block_m 128: their columns
 // fit beside one another, so the second tile's are there when the softmax of the first is done, and the first's product
-// with V runs under the second's exponentials: forest of 65532 nodes 1745 -> 1403 us, of 8188 217 -> 179.  The
-// roundings are those of the tiles one by one.  One softmax over both (1332 us) rounded the own tile's largest weight too,
-// 1.2 to 2.8 % more error; with the second tile's output in columns of its own, scaled when O is read, it had the
-// error of now and the speed, but not the bits.  One softmax lost elsewhere: longer lists (dynamic trees of 1024 nodes, D 128
-// 54.4 / 56.0; further rounds of 64 or 128 slots 24.4 / 27.1 and 68 / 79), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118).
+// with V runs under the second's exponentials: forest of 65532 nodes 1745 -> 1360 us, of 8188 218 -> 175 (1400 and 179 with O
+// rescaled ahead of the exponentials, as in the other rounds).  The roundings are those of the tiles one by one.  One
+// softmax over both (1335 us) rounded the own tile's largest weight too, 1.2 to 2.8 % more error; with the second tile's
+// output in columns of its own, scaled when O is read, it had the error of now and the speed, but not the bits.  One
+// softmax lost elsewhere: longer lists (dynamic trees of 1024 nodes, D 128 54.4 / 56.0; further rounds of 64 or 128 slots
+// 24.4 / 27.1 and 68 / 79), block_m 64 at D 64 (140 / 155), block_m 32 (104 / 118).
 // tree_umma_pays (fst_plan.h) has the line between the two kernels.
 #pragma once
 
@@ -689,7 +690,8 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                 // (two words to a turn at block_m 128: 1760 -> 1892 us on the forest of 65532 nodes; both words of
                 // a row in one turn at block_m 64: 69.0 -> 67.5 us on the deep tree).
                 constexpr int WT = NW == 2 ? 2 : 1;
-                bool second = false, settled = !BOTH || t == 0;       // the earlier products of O have landed
+                bool second = false;
+                float alpha = 1.f;                        // what my row of O is to be scaled by
                 if constexpr (BOTH) {
                     // A row that attends to nobody in its block but itself, as where the tree is numbered breadth first, needs no 32
                     // exponentials: where one word is all that a warp has, and one column of it all that a row has, the score is
@@ -748,14 +750,9 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                         mx = fmaxf(mx, m);
                         if (rest != 0u) continue;
                         const bool up = mx > m_ref;
-                        if (!settled) {
-                            settled = true;
-                            alive = __all_sync(0xffffffffu, wait(bar_m + g * 8, pairs & 1, a.status, item));
-                            fence_after_sync();
-                        }
-                        if (__any_sync(0xffffffffu, up)) {
-                            if (t > 0) {                  // rescale my row of O (the stores are awaited with P's)
-                                const float alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
+                        if (BOTH ? up : __any_sync(0xffffffffu, up)) {
+                            if (t > 0) alpha = up ? fast_exp2((m_ref - mx) * c2) : 1.f;
+                            if (!BOTH && t > 0) {         // rescale my row of O (the stores are awaited with P's)
 #pragma unroll 1
                                 for (int c0 = 0; c0 < D; c0 += 16) {
                                     uint32_t o[16];
@@ -790,11 +787,23 @@ tree_umma_kernel(const AttnArgs a, const TreeUmmaArgs ta, const __grid_constant_
                         tmem_st16(tmem_s + (col_my >> 1) + wi[k] * 16, pk);
                     }
                 }
-                if (!settled) {                           // no row of my warp has ancestors, but it keeps step with the barrier
+                if (BOTH && t > 0) {                      // rescale it here, once the first tile's product has landed
                     alive = __all_sync(0xffffffffu, wait(bar_m + g * 8, pairs & 1, a.status, item));
+                    if (!alive) break;
+                    ++pairs;
+                    fence_after_sync();
+                    if (__any_sync(0xffffffffu, alpha != 1.f)) {
+#pragma unroll 1
+                        for (int c0 = 0; c0 < D; c0 += 16) {
+                            uint32_t o[16];
+                            tmem_ld16(o, tmem_o + c0);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                            tmem_st16(tmem_o + c0, o);
+                        }
+                        l *= alpha;
+                    }
                 }
-                if (!alive) break;
-                pairs += int(BOTH && t > 0);
                 l += sum[0] + sum[1];
                 tmem_st_wait();
                 fence_before_sync();
