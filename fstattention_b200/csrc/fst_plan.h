@@ -113,7 +113,7 @@ inline int tma_tile_cols(int64_t ctas, int D, int bm, int ma, int sms) {
 //                        96 slots: 0.84 - 1.02 up to 420, 0.97 - 1.08 at 500, 1.06 - 1.21 above.  Bound 2 and 3: 0.56 - 1.08 up to 224; deep trees
 //                        1.07 at 250 to 310, others 0.83 - 1.00; 0.86 - 1.16 up to 420, 0.93 - 1.21 at 500, 0.98 - 1.43 above.  Bound 4 and
 //                        up: 0.63 - 1.11 up to 224; with 700 nodes and more 1.02 - 1.18 at 250 to 310 (in a decode step of 1024 window
-//                        nodes, 256 items, 103.8 / 99.8), 0.98 - 1.22 up to 420 (scored trees 0.90 at 312), 1.01 - 1.44 above; with fewer
+//                        nodes, 256 items, 1.00 - 1.04 on five GPUs), 0.98 - 1.22 up to 420 (scored trees 0.90 at 312), 1.01 - 1.44 above; with fewer
 //                        0.86 - 1.17 up to 420, 1.00 - 1.22 at 500, 1.05 - 1.39 above
 //   D 128, block_m 32    64 slots: 0.53 - 0.99 up to 530, 1.00 - 1.03 up to 900, 1.09 - 1.23 above; bound 4 to 7: 0.54 - 1.03 up to 420, 0.88 - 1.07 at 500,
 //                        0.96 - 1.10 up to 900, 0.98 - 1.27 above (256-node deep trees 0.93 - 1.04); 0.62 - 1.01 with 320 slots.  64 nodes

@@ -123,7 +123,7 @@ def test_tree_umma_rounds_like_the_other_kernel(fst, D, bm, dtype):
     for kernel in ("tree_umma", "tma"):
         o = fst.fst_attention(q.cuda(), k.cuda(), v.cuda(), meta, sm_scale=D ** -0.5, kernel=kernel).cpu().double()
         err[kernel] = (o - want).norm().item() / want.norm().item()
-    assert err["tree_umma"] <= 1.04 * err["tma"], err
+    assert err["tree_umma"] <= 1.01 * err["tma"], err      # 0.998 to 1.008 here
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
